@@ -143,3 +143,25 @@ def test_single_token_cache_through_the_gather_path(d):
     # and the consumers of a compressed dictionary refuse arrays that do not match its shape
     with pytest.raises(ValueError):
         fused_attention(q, dict(ck, packed_key_indices=ck["packed_key_indices"][:-1]), cv, kc, vc)
+
+
+@pytest.mark.parametrize("d,bits,Hq,Hkv", [(128, 3, 8, 2), (128, 2, 3, 3), (64, 3, 4, 4), (64, 4, 6, 2), (64, 2, 5, 1)])
+@pytest.mark.parametrize("cached,new", [(0, 17), (131, 1), (300, 128), (127, 130)])
+def test_chunk_attends_in_place_over_a_strided_cache(d, bits, Hq, Hkv, cached, new):
+    """Chunks of a prompt behind a prefix: the kernels read the cache rows where they are (a token stride of the
+    capacity, odd here) and give bit for bit what they give on the gathered prefix."""
+    from turboquant_b200 import CompressedKVCache, fused_attention
+    kc, vc = device_compressors(d, bits, mode="bf16")
+    n = cached + new
+    k, v = _tokens(2, Hkv, n, d, cached + d).cuda(), _tokens(2, Hkv, n, d, new + d).cuda()
+    q = _tokens(2, Hq, new, d, bits).cuda()
+    cache = CompressedKVCache(kc, vc, 2, Hkv, n + 37)
+    cache.append(k[:, :, :cached], v[:, :, :cached])
+    cache.append(k[:, :, cached:], v[:, :, cached:])
+    ck, cv = cache._contiguous_prefix()
+    got = cache.attend(q)
+    want = fused_attention(q, ck, cv, kc, vc)
+    if d == 128 and (Hq // Hkv) * new <= 16 and n < 256:
+        assert rel_err(got, want) < 1e-2  # a short contiguous call of this size takes the prefill kernel instead
+    else:
+        assert torch.equal(got, want)

@@ -57,7 +57,7 @@ struct AttnArgs {
   int out_dtype;
   int64_t o_stride_b, o_stride_h, o_stride_s;
   // keys between the packed rows of consecutive (batch, KV head) pairs in every packed array: Sk for the
-  // contiguous [B, Hkv, Sk] layout, the capacity of a persistent cache otherwise (split-KV kernel only)
+  // contiguous [B, Hkv, Sk] layout, the capacity of a persistent cache otherwise (tensor-core mode only)
   int64_t kv_stride;
 };
 

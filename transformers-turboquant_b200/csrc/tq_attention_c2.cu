@@ -204,7 +204,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   }
   // 32-bit division (head counts are below 65536): the 64-bit form is a subroutine of ~100 instructions, twice,
   // on every thread's way to its first load
-  const int64_t kv_base = (b * a.Hkv + (int)head / ((int)a.Hq / (int)a.Hkv)) * a.Sk;
+  const int64_t kv_base = (b * a.Hkv + (int)head / ((int)a.Hq / (int)a.Hkv)) * a.kv_stride;
   const int shift = (int)(a.Sk - a.Sq);
   int k_end = (int)a.Sk;
   if (a.causal) k_end = min(k_end, min(q0_last + kBM - 1, (int)a.Sq - 1) + shift + 1);

@@ -365,7 +365,7 @@ attention_ws_kernel(const AttnArgs a, __nv_bfloat16* __restrict__ o_rot, const i
     head[0] = head[1] = blockIdx.y;
     q0[0] = 2 * xblk * kBM; q0[1] = q0[0] + kBM;
   }
-  const int64_t kv_base = (b * a.Hkv + head[0] / (a.Hq / a.Hkv)) * a.Sk;
+  const int64_t kv_base = (b * a.Hkv + head[0] / (a.Hq / a.Hkv)) * a.kv_stride;
   const int shift = (int)(a.Sk - a.Sq);
   int k_end = (int)a.Sk;
   if (a.causal) k_end = min(k_end, min(q0[1] + kBM - 1, (int)a.Sq - 1) + shift + 1);
@@ -910,9 +910,6 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
   TQ_REQUIRE(B <= 65535 && Hq <= 65535, "batch and head counts are limited to 65535 in bf16 mode");
   TQ_REQUIRE(a.sm_scale > 0.f && a.sm_scale < 1e30f, "sm_scale must be positive and finite in bf16 mode");
   const Bf16Path path = bf16_path(a, Sq, d);
-  TQ_REQUIRE(path == Bf16Path::kDecode || a.kv_stride == a.Sk,
-             "a cache with capacity %lld > Sk is served by the split-KV kernel only: head_dim 128, "
-             "(Hq / Hkv) * Sq <= 16", (long long)a.kv_stride);
   const bool pairs = path == Bf16Path::kPairs;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   const __nv_bfloat16 *w_cat, *w_unrot;
