@@ -286,6 +286,26 @@ int tq_attention_fwd_prepared(const void* q, int dtype, int64_t B, int64_t Hq, i
                               void* out, int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s,
                               void* workspace, size_t workspace_bytes, int mode, void* stream);
 
+/* tq_attention_fwd_prepared under a mask the library first summarises into visibility bits (one small launch): additive
+ * fp32 (TQ_MASK_ADDITIVE) or bytes of which 0 hides a key (TQ_MASK_BOOL, what HF's sdpa path hands over for padded
+ * batches).  `mask_batches` is 1 (one mask for every batch element) or B; strides in elements, rows contiguous.
+ * Tiles of keys that no row of a tile of queries sees are not computed. */
+#define TQ_MASK_ADDITIVE 0
+#define TQ_MASK_BOOL 1
+size_t tq_attention_masked_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
+                                           int64_t kv_capacity, int d, int mode, int64_t mask_batches);
+int tq_attention_fwd_masked(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d,
+                            int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_s,
+                            int64_t Hkv, int64_t Sk, int64_t kv_capacity,
+                            const uint8_t* key_idx, const uint8_t* key_signs,
+                            const uint16_t* key_vec_norms, const uint16_t* key_residual_norms,
+                            const uint8_t* val_idx, const uint16_t* val_vec_norms,
+                            const void* constants, int bits, float sm_scale, int causal,
+                            const void* mask, int mask_kind, int64_t mask_batches, int64_t mask_stride_b,
+                            int64_t mask_stride_q,
+                            void* out, int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s,
+                            void* workspace, size_t workspace_bytes, int mode, void* stream);
+
 /* tq_attention_fwd for callers that cannot hand over scratch memory (no counterpart in the
  * reference).  Meant for hosts that may not call cudaMalloc or any other allocator: a plugin
  * inside a serving process whose device memory belongs to someone else, or a call site that

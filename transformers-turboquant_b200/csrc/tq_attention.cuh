@@ -37,6 +37,19 @@ inline ConstLayout const_layout(int d) {
 int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k, const float* bnd_k, const float* Pi_v,
                       const float* cen_v, const float* bnd_v, int bits, int d, void* constants, cudaStream_t stream);
 
+// Summary of a mask (tq_mask.cu): visibility bits, classes of 16 rows x 128 keys, rows with a visible key.
+struct MaskBits {
+  const uint32_t* words;  // [batch][Sq][4 T]; NULL: no summary
+  const uint32_t* rows;   // [batch][NG][NC]: bit r set when row 16 g + r has a visible key in this chunk of 64 tiles
+  const uint8_t* tiles;   // [batch][NG][T]: 1 some key visible, 2 some hidden, 4 some other additive value
+  int T, NG, NC;          // 128-key tiles, 16-row groups, chunks of 64 tiles
+  int batch;              // 0: one mask for every batch element
+};
+// The pointers of a summary of `nb` masks at `base` (which may be NULL to ask for the size only).
+MaskBits mask_bits_layout(int64_t nb, int64_t Sq, int64_t Sk, void* base, size_t* bytes);
+int summarize_mask(const void* mask, bool boolean, int64_t nb, int64_t stride_b, int64_t stride_q, int64_t Sq, int64_t Sk,
+                   int causal, const MaskBits& m, cudaStream_t stream);
+
 struct AttnArgs {
   const void* q_cat;   // fp32 [n, 2d] (fp32 mode) or bf16 [n, 2d] (bf16 mode), row n = (b*Hq+h)*Sq+s
   int64_t Hq, Sq, Hkv, Sk;
@@ -59,6 +72,7 @@ struct AttnArgs {
   // keys between the packed rows of consecutive (batch, KV head) pairs in every packed array: Sk for the
   // contiguous [B, Hkv, Sk] layout, the capacity of a persistent cache otherwise (tensor-core mode only)
   int64_t kv_stride;
+  MaskBits mb;  // summary of the mask; where it exists, `mask` is read in tiles of its third class only
 };
 
 int check_attention_args(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,

@@ -114,6 +114,7 @@ constexpr int kProducers = 256;    // 8 producer warps
 constexpr int kThreads = kSoftmax + kProducers + 64;
 constexpr int kCtlWarp = kThreads / 32 - 2;   // tensor-memory allocation; issues the score MMAs in the leader CTA
 constexpr int kPvWarp = kThreads / 32 - 1;    // issues the P V_hat MMAs in the leader CTA
+constexpr int kMapWords = 64;                 // tiles of the mask maps / 32: masks of more keys are read without skipping
 constexpr int kSoftmaxArrivals = 2 * kSoftmax / 32;     // softmax warps of both CTAs
 constexpr int kProducerArrivals = 2 * kProducers / 32;  // producer warps of both CTAs
 
@@ -164,7 +165,8 @@ struct C2Smem {
   static_assert(2 * D <= 2 * kBN, "the Q_cat accumulator borrows both score tiles");
 };
 
-template <int D, int BITS, bool TRACE>
+// MASK: the call has an additive mask or a mask summary (a kernel of its own: the mask handling costs the plain one 1.5 %)
+template <int D, int BITS, bool MASK, bool TRACE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   using L = C2Smem<D, BITS>;
@@ -183,6 +185,9 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   __shared__ __align__(8) uint64_t bars[4 * kStages + 22];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
+  // bit t of each map, from the mask's summary over the rows of both CTAs: key tile t is computed at all / has hidden
+  // keys / has additive values that are neither 0 nor minus infinity
+  __shared__ uint32_t map_live[MASK ? kMapWords : 1], map_hidden[MASK ? kMapWords : 1], map_other[MASK ? kMapWords : 1];
   volatile int* abort_flag = &s_abort;
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
@@ -290,6 +295,37 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     }
   }
   if (warp == kCtlWarp) tc::tmem_alloc2(tc::smem_u32(&tmem_slot), L::kCols);
+  // Maps of the masked key tiles, by the producer warps (32 tiles each at a time).  Rows without a visible key
+  // average all keys of their causal range: a cluster that has one computes every tile.
+  const bool mapped = MASK && a.mb.words != nullptr && n_tiles_live <= 32 * kMapWords;
+  if (mapped && warp >= kSoftmax / 32 && warp < kCtlWarp) {
+    const int g0 = (pair_heads ? q0 : 2 * xpair * kBM) / 16, ng = min((pair_heads ? kBM : 2 * kBM) / 16, a.mb.NG - g0);
+    const int64_t gb = (a.mb.batch ? b * a.mb.NG : 0) + g0;
+    bool blind = false;  // lane = row group
+    if (lane < ng) {
+      uint32_t seen = 0;
+      for (int c = 0; c < a.mb.NC; ++c) seen |= a.mb.rows[(gb + lane) * a.mb.NC + c];
+      const int rows = min(16, (int)a.Sq - 16 * (g0 + lane));
+      blind = (~seen & ((1u << rows) - 1u)) != 0u;
+    }
+    blind = __any_sync(0xffffffffu, blind);
+    for (int w = warp - kSoftmax / 32; w * 32 < n_tiles_live; w += kProducers / 32) {
+      const int t = w * 32 + lane;
+      uint32_t cls = 0;
+      if (t < n_tiles_live) {
+        for (int g = 0; g < ng; ++g) cls |= a.mb.tiles[(gb + g) * a.mb.T + t];
+        if (blind) cls |= 1u;
+      }
+      const uint32_t live = __ballot_sync(0xffffffffu, (cls & 1u) != 0u);
+      const uint32_t hidden = __ballot_sync(0xffffffffu, (cls & 2u) != 0u);
+      const uint32_t other = __ballot_sync(0xffffffffu, (cls & 4u) != 0u);
+      if (lane == 0) {
+        map_live[w] = live;
+        map_hidden[w] = hidden;
+        map_other[w] = other;
+      }
+    }
+  }
   const long long t_i = TRACE ? clock64() : 0;
   tc::fence_before_sync();
   __syncthreads();
@@ -297,7 +333,22 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   tc::cluster_sync_relaxed();  // the peer's barriers and tensor memory exist before anyone signals or issues
   tc::fence_after_sync();
   const bool dead = s_abort != 0;  // an earlier bounded wait expired: do nothing but keep the cluster barriers paired
-  const int n_tiles = dead ? 0 : n_tiles_live;
+  int n_tiles = dead ? 0 : n_tiles_live;
+  if (mapped && !dead) {
+    n_tiles = 0;
+    for (int w = 0; w * 32 < n_tiles_live; ++w) n_tiles += __popc(map_live[w]);
+  }
+  // the key tile computed after tile `t` (-1: the first one)
+  auto next_tile = [&](int t) -> int {
+    ++t;
+    if (mapped) {
+      for (; t < n_tiles_live; t = (t | 31) + 1) {
+        const uint32_t w = map_live[t >> 5] >> (t & 31);
+        if (w != 0u) return t + __ffs((int)w) - 1;
+      }
+    }
+    return t;
+  };
   const uint32_t tmem_base = tmem_slot;
   const uint32_t tmem_o = tmem_base + L::kColO;
   bool ok = true;
@@ -364,11 +415,21 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     }
     float m_run = -INFINITY, l_run = 0.f;
     const float cexp = a.sm_scale * kLog2e, rcexp = 1.f / cexp;  // K_hat carries the key norms: S is the raw score
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int bb = j & 1, u = j >> 1, k0 = j * kBN;
+    int kt = next_tile(-1);
+    for (int j = 0; j < n_tiles && ok; ++j, kt = next_tile(kt)) {
+      const int bb = j & 1, u = j >> 1, k0 = kt * kBN;
       const int kc0 = k0 + chalf * HC;
       const uint32_t tmem_s = tmem_base + L::kColS + bb * kBN;
       tr.mark(0, j);
+      bool hidden = false, other = MASK && a.mask != nullptr;
+      uint2 seen = make_uint2(0u, 0u);  // visibility bits of this thread's 64 columns
+      if (MASK && a.mb.words != nullptr) {
+        hidden = !mapped || ((map_hidden[kt >> 5] >> (kt & 31)) & 1u) != 0u;
+        other = other && (!mapped || ((map_other[kt >> 5] >> (kt & 31)) & 1u) != 0u);
+        if (hidden && !other && qi < a.Sq)
+          seen = *reinterpret_cast<const uint2*>(a.mb.words + ((a.mb.batch ? b * a.Sq : 0) + qi) * (4 * (int64_t)a.mb.T) +
+                                                 4 * kt + 2 * chalf);
+      }
       if (!(ok = tc::mbar_wait_or_abort(s_full(bb), u & 1, abort_flag))) break;
       tc::fence_after_sync();
       tr.mark(1, j);
@@ -385,7 +446,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
           t[32 + c] = __uint_as_float(raw1[c]);
         }
       }
-      const bool edge = (k0 + kBN > a.Sk) || (a.causal && k0 + kBN - 1 > q0 + shift) || a.mask != nullptr;
+      const bool edge = (k0 + kBN > a.Sk) || (a.causal && k0 + kBN - 1 > q0 + shift) || hidden || other;
       if (edge) {
         // Tiles that cross the end of the keys or the causal diagonal, and every tile under an additive mask.  A
         // thread's 64 columns are the keys kc0 .. kc0 + 63: `vsk` is the last column that exists, `vis` the last one
@@ -394,16 +455,20 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
         // select per score here, where a branchy per-element form cost more than two whole tile periods.
         const int vsk = (int)a.Sk - 1 - kc0;
         const int vis = a.causal ? min(vsk, qi + shift - kc0) : vsk;
-        if (a.mask != nullptr && qi < a.Sq) {
+        // The large negative value HF masks with is clamped to -60000 in log2 units (exp2 of it is still exactly 0
+        // beside any real score) so that it stays finite: a row whose visible keys are all masked then averages
+        // them uniformly, as a softmax over equal finite scores does in the reference, instead of coming out as zeros.
+        const float floor_raw = -60000.f * rcexp;
+        if (MASK && other && qi < a.Sq) {
           const float* mrow = a.mask + b * a.mask_stride_b + (int64_t)qi * a.mask_stride_q + kc0;
-          // The large negative value HF masks with is clamped to -60000 in log2 units (exp2 of it is still exactly
-          // 0 beside any real score) so that it stays finite: a row whose visible keys are all masked then averages
-          // them uniformly, as a softmax over equal finite scores does in the reference, instead of coming out as
-          // zeros.
-          const float m_unit = kLog2e * rcexp, floor_raw = -60000.f * rcexp;
+          const float m_unit = kLog2e * rcexp;
 #pragma unroll
           for (int c = 0; c < HC; ++c)
             if (c <= vsk) t[c] = fmaxf(fmaf(mrow[c], m_unit, t[c]), floor_raw);
+        } else if (MASK && hidden) {
+          // a hidden key's score is the floor, as the clamp above leaves it
+#pragma unroll
+          for (int c = 0; c < HC; ++c) t[c] = (((c < 32 ? seen.x : seen.y) >> (c & 31)) & 1u) != 0u ? fmaxf(t[c], floor_raw) : floor_raw;
         }
 #pragma unroll
         for (int c = 0; c < HC; ++c) t[c] = c <= vis ? t[c] : -INFINITY;
@@ -419,6 +484,13 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
           m3 = tc::fmax3(m3, t[c8 + 6], t[c8 + 7]);
         }
         mx = fmaxf(tc::fmax3(m0, m1, m2), m3) * cexp;
+      }
+      if (MASK && !edge && a.mb.words != nullptr && mx < -59000.f) {
+        // scores as low as the hidden keys' floor: clamped there in every tile of a masked call
+        const float floor_raw = -60000.f * rcexp;
+#pragma unroll
+        for (int c = 0; c < HC; ++c) t[c] = fmaxf(t[c], floor_raw);
+        mx = fmaxf(mx, -60000.f);
       }
       // exchange half-row maxima with the partner warp (slots alternate with the tile parity)
       tr.mark(2, j);
@@ -629,8 +701,9 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       vsrc[i] = (int)(L::kIdxK + L::kSgn) + key * VROW + gp * 2 * VB;
       vdst[i] = (key / 8) * (int)L::kLboV + (key % 8) * 16 + 2 * gp * (int)L::kSboV;
     }
+    int kt = next_tile(-1);
     if (n_tiles > 0) {
-      prefetch(0);
+      prefetch(kt * kBN);
       ok = tc::mbar_wait_or_abort(lut_full, 0, abort_flag);  // the decode tables have landed
     }
     for (int j = 0; j < n_tiles && ok; ++j) {
@@ -656,7 +729,8 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       if (lane == 0) tc::mbar_arrive(pk_full(ps));
       if (!(ok = tc::mbar_wait_or_abort(pk_full(ps), (j >> 1) & 1, abort_flag))) break;
       tr.mark(1, j);
-      if (j + 1 < n_tiles) prefetch((j + 1) * kBN);
+      kt = next_tile(kt);
+      if (j + 1 < n_tiles) prefetch(kt * kBN);
       tr.mark(6, j);
       if (u >= 1 && !(ok = tc::mbar_wait_or_abort(k_empty(st), (u - 1) & 1, abort_flag))) break;
       if (j == 2 && !(ok = tc::mbar_wait_or_abort(qp_done, 0, abort_flag))) break;  // stage 2 held a prologue operand
@@ -849,9 +923,12 @@ template <int D, int BITS>
 int launch_c2(const AttnArgs& a, const PairArgs& x, int64_t B, cudaStream_t stream) {
   constexpr size_t smem = C2Smem<D, BITS>::kTotal > 120 * 1024 ? C2Smem<D, BITS>::kTotal : 120 * 1024;
 #ifdef TQ_B200_TRACE  // diagnostics build only: the product library carries one instantiation per (d, bits)
-  auto kern = g_trace2_host_on ? attention_c2_kernel<D, BITS, true> : attention_c2_kernel<D, BITS, false>;
+  const bool masked = a.mask != nullptr || a.mb.words != nullptr;
+  auto kern = masked ? (g_trace2_host_on ? attention_c2_kernel<D, BITS, true, true> : attention_c2_kernel<D, BITS, true, false>)
+                     : (g_trace2_host_on ? attention_c2_kernel<D, BITS, false, true> : attention_c2_kernel<D, BITS, false, false>);
 #else
-  auto kern = attention_c2_kernel<D, BITS, false>;
+  auto kern = a.mask != nullptr || a.mb.words != nullptr ? attention_c2_kernel<D, BITS, true, false>
+                                                         : attention_c2_kernel<D, BITS, false, false>;
 #endif
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pair_heads = ((a.Hq / a.Hkv) % 2 == 0) ? 1 : 0;

@@ -67,8 +67,9 @@ struct DecodeArgs {
   int causal;
   const float* mask;  // optional additive mask, element (b, s, k) at mask[b * mask_stride_b + s * mask_stride_q + k]
   int64_t mask_stride_b, mask_stride_q;
-  float* part_o;   // [B*Hkv, nsplit, 16, d]
-  float* part_ml;  // [B*Hkv, nsplit, 16, 2]  (running maximum, row sum)
+  MaskBits mb;     // the mask's summary (words == NULL: none); `mask` is then read only where it says so
+  float* part_o;   // [B*Hkv, nsplit, R, d]  (R = query rows per KV head)
+  float* part_ml;  // [B*Hkv, nsplit, R, 2]  (running maximum, row sum)
   int nsplit, keys_per_split;
 };
 
@@ -262,8 +263,35 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
       m_run[t][e] = -INFINITY;
       l_run[t][e] = 0.f;
     }
-  const int k_lo = split * a.keys_per_split;
-  const int k_hi = min((int)a.Sk, k_lo + a.keys_per_split);
+  int k_lo = split * a.keys_per_split;
+  int k_hi = min((int)a.Sk, k_lo + a.keys_per_split);
+  if constexpr (MASK) {
+    // Hidden keys at either end of the range weigh exactly 0 beside a visible one: trimmed, in steps of the mask
+    // summary's 128-key tiles, unless some row has no visible key (it then averages all its keys).  At most 16 query
+    // rows: one row group.  (Decode-sized calls over left-padded batches: a quarter of the keys and more.)
+    if (a.mb.words != nullptr && k_lo < k_hi) {
+      const int64_t mbat = a.mb.batch ? b : 0;
+      uint32_t rows_seen = 0;
+      for (int c = lane; c < a.mb.NC; c += 32) rows_seen |= a.mb.rows[mbat * a.mb.NC + c];
+      rows_seen = __reduce_or_sync(0xffffffffu, rows_seen);
+      if ((~rows_seen & ((1u << (int)a.Sq) - 1u)) == 0u) {
+        const uint8_t* cls = a.mb.tiles + mbat * a.mb.T;
+        int first = 1 << 30, last = -1;
+        for (int t = k_lo / 128 + lane; t <= (k_hi - 1) / 128; t += 32)
+          if (cls[t] & 1u) {
+            first = min(first, t);
+            last = t;
+          }
+        first = __reduce_min_sync(0xffffffffu, first);
+        last = __reduce_max_sync(0xffffffffu, last);
+        if (last < 0) k_hi = k_lo;
+        else {
+          k_lo = max(k_lo, first * 128);
+          k_hi = min(k_hi, (last + 1) * 128);
+        }
+      }
+    }
+  }
   const uint8_t* kidx_base = a.key_idx + kv_base * (16 * KB);
   const uint8_t* ksgn_base = a.key_sgn + kv_base * 16;
   const uint8_t* vidx_base = a.val_idx + kv_base * (16 * VB);
@@ -356,17 +384,31 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
     // the decode work that hides its latency
     float mk[MASK ? NT : 1][4];
     if constexpr (MASK) {
+      const int64_t mbat = a.mb.batch ? b : 0;
+      const bool read_mask = a.mask != nullptr && (a.mb.words == nullptr || (a.mb.tiles[mbat * a.mb.T + blk / 128] & 4u) != 0u);
 #pragma unroll
       for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = 8 * t + 2 * tq + (i & 1), key = blk + gq + 8 * (i >> 1);
-          // kept finite, as the large negative value HF masks with is: a row whose keys are all masked then
-          // averages them uniformly, as it does in the prefill kernels and in the reference's softmax
-          mk[t][i] = (r < R && key < (int)a.Sk)
-                         ? fmaxf(__ldg(a.mask + b * a.mask_stride_b + (r % (int)a.Sq) * a.mask_stride_q + key) * kLog2e,
-                                 -3.0e38f)
-                         : 0.f;
+        for (int e = 0; e < 2; ++e) {
+          const int r = 8 * t + 2 * tq + e;
+          uint32_t seen = ~0u;  // visibility of the block's 16 keys
+          if (!read_mask && r < R) {
+            const uint32_t w = a.mb.words[(mbat * a.Sq + r % (int)a.Sq) * (4 * (int64_t)a.mb.T) + blk / 32];
+            seen = w >> (blk % 32);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int key = blk + gq + 8 * h;
+            // kept finite, as the large negative value HF masks with is: a row whose keys are all masked then
+            // averages them uniformly, as it does in the prefill kernels and in the reference's softmax
+            float v = ((seen >> (gq + 8 * h)) & 1u) != 0u ? 0.f : -3.0e38f;
+            if (read_mask)
+              v = (r < R && key < (int)a.Sk)
+                      ? fmaxf(__ldg(a.mask + b * a.mask_stride_b + (r % (int)a.Sq) * a.mask_stride_q + key) * kLog2e,
+                              -3.0e38f)
+                      : 0.f;
+            mk[t][2 * h + e] = v;
+          }
         }
     }
     // ============ scores, transposed: S^T (16 keys x 8 query rows per tile); centroid half s1, sign half s2 ============
@@ -568,6 +610,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
     __syncthreads();
     for (int e = tid; e < 8 * D; e += kWarps * 32) {
       const int r8 = e / D, c = e % D, r = r8 + 8 * t;
+      if (r >= R) break;
       float m = -INFINITY;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) m = fmaxf(m, mrg_ml[w][r][0]);
@@ -579,10 +622,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
         acc = fmaf(mrg_o[w][r8][c], f, acc);
         l = fmaf(mrg_ml[w][r][1], f, l);
       }
-      a.part_o[(unit * kRows + r) * D + c] = acc;
+      a.part_o[(unit * R + r) * D + c] = acc;
       if (c == 0) {
-        a.part_ml[(unit * kRows + r) * 2] = m;
-        a.part_ml[(unit * kRows + r) * 2 + 1] = l;
+        a.part_ml[(unit * R + r) * 2] = m;
+        a.part_ml[(unit * R + r) * 2 + 1] = l;
       }
     }
   }
@@ -664,25 +707,26 @@ __global__ void __launch_bounds__(512) decode_finish_kernel(const float* __restr
 #pragma unroll
   for (int c = 0; c < D / 4; ++c) pv[c] = __ldg(Pi_v + (32 * p + c) * D + j);
   grid_dependency_wait();
-  const float* ml = part_ml + (unit * nsplit * kRows + r) * 2;  // split s: ml[s * kRows * 2], + 1
+  const int R = G * (int)Sq;
+  const float* ml = part_ml + (unit * nsplit * R + r) * 2;  // split s: ml[s * R * 2], + 1
   // every warp finds the maximum and the total weight by itself; warp 0 also publishes the factors
   float m = -INFINITY;
-  for (int s = lane; s < nsplit; s += 32) m = fmaxf(m, ml[(int64_t)s * kRows * 2]);
+  for (int s = lane; s < nsplit; s += 32) m = fmaxf(m, ml[(int64_t)s * R * 2]);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
   float l = 0.f;
   for (int s = lane; s < nsplit; s += 32) {
-    const float ms = ml[(int64_t)s * kRows * 2];
+    const float ms = ml[(int64_t)s * R * 2];
     const float f = (ms == -INFINITY) ? 0.f : exp2f(ms - m);
     if (tid < 32) f_s[s] = f;
-    l = fmaf(ml[(int64_t)s * kRows * 2 + 1], f, l);
+    l = fmaf(ml[(int64_t)s * R * 2 + 1], f, l);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
   __syncthreads();
   float acc = 0.f;
 #pragma unroll 4
-  for (int s = p; s < nsplit; s += 4) acc = fmaf(part_o[((unit * nsplit + s) * kRows + r) * D + j], f_s[s], acc);
+  for (int s = p; s < nsplit; s += 4) acc = fmaf(part_o[((unit * nsplit + s) * R + r) * D + j], f_s[s], acc);
   part[p][j] = acc;
   __syncthreads();
   if (tid < D) o_s[tid] = l > 0.f ? (part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid]) / l : 0.f;
@@ -786,20 +830,32 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
       nsplit = (int)n;
     }
   }
-  TQ_REQUIRE(units * nsplit <= kMaxExtraUnits + B * a.Hq, "partial-result workspace too small for %d splits", nsplit);
+  if (a.mb.words != nullptr) {
+    // Under a summarised mask the splits' live ranges differ (padding), so that equal shares of the keys are not equal
+    // work: up to four waves of smaller splits, which the SMs take as they become free, of at least 256 keys each.
+    // Append and attend of batch 16 x 32 KV heads x 4000 keys, half to all of them live: 253 us reading the additive
+    // mask in one wave, 201 us with the summary, the trimmed ranges and these splits.
+    const int64_t most = (kMaxExtraUnits + B * a.Hq) * kRows / R / units;  // what the partial-result workspace holds
+    int64_t n = (4 * slots + units - 1) / units;
+    n = n < (a.Sk + 255) / 256 ? n : (a.Sk + 255) / 256;
+    n = n < kMaxExtraUnits ? n : kMaxExtraUnits;
+    n = n < most ? n : most;
+    if (n > nsplit) nsplit = (int)n;
+  }
+  TQ_REQUIRE(units * nsplit * R <= (kMaxExtraUnits + B * a.Hq) * kRows, "partial-result workspace too small for %d splits", nsplit);
   int per = (int)((a.Sk + nsplit - 1) / nsplit);
   per = (per + kBlockKeys * kWarps - 1) / (kBlockKeys * kWarps) * (kBlockKeys * kWarps);
   nsplit = (int)((a.Sk + per - 1) / per);
   float* part_o = static_cast<float*>(part_ws);
-  float* part_ml = part_o + (size_t)units * nsplit * kRows * 128;
+  float* part_ml = part_o + (size_t)units * nsplit * R * 128;
   DecodeArgs da{static_cast<const __nv_bfloat16*>(q_cat), a.Hq, a.Hkv, a.Sq, a.Sk, a.kv_stride, a.key_idx, a.key_sgn, a.key_vn,
                 a.key_rn, a.val_idx, a.val_vn, a.cen_k, a.cen_v, a.sm_scale, a.causal, a.mask, a.mask_stride_b,
-                a.mask_stride_q, part_o, part_ml, nsplit, per};
+                a.mask_stride_q, a.mb, part_o, part_ml, nsplit, per};
   dim3 grid((unsigned)nsplit, (unsigned)a.Hkv, (unsigned)B);
   {
     ProfScope prof(kProfAttention, stream);
     void (*kern)(DecodeArgs);
-    if (a.mask == nullptr)
+    if (a.mask == nullptr && a.mb.words == nullptr)
       kern = nt == 1 ? (bits == 2 ? decode_kernel<2, 1, false> : bits == 3 ? decode_kernel<3, 1, false> : decode_kernel<4, 1, false>)
                      : (bits == 2 ? decode_kernel<2, 2, false> : bits == 3 ? decode_kernel<3, 2, false> : decode_kernel<4, 2, false>);
     else

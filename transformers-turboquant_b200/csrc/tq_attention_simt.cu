@@ -310,6 +310,11 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
         float t = s[r][c] * a.sm_scale;
         if (a.mask != nullptr && i < a.Sq && k < a.Sk)
           t += a.mask[b * a.mask_stride_b + (int64_t)i * a.mask_stride_q + k];
+        if (a.mask == nullptr && a.mb.words != nullptr && i < a.Sq && k < a.Sk) {
+          // a boolean mask: a hidden key has the score that adding the most negative float gives
+          const uint32_t w = a.mb.words[((a.mb.batch ? b * a.Sq : 0) + i) * (4 * (int64_t)a.mb.T) + k / 32];
+          if (((w >> (k & 31)) & 1u) == 0u) t = -3.402823466e38f;
+        }
         if (k >= a.Sk || (a.causal && k > i + shift)) t = -INFINITY;
         s[r][c] = t;
         mx = fmaxf(mx, t);
@@ -642,6 +647,13 @@ extern "C" int tq_prepare_queries(const void* q, int dtype, int64_t B, int64_t H
                               q_cat, s);
 }
 
+// A mask to be summarised: additive fp32 or boolean bytes, `nb` = 1 (for every batch element) or B of them.
+struct MaskSource {
+  const void* data;
+  bool boolean;
+  int64_t nb, stride_b, stride_q;
+};
+
 static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t q_stride_b,
                                 int64_t q_stride_h, int64_t q_stride_s, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                 const uint8_t* key_idx, const uint8_t* key_signs, const uint16_t* key_vec_norms,
@@ -651,7 +663,7 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
                                 float sm_scale, int causal, const float* mask, int64_t mask_stride_b,
                                 int64_t mask_stride_q, void* out, int64_t o_stride_b, int64_t o_stride_h,
                                 int64_t o_stride_s, void* workspace, size_t workspace_bytes, int mode, void* stream,
-                                const uint8_t* prepared = nullptr) {
+                                const uint8_t* prepared = nullptr, const MaskSource* src = nullptr) {
   if (int st = check_attention_common(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Hkv, Sk, bits,
                                       mode))
     return st;
@@ -675,9 +687,12 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   TQ_REQUIRE(o_stride_b % al == 0 && o_stride_h % al == 0 && o_stride_s % al == 0,
              "out strides must keep every row 16-byte aligned");
   TQ_REQUIRE(sm_scale == sm_scale, "sm_scale is NaN");
-  const size_t need = prepared != nullptr
-                          ? tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, kv_stride, d, mode)
-                          : tq_attention_workspace_bytes(B, Hq, Sq, d, mode);
+  const size_t call_need = prepared != nullptr
+                               ? tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, kv_stride, d, mode)
+                               : tq_attention_workspace_bytes(B, Hq, Sq, d, mode);
+  size_t mask_need = 0;
+  if (src != nullptr) mask_bits_layout(src->nb, Sq, Sk, nullptr, &mask_need);
+  const size_t need = call_need + mask_need;
   if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
     return fail(TQ_ERR_WORKSPACE, "workspace of %zu bytes needed (256-byte aligned), got %zu", need,
                 workspace_bytes);
@@ -685,8 +700,18 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   if (scope.status()) return scope.status();
   AttnArgs a{nullptr, Hq, Sq, Hkv, Sk, key_idx, key_signs, key_vec_norms, key_residual_norms, val_idx,
              val_vec_norms, centroids_k, centroids_v, Pi_v, sm_scale, causal, mask, mask_stride_b, mask_stride_q,
-             out, dtype, o_stride_b, o_stride_h, o_stride_s, kv_stride};
+             out, dtype, o_stride_b, o_stride_h, o_stride_s, kv_stride, MaskBits{}};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (src != nullptr) {
+    a.mb = mask_bits_layout(src->nb, Sq, Sk, static_cast<uint8_t*>(workspace) + call_need, nullptr);
+    if (!src->boolean) {
+      a.mask = static_cast<const float*>(src->data);
+      a.mask_stride_b = src->nb > 1 ? src->stride_b : 0;
+      a.mask_stride_q = src->stride_q;
+    }
+    if (int st = summarize_mask(src->data, src->boolean, src->nb, src->stride_b, src->stride_q, Sq, Sk, causal, a.mb, s))
+      return st;
+  }
   if (mode == TQ_MODE_FP32) {
     TQ_REQUIRE(kv_stride == Sk, "a cache with capacity > Sk needs TQ_MODE_BF16");
     return attention_fwd_fp32(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
@@ -746,6 +771,40 @@ extern "C" int tq_attention_fwd_prepared(const void* q, int dtype, int64_t B, in
                          dummy, dummy, bits, sm_scale, causal, mask, mask_stride_b, mask_stride_q, out, o_stride_b,
                          o_stride_h, o_stride_s, workspace, workspace_bytes, mode, stream,
                          static_cast<const uint8_t*>(constants));
+}
+
+extern "C" size_t tq_attention_masked_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
+                                                      int64_t kv_capacity, int d, int mode, int64_t mask_batches) {
+  if (B <= 0 || Hq <= 0 || Sq <= 0 || d <= 0 || Hkv <= 0 || Sk <= 0 || mask_batches <= 0) return 0;
+  size_t mask_bytes = 0;
+  mask_bits_layout(mask_batches, Sq, Sk, nullptr, &mask_bytes);
+  return tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, kv_capacity, d, mode) + mask_bytes;
+}
+
+extern "C" int tq_attention_fwd_masked(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d,
+                                       int64_t q_stride_b, int64_t q_stride_h, int64_t q_stride_s, int64_t Hkv,
+                                       int64_t Sk, int64_t kv_capacity, const uint8_t* key_idx,
+                                       const uint8_t* key_signs, const uint16_t* key_vec_norms,
+                                       const uint16_t* key_residual_norms, const uint8_t* val_idx,
+                                       const uint16_t* val_vec_norms, const void* constants, int bits,
+                                       float sm_scale, int causal, const void* mask, int mask_kind,
+                                       int64_t mask_batches, int64_t mask_stride_b, int64_t mask_stride_q, void* out,
+                                       int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, void* workspace,
+                                       size_t workspace_bytes, int mode, void* stream) {
+  TQ_REQUIRE(constants != nullptr && (reinterpret_cast<uintptr_t>(constants) & 255u) == 0,
+             "constants must be a 256-byte aligned buffer filled by tq_prepare_constants");
+  TQ_REQUIRE(kv_capacity >= Sk, "cache capacity %lld is smaller than the %lld keys in use", (long long)kv_capacity,
+             (long long)Sk);
+  TQ_REQUIRE((mask != nullptr || B * Hq * Sq == 0) && (mask_kind == TQ_MASK_ADDITIVE || mask_kind == TQ_MASK_BOOL),
+             "a mask of kind %d (or NULL) is not one the library knows", mask_kind);
+  TQ_REQUIRE(mask_batches == 1 || mask_batches == B, "%lld masks for a batch of %lld", (long long)mask_batches, (long long)B);
+  TQ_REQUIRE(mask_kind == TQ_MASK_BOOL || (reinterpret_cast<uintptr_t>(mask) & 3u) == 0, "an additive mask must be 4-byte aligned");
+  const MaskSource src{mask, mask_kind == TQ_MASK_BOOL, mask_batches, mask_stride_b, mask_stride_q};
+  const float* dummy = reinterpret_cast<const float*>(constants);  // replaced from the buffer inside
+  return attention_entry(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Hkv, Sk, kv_capacity, key_idx,
+                         key_signs, key_vec_norms, key_residual_norms, val_idx, val_vec_norms, dummy, dummy, dummy,
+                         dummy, dummy, bits, sm_scale, causal, nullptr, 0, 0, out, o_stride_b, o_stride_h, o_stride_s,
+                         workspace, workspace_bytes, mode, stream, static_cast<const uint8_t*>(constants), &src);
 }
 
 extern "C" int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t q_stride_b,

@@ -467,7 +467,8 @@ attention_ws_kernel(const AttnArgs a, __nv_bfloat16* __restrict__ o_rot, const i
       }
       tr.mark(2, j);
       float mx = -INFINITY;
-      const bool edge = (k0 + kBN > a.Sk) || (a.causal && k0 + kBN - 1 > q0[tl] + shift) || a.mask != nullptr;
+      const bool edge = (k0 + kBN > a.Sk) || (a.causal && k0 + kBN - 1 > q0[tl] + shift) || a.mask != nullptr ||
+                        a.mb.words != nullptr;
       if (!edge) {
         // raw scores: the positive constant sm_scale*log2(e) is applied to the maximum and inside the exp2
 #pragma unroll
@@ -478,6 +479,10 @@ attention_ws_kernel(const AttnArgs a, __nv_bfloat16* __restrict__ o_rot, const i
         const float* mrow = (a.mask != nullptr && qi < a.Sq)
                                 ? a.mask + b * a.mask_stride_b + (int64_t)qi * a.mask_stride_q + k0
                                 : nullptr;
+        // a boolean mask comes as visibility bits only
+        uint2 seen = make_uint2(~0u, ~0u);
+        if (a.mb.words != nullptr && a.mask == nullptr && qi < a.Sq)
+          seen = *reinterpret_cast<const uint2*>(a.mb.words + ((a.mb.batch ? b * a.Sq : 0) + qi) * (4 * (int64_t)a.mb.T) + k0 / 32);
 #pragma unroll
         for (int c = 0; c < kBN; ++c) {
           const int k = k0 + c;
@@ -487,6 +492,7 @@ attention_ws_kernel(const AttnArgs a, __nv_bfloat16* __restrict__ o_rot, const i
           // accurate: a row whose visible keys are all masked then averages them uniformly, as a softmax over equal
           // finite scores does in the reference, instead of coming out as zeros.
           if (mrow != nullptr && k < a.Sk) v = fmaxf(fmaf(mrow[c], kLog2e, v), -60000.f);
+          if ((((c < 32 ? seen.x : seen.y) >> (c & 31)) & 1u) == 0u) v = -60000.f;
           if (k >= a.Sk || (a.causal && k > qi + shift)) v = -INFINITY;
           t[c] = v * rcexp;  // back to raw units: the exp2 below rescales (-inf stays -inf)
           mx = fmaxf(mx, v);

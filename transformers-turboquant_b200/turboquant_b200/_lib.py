@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(_HERE, "libtq_b200.so")
 TQ_OK = 0
 TQ_F32, TQ_BF16, TQ_F16 = 0, 1, 2
 TQ_MODE_FP32, TQ_MODE_BF16 = 0, 1
+TQ_MASK_ADDITIVE, TQ_MASK_BOOL = 0, 1
 
 
 class TurboQuantError(RuntimeError):
@@ -55,6 +56,9 @@ SIGNATURES = {
     "tq_attention_prepared_workspace_bytes": (_z, [_l, _l, _l, _l, _l, _l, _i, _i]),
     "tq_attention_fwd_prepared": (_i, [_p, _i, _l, _l, _l, _i, _l, _l, _l, _l, _l, _l, _p, _p, _p, _p, _p, _p,
                                        _p, _i, _f, _i, _p, _l, _l, _p, _l, _l, _l, _p, _z, _i, _p]),
+    "tq_attention_masked_workspace_bytes": (_z, [_l, _l, _l, _l, _l, _l, _i, _i, _l]),
+    "tq_attention_fwd_masked": (_i, [_p, _i, _l, _l, _l, _i, _l, _l, _l, _l, _l, _l, _p, _p, _p, _p, _p, _p,
+                                     _p, _i, _f, _i, _p, _i, _l, _l, _l, _p, _l, _l, _l, _p, _z, _i, _p]),
     "tq_compress_keys": (_i, [_p, _i, _l, _l, _l, _i, _l, _l, _l, _p, _p, _p, _p, _i, _p, _p, _p, _p, _i, _p]),
     "tq_compress_values": (_i, [_p, _i, _l, _l, _l, _i, _l, _l, _l, _p, _p, _i, _p, _p, _i, _p]),
     "tq_append_keys": (_i, [_p, _i, _l, _l, _l, _i, _l, _l, _l, _p, _p, _p, _p, _i, _p, _p, _p, _p, _l, _l, _i, _p]),

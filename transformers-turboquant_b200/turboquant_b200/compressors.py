@@ -313,15 +313,12 @@ class TurboQuantCompressorMSE(_Constants):
         return out
 
 
-def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
-    """A mask broadcastable to [B, 1, Sq, Sk] as (tensor, pointer, batch stride, row stride) of an additive
-    fp32 tensor with unit inner stride; (None, None, 0, 0) for no mask.
+def _mask_rows(attention_mask: torch.Tensor, B: int, Sq: int, Sk: int, dev):
+    """A mask broadcastable to [B, 1, Sq, Sk] as a [1 or B, Sq, Sk] tensor with unit inner stride and its kind.
 
     Floating-point masks are additive (0 = visible, large negative = hidden), as HF's eager path builds them.
-    Boolean masks mean True = visible, which is what HF's sdpa path hands over for padded batches; they are
-    turned into the additive form here.  Integer masks are refused: their meaning would be a guess."""
-    if attention_mask is None:
-        return None, None, 0, 0
+    Boolean masks mean True = visible, which is what HF's sdpa path hands over for padded batches; the kernels
+    read their bytes.  Integer masks are refused: their meaning would be a guess."""
     mk = attention_mask
     if mk.dim() == 4:
         if mk.shape[1] != 1:
@@ -330,10 +327,9 @@ def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
     elif mk.dim() == 2:
         mk = mk.unsqueeze(0)
     if mk.dtype == torch.bool:
-        keep = mk.to(device=dev)
-        mk = torch.zeros(keep.shape, dtype=torch.float32, device=dev).masked_fill_(~keep, torch.finfo(torch.float32).min)
+        mk, kind = mk.to(device=dev), _lib.TQ_MASK_BOOL
     elif mk.dtype.is_floating_point:
-        mk = mk.to(device=dev, dtype=torch.float32)
+        mk, kind = mk.to(device=dev, dtype=torch.float32), _lib.TQ_MASK_ADDITIVE
     else:
         raise TypeError(f"attention mask of dtype {mk.dtype} is ambiguous: pass a bool mask (True = visible) or an "
                         "additive floating-point mask")
@@ -341,7 +337,43 @@ def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
         raise ValueError(f"mask shape {tuple(attention_mask.shape)} does not broadcast to [B,1,{Sq},{Sk}]")
     if mk.stride(-1) != 1:
         mk = mk.contiguous()
+    return mk, kind
+
+
+def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
+    """A mask as the C entry points with an additive fp32 mask take it: (tensor, pointer, batch stride, row stride),
+    boolean masks turned into the additive form; (None, None, 0, 0) for no mask."""
+    if attention_mask is None:
+        return None, None, 0, 0
+    mk, kind = _mask_rows(attention_mask, B, Sq, Sk, dev)
+    if kind == _lib.TQ_MASK_BOOL:
+        mk = torch.zeros(mk.shape, dtype=torch.float32, device=dev).masked_fill_(~mk, torch.finfo(torch.float32).min)
     return mk, mk.data_ptr(), (mk.stride(0) if mk.shape[0] == B and B > 1 else 0), mk.stride(1)
+
+
+def _attend(qv: torch.Tensor, Hkv: int, Sk: int, capacity: int, packed: tuple, kc, vc, sm_scale, causal: bool,
+            attention_mask, mode: int) -> torch.Tensor:
+    """One attention call over `packed` = (key indices, signs, norms, residual norms, value indices, norms)."""
+    B, Hq, Sq, D = qv.shape
+    dev = qv.device
+    # [B, Hq, Sq, D] as a view of a [B, Sq, Hq, D] buffer: the adapters' `out.transpose(1, 2).reshape(B, Sq, Hq * D)`
+    # in front of the output projection is then a view, not a copy (the kernels write through the strides)
+    out = torch.empty((B, Sq, Hq, D), dtype=qv.dtype, device=dev).transpose(1, 2)
+    scale = float(sm_scale) if sm_scale is not None else 1.0 / math.sqrt(D)
+    head = (qv.data_ptr(), _DTYPES[qv.dtype], B, Hq, Sq, D, qv.stride(0), qv.stride(1), qv.stride(2), Hkv, Sk, capacity,
+            *[t.data_ptr() for t in packed], prepared_constants(kc, vc).data_ptr(), kc.bits, scale, 1 if causal else 0)
+    tail = (out.data_ptr(), out.stride(0), out.stride(1), out.stride(2))
+    if attention_mask is None:
+        ws = _workspace(dev, _lib.lib.tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, capacity, D, mode))
+        _lib.check(_lib.lib.tq_attention_fwd_prepared(*head, None, 0, 0, *tail, ws.data_ptr(), ws.numel(), mode,
+                                                      _stream_ptr(dev)))
+    else:
+        mk, kind = _mask_rows(attention_mask, B, Sq, Sk, dev)  # mk keeps a converted mask alive
+        ws = _workspace(dev, _lib.lib.tq_attention_masked_workspace_bytes(B, Hq, Sq, Hkv, Sk, capacity, D, mode,
+                                                                          mk.shape[0]))
+        _lib.check(_lib.lib.tq_attention_fwd_masked(*head, mk.data_ptr(), kind, mk.shape[0], mk.stride(0), mk.stride(1),
+                                                    *tail, ws.data_ptr(), ws.numel(), mode, _stream_ptr(dev)))
+    return out
 
 
 @torch.no_grad()
@@ -368,24 +400,10 @@ def fused_attention(q: torch.Tensor, compressed_k: dict, compressed_v: dict,
         raise ValueError("key and value compressors must use the same bit width")
     compressed_k, compressed_v = _dense_packed(compressed_k, _KEY_ARRAYS), _dense_packed(compressed_v, _VALUE_ARRAYS)
     qv = _rows_view(q)
-    dev = qv.device
-    m = resolve_mode(qv.dtype, mode or key_compressor.mode)
-    # [B, Hq, Sq, D] as a view of a [B, Sq, Hq, D] buffer: the adapters' `out.transpose(1, 2).reshape(B, Sq, Hq * D)`
-    # in front of the output projection is then a view, not a copy (the kernels write through the strides)
-    out = torch.empty((B, Sq, Hq, D), dtype=qv.dtype, device=dev).transpose(1, 2)
-    consts = prepared_constants(key_compressor, val_compressor)
-    ws = _workspace(dev, _lib.lib.tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, Sk, D, m))
-    mk, mask_ptr, msb, msq = _mask_args(attention_mask, B, Sq, Sk, dev)  # mk keeps the converted mask alive
-    scale = float(sm_scale) if sm_scale is not None else 1.0 / math.sqrt(D)
-    _lib.check(_lib.lib.tq_attention_fwd_prepared(
-        qv.data_ptr(), _DTYPES[qv.dtype], B, Hq, Sq, D, qv.stride(0), qv.stride(1), qv.stride(2), Hkv, Sk, Sk,
-        compressed_k["packed_key_indices"].data_ptr(), compressed_k["packed_qjl_signs"].data_ptr(),
-        compressed_k["vec_norms"].data_ptr(), compressed_k["residual_norm"].data_ptr(),
-        compressed_v["packed_indices"].data_ptr(), compressed_v["vec_norms"].data_ptr(),
-        consts.data_ptr(), key_compressor.bits, scale, 1 if causal else 0, mask_ptr, msb, msq,
-        out.data_ptr(), out.stride(0), out.stride(1), out.stride(2),
-        ws.data_ptr(), ws.numel(), m, _stream_ptr(dev)))
-    return out
+    packed = (*[compressed_k[n] for n in ("packed_key_indices", "packed_qjl_signs", "vec_norms", "residual_norm")],
+              *[compressed_v[n] for n in ("packed_indices", "vec_norms")])
+    return _attend(qv, Hkv, Sk, Sk, packed, key_compressor, val_compressor, sm_scale, causal, attention_mask,
+                   resolve_mode(qv.dtype, mode or key_compressor.mode))
 
 
 def device_fault_count(device=None) -> int:

@@ -11,12 +11,10 @@ the buffers in place, so a decode step touches each packed byte once and copies 
 
 from __future__ import annotations
 
-import math
-
 import torch
 
 from . import _lib
-from .compressors import (_DTYPES, _mask_args, _require_cuda, _rows_view, _stream_ptr, _workspace,
+from .compressors import (_attend, _DTYPES, _require_cuda, _rows_view, _stream_ptr,
                           TurboQuantCompressorMSE, TurboQuantCompressorV2, fused_attention, prepared_constants,
                           resolve_mode)
 
@@ -127,18 +125,7 @@ class CompressedKVCache:
         # The prefill kernels follow the token stride of the cache as the split-KV kernel does: gathering the prefix
         # first took six strided copies per call (a 300-token chunk behind 8 000 tokens: 149 us with, 115 us without;
         # a step of a GPT-2-shaped layer over 700 tokens: 140 us with, 55 us without).
-        dev = qv.device
-        out = torch.empty((B, Sq, Hq, D), dtype=qv.dtype, device=dev).transpose(1, 2)  # position-major, as fused_attention
-        ws = _workspace(dev, _lib.lib.tq_attention_prepared_workspace_bytes(B, Hq, Sq, self.kv_heads, self.length,
-                                                                            self.capacity, D, _lib.TQ_MODE_BF16))
-        scale = float(sm_scale) if sm_scale is not None else 1.0 / math.sqrt(D)
-        mk, mask_ptr, msb, msq = _mask_args(attention_mask, B, Sq, self.length, dev)  # mk keeps the mask alive
-        _lib.check(_lib.lib.tq_attention_fwd_prepared(
-            qv.data_ptr(), _DTYPES[qv.dtype], B, Hq, Sq, D, qv.stride(0), qv.stride(1), qv.stride(2),
-            self.kv_heads, self.length, self.capacity,
-            self.key_indices.data_ptr(), self.key_signs.data_ptr(), self.key_norms.data_ptr(),
-            self.key_residual_norms.data_ptr(), self.value_indices.data_ptr(), self.value_norms.data_ptr(),
-            prepared_constants(kc, vc).data_ptr(), kc.bits, scale, 1 if causal else 0, mask_ptr, msb, msq,
-            out.data_ptr(), out.stride(0), out.stride(1), out.stride(2),
-            ws.data_ptr(), ws.numel(), _lib.TQ_MODE_BF16, _stream_ptr(dev)))
-        return out
+        packed = (self.key_indices, self.key_signs, self.key_norms, self.key_residual_norms, self.value_indices,
+                  self.value_norms)
+        return _attend(qv, self.kv_heads, self.length, self.capacity, packed, kc, vc, sm_scale, causal, attention_mask,
+                       _lib.TQ_MODE_BF16)
