@@ -1,0 +1,50 @@
+"""Tiles of the fused compression kernel that hold short sequences of several heads and batch elements, both 16-bit input
+types and both head dimensions, against the fp32 kernels on the same data."""
+
+import pytest
+import torch
+
+from helpers import device_compressors
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits_differ(a, b):
+    x = (a ^ b).to(torch.int32)
+    return float(sum(((x >> i) & 1).sum() for i in range(8))) / (8 * a.numel())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d,bits", [(128, 2), (128, 4), (64, 2), (64, 3), (64, 4)])
+@pytest.mark.parametrize("B,H,S", [(1, 1, 1), (3, 5, 1), (16, 32, 1), (2, 200, 1), (5, 3, 7), (3, 7, 30), (2, 3, 64), (2, 3, 65),
+                                   (1, 2, 128), (2, 2, 129), (1, 3, 700)])
+def test_short_sequences_share_tiles(B, H, S, d, bits, dtype):
+    from turboquant_b200 import CompressedKVCache, compress_kv
+
+    g = torch.Generator().manual_seed(B * H + S + d)
+    # rows as a fused projection leaves them: heads side by side, keys and values interleaved
+    x = torch.randn(B, S, 2, H, d, generator=g)
+    x[0, 0, :, 0] = 0.0
+    k, v = (t.transpose(1, 2) for t in x.cuda().to(dtype).unbind(2))
+    kc, vc = device_compressors(d, bits)
+    ck, cv = compress_kv(k, v, kc, vc)
+    kf, vf = device_compressors(d, bits, mode="fp32")
+    fk, fv = kf.compress(k), vf.compress(v)
+    # operands of 22 (fp16) and 16 (bf16) mantissa bits: coordinates within rounding of a boundary may move; an index
+    # that moved moves its residual, and with it a few signs of that row
+    n = k.numel()
+    tight = dtype == torch.float16
+    assert _bits_differ(ck["packed_key_indices"], fk["packed_key_indices"]) <= (1e-6 if tight else 3e-5) + 4 / n
+    assert _bits_differ(cv["packed_indices"], fv["packed_indices"]) <= (1e-6 if tight else 3e-5) + 4 / n
+    assert _bits_differ(ck["packed_qjl_signs"], fk["packed_qjl_signs"]) <= (2e-5 if tight else 2e-4) + 40 / n
+    for a, b in ((ck["vec_norms"], fk["vec_norms"]), (ck["residual_norm"], fk["residual_norm"]), (cv["vec_norms"], fv["vec_norms"])):
+        assert int((a.view(torch.int16).int() - b.view(torch.int16).int()).abs().max()) <= 1
+    # the same rows behind others in a cache, one token short of its end
+    cache = CompressedKVCache(kc, vc, B, H, S + 4)
+    cache.length = 3
+    cache.append(k, v)
+    for buf, ref in ((cache.key_indices, ck["packed_key_indices"]), (cache.key_signs, ck["packed_qjl_signs"]),
+                     (cache.key_norms, ck["vec_norms"]), (cache.key_residual_norms, ck["residual_norm"]),
+                     (cache.value_indices, cv["packed_indices"]), (cache.value_norms, cv["vec_norms"])):
+        assert torch.equal(buf[:, :, 3:3 + S].reshape(-1), ref.reshape(-1))
+        assert not buf[:, :, :3].any() and not buf[:, :, 3 + S:].any()

@@ -16,8 +16,11 @@ struct ConstLayout {
   size_t pi_k, s_eff, pi_v, cen_k, bnd_k, cen_v, bnd_v;           // fp32 originals
   size_t w_cat_pair, w_unrot_pair, luts, w_cat_plain, w_unrot_plain;  // attention: bf16 operand images, fp16 pair tables
   size_t pik_hi, pik_lo, se_hi, se_lo, piv_hi, piv_lo;            // compression: split-bf16 K-major operand images
+  size_t pik16_hi, pik16_lo, se16_hi, se16_lo, piv16_hi, piv16_lo;  // ... and split-fp16 ones (Pi x kPi16Scale)
   size_t total;
 };
+// The fp16 images of the rotations hold Pi x 128: entries of about 0.1 would put the low parts into fp16's subnormals.
+constexpr float kPi16Scale = 128.f;
 constexpr uint32_t kConstMagic = 0x31425154u;  // "TQB1"
 inline ConstLayout const_layout(int d) {
   ConstLayout L{};
@@ -31,6 +34,8 @@ inline ConstLayout const_layout(int d) {
   L.w_cat_plain = take(2 * m16); L.w_unrot_plain = take(m16);
   L.pik_hi = take(m16); L.pik_lo = take(m16); L.se_hi = take(m16); L.se_lo = take(m16);
   L.piv_hi = take(m16); L.piv_lo = take(m16);
+  L.pik16_hi = take(m16); L.pik16_lo = take(m16); L.se16_hi = take(m16); L.se16_lo = take(m16);
+  L.piv16_hi = take(m16); L.piv16_lo = take(m16);
   L.total = off;
   return L;
 }

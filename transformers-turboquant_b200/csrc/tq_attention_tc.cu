@@ -116,6 +116,16 @@ __global__ void build_split_image_kernel(const float* __restrict__ M, int d, __n
   hi[at] = h;
   lo[at] = __float2bfloat16_rn(v - __bfloat162float(h));
 }
+// The same image split into fp16 parts of M x scale: hi + lo carries 22 mantissa bits.
+__global__ void build_split16_image_kernel(const float* __restrict__ M, int d, float scale, __half* __restrict__ hi,
+                                           __half* __restrict__ lo) {
+  const int j = blockIdx.x, i = threadIdx.x;
+  const float v = M[j * d + i] * scale;
+  const __half h = __float2half_rn(v);
+  const int at = operand_index(j, i, d, d);
+  hi[at] = h;
+  lo[at] = __float2half_rn(v - __half2float(h));
+}
 __global__ void copy_floats_kernel(const float* __restrict__ src, float* __restrict__ dst, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
 }
@@ -148,6 +158,10 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
   build_split_image_kernel<<<d, d, 0, stream>>>(Pi_k, d, b16(L.pik_hi), b16(L.pik_lo));
   build_split_image_kernel<<<d, d, 0, stream>>>(S_eff, d, b16(L.se_hi), b16(L.se_lo));
   build_split_image_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.piv_hi), b16(L.piv_lo));
+  auto h16 = [&](size_t off) { return reinterpret_cast<__half*>(c + off); };
+  build_split16_image_kernel<<<d, d, 0, stream>>>(Pi_k, d, kPi16Scale, h16(L.pik16_hi), h16(L.pik16_lo));
+  build_split16_image_kernel<<<d, d, 0, stream>>>(S_eff, d, 1.f, h16(L.se16_hi), h16(L.se16_lo));
+  build_split16_image_kernel<<<d, d, 0, stream>>>(Pi_v, d, kPi16Scale, h16(L.piv16_hi), h16(L.piv16_lo));
   write_header_kernel<<<1, 1, 0, stream>>>(reinterpret_cast<uint32_t*>(c + L.header), d, bits);
   TQ_CUDA_OK(cudaGetLastError());
   return TQ_OK;

@@ -265,7 +265,7 @@ int tq_compress_kv(const void* keys, const void* values, int dtype, int64_t B, i
     CallScope scope(keys != nullptr ? keys : values, "keys/values", static_cast<cudaStream_t>(stream));
     if (scope.status()) return scope.status();
     const int64_t ks[3] = {k_stride_b, k_stride_h, k_stride_s}, vs[3] = {v_stride_b, v_stride_h, v_stride_s};
-    const int st = compress_kv(keys, values, B, H, S, ks, vs, c, bits, key_idx, key_signs, key_vec_norms,
+    const int st = compress_kv(keys, values, dtype, d, B, H, S, ks, vs, c, bits, key_idx, key_signs, key_vec_norms,
                                key_residual_norms, val_idx, val_vec_norms, kv_capacity, kv_offset,
                                static_cast<cudaStream_t>(stream));
     if (st != TQ_ERR_UNSUPPORTED) return st;  // strides no tensor map describes: the per-side kernels read them

@@ -1,4 +1,4 @@
-// Fused key + value compression, one launch (TQ_MODE_BF16, bf16 inputs, head_dim 128).
+// Fused key + value compression, one launch (TQ_MODE_BF16, bf16 or fp16 inputs).
 //
 // Replaces TurboQuantCompressorV2.compress and TurboQuantCompressorMSE.compress of the reference
 // (src/turboquant_pytorch/compressors.py:98-161, :270-294) with the packed result layout of compressors.py:132-138,
@@ -17,6 +17,12 @@
 //     MMA there, so it costs no shared memory and no proxy fence; its projection overwrites the rotated
 //     coordinates it came from.  The sign pass of tile i runs after the index pass of tile i+1, under which the
 //     sketch MMA of tile i has finished;
+//   * fp16 inputs are exact operands of fp16 MMAs against fp16 hi + lo images of the rotations (x 128, to keep the low
+//     parts out of the subnormals) and of the sketch: 22 mantissa bits, small products first.  Against fp64 as many
+//     indices and signs differ as with the fp32 CUDA-core kernel (53 / 113 / 132 of 3.8e8 key indices, signs and value
+//     indices; fp32: 53 / 110 / 131), in 25 us instead of 171 us for the 6 x 8 x 777 keys and values of a padded prompt;
+//   * head_dim 64 takes half of tensor and shared memory, so two CTAs share an SM (8 x 12 x 1024 keys and values: 15 us
+//     instead of 38 us for a launch per side of the kernel in tq_compress_tc.cu);
 //   * the constant operands (Pi hi/lo, S_eff hi/lo for keys; Pi_v hi/lo for values) are bulk-copied from images
 //     built once per compressor pair (tq_prepare_constants).
 //
@@ -46,25 +52,32 @@ int read_compress_kv_faults(unsigned long long* out) {
 
 namespace {
 
-constexpr int kD = 128;
-constexpr int kEpiWarps = 16;
-constexpr int kKvThreads = (kEpiWarps + 1) * 32;
 constexpr int kSlots = 3;
-constexpr uint32_t kTileBytes = 128 * kD * 2;      // one bf16 tile, two 64-column halves of 16 KB
-constexpr uint32_t kMatBytes = kD * kD * 2;        // one bf16 operand image
-constexpr uint32_t kOffX = 0;
-constexpr uint32_t kOffConst = kSlots * kTileBytes;
-constexpr uint32_t kOffExch = kOffConst + 4 * kMatBytes;
-constexpr uint32_t kOffMisc = kOffExch + 4 * 128 * 4;   // barriers, tensor-memory slot, abort flag, centroids
-constexpr uint32_t kSmemBytes = kOffMisc + 256;
-static_assert(kSmemBytes <= 227 * 1024, "shared memory over-subscribed");
-// tensor memory: three accumulator slots (rotated coordinates, later the sketch projection), residual hi, lo
-constexpr uint32_t kColYP = 0, kColRH = 3 * kD, kColRL = 3 * kD + kD / 2;
+template <int D>
+struct KvShape {
+  static constexpr int kParts = D / 32;                 // threads per row
+  static constexpr int kEpiWarps = 4 * kParts;
+  static constexpr int kThreads = (kEpiWarps + 1) * 32;
+  // head_dim 128: all of tensor memory, nearly all of shared memory; head_dim 64: half of either
+  static constexpr int kCtasPerSm = D == 64 ? 2 : 1;
+  static constexpr uint32_t kTileBytes = 128 * D * 2;   // one 16-bit tile: one or two 64-column boxes of 16 KB
+  static constexpr uint32_t kBoxBytes = 128 * 64 * 2;
+  static constexpr uint32_t kMatBytes = D * D * 2;      // one 16-bit operand image
+  static constexpr uint32_t kOffX = 0;
+  static constexpr uint32_t kOffConst = kSlots * kTileBytes;
+  static constexpr uint32_t kOffExch = kOffConst + 4 * kMatBytes;
+  static constexpr uint32_t kOffMisc = kOffExch + kParts * 128 * 4;  // barriers, tensor-memory slot, abort flag, centroids
+  static constexpr uint32_t kSmemBytes = kOffMisc + 256;
+  // tensor memory: three accumulator slots (rotated coordinates, later the sketch projection), residual hi, lo
+  static constexpr uint32_t kColYP = 0, kColRH = 3 * D, kColRL = 3 * D + D / 2, kCols = 4 * D;
+  static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "shared memory over-subscribed");
+};
 
 struct KvArgs {
-  uint32_t units_k, units_v;  // 128-vector tiles on either side (32-bit: unit arithmetic runs per thread and tile)
-  uint32_t tiles_per_head;    // ceil(S / 128)
-  uint32_t S, H;
+  uint32_t units_k, units_v;  // tiles on either side (32-bit: unit arithmetic runs per thread and tile)
+  uint32_t tiles_s, tiles_h;  // tiles along the positions and along the heads (times those along the batch)
+  uint32_t box_s, box_h, box_b;  // positions x heads x batch elements of one tile, at most 128 vectors
+  uint32_t S, H, B;
   const uint8_t* consts;      // constants buffer of tq_prepare_constants
   uint8_t* key_idx;
   uint8_t* key_sgn;
@@ -145,9 +158,19 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
          (1ull << 46) | (2ull << 61);
 }
 
-template <int BITS>
-__global__ void __launch_bounds__(kKvThreads, 1)
+// F16: fp16 inputs (and fp16 operand images of the rotations), else bf16.
+template <int D, int BITS, bool F16>
+__global__ void __launch_bounds__(KvShape<D>::kThreads, KvShape<D>::kCtasPerSm)
 compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const KvArgs a) {
+  using L = KvShape<D>;
+  constexpr int kD = D, kParts = L::kParts, kEpiWarps = L::kEpiWarps;
+  constexpr uint32_t kTileBytes = L::kTileBytes, kMatBytes = L::kMatBytes, kOffX = L::kOffX, kOffConst = L::kOffConst;
+  constexpr uint32_t kOffExch = L::kOffExch, kOffMisc = L::kOffMisc;
+  constexpr uint32_t kColYP = L::kColYP, kColRH = L::kColRH, kColRL = L::kColRL;
+  // Split of the residual for the sketch: fp16 hi + lo of the residual scaled by a power of two (22 mantissa bits), or
+  // bf16 hi + lo (16 bits), which needs no scaling and two operations fewer per coordinate.
+  constexpr bool SK16 = F16 || D == 64;
+  constexpr float kYScale = F16 ? kPi16Scale : 1.f;  // the rotated coordinates come out times this
   constexpr int KB = BITS - 1, VB = BITS;
   constexpr uint32_t SBO = (kD / 8) * 128;  // canonical (unswizzled) K-major images of the constant operands
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -189,27 +212,29 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     }
     tc::mbar_init(r_full, kEpiWarps);
     for (int q = 0; q < 4; ++q) {
-      tc::mbar_init(xch(q), 4);
-      tc::mbar_init(xfree(q), 4);
+      tc::mbar_init(xch(q), kParts);
+      tc::mbar_init(xfree(q), kParts);
     }
     tc::fence_mbar_init();
   }
   if (tid < (1 << KB)) cen_s[tid] = __ldg(reinterpret_cast<const float*>(a.consts + a.L.cen_k) + tid);
-  if (warp == kEpiWarps) tc::tmem_alloc(tc::smem_u32(tmem_slot), 512);
+  if (warp == kEpiWarps) tc::tmem_alloc(tc::smem_u32(tmem_slot), L::kCols);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool ok = true;
 
-  // global unit of this CTA's i-th unit -> side, (batch * head), first row
-  auto unit_of = [&](int i, bool& is_key, int64_t& bh, int& s0) {
+  // this CTA's i-th unit -> side, first batch element, head and position of the tile
+  auto unit_of = [&](int i, bool& is_key, uint32_t& b0, uint32_t& h0, uint32_t& s0) {
     const uint32_t g = c + (uint32_t)i * G;
     is_key = g < a.units_k;
     const uint32_t t = is_key ? g : g - a.units_k;
-    const uint32_t h = t / a.tiles_per_head;
-    bh = h;
-    s0 = (int)(t - h * a.tiles_per_head) * 128;
+    const uint32_t th = t / a.tiles_s;
+    s0 = (t - th * a.tiles_s) * a.box_s;
+    b0 = th / a.tiles_h;
+    h0 = (th - b0 * a.tiles_h) * a.box_h;
+    b0 *= a.box_b;
   };
 
   if (warp == kEpiWarps) {
@@ -218,33 +243,33 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       int issued = 0;  // tiles whose copies have been issued
       auto issue_tile = [&](int i) {
         bool is_key;
-        int64_t bh;
-        int s0;
-        unit_of(i, is_key, bh, s0);
+        uint32_t b0, h0, s0;
+        unit_of(i, is_key, b0, h0, s0);
         const int s = i % kSlots;
         const CUtensorMap* map = is_key ? &map_k : &map_v;
         const uint32_t dst = tc::smem_u32(smem + kOffX + s * kTileBytes);
-        tc::mbar_arrive_expect_tx(x_full(s), kTileBytes);
-        const uint32_t bi = (uint32_t)bh / a.H, hi = (uint32_t)bh - bi * a.H;
-        tma_load_tile(dst, map, 0, s0, (int)hi, (int)bi, x_full(s));
-        tma_load_tile(dst + kTileBytes / 2, map, 64, s0, (int)hi, (int)bi, x_full(s));
+        tc::mbar_arrive_expect_tx(x_full(s), a.box_s * a.box_h * a.box_b * (D * 2));
+#pragma unroll
+        for (int x = 0; x < D / 64; ++x)
+          tma_load_tile(dst + x * L::kBoxBytes, map, 64 * x, (int)s0, (int)h0, (int)b0, x_full(s));
         issued = i + 1;
       };
       auto load_consts = [&](bool keys) {
         const uint32_t dst = tc::smem_u32(smem + kOffConst);
         if (keys) {
           tc::mbar_arrive_expect_tx(const_full, 4 * kMatBytes);
-          tc::bulk_load(dst, a.consts + a.L.pik_hi, kMatBytes, const_full);
-          tc::bulk_load(dst + kMatBytes, a.consts + a.L.pik_lo, kMatBytes, const_full);
-          tc::bulk_load(dst + 2 * kMatBytes, a.consts + a.L.se_hi, kMatBytes, const_full);
-          tc::bulk_load(dst + 3 * kMatBytes, a.consts + a.L.se_lo, kMatBytes, const_full);
+          tc::bulk_load(dst, a.consts + (F16 ? a.L.pik16_hi : a.L.pik_hi), kMatBytes, const_full);
+          tc::bulk_load(dst + kMatBytes, a.consts + (F16 ? a.L.pik16_lo : a.L.pik_lo), kMatBytes, const_full);
+          tc::bulk_load(dst + 2 * kMatBytes, a.consts + (SK16 ? a.L.se16_hi : a.L.se_hi), kMatBytes, const_full);
+          tc::bulk_load(dst + 3 * kMatBytes, a.consts + (SK16 ? a.L.se16_lo : a.L.se_lo), kMatBytes, const_full);
         } else {
           tc::mbar_arrive_expect_tx(const_full, 2 * kMatBytes);
-          tc::bulk_load(dst, a.consts + a.L.piv_hi, kMatBytes, const_full);
-          tc::bulk_load(dst + kMatBytes, a.consts + a.L.piv_lo, kMatBytes, const_full);
+          tc::bulk_load(dst, a.consts + (F16 ? a.L.piv16_hi : a.L.piv_hi), kMatBytes, const_full);
+          tc::bulk_load(dst + kMatBytes, a.consts + (F16 ? a.L.piv16_lo : a.L.piv_lo), kMatBytes, const_full);
         }
       };
-      constexpr uint32_t idesc = tc::idesc_bf16(128, kD, false, false);
+      constexpr uint32_t idesc = F16 ? tc::idesc_f16(128, kD, false, false) : tc::idesc_bf16(128, kD, false, false);
+      constexpr uint32_t idesc_p = SK16 ? tc::idesc_f16(128, kD, false, false) : tc::idesc_bf16(128, kD, false, false);
       const uint32_t cbase = tc::smem_u32(smem + kOffConst);
       const uint64_t b_hi = tc::smem_desc(cbase, 128, SBO), b_lo = tc::smem_desc(cbase + kMatBytes, 128, SBO);
       const uint64_t se_hi = tc::smem_desc(cbase + 2 * kMatBytes, 128, SBO);
@@ -255,15 +280,21 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (!(ok = tc::mbar_wait_or_abort(r_full, i & 1, abort_flag))) return;
         tc::fence_after_sync();
         const uint32_t d_p = tmem + kColYP + (i % kSlots) * kD;
+        auto product = [&](uint32_t col, uint64_t b, uint32_t first) {
 #pragma unroll
-        for (int ks = 0; ks < kD / 16; ++ks)
-          tc::mma_bf16_ts(d_p, tmem + kColRH + ks * 8, se_hi + (uint64_t)(ks * 256 >> 4), idesc, ks > 0);
-#pragma unroll
-        for (int ks = 0; ks < kD / 16; ++ks)
-          tc::mma_bf16_ts(d_p, tmem + kColRH + ks * 8, se_lo + (uint64_t)(ks * 256 >> 4), idesc, 1u);
-#pragma unroll
-        for (int ks = 0; ks < kD / 16; ++ks)
-          tc::mma_bf16_ts(d_p, tmem + kColRL + ks * 8, se_hi + (uint64_t)(ks * 256 >> 4), idesc, 1u);
+          for (int ks = 0; ks < kD / 16; ++ks)
+            tc::mma_bf16_ts(d_p, tmem + col + ks * 8, b + (uint64_t)(ks * 256 >> 4), idesc_p, ks > 0 ? 1u : first ^ 1u);
+        };
+        // the accumulator is truncated at every step, so the 22-bit form adds the large product to the small ones
+        if constexpr (SK16) {
+          product(kColRL, se_hi, 1u);
+          product(kColRH, se_lo, 0u);
+          product(kColRH, se_hi, 0u);
+        } else {
+          product(kColRH, se_hi, 1u);
+          product(kColRH, se_lo, 0u);
+          product(kColRL, se_hi, 0u);
+        }
         tc::mma_commit(p_done(i % kSlots));
       };
       bool keys_loaded = nk > 0;
@@ -295,14 +326,14 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           // rotation: Y_raw = X Pi_hi^T + X Pi_lo^T; K step ks reads 32 bytes of each 128-byte row of half ks / 4
           const uint32_t xb = tc::smem_u32(smem + kOffX + s * kTileBytes);
           const uint32_t d_y = tmem + kColYP + s * kD;
+          auto product = [&](uint64_t b, uint32_t first) {
 #pragma unroll
-          for (int ks = 0; ks < kD / 16; ++ks)
-            tc::mma_bf16(d_y, smem_desc_sw128(xb + (ks / 4) * (kTileBytes / 2) + (ks % 4) * 32),
-                         b_hi + (uint64_t)(ks * 256 >> 4), idesc, ks > 0);
-#pragma unroll
-          for (int ks = 0; ks < kD / 16; ++ks)
-            tc::mma_bf16(d_y, smem_desc_sw128(xb + (ks / 4) * (kTileBytes / 2) + (ks % 4) * 32),
-                         b_lo + (uint64_t)(ks * 256 >> 4), idesc, 1u);
+            for (int ks = 0; ks < kD / 16; ++ks)
+              tc::mma_bf16(d_y, smem_desc_sw128(xb + (ks / 4) * L::kBoxBytes + (ks % 4) * 32), b + (uint64_t)(ks * 256 >> 4),
+                           idesc, ks > 0 ? 1u : first ^ 1u);
+          };
+          product(F16 ? b_lo : b_hi, 1u);
+          product(F16 ? b_hi : b_lo, 0u);
           tc::mma_commit(y_done(s));
         }
         if (sketch_pending) {
@@ -336,6 +367,15 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     for (int j = 0; j < (1 << KB) - 1; ++j) bnd_k[j] = __ldg(reinterpret_cast<const float*>(a.consts + a.L.bnd_k) + j);
 #pragma unroll
     for (int j = 0; j < (1 << VB) - 1; ++j) bnd_v[j] = __ldg(reinterpret_cast<const float*>(a.consts + a.L.bnd_v) + j);
+    // this row of a tile: batch element, head and position relative to the tile's first (rows past the box hold nothing)
+    const uint32_t row_h = (uint32_t)row / a.box_s, row_s = (uint32_t)row - row_h * a.box_s;
+    const uint32_t row_b = row_h / a.box_h, row_hh = row_h - row_b * a.box_h;
+    auto live_row = [&](uint32_t b0, uint32_t h0, uint32_t s0) {
+      return row_b < a.box_b && b0 + row_b < a.B && h0 + row_hh < a.H && s0 + row_s < a.S;
+    };
+    auto out_row = [&](uint32_t b0, uint32_t h0, uint32_t s0) {
+      return ((int64_t)(b0 + row_b) * a.H + h0 + row_hh) * a.out_stride + a.out_offset + s0 + row_s;
+    };
     int n_xch = 0;    // exchanges through `exch` so far in this quarter (phase of xch / xfree)
     // sum of the four parts' values of this row, in a fixed order; every part gets the same total
     auto exchange = [&](float mine, float& total_out) -> bool {
@@ -345,7 +385,8 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(xch(q));
       if (!tc::mbar_wait_or_abort(xch(q), n_xch & 1, abort_flag)) return false;
-      total_out = ((exch[0][row] + exch[1][row]) + exch[2][row]) + exch[3][row];
+      total_out = exch[0][row] + exch[1][row];
+      if constexpr (kParts == 4) total_out = (total_out + exch[2][row]) + exch[3][row];
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(xfree(q));
       ++n_xch;
@@ -355,16 +396,15 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       if (i < n) {
         const int s = i % kSlots, u = i / kSlots;
         bool is_key;
-        int64_t bh;
-        int s0;
-        unit_of(i, is_key, bh, s0);
-        const bool live = (uint32_t)(s0 + row) < a.S;
-        const int64_t no = bh * a.out_stride + a.out_offset + s0 + row;
+        uint32_t b0, h0, s0;
+        unit_of(i, is_key, b0, h0, s0);
+        const bool live = live_row(b0, h0, s0);
+        const int64_t no = out_row(b0, h0, s0);
         // ---- norm of the row: this thread's 64 bytes of the tile as it landed (128-byte swizzle) ----
         if (!(ok = tc::mbar_wait_or_abort(x_full(s), u & 1, abort_flag))) break;
         float ss = 0.f;
         {
-          const uint8_t* xrow = smem + kOffX + s * kTileBytes + (part / 2) * (kTileBytes / 2) + row * 128;
+          const uint8_t* xrow = smem + kOffX + s * kTileBytes + (part / 2) * L::kBoxBytes + row * 128;
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {
             const int chunk = 4 * (part % 2) + cc;  // 16-byte chunk of the row's half
@@ -372,7 +412,15 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xffff0000u);
+              float lo, hi;
+              if constexpr (F16) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                lo = f.x;
+                hi = f.y;
+              } else {
+                lo = __uint_as_float(w[e] << 16);
+                hi = __uint_as_float(w[e] & 0xffff0000u);
+              }
               ss = fmaf(lo, lo, ss);
               ss = fmaf(hi, hi, ss);
             }
@@ -382,7 +430,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (lane == 0) tc::mbar_arrive(x_read(s));
         float ss_tot;
         if (!(ok = exchange(ss, ss_tot))) break;
-        const float nv = sqrtf(ss_tot), den = nv + 1e-8f;
+        const float nv = sqrtf(ss_tot), den1 = nv + 1e-8f, den = kYScale * den1;
         if (!(ok = tc::mbar_wait_or_abort(y_done(s), u & 1, abort_flag))) break;
         tc::fence_after_sync();
         uint32_t raw[32];
@@ -397,7 +445,10 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           uint32_t packed[KB], rh[16], rl[16];
 #pragma unroll
           for (int j = 0; j < KB; ++j) packed[j] = 0;
-          const float neg_nv = -nv;
+          const float neg_nv = -kYScale * nv;
+          // brings the residual's coordinates (at most about the norm) to at most about 64: a power of two
+          const float r_scale = __uint_as_float(
+              (uint32_t)max(127 + 6 - (F16 ? 7 : 0) + 127 - (int)(__float_as_uint(den1) >> 23), 1) << 23);
           static_for<0, 16>([&](auto pc) {
             constexpr int pr = decltype(pc)::value;  // coordinates 2 pr, 2 pr + 1 of this thread's 32
             float res[2];
@@ -412,9 +463,16 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             }
             // split into bf16 hi (truncated: the upper halves of the two words, one byte permute) and lo = the
             // exact remainder, rounded; hi + lo carries ~16 mantissa bits
-            const uint32_t b0 = __float_as_uint(res[0]), b1 = __float_as_uint(res[1]);
-            rh[pr] = __byte_perm(b0, b1, 0x7632);
-            rl[pr] = tc::pack_bf16x2(res[0] - __uint_as_float(b0 & 0xffff0000u), res[1] - __uint_as_float(b1 & 0xffff0000u));
+            if constexpr (SK16) {
+              const float r0 = res[0] * r_scale, r1 = res[1] * r_scale;
+              rh[pr] = tc::pack_f16x2(r0, r1);
+              const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&rh[pr]));
+              rl[pr] = tc::pack_f16x2(r0 - h.x, r1 - h.y);
+            } else {
+              const uint32_t w0 = __float_as_uint(res[0]), w1 = __float_as_uint(res[1]);
+              rh[pr] = __byte_perm(w0, w1, 0x7632);
+              rl[pr] = tc::pack_bf16x2(res[0] - __uint_as_float(w0 & 0xffff0000u), res[1] - __uint_as_float(w1 & 0xffff0000u));
+            }
           });
           if (live) {
             uint32_t* dst = reinterpret_cast<uint32_t*>(a.key_idx + no * (kD * KB / 8) + 4 * KB * part);
@@ -427,7 +485,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           }
           float rr_tot;
           if (!(ok = exchange(rr, rr_tot))) break;
-          if (live && part == 0) a.key_rn[no] = fp16_bits(sqrtf(rr_tot));
+          if (live && part == 0) a.key_rn[no] = fp16_bits(sqrtf(rr_tot) * (1.f / kYScale));
           // the residual operand of the previous key tile must have been consumed by its sketch MMAs
           if (i >= 1 && !(ok = tc::mbar_wait_or_abort(p_done((i - 1) % kSlots), ((i - 1) / kSlots) & 1, abort_flag))) break;
           tc::tmem_st16(tmem + kColRH + lane_base + 16 * part, rh);
@@ -466,9 +524,8 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       if (i >= 1 && i - 1 < nk) {
         const int s1 = (i - 1) % kSlots;
         bool is_key;
-        int64_t bh;
-        int s0;
-        unit_of(i - 1, is_key, bh, s0);
+        uint32_t b0, h0, s0;
+        unit_of(i - 1, is_key, b0, h0, s0);
         if (!(ok = tc::mbar_wait_or_abort(p_done(s1), ((i - 1) / kSlots) & 1, abort_flag))) break;
         tc::fence_after_sync();
         uint32_t raw[32];
@@ -485,8 +542,8 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           const uint32_t sb = raw[e] & 0x80000000u;
           neg = (e == 31 ? sb : __umulhi(sb, 2u << e)) + neg;
         }
-        if ((uint32_t)(s0 + row) < a.S)
-          *reinterpret_cast<uint32_t*>(a.key_sgn + (bh * a.out_stride + a.out_offset + s0 + row) * (kD / 8) + 4 * part) = ~neg;
+        if (live_row(b0, h0, s0))
+          *reinterpret_cast<uint32_t*>(a.key_sgn + out_row(b0, h0, s0) * (kD / 8) + 4 * part) = ~neg;
       }
     }
   }
@@ -496,7 +553,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == kEpiWarps) tc::tmem_dealloc(tmem, 512);
+  if (warp == kEpiWarps) tc::tmem_dealloc(tmem, L::kCols);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -518,59 +575,71 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// Tensor map over a bf16 [B, H, S, 128] view with element strides (sb, sh, ss): box = 64 columns x 128 rows of one
-// (batch, head), 128-byte swizzle, zero fill past the end of S.
-int make_map(CUtensorMap* map, const void* base, int64_t B, int64_t H, int64_t S, int64_t sb, int64_t sh, int64_t ss) {
+// Tensor map over a 16-bit [B, H, S, d] view with element strides (sb, sh, ss): box = 64 columns x the positions, heads
+// and batch elements of a tile, 128-byte swizzle, zero fill past the ends.
+int make_map(CUtensorMap* map, const void* base, bool f16, int d, const KvArgs& a, const int64_t* st) {
   EncodeTiledFn enc = encode_tiled();
   if (enc == nullptr) return fail(TQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  const cuuint64_t dims[4] = {(cuuint64_t)kD, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
+  const cuuint64_t dims[4] = {(cuuint64_t)d, a.S, a.H, a.B};
   // a dimension of extent 1 may carry any stride; the encoder still wants a multiple of 16 bytes
-  const cuuint64_t strides[3] = {(cuuint64_t)(S > 1 ? ss : kD) * 2, (cuuint64_t)(H > 1 ? sh : kD) * 2,
-                                 (cuuint64_t)(B > 1 ? sb : kD) * 2};
-  const cuuint32_t box[4] = {64, 128, 1, 1}, estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint64_t strides[3] = {(cuuint64_t)(a.S > 1 ? st[2] : d) * 2, (cuuint64_t)(a.H > 1 ? st[1] : d) * 2,
+                                 (cuuint64_t)(a.B > 1 ? st[0] : d) * 2};
+  const cuuint32_t box[4] = {64, a.box_s, a.box_h, a.box_b}, estr[4] = {1, 1, 1, 1};
+  const CUresult r = enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TQ_ERR_UNSUPPORTED, "tensor map for strides (%lld, %lld, %lld) refused (CUresult %d)",
-                                     (long long)sb, (long long)sh, (long long)ss, (int)r);
+                                     (long long)st[0], (long long)st[1], (long long)st[2], (int)r);
   return TQ_OK;
+}
+
+template <int D, int BITS, bool F16>
+int launch_kv(const CUtensorMap& map_k, const CUtensorMap& map_v, const KvArgs& a, cudaStream_t stream) {
+  auto kern = compress_kv_kernel<D, BITS, F16>;
+  constexpr uint32_t smem = KvShape<D>::kSmemBytes;
+  TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t total = (int64_t)a.units_k + a.units_v;
+  int grid = sm_count() * KvShape<D>::kCtasPerSm;
+  if (grid > total) grid = (int)total;
+  {
+    ProfScope prof(a.units_k != 0 ? kProfCompressKeys : kProfCompressValues, stream);
+    kern<<<grid, KvShape<D>::kThreads, smem, stream>>>(map_k, map_v, a);
+  }
+  TQ_CUDA_OK(cudaGetLastError());
+  return TQ_OK;
+}
+template <int D, bool F16>
+int launch_bits(int bits, const CUtensorMap& map_k, const CUtensorMap& map_v, const KvArgs& a, cudaStream_t stream) {
+  return bits == 2 ? launch_kv<D, 2, F16>(map_k, map_v, a, stream)
+         : bits == 3 ? launch_kv<D, 3, F16>(map_k, map_v, a, stream) : launch_kv<D, 4, F16>(map_k, map_v, a, stream);
 }
 
 }  // namespace
 
-bool compress_kv_applies(int dtype, int d, int mode) { return dtype == TQ_BF16 && d == kD && mode == TQ_MODE_BF16; }
+bool compress_kv_applies(int dtype, int d, int mode) {
+  return (dtype == TQ_BF16 || dtype == TQ_F16) && (d == 128 || d == 64) && mode == TQ_MODE_BF16;
+}
 
-int compress_kv(const void* k, const void* v, int64_t B, int64_t H, int64_t S, const int64_t* k_strides,
+int compress_kv(const void* k, const void* v, int dtype, int d, int64_t B, int64_t H, int64_t S, const int64_t* k_strides,
                 const int64_t* v_strides, const uint8_t* consts, int bits, uint8_t* key_idx, uint8_t* key_sgn,
                 uint16_t* key_vn, uint16_t* key_rn, uint8_t* val_idx, uint16_t* val_vn, int64_t out_stride,
                 int64_t out_offset, cudaStream_t stream) {
-  const int64_t tiles_per_head = (S + 127) / 128, units = B * H * tiles_per_head;
-  TQ_REQUIRE(units < ((int64_t)1 << 31) && S < ((int64_t)1 << 31) && H < ((int64_t)1 << 31) && B < ((int64_t)1 << 31),
-             "problem too large");
+  const bool f16 = dtype == TQ_F16;
+  TQ_REQUIRE(S < ((int64_t)1 << 31) && H < ((int64_t)1 << 31) && B < ((int64_t)1 << 31), "problem too large");
+  // A tile is up to 128 vectors of one head, or whole short sequences of several heads and batch elements (a generation
+  // step of 16 x 32 heads: 24 us with a tile per head).
+  const int64_t bs = S < 128 ? S : 128, bh = H < 128 / bs ? H : 128 / bs, bb = B < 128 / (bs * bh) ? B : 128 / (bs * bh);
+  const int64_t tiles_s = (S + bs - 1) / bs, tiles_h = (H + bh - 1) / bh, tiles_b = (B + bb - 1) / bb;
+  const int64_t units = tiles_s * tiles_h * tiles_b;
+  TQ_REQUIRE(tiles_s * tiles_h < ((int64_t)1 << 31) && 2 * units < ((int64_t)1 << 31), "problem too large");
+  const KvArgs a{(uint32_t)(k != nullptr ? units : 0), (uint32_t)(v != nullptr ? units : 0), (uint32_t)tiles_s,
+                 (uint32_t)tiles_h, (uint32_t)bs, (uint32_t)bh, (uint32_t)bb, (uint32_t)S, (uint32_t)H, (uint32_t)B, consts,
+                 key_idx, key_sgn, key_vn, key_rn, val_idx, val_vn, out_stride, out_offset, const_layout(d)};
   CUtensorMap map_k, map_v;
-  const void* any = k != nullptr ? k : v;
-  const int64_t* any_strides = k != nullptr ? k_strides : v_strides;
-  if (int st = make_map(&map_k, k != nullptr ? k : any, B, H, S, (k ? k_strides : any_strides)[0],
-                        (k ? k_strides : any_strides)[1], (k ? k_strides : any_strides)[2]))
-    return st;
-  if (int st = make_map(&map_v, v != nullptr ? v : any, B, H, S, (v ? v_strides : any_strides)[0],
-                        (v ? v_strides : any_strides)[1], (v ? v_strides : any_strides)[2]))
-    return st;
-  TQ_REQUIRE(2 * units < ((int64_t)1 << 31), "problem too large");
-  KvArgs a{(uint32_t)(k != nullptr ? units : 0), (uint32_t)(v != nullptr ? units : 0), (uint32_t)tiles_per_head,
-           (uint32_t)S, (uint32_t)H, consts, key_idx, key_sgn, key_vn, key_rn, val_idx, val_vn, out_stride, out_offset,
-           const_layout(kD)};
-  const int64_t total = (int64_t)a.units_k + a.units_v;
-  int grid = sm_count();
-  if (grid > total) grid = (int)total;
-  auto kern = bits == 2 ? compress_kv_kernel<2> : bits == 3 ? compress_kv_kernel<3> : compress_kv_kernel<4>;
-  TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-  {
-    ProfScope prof(k != nullptr ? kProfCompressKeys : kProfCompressValues, stream);
-    kern<<<grid, kKvThreads, kSmemBytes, stream>>>(map_k, map_v, a);
-  }
-  TQ_CUDA_OK(cudaGetLastError());
-  return TQ_OK;
+  if (int st = make_map(&map_k, k != nullptr ? k : v, f16, d, a, k != nullptr ? k_strides : v_strides)) return st;
+  if (int st = make_map(&map_v, v != nullptr ? v : k, f16, d, a, v != nullptr ? v_strides : k_strides)) return st;
+  if (d == 64) return f16 ? launch_bits<64, true>(bits, map_k, map_v, a, stream) : launch_bits<64, false>(bits, map_k, map_v, a, stream);
+  return f16 ? launch_bits<128, true>(bits, map_k, map_v, a, stream) : launch_bits<128, false>(bits, map_k, map_v, a, stream);
 }
 
 }  // namespace tq
