@@ -45,9 +45,9 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
 // Summary of a mask (tq_mask.cu): visibility bits, classes of 16 rows x 128 keys, rows with a visible key.
 struct MaskBits {
   const uint32_t* words;  // [batch][Sq][4 T]; NULL: no summary
-  const uint32_t* rows;   // [batch][NG][NC]: bit r set when row 16 g + r has a visible key in this chunk of 64 tiles
+  const uint32_t* rows;   // [batch][NG][NC]: bit r set when row 16 g + r has a visible key in this chunk of 16 tiles
   const uint8_t* tiles;   // [batch][NG][T]: 1 some key visible, 2 some hidden, 4 some other additive value
-  int T, NG, NC;          // 128-key tiles, 16-row groups, chunks of 64 tiles
+  int T, NG, NC;          // 128-key tiles, 16-row groups, chunks of 16 tiles
   int batch;              // 0: one mask for every batch element
 };
 // The pointers of a summary of `nb` masks at `base` (which may be NULL to ask for the size only).
@@ -82,6 +82,11 @@ struct AttnArgs {
 
 int check_attention_args(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                          int64_t ss, int64_t Hkv, int64_t Sk, int bits, int mode);
+
+// q_cat rows [q Pi^T | coeff (q Pi^T) S_eff^T] of few query rows (fp32 arithmetic; bf16 or fp32 result), any dtype and
+// strides of q; row n = (b * Hq + h) * Sq + s.
+int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh, int64_t ss,
+               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream);
 
 // fp32 mode: query preparation + CUDA-core flash kernel.  `workspace` holds q_cat fp32.
 int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,

@@ -2,7 +2,7 @@
 // keys.  There is no counterpart in the reference, which disables the KV cache and recomputes full
 // attention per generated token (patch.py:80-81); this serves a cache kept in the library's wire format.
 //
-// Three launches per call: `decode_prepare_kernel` (q_cat = [q Pi^T | coeff q Pi^T S^T], fp32), `decode_kernel`
+// Three launches per call: `qprep_rows` (q_cat = [q Pi^T | coeff q Pi^T S^T], fp32 arithmetic), `decode_kernel`
 // (below) and `decode_finish_kernel` (merge of the splits + back-rotation by Pi_v, fp32).
 //
 // The work is bound by the packed bytes (about 100 B per key at 3 bits) and by the instructions that turn them
@@ -631,61 +631,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
   }
 }
 
-__device__ __forceinline__ float load_elem(const void* base, int dtype, int64_t off) {
-  if (dtype == TQ_F32) return static_cast<const float*>(base)[off];
-  if (dtype == TQ_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[off]);
-  return __half2float(static_cast<const __half*>(base)[off]);
-}
 __device__ __forceinline__ void store_elem(void* base, int dtype, int64_t off, float v) {
   if (dtype == TQ_F32) static_cast<float*>(base)[off] = v;
   else if (dtype == TQ_BF16) static_cast<__nv_bfloat16*>(base)[off] = __float2bfloat16_rn(v);
   else static_cast<__half*>(base)[off] = __float2half_rn(v);
-}
-
-// q_cat rows of one (batch, KV head): [q_rot | coeff q_rot S_eff^T] with q_rot = q Pi_k^T (the residual sketch
-// lives in rotated coordinates), fp32 arithmetic on the fp32 matrices, rounded to bf16 once.  A decode-sized
-// call has a few hundred query rows at most, which is no work for a tensor-core tile pipeline: one CTA per
-// (batch, KV head); a warp takes four matrix rows (coalesced 512-byte loads, all in flight at once) and reduces
-// each dot product across its lanes.
-__global__ void __launch_bounds__(1024) decode_prepare_kernel(const void* __restrict__ q, int dtype, int64_t sb, int64_t sh,
-                                                              int64_t ss, int64_t Hq, int64_t Hkv, int64_t Sq,
-                                                              const float* __restrict__ Pi_k, const float* __restrict__ S_eff,
-                                                              float coeff, __nv_bfloat16* __restrict__ q_cat) {
-  constexpr int D = 128;
-  __shared__ __align__(16) float buf[3][kRows][D];  // raw queries, rotated queries, sketch projections
-  grid_launch_dependents();  // the split-KV kernel builds its tables and starts copying packed rows meanwhile
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int64_t b = blockIdx.x / Hkv, kvh = blockIdx.x % Hkv;
-  const int G = (int)(Hq / Hkv), R = G * (int)Sq;
-  for (int e = tid; e < R * D; e += 1024) {
-    const int r = e / D, c = e % D;
-    buf[0][r][c] = load_elem(q, dtype, b * sb + (kvh * G + r / Sq) * sh + (r % Sq) * ss + c);
-  }
-#pragma unroll
-  for (int stage = 0; stage < 2; ++stage) {
-    const float* W = stage == 0 ? Pi_k : S_eff;
-    float4 w[4];
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) w[jj] = __ldg(reinterpret_cast<const float4*>(W + (int64_t)(4 * warp + jj) * D) + lane);
-    __syncthreads();  // the stage's input rows are complete
-    for (int r = 0; r < R; ++r) {
-      const float4 x = *reinterpret_cast<const float4*>(&buf[stage][r][4 * lane]);
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        float p = fmaf(w[jj].x, x.x, fmaf(w[jj].y, x.y, fmaf(w[jj].z, x.z, w[jj].w * x.w)));
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) p += __shfl_xor_sync(0xffffffffu, p, d);
-        if (lane == jj) buf[stage + 1][r][4 * warp + jj] = p;
-      }
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < R * 2 * D; e += 1024) {
-    const int r = e / (2 * D), c = e % (2 * D);
-    const int64_t row = (b * Hq + kvh * G + r / Sq) * Sq + r % Sq;
-    const float v = c < D ? buf[1][r][c] : coeff * buf[2][r][c - D];
-    q_cat[row * (2 * D) + c] = __float2bfloat16_rn(v);
-  }
 }
 
 // One query row per CTA: merge the splits (O = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m)), rotate back
@@ -803,13 +752,8 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
                      int64_t ss, const float* Pi_k, const float* S_eff, void* q_cat, void* part_ws, cudaStream_t stream) {
   const int64_t units = B * a.Hkv;
   const int R = (int)((a.Hq / a.Hkv) * a.Sq);
-  {
-    ProfScope prof(kProfPrepareQueries, stream);
-    decode_prepare_kernel<<<(unsigned)units, 1024, 0, stream>>>(q, q_dtype, sb, sh, ss, a.Hq, a.Hkv, a.Sq, Pi_k, S_eff,
-                                                               sqrtf(1.5707963267948966f) / 128.f,
-                                                               static_cast<__nv_bfloat16*>(q_cat));
-    TQ_CUDA_OK(cudaGetLastError());
-  }
+  // spread over all SMs: 8 x 32 rows take 5 us (8 us with a CTA per KV head)
+  if (int st = qprep_rows(q, q_dtype, B * a.Hq * a.Sq, a.Hq, a.Sq, 128, sb, sh, ss, Pi_k, S_eff, q_cat, true, stream)) return st;
   // One wave of CTAs, each with at least 64 keys (one 16-key block per warp).  The SMs run their resident
   // CTAs side by side and finish with the fullest one, so among the split counts that fit, take the one that
   // fills the SMs most evenly (the largest such count: more warps per SM hide more latency).
@@ -834,7 +778,7 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
     // Under a summarised mask the splits' live ranges differ (padding), so that equal shares of the keys are not equal
     // work: up to four waves of smaller splits, which the SMs take as they become free, of at least 256 keys each.
     // Append and attend of batch 16 x 32 KV heads x 4000 keys, half to all of them live: 253 us reading the additive
-    // mask in one wave, 201 us with the summary, the trimmed ranges and these splits.
+    // mask in one wave, 201 us (159 us now) with the summary, the trimmed ranges and these splits.
     const int64_t most = (kMaxExtraUnits + B * a.Hq) * kRows / R / units;  // what the partial-result workspace holds
     int64_t n = (4 * slots + units - 1) / units;
     n = n < (a.Sk + 255) / 256 ? n : (a.Sk + 255) / 256;

@@ -15,6 +15,7 @@
 namespace tq {
 
 constexpr int kRows = 64;  // query rows and keys per tile
+constexpr int kFewRows = 16;  // query rows per CTA of the few-rows preparation
 
 __device__ __forceinline__ void store8(void* base, int dtype, int64_t off, const float (&v)[8]) {
   if (dtype == TQ_F32) {
@@ -101,6 +102,83 @@ __global__ void __launch_bounds__(16 * (D / 8)) qprep_simt_kernel(const QPrepArg
   }
 }
 
+// ---- query preparation of few rows -----------------------------------------------------
+//
+// The tile kernel above needs both matrices in shared memory before its first product: 33 us for the two rows of an
+// inspection call.  Here eight threads share an output coordinate and hold their part of its two matrix rows in registers
+// (all loads in flight at once), for up to 16 query rows per CTA.  Bound by one trip to L2 and two short reductions:
+// 3.6 us for two rows, 4.9 us for 8 x 32 (8.4 us for the kernel that had one CTA per KV head).
+template <int D, bool BF16_OUT>
+__global__ void __launch_bounds__(8 * D) qprep_rows_kernel(const void* __restrict__ q, int dtype, int64_t n_q, int64_t Hq,
+                                                           int64_t Sq, int64_t sb, int64_t sh, int64_t ss,
+                                                           const float* __restrict__ Pi, const float* __restrict__ S_eff,
+                                                           float coeff, void* __restrict__ q_cat, int rows_per_cta) {
+  constexpr int NV = D / 32;  // float4s of a matrix row per thread: columns 4 part + 32 i .. + 3
+  __shared__ __align__(16) float x[kFewRows][D], y[kFewRows][D];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the split-KV kernel may start its own set-up
+  const int tid = threadIdx.x, j = tid / 8, part = tid % 8;
+  float4 w1[NV], w2[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) w1[i] = __ldg(reinterpret_cast<const float4*>(Pi + j * D + 4 * part + 32 * i));
+#pragma unroll
+  for (int i = 0; i < NV; ++i) w2[i] = __ldg(reinterpret_cast<const float4*>(S_eff + j * D + 4 * part + 32 * i));
+  const int64_t n0 = (int64_t)blockIdx.x * rows_per_cta;
+  const int R = (int)(n_q - n0 < rows_per_cta ? n_q - n0 : rows_per_cta);
+  for (int e = tid; e < R * D; e += 8 * D) {
+    const int r = e / D, c = e % D;
+    const int64_t n = n0 + r, h = (n / Sq) % Hq, b = n / Sq / Hq;
+    const int64_t off = b * sb + h * sh + (n % Sq) * ss + c;
+    x[r][c] = dtype == TQ_F32 ? static_cast<const float*>(q)[off]
+              : dtype == TQ_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(q)[off])
+                                 : __half2float(static_cast<const __half*>(q)[off]);
+  }
+  auto put = [&](int r, int c, float v) {
+    const int64_t at = (n0 + r) * 2 * D + c;
+    if constexpr (BF16_OUT) static_cast<__nv_bfloat16*>(q_cat)[at] = __float2bfloat16_rn(v);
+    else static_cast<float*>(q_cat)[at] = v;
+  };
+  auto project = [&](const float (*in)[D], const float4 (&w)[NV], int r) {
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(&in[r][4 * part + 32 * i]);
+      acc = fmaf(w[i].x, v.x, fmaf(w[i].y, v.y, fmaf(w[i].z, v.z, fmaf(w[i].w, v.w, acc))));
+    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    return acc + __shfl_xor_sync(0xffffffffu, acc, 4);
+  };
+  __syncthreads();
+#pragma unroll 2
+  for (int r = 0; r < R; ++r) {
+    const float v = project(x, w1, r);
+    if (part == 0) {
+      y[r][j] = v;
+      put(r, j, v);
+    }
+  }
+  __syncthreads();
+#pragma unroll 2
+  for (int r = 0; r < R; ++r) {
+    const float v = project(y, w2, r);
+    if (part == 0) put(r, D + j, coeff * v);
+  }
+}
+
+int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh, int64_t ss,
+               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream) {
+  const int64_t sms = sm_count();
+  const int64_t even = (n_q + sms - 1) / sms;  // one wave of CTAs, while they hold that many rows
+  const int per = (int)(even < kFewRows ? even : kFewRows);
+  const unsigned grid = (unsigned)((n_q + per - 1) / per);
+  const float coeff = sqrtf(1.5707963267948966f) / (float)d;
+  auto kern = d == 128 ? (bf16_out ? qprep_rows_kernel<128, true> : qprep_rows_kernel<128, false>)
+                       : (bf16_out ? qprep_rows_kernel<64, true> : qprep_rows_kernel<64, false>);
+  ProfScope prof(kProfPrepareQueries, stream);
+  kern<<<grid, 8 * d, 0, stream>>>(q, dtype, n_q, Hq, Sq, sb, sh, ss, Pi, S_eff, coeff, q_cat, per);
+  TQ_CUDA_OK(cudaGetLastError());
+  return TQ_OK;
+}
 // ---- tile decode helpers -------------------------------------------------------------
 
 // Decode keys [k0, k0+64) of one head into Ks[j][0:D] = C[idx], Ks[j][D:2D] = +-1, and
@@ -238,10 +316,74 @@ __global__ void __launch_bounds__(256) scores_simt_kernel(const ScoreArgs a) {
     }
 }
 
+// Few query rows per head (inspection of single queries, SQ <= 4): the tile kernel above decodes 64 keys for a tile of 64
+// query rows that are not there (24 us for one query over 2 x 8192 keys; 5 us here).  Here four lanes share a key: each decodes a
+// quarter of its coordinates into registers once, multiplies them by the query rows in shared memory and the four meet by
+// two shuffles.
+template <int D, int IB, int SQ>
+__global__ void __launch_bounds__(256) scores_rows_kernel(const ScoreArgs a) {
+  constexpr int PER = D / 4;  // coordinates per lane
+  __shared__ __align__(16) float q_s[SQ][2 * D];
+  __shared__ float cen[1 << IB];
+  const int tid = threadIdx.x, part = tid % 4;
+  const int64_t bh = blockIdx.y, b = bh / a.Hq, h = bh % a.Hq;
+  const int64_t kv_base = (b * a.Hkv + h / (a.Hq / a.Hkv)) * a.Sk;
+  if (tid < (1 << IB)) cen[tid] = a.cen_k[tid];
+  for (int e = tid; e < SQ * 2 * D; e += 256)
+    q_s[e / (2 * D)][e % (2 * D)] = e / (2 * D) < a.Sq ? a.q_cat[bh * a.Sq * 2 * D + e] : 0.f;
+  __syncthreads();
+  const int k = blockIdx.x * 64 + tid / 4;
+  float a1[SQ], a2[SQ];
+#pragma unroll
+  for (int r = 0; r < SQ; ++r) a1[r] = a2[r] = 0.f;
+  if (k < a.Sk) {
+    const int64_t n = kv_base + k;
+    // PER IB-bit indices and PER sign bits: whole 16-bit units at 2-byte aligned addresses
+    const uint16_t* ip = reinterpret_cast<const uint16_t*>(a.key_idx + n * (D * IB / 8)) + part * (PER * IB / 16);
+    const uint16_t* sp = reinterpret_cast<const uint16_t*>(a.key_sgn + n * (D / 8)) + part * (PER / 16);
+#pragma unroll
+    for (int g = 0; g < PER / 16; ++g) {
+      uint64_t w = 0;
+#pragma unroll
+      for (int x = 0; x < IB; ++x) w |= (uint64_t)ip[g * IB + x] << (16 * x);
+      const uint32_t sb = sp[g];
+#pragma unroll
+      for (int c4 = 0; c4 < 16; c4 += 4) {
+        float v[4], sg[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[e] = cen[(uint32_t)(w >> ((c4 + e) * IB)) & ((1u << IB) - 1)];
+          sg[e] = ((sb >> (c4 + e)) & 1u) ? 1.f : -1.f;
+        }
+#pragma unroll
+        for (int r = 0; r < SQ; ++r) {
+          const float4 q1 = *reinterpret_cast<const float4*>(&q_s[r][part * PER + 16 * g + c4]);
+          const float4 q2 = *reinterpret_cast<const float4*>(&q_s[r][D + part * PER + 16 * g + c4]);
+          a1[r] = fmaf(q1.x, v[0], fmaf(q1.y, v[1], fmaf(q1.z, v[2], fmaf(q1.w, v[3], a1[r]))));
+          a2[r] = fmaf(q2.x, sg[0], fmaf(q2.y, sg[1], fmaf(q2.z, sg[2], fmaf(q2.w, sg[3], a2[r]))));
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < SQ; ++r) {
+    a1[r] += __shfl_xor_sync(0xffffffffu, a1[r], 1);
+    a2[r] += __shfl_xor_sync(0xffffffffu, a2[r], 1);
+    a1[r] += __shfl_xor_sync(0xffffffffu, a1[r], 2);
+    a2[r] += __shfl_xor_sync(0xffffffffu, a2[r], 2);
+  }
+  if (k < a.Sk && part == 0) {
+    const float n1 = fp16_value(a.key_vn[kv_base + k]), n2 = fp16_value(a.key_rn[kv_base + k]);
+#pragma unroll
+    for (int r = 0; r < SQ; ++r)
+      if (r < a.Sq) a.scores[(bh * a.Sq + r) * a.Sk + k] = fmaf(n1, a1[r], n2 * a2[r]);
+  }
+}
+
 // ---- fused attention -----------------------------------------------------------------
 
 
-template <int D, int KB, int VB>
+template <int D, int KB, int VB, bool MASK>
 __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
   constexpr int KS = 2 * D + 4, VS = D + 4, PS = kRows + 4, G = D / 8;
   constexpr int NC = D / 16;  // output coordinates per thread in the P V product
@@ -308,12 +450,16 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
       for (int c = 0; c < 4; ++c) {
         const int k = k0 + tx + 16 * c;
         float t = s[r][c] * a.sm_scale;
-        if (a.mask != nullptr && i < a.Sq && k < a.Sk)
-          t += a.mask[b * a.mask_stride_b + (int64_t)i * a.mask_stride_q + k];
-        if (a.mask == nullptr && a.mb.words != nullptr && i < a.Sq && k < a.Sk) {
-          // a boolean mask: a hidden key has the score that adding the most negative float gives
-          const uint32_t w = a.mb.words[((a.mb.batch ? b * a.Sq : 0) + i) * (4 * (int64_t)a.mb.T) + k / 32];
-          if (((w >> (k & 31)) & 1u) == 0u) t = -3.402823466e38f;
+        if constexpr (MASK) {
+          if (i < a.Sq && k < a.Sk) {
+            if (a.mask != nullptr) {
+              t += a.mask[b * a.mask_stride_b + (int64_t)i * a.mask_stride_q + k];
+            } else {
+              // a boolean mask: a hidden key has the score that adding the most negative float gives
+              const uint32_t w = a.mb.words[((a.mb.batch ? b * a.Sq : 0) + i) * (4 * (int64_t)a.mb.T) + k / 32];
+              if (((w >> (k & 31)) & 1u) == 0u) t = -3.402823466e38f;
+            }
+          }
         }
         if (k >= a.Sk || (a.causal && k > i + shift)) t = -INFINITY;
         s[r][c] = t;
@@ -452,6 +598,8 @@ static int launch_qprep(const QPrepArgs& a, cudaStream_t stream) {
 int qprep_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                int64_t ss, const float* Pi, const float* S_eff, float* q_cat, cudaStream_t stream) {
   const int64_t n = B * Hq * Sq;
+  if (n <= (int64_t)kFewRows * sm_count())  // one wave of the few-rows kernel costs less than loading the tile kernel's matrices
+    return qprep_rows(q, dtype, n, Hq, Sq, d, sb, sh, ss, Pi, S_eff, q_cat, false, stream);
   QPrepArgs a{q, n, Hq, Sq, sb, sh, ss, Pi, S_eff, sqrtf(1.5707963267948966f) / (float)d, q_cat,
               (int)((n + kRows - 1) / kRows)};
 #define TQ_CASE(TYPE) return d == 128 ? launch_qprep<TYPE, 128>(a, stream) : launch_qprep<TYPE, 64>(a, stream);
@@ -463,6 +611,14 @@ int qprep_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int 
 
 template <int D, int IB>
 static int launch_scores(const ScoreArgs& a, int64_t B, cudaStream_t stream) {
+  // (16-bit loads of the packed rows)
+  const bool even = ((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn)) & 1u) == 0;
+  if (a.Sq <= 4 && B * a.Hq <= 65535 && even) {
+    auto kern = a.Sq == 1 ? scores_rows_kernel<D, IB, 1> : scores_rows_kernel<D, IB, 4>;
+    kern<<<dim3((unsigned)((a.Sk + 63) / 64), (unsigned)(B * a.Hq)), 256, 0, stream>>>(a);
+    TQ_CUDA_OK(cudaGetLastError());
+    return TQ_OK;
+  }
   constexpr size_t smem = sizeof(float) * (2 * kRows * (2 * D + 4) + 2 * kRows);
   auto kern = scores_simt_kernel<D, IB>;
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -488,7 +644,8 @@ template <int D, int BITS>
 static int launch_attention(const AttnArgs& a, int64_t B, cudaStream_t stream) {
   constexpr size_t smem =
       sizeof(float) * (2 * kRows * (2 * D + 4) + kRows * (D + 4) + kRows * (kRows + 4) + 2 * kRows);
-  auto kern = attention_simt_kernel<D, BITS - 1, BITS>;
+  auto kern = a.mask != nullptr || a.mb.words != nullptr ? attention_simt_kernel<D, BITS - 1, BITS, true>
+                                                         : attention_simt_kernel<D, BITS - 1, BITS, false>;
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((unsigned)((a.Sq + kRows - 1) / kRows), (unsigned)a.Hq, (unsigned)B);
   ProfScope prof(kProfAttention, stream);

@@ -11,7 +11,7 @@
 // unmasked path, and tiles nobody can see are not computed: a hidden score weighs exactly 0 beside a visible one.
 // (Rows with no visible key average all keys of their causal range, so nothing is skipped for their tiles.)
 //
-// A layer's prefill of 6 x 777 padded tokens (32 heads, boolean mask) went from 507 to 371 us: the three elementwise
+// A layer's prefill of 6 x 777 padded tokens (32 heads, boolean mask) went from 507 to 371 us when it came: the three elementwise
 // kernels that made the mask additive (12 us) became this one, and the attention kernel no longer waits for 64 scattered
 // loads per thread and tile.
 //
@@ -22,7 +22,7 @@
 namespace tq {
 namespace {
 
-constexpr int kTileKeys = 128, kGroupRows = 16, kChunkTiles = 64;  // keys per tile, rows per group, tiles per CTA
+constexpr int kTileKeys = 128, kGroupRows = 16, kChunkTiles = 16;  // keys per tile, rows per group, tiles per CTA
 
 struct MaskArgs {
   const void* mask;
@@ -50,35 +50,49 @@ __global__ void __launch_bounds__(kGroupRows * 32) mask_summary_kernel(const Mas
     const int last = a.causal ? min(a.Sk - 1, s + a.shift) : a.Sk - 1;  // last key of the row's causal range
     const int64_t row_off = b * a.stride_b + (int64_t)s * a.stride_q;
     bool any_row = false;
-    for (int t = t0; t < t1; ++t) {
-      const int k = t * kTileKeys + 4 * lane;  // this lane's four keys
-      uint32_t vis = 0, oth = 0;
+    // kAhead tiles' loads in flight: a row is a chain of latencies otherwise (4000 keys: 23 us)
+    constexpr int kAhead = 4;
+    for (int ta = t0; ta < t1; ta += kAhead) {
+    uint32_t raw[kAhead][BOOL ? 2 : 4];
+#pragma unroll
+    for (int x = 0; x < kAhead; ++x) {
+      const int k = (ta + x) * kTileKeys + 4 * lane;  // this lane's four keys
+      const int n = ta + x < t1 ? a.Sk - k : 0;       // how many of them (and after them) exist
       if constexpr (BOOL) {
         // four bytes at any alignment: the aligned words around them, each loaded only if it holds a byte of the row
         const uint8_t* p = static_cast<const uint8_t*>(a.mask) + row_off + k;
-        const int n = a.Sk - k;  // bytes of this lane that exist
-        if (n > 0) {
-          const uint32_t m = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
-          const uint32_t* w = reinterpret_cast<const uint32_t*>(p - m);
-          const uint32_t lo = __ldg(w), hi = (m != 0 && n > (int)(4 - m)) ? __ldg(w + 1) : 0u;
-          const uint32_t v = __funnelshift_r(lo, hi, 8 * m);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) vis |= (e < n && ((v >> (8 * e)) & 0xffu) != 0u) ? 1u << e : 0u;
-        }
+        const uint32_t m = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3u);
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(p - m);
+        raw[x][0] = n > 0 ? __ldg(w) : 0u;
+        raw[x][1] = (m != 0 && n > (int)(4 - m)) ? __ldg(w + 1) : 0u;
       } else {
         const float* p = static_cast<const float*>(a.mask) + row_off + k;
-        float v[4];
-        if (k + 4 <= a.Sk && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(p));
-          v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+          const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+          raw[x][0] = q.x; raw[x][1] = q.y; raw[x][2] = q.z; raw[x][3] = q.w;
         } else {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) v[e] = k + e < a.Sk ? __ldg(p + e) : -INFINITY;
+          for (int e = 0; e < 4; ++e) raw[x][e] = e < n ? __float_as_uint(__ldg(p + e)) : 0xff800000u;
         }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kAhead; ++x) {
+      const int t = ta + x;
+      if (t >= t1) break;
+      const int k = t * kTileKeys + 4 * lane, n = a.Sk - k;
+      uint32_t vis = 0, oth = 0;
+      if constexpr (BOOL) {
+        const uint32_t m = (uint32_t)((reinterpret_cast<uintptr_t>(a.mask) + (uintptr_t)(row_off + k)) & 3u);
+        const uint32_t v = __funnelshift_r(raw[x][0], raw[x][1], 8 * m);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) vis |= (e < n && ((v >> (8 * e)) & 0xffu) != 0u) ? 1u << e : 0u;
+      } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          vis |= v[e] == 0.f ? 1u << e : 0u;
-          oth |= (v[e] == 0.f || v[e] <= -1e30f) ? 0u : 1u << e;  // (a NaN is neither)
+          const float f = __uint_as_float(raw[x][e]);
+          vis |= f == 0.f ? 1u << e : 0u;
+          oth |= (f == 0.f || f <= -1e30f) ? 0u : 1u << e;  // (a NaN is neither)
         }
       }
       const uint32_t seen = vis | oth;  // keys that are not hidden
@@ -93,6 +107,7 @@ __global__ void __launch_bounds__(kGroupRows * 32) mask_summary_kernel(const Mas
       w |= __shfl_xor_sync(0xffffffffu, w, 4);
       if (lane % 8 == 0) a.words[(b * a.Sq + s) * (4 * (int64_t)a.T) + 4 * t + lane / 8] = w;
       if (lane == 0 && all != 0u) atomicOr(&s_cls[t - t0], all);
+    }
     }
     if (__any_sync(0xffffffffu, any_row) && lane == 0) atomicOr(&s_rows, 1u << warp);
   }
