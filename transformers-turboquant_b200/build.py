@@ -3,7 +3,7 @@
     python transformers-turboquant_b200/build.py [--force] [--verbose] [--trace]
 
 Each csrc/*.cu is compiled to an object in build/ (only when its sources changed) and
-the objects are linked into turboquant_b200/libtq_b200.so.  nvcc cross-compiles, so no
+the objects are linked into turboquant_b200/libtq_b200.so; csrc/host/tq_host.cpp becomes turboquant_b200/_tq_host.so.  nvcc cross-compiles, so no
 GPU is needed.  `-Xptxas -v` output (registers, spills, shared memory per kernel) is
 kept in build/ptxas_<file>.log.  `--trace` (implies a full rebuild) adds the diagnostic
 instantiations of the attention kernels that tq_trace_enable / tq_trace_read need; the
@@ -22,6 +22,8 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "turboquant_b200", "libtq_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "tq_host.cpp")
+HOST_LIB = os.path.join(HERE, "turboquant_b200", "_tq_host.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-Xptxas", "-v", "-I", INCLUDE, "-I", CSRC]
@@ -29,6 +31,29 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 
 def _newest(paths):
     return max(os.path.getmtime(p) for p in paths)
+
+
+def build_host(force: bool = False) -> str:
+    """The CPython module with the native tails of the entry points (linked against libtq_b200.so beside it; torch's own
+    libraries are in the process already when it is imported)."""
+    deps = [HOST_SRC, os.path.join(INCLUDE, "tq_b200.h"), LIB, os.path.abspath(__file__)]
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) > _newest(deps):
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+
+    root = os.path.join(os.path.dirname(torch.__file__), "include")
+    includes = [INCLUDE, root, os.path.join(root, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+                os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    res = subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
+                          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[x for i in includes for x in ("-I", i)], HOST_SRC, "-o", HOST_LIB, "-L", os.path.dirname(LIB),
+                          "-l:libtq_b200.so", "-L", os.path.join(os.path.dirname(torch.__file__), "lib"), "-lc10", "-lc10_cuda",
+                          "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"],
+                         capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
+    return HOST_LIB
 
 
 def build(force: bool = False, verbose: bool = False, trace: bool = False) -> str:
@@ -70,6 +95,7 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> st
                               "-lcudart"], capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_host(force)
     return LIB
 
 

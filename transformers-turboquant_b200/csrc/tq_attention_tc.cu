@@ -80,23 +80,31 @@ __device__ __forceinline__ int operand_index(int row, int col, int d, int tile_r
   return (row / tile_rows) * tile_rows * d + (r / 8) * (d * 8) + (col / 8) * 64 + (r % 8) * 8 + col % 8;
 }
 __global__ void build_wcat_kernel(const float* __restrict__ Pi, const float* __restrict__ S_eff, int d, float coeff,
-                                  __nv_bfloat16* __restrict__ w_cat, int tile_rows) {
-  const int j = blockIdx.x, i = threadIdx.x;  // one block per row, d threads
-  w_cat[operand_index(j, i, d, tile_rows)] = __float2bfloat16_rn(Pi[j * d + i]);
+                                  __nv_bfloat16* __restrict__ w_cat, int tile_rows, __nv_bfloat16* __restrict__ w_cat2, int tile_rows2) {
+  const int j = blockIdx.x, i = threadIdx.x;  // one block per row, d threads; a second layout where w_cat2 is given
+  const __nv_bfloat16 top = __float2bfloat16_rn(Pi[j * d + i]);
   float acc = 0.f;
   for (int c = 0; c < d; ++c) acc = fmaf(S_eff[j * d + c], Pi[c * d + i], acc);
-  w_cat[operand_index(d + j, i, d, tile_rows)] = __float2bfloat16_rn(coeff * acc);
+  const __nv_bfloat16 low = __float2bfloat16_rn(coeff * acc);
+  w_cat[operand_index(j, i, d, tile_rows)] = top;
+  w_cat[operand_index(d + j, i, d, tile_rows)] = low;
+  if (w_cat2 != nullptr) {
+    w_cat2[operand_index(j, i, d, tile_rows2)] = top;
+    w_cat2[operand_index(d + j, i, d, tile_rows2)] = low;
+  }
 }
 __global__ void build_wunrot_kernel(const float* __restrict__ Pi_v, int d, __nv_bfloat16* __restrict__ w_unrot,
-                                    int tile_rows) {
+                                    int tile_rows, __nv_bfloat16* __restrict__ w_unrot2, int tile_rows2) {
   const int j = blockIdx.x, i = threadIdx.x;
-  w_unrot[operand_index(j, i, d, tile_rows)] = __float2bfloat16_rn(Pi_v[i * d + j]);
+  const __nv_bfloat16 v = __float2bfloat16_rn(Pi_v[i * d + j]);
+  w_unrot[operand_index(j, i, d, tile_rows)] = v;
+  if (w_unrot2 != nullptr) w_unrot2[operand_index(j, i, d, tile_rows2)] = v;
 }
 
 // Pair tables of the SM-pair kernel: entry (i1 << B | i0) = bf16x2 (C[i0], C[i1]); 4^(bits-1) key entries
 // followed by 4^bits value entries, so that the kernel can bulk-copy them into shared memory.
-__global__ void build_luts_kernel(const float* __restrict__ cen_k, const float* __restrict__ cen_v, int kb, int vb,
-                                  uint32_t* __restrict__ luts) {
+__device__ __forceinline__ void build_luts(const float* __restrict__ cen_k, const float* __restrict__ cen_v, int kb, int vb,
+                                           uint32_t* __restrict__ luts) {
   const int nk = 1 << (2 * kb), nv = 1 << (2 * vb);
   for (int e = threadIdx.x; e < nk + nv; e += blockDim.x) {
     const float* cen = e < nk ? cen_k : cen_v;
@@ -104,35 +112,53 @@ __global__ void build_luts_kernel(const float* __restrict__ cen_k, const float* 
     luts[e] = tc::pack_f16x2(cen[i & ((1 << b) - 1)], cen[i >> b]);
   }
 }
+__global__ void build_luts_kernel(const float* __restrict__ cen_k, const float* __restrict__ cen_v, int kb, int vb,
+                                  uint32_t* __restrict__ luts) {
+  build_luts(cen_k, cen_v, kb, vb, luts);
+}
 
-// Canonical K-major operand image of a row-major fp32 [d, d] matrix, split into bf16 hi = bf16(m) and
-// lo = bf16(m - hi): what the compression kernel's MMAs take as B operands (x (hi + lo)^T carries ~16 mantissa bits).
-__global__ void build_split_image_kernel(const float* __restrict__ M, int d, __nv_bfloat16* __restrict__ hi,
-                                         __nv_bfloat16* __restrict__ lo) {
-  const int j = blockIdx.x, i = threadIdx.x;
-  const float v = M[j * d + i];
+// Canonical K-major operand images of the three fp32 [d, d] matrices (blockIdx.y: Pi_k, S_eff, Pi_v), each split into
+// bf16 hi = bf16(m), lo = bf16(m - hi) (x (hi + lo)^T carries ~16 mantissa bits) and, scaled, into fp16 parts (22 bits):
+// what the compression kernel's MMAs take as B operands; and the matrices themselves.
+struct ImageArgs {
+  const float* src[3];
+  float* copy[3];
+  __nv_bfloat16 *hi[3], *lo[3];
+  __half *hi16[3], *lo16[3];
+  float scale16[3];
+};
+__global__ void build_split_images_kernel(const ImageArgs a, int d) {
+  const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
+  const float v = a.src[m][j * d + i];
+  const int at = operand_index(j, i, d, d);
+  a.copy[m][j * d + i] = v;
   const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  const int at = operand_index(j, i, d, d);
-  hi[at] = h;
-  lo[at] = __float2bfloat16_rn(v - __bfloat162float(h));
+  a.hi[m][at] = h;
+  a.lo[m][at] = __float2bfloat16_rn(v - __bfloat162float(h));
+  const float w = v * a.scale16[m];
+  const __half g = __float2half_rn(w);
+  a.hi16[m][at] = g;
+  a.lo16[m][at] = __float2half_rn(w - __half2float(g));
 }
-// The same image split into fp16 parts of M x scale: hi + lo carries 22 mantissa bits.
-__global__ void build_split16_image_kernel(const float* __restrict__ M, int d, float scale, __half* __restrict__ hi,
-                                           __half* __restrict__ lo) {
-  const int j = blockIdx.x, i = threadIdx.x;
-  const float v = M[j * d + i] * scale;
-  const __half h = __float2half_rn(v);
-  const int at = operand_index(j, i, d, d);
-  hi[at] = h;
-  lo[at] = __float2half_rn(v - __half2float(h));
-}
-__global__ void copy_floats_kernel(const float* __restrict__ src, float* __restrict__ dst, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
-}
-__global__ void write_header_kernel(uint32_t* hdr, int d, int bits) {
-  hdr[0] = kConstMagic;
-  hdr[1] = (uint32_t)d;
-  hdr[2] = (uint32_t)bits;
+// The header, the codebooks and the pair tables (one block).
+struct CodebookArgs {
+  const float* src[4];
+  float* dst[4];
+  int n[4];
+  uint32_t *header, *luts;
+  int d, bits;
+};
+__global__ void copy_codebooks_kernel(const CodebookArgs a) {
+  const int i = threadIdx.x;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (i < a.n[c]) a.dst[c][i] = a.src[c][i];
+  if (i == 0) {
+    a.header[0] = kConstMagic;
+    a.header[1] = (uint32_t)a.d;
+    a.header[2] = (uint32_t)a.bits;
+  }
+  build_luts(a.src[0], a.src[2], a.bits - 1, a.bits, a.luts);
 }
 
 int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k, const float* bnd_k, const float* Pi_v,
@@ -141,28 +167,23 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
   uint8_t* c = static_cast<uint8_t*>(constants);
   auto f32 = [&](size_t off) { return reinterpret_cast<float*>(c + off); };
   auto b16 = [&](size_t off) { return reinterpret_cast<__nv_bfloat16*>(c + off); };
-  const int kb = bits - 1, vb = bits;
-  const struct { const float* src; size_t off; int n; } copies[] = {
-      {Pi_k, L.pi_k, d * d}, {S_eff, L.s_eff, d * d}, {Pi_v, L.pi_v, d * d}, {cen_k, L.cen_k, 1 << kb},
-      {bnd_k, L.bnd_k, (1 << kb) - 1}, {cen_v, L.cen_v, 1 << vb}, {bnd_v, L.bnd_v, (1 << vb) - 1}};
-  for (const auto& cp : copies) {
-    copy_floats_kernel<<<cp.n >= 4096 ? 16 : 1, 256, 0, stream>>>(cp.src, f32(cp.off), cp.n);
-    TQ_CUDA_OK(cudaGetLastError());
-  }
-  const float coeff = sqrtf(1.5707963267948966f) / (float)d;
-  build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, coeff, b16(L.w_cat_pair), d);
-  build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, coeff, b16(L.w_cat_plain), 0);
-  build_wunrot_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.w_unrot_pair), d / 2);
-  build_wunrot_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.w_unrot_plain), 0);
-  build_luts_kernel<<<1, 128, 0, stream>>>(cen_k, cen_v, kb, vb, reinterpret_cast<uint32_t*>(c + L.luts));
-  build_split_image_kernel<<<d, d, 0, stream>>>(Pi_k, d, b16(L.pik_hi), b16(L.pik_lo));
-  build_split_image_kernel<<<d, d, 0, stream>>>(S_eff, d, b16(L.se_hi), b16(L.se_lo));
-  build_split_image_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.piv_hi), b16(L.piv_lo));
   auto h16 = [&](size_t off) { return reinterpret_cast<__half*>(c + off); };
-  build_split16_image_kernel<<<d, d, 0, stream>>>(Pi_k, d, kPi16Scale, h16(L.pik16_hi), h16(L.pik16_lo));
-  build_split16_image_kernel<<<d, d, 0, stream>>>(S_eff, d, 1.f, h16(L.se16_hi), h16(L.se16_lo));
-  build_split16_image_kernel<<<d, d, 0, stream>>>(Pi_v, d, kPi16Scale, h16(L.piv16_hi), h16(L.piv16_lo));
-  write_header_kernel<<<1, 1, 0, stream>>>(reinterpret_cast<uint32_t*>(c + L.header), d, bits);
+  const int kb = bits - 1, vb = bits;
+  const ImageArgs img{{Pi_k, S_eff, Pi_v},
+                      {f32(L.pi_k), f32(L.s_eff), f32(L.pi_v)},
+                      {b16(L.pik_hi), b16(L.se_hi), b16(L.piv_hi)},
+                      {b16(L.pik_lo), b16(L.se_lo), b16(L.piv_lo)},
+                      {h16(L.pik16_hi), h16(L.se16_hi), h16(L.piv16_hi)},
+                      {h16(L.pik16_lo), h16(L.se16_lo), h16(L.piv16_lo)},
+                      {kPi16Scale, 1.f, kPi16Scale}};
+  build_split_images_kernel<<<dim3(d, 3), d, 0, stream>>>(img, d);
+  const CodebookArgs cb{{cen_k, bnd_k, cen_v, bnd_v}, {f32(L.cen_k), f32(L.bnd_k), f32(L.cen_v), f32(L.bnd_v)},
+                        {1 << kb, (1 << kb) - 1, 1 << vb, (1 << vb) - 1}, reinterpret_cast<uint32_t*>(c + L.header),
+                        reinterpret_cast<uint32_t*>(c + L.luts), d, bits};
+  copy_codebooks_kernel<<<1, 128, 0, stream>>>(cb);
+  const float coeff = sqrtf(1.5707963267948966f) / (float)d;
+  build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, coeff, b16(L.w_cat_pair), d, b16(L.w_cat_plain), 0);
+  build_wunrot_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.w_unrot_pair), d / 2, b16(L.w_unrot_plain), 0);
   TQ_CUDA_OK(cudaGetLastError());
   return TQ_OK;
 }
@@ -884,7 +905,7 @@ int prepare_queries_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_
   ProfScope prof(kProfPrepareQueries, stream);
   __nv_bfloat16* w_cat = static_cast<__nv_bfloat16*>(w_cat_scratch);
   if (Pi_k != nullptr) {  // NULL: `w_cat_scratch` already holds the row-major operand (a prepared constants buffer)
-    build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, sqrtf(1.5707963267948966f) / (float)d, w_cat, 0);
+    build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, sqrtf(1.5707963267948966f) / (float)d, w_cat, 0, nullptr, 0);
     TQ_CUDA_OK(cudaGetLastError());
   }
   const int tiles = (int)((n_q + 127) / 128);
@@ -958,7 +979,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
                                                 : reinterpret_cast<uint8_t*>(o_rot) + round256((size_t)n_q * d * 2),
                             stream);
   if (prepared == nullptr) {
-    build_wunrot_kernel<<<d, d, 0, stream>>>(a.Pi_v, d, const_cast<__nv_bfloat16*>(w_unrot), pairs ? d / 2 : 0);
+    build_wunrot_kernel<<<d, d, 0, stream>>>(a.Pi_v, d, const_cast<__nv_bfloat16*>(w_unrot), pairs ? d / 2 : 0, nullptr, 0);
     TQ_CUDA_OK(cudaGetLastError());
   }
   if (pairs) {
@@ -966,7 +987,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
     // bulk-copies its half of either constant operand (d rows of w_cat, d/2 rows of w_unrot)
     if (prepared == nullptr) {
       build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, sqrtf(1.5707963267948966f) / (float)d,
-                                             const_cast<__nv_bfloat16*>(w_cat), d);
+                                             const_cast<__nv_bfloat16*>(w_cat), d, nullptr, 0);
       TQ_CUDA_OK(cudaGetLastError());
       build_luts_kernel<<<1, 128, 0, stream>>>(a.cen_k, a.cen_v, bits - 1, bits, const_cast<uint32_t*>(luts));
       TQ_CUDA_OK(cudaGetLastError());

@@ -95,3 +95,14 @@ def check(status: int) -> None:
 
 def version() -> int:
     return int(lib.tq_version())
+
+
+# the native tails of the Python entry points (torch has to be in the process before it is loaded)
+import torch  # noqa: E402,F401
+
+try:
+    from . import _tq_host as host  # noqa: E402
+except ImportError as e:
+    raise ImportError("the native module _tq_host is missing or does not match this torch: build it with "
+                      "`python transformers-turboquant_b200/build.py --force`") from e
+host.set_error_type(TurboQuantError)

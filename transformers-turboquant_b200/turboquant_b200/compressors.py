@@ -28,8 +28,8 @@ def resolve_mode(dtype: torch.dtype, mode: str | None = None) -> int:
     variable ("fp32" | "bf16"), else by input type: fp32 inputs run the fp32 parity
     kernels, 16-bit inputs the tensor-core kernels."""
     mode = mode or os.environ.get("TQ_B200_MODE") or "auto"
-    if mode == "auto":
-        return _lib.TQ_MODE_FP32 if dtype == torch.float32 else _lib.TQ_MODE_BF16
+    if mode == "auto":  # (types the kernels do not know are read as fp32)
+        return _lib.TQ_MODE_BF16 if dtype in (torch.bfloat16, torch.float16) else _lib.TQ_MODE_FP32
     if mode not in _MODES:
         raise ValueError(f"mode must be 'fp32', 'bf16' or 'auto', got {mode!r}")
     return _MODES[mode]
@@ -60,16 +60,6 @@ def _dense_packed(compressed: dict, keys: tuple) -> dict:
             raise ValueError(f"{name} holds {tuple(t.shape)} entries for a compressed shape {compressed['shape']}")
         out[name] = t if t.is_contiguous() else t.contiguous()
     return out
-
-
-def _rows_view(t: torch.Tensor) -> torch.Tensor:
-    """[B, H, S, D] tensor whose rows the kernels can read in place: supported dtype, unit
-    inner stride, 16-byte aligned rows.  Anything else is copied once."""
-    if t.dtype not in _DTYPES:
-        t = t.float()
-    esz = t.element_size()
-    ok = t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all((s * esz) % 16 == 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
 
 
 def _haar_rotation(d: int, seed: int) -> torch.Tensor:
@@ -148,37 +138,6 @@ def prepared_constants(kc=None, vc=None) -> torch.Tensor:
     return hit[1]
 
 
-_WORKSPACES: dict = {}
-
-
-def _workspace(dev, nbytes: int) -> torch.Tensor:
-    """Scratch for one call.  One buffer per (device, stream) is kept and grown: calls on a stream run in order,
-    so they can share it; during stream capture a fresh tensor is taken from the graph's pool instead."""
-    nbytes = max(int(nbytes), 256)
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), _stream_ptr(dev))
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        _WORKSPACES[key] = ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    return ws
-
-
-def _packed_buffers(kc, vc, B: int, H: int, S: int, D: int, dev):
-    ck = cv = None
-    n = B * H * S
-    if kc is not None:
-        ck = {"packed_key_indices": torch.empty((n, D * kc.mse_bits // 8), dtype=torch.uint8, device=dev),
-              "packed_qjl_signs": torch.empty((n, D // 8), dtype=torch.uint8, device=dev),
-              "residual_norm": torch.empty((B, H, S), dtype=torch.float16, device=dev),
-              "vec_norms": torch.empty((B, H, S), dtype=torch.float16, device=dev), "shape": (B, H, S, D)}
-    if vc is not None:
-        cv = {"packed_indices": torch.empty((n, D * vc.bits // 8), dtype=torch.uint8, device=dev),
-              "vec_norms": torch.empty((n,), dtype=torch.float16, device=dev), "shape": (B, H, S, D)}
-    return ck, cv
-
-
-@torch.no_grad()
 def compress_kv(keys, values, key_compressor=None, val_compressor=None):
     """Compress keys and values [B, H, S, D] in ONE launch (either may be None): what the family adapters do with
     `key_compressor.compress(k)` and `val_compressor.compress(v)` back to back (families/llama.py:103-104 of
@@ -195,23 +154,13 @@ def compress_kv(keys, values, key_compressor=None, val_compressor=None):
     owner = kc or vc
     if D != owner.head_dim or (keys is not None and values is not None and values.shape != keys.shape):
         raise ValueError(f"expected [B, H, S, {owner.head_dim}] keys and values of one shape")
-    k = _rows_view(keys) if kc is not None else None
-    v = _rows_view(values) if vc is not None else None
-    if k is not None and v is not None and k.dtype != v.dtype:
-        v = v.to(k.dtype)
-    x = k if k is not None else v
-    dev = x.device
-    ck, cv = _packed_buffers(kc, vc, B, H, S, D, dev)
-    consts = prepared_constants(kc, vc)
-    ks = k.stride() if k is not None else (0, 0, D, 1)
-    vs = v.stride() if v is not None else (0, 0, D, 1)
-    _lib.check(_lib.lib.tq_compress_kv(
-        k.data_ptr() if k is not None else None, v.data_ptr() if v is not None else None, _DTYPES[x.dtype],
-        B, H, S, D, ks[0], ks[1], ks[2], vs[0], vs[1], vs[2], consts.data_ptr(), owner.bits,
-        ck["packed_key_indices"].data_ptr() if ck else None, ck["packed_qjl_signs"].data_ptr() if ck else None,
-        ck["vec_norms"].data_ptr() if ck else None, ck["residual_norm"].data_ptr() if ck else None,
-        cv["packed_indices"].data_ptr() if cv else None, cv["vec_norms"].data_ptr() if cv else None,
-        S, 0, resolve_mode(x.dtype, owner.mode), _stream_ptr(dev)))
+    ki, ks, rn, vn, vi, vv = _lib.host.compress(keys if kc is not None else None, values if vc is not None else None,
+                                                prepared_constants(kc, vc), owner.bits, resolve_mode(ref.dtype, owner.mode))
+    ck = cv = None
+    if kc is not None:
+        ck = {"packed_key_indices": ki, "packed_qjl_signs": ks, "residual_norm": rn, "vec_norms": vn, "shape": (B, H, S, D)}
+    if vc is not None:
+        cv = {"packed_indices": vi, "vec_norms": vv, "shape": (B, H, S, D)}
     return ck, cv
 
 
@@ -239,14 +188,12 @@ class TurboQuantCompressorV2(_Constants):
         self.S_eff = self.S @ self.Pi.T  # sketch matrix in rotated coordinates
         self.to(device)
 
-    @torch.no_grad()
     def compress(self, states: torch.Tensor) -> dict:
         """[B, H, S, D] -> packed dict (one fused kernel)."""
         if states.dim() != 4 or states.shape[-1] != self.head_dim:
             raise ValueError(f"expected [B, H, S, {self.head_dim}] states, got {tuple(states.shape)}")
         return compress_kv(states, None, key_compressor=self)[0]
 
-    @torch.no_grad()
     def asymmetric_attention_scores(self, queries: torch.Tensor, compressed: dict) -> torch.Tensor:
         """Unscaled, unmasked estimator scores fp32 [B, Hq, Sq, Sk] (compressors.py:163-224).
         Materialises the whole matrix; the adapters use `fused_attention` instead."""
@@ -257,18 +204,9 @@ class TurboQuantCompressorV2(_Constants):
         if (Bk, Dk) != (B, D) or D != self.head_dim:
             raise ValueError(f"queries {tuple(queries.shape)} do not match compressed keys {compressed['shape']}")
         compressed = _dense_packed(compressed, _KEY_ARRAYS)
-        q = _rows_view(queries)
-        dev = q.device
-        scores = torch.empty((B, Hq, Sq, Sk), dtype=torch.float32, device=dev)
-        ws_bytes = _lib.lib.tq_attention_workspace_bytes(B, Hq, Sq, D, _lib.TQ_MODE_FP32)
-        ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-        _lib.check(_lib.lib.tq_attention_scores(
-            q.data_ptr(), _DTYPES[q.dtype], B, Hq, Sq, D, q.stride(0), q.stride(1), q.stride(2), Hkv, Sk,
-            compressed["packed_key_indices"].data_ptr(), compressed["packed_qjl_signs"].data_ptr(),
-            compressed["vec_norms"].data_ptr(), compressed["residual_norm"].data_ptr(),
-            self.Pi.data_ptr(), self.S_eff.data_ptr(), self.centroids.data_ptr(), self.bits,
-            scores.data_ptr(), ws.data_ptr(), ws.numel(), _lib.TQ_MODE_FP32, _stream_ptr(dev)))
-        return scores
+        return _lib.host.scores(queries, Hkv, Sk, *[compressed[n] for n in ("packed_key_indices", "packed_qjl_signs", "vec_norms",
+                                                                            "residual_norm")],
+                                self.Pi, self.S_eff, self.centroids, self.bits)
 
 
 class TurboQuantCompressorMSE(_Constants):
@@ -292,13 +230,11 @@ class TurboQuantCompressorMSE(_Constants):
         self.boundaries = midpoints(self.centroids)
         self.to(device)
 
-    @torch.no_grad()
     def compress(self, states: torch.Tensor) -> dict:
         if states.dim() != 4 or states.shape[-1] != self.head_dim:
             raise ValueError(f"expected [B, H, S, {self.head_dim}] states, got {tuple(states.shape)}")
         return compress_kv(None, states, val_compressor=self)[1]
 
-    @torch.no_grad()
     def decompress(self, compressed: dict) -> torch.Tensor:
         """packed dict -> fp32 [B, H, S, D] (compressors.py:296-317)."""
         B, H, S, D = compressed["shape"]
@@ -306,11 +242,7 @@ class TurboQuantCompressorMSE(_Constants):
         idx = compressed["packed_indices"]
         _require_cuda(idx, "compressed values")
         self._check_device(idx)
-        out = torch.empty((B, H, S, D), dtype=torch.float32, device=idx.device)
-        _lib.check(_lib.lib.tq_decompress_values(
-            idx.data_ptr(), compressed["vec_norms"].data_ptr(), B * H * S, D, self.Pi.data_ptr(),
-            self.centroids.data_ptr(), self.bits, out.data_ptr(), _stream_ptr(idx.device)))
-        return out
+        return _lib.host.decompress(idx, compressed["vec_norms"], self.Pi, self.centroids, self.bits, B, H, S, D)
 
 
 def _mask_rows(attention_mask: torch.Tensor, B: int, Sq: int, Sk: int, dev):
@@ -351,32 +283,15 @@ def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
     return mk, mk.data_ptr(), (mk.stride(0) if mk.shape[0] == B and B > 1 else 0), mk.stride(1)
 
 
-def _attend(qv: torch.Tensor, Hkv: int, Sk: int, capacity: int, packed: tuple, kc, vc, sm_scale, causal: bool,
+def _attend(q: torch.Tensor, Hkv: int, Sk: int, capacity: int, packed: tuple, kc, vc, sm_scale, causal: bool,
             attention_mask, mode: int) -> torch.Tensor:
     """One attention call over `packed` = (key indices, signs, norms, residual norms, value indices, norms)."""
-    B, Hq, Sq, D = qv.shape
-    dev = qv.device
-    # [B, Hq, Sq, D] as a view of a [B, Sq, Hq, D] buffer: the adapters' `out.transpose(1, 2).reshape(B, Sq, Hq * D)`
-    # in front of the output projection is then a view, not a copy (the kernels write through the strides)
-    out = torch.empty((B, Sq, Hq, D), dtype=qv.dtype, device=dev).transpose(1, 2)
-    scale = float(sm_scale) if sm_scale is not None else 1.0 / math.sqrt(D)
-    head = (qv.data_ptr(), _DTYPES[qv.dtype], B, Hq, Sq, D, qv.stride(0), qv.stride(1), qv.stride(2), Hkv, Sk, capacity,
-            *[t.data_ptr() for t in packed], prepared_constants(kc, vc).data_ptr(), kc.bits, scale, 1 if causal else 0)
-    tail = (out.data_ptr(), out.stride(0), out.stride(1), out.stride(2))
-    if attention_mask is None:
-        ws = _workspace(dev, _lib.lib.tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, capacity, D, mode))
-        _lib.check(_lib.lib.tq_attention_fwd_prepared(*head, None, 0, 0, *tail, ws.data_ptr(), ws.numel(), mode,
-                                                      _stream_ptr(dev)))
-    else:
-        mk, kind = _mask_rows(attention_mask, B, Sq, Sk, dev)  # mk keeps a converted mask alive
-        ws = _workspace(dev, _lib.lib.tq_attention_masked_workspace_bytes(B, Hq, Sq, Hkv, Sk, capacity, D, mode,
-                                                                          mk.shape[0]))
-        _lib.check(_lib.lib.tq_attention_fwd_masked(*head, mk.data_ptr(), kind, mk.shape[0], mk.stride(0), mk.stride(1),
-                                                    *tail, ws.data_ptr(), ws.numel(), mode, _stream_ptr(dev)))
-    return out
+    B, _, Sq, D = q.shape
+    mk, kind = (None, 0) if attention_mask is None else _mask_rows(attention_mask, B, Sq, Sk, q.device)
+    return _lib.host.attend(q, Hkv, Sk, capacity, packed, prepared_constants(kc, vc), kc.bits,
+                            float(sm_scale) if sm_scale is not None else 1.0 / math.sqrt(D), 1 if causal else 0, mode, mk, kind)
 
 
-@torch.no_grad()
 def fused_attention(q: torch.Tensor, compressed_k: dict, compressed_v: dict,
                     key_compressor: TurboQuantCompressorV2, val_compressor: TurboQuantCompressorMSE,
                     causal: bool = True, attention_mask: torch.Tensor | None = None,
@@ -399,11 +314,10 @@ def fused_attention(q: torch.Tensor, compressed_k: dict, compressed_v: dict,
     if key_compressor.bits != val_compressor.bits:
         raise ValueError("key and value compressors must use the same bit width")
     compressed_k, compressed_v = _dense_packed(compressed_k, _KEY_ARRAYS), _dense_packed(compressed_v, _VALUE_ARRAYS)
-    qv = _rows_view(q)
     packed = (*[compressed_k[n] for n in ("packed_key_indices", "packed_qjl_signs", "vec_norms", "residual_norm")],
               *[compressed_v[n] for n in ("packed_indices", "vec_norms")])
-    return _attend(qv, Hkv, Sk, Sk, packed, key_compressor, val_compressor, sm_scale, causal, attention_mask,
-                   resolve_mode(qv.dtype, mode or key_compressor.mode))
+    return _attend(q, Hkv, Sk, Sk, packed, key_compressor, val_compressor, sm_scale, causal, attention_mask,
+                   resolve_mode(q.dtype, mode or key_compressor.mode))
 
 
 def device_fault_count(device=None) -> int:

@@ -14,9 +14,8 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .compressors import (_attend, _DTYPES, _require_cuda, _rows_view, _stream_ptr,
-                          TurboQuantCompressorMSE, TurboQuantCompressorV2, fused_attention, prepared_constants,
-                          resolve_mode)
+from .compressors import (_attend, _require_cuda, TurboQuantCompressorMSE, TurboQuantCompressorV2, fused_attention,
+                          prepared_constants, resolve_mode)
 
 
 class CompressedKVCache:
@@ -59,7 +58,6 @@ class CompressedKVCache:
     def reset(self) -> None:
         self.length = 0
 
-    @torch.no_grad()
     def append(self, keys: torch.Tensor, values: torch.Tensor) -> None:
         """Compress [B, Hkv, S_new, D] keys and values and store them behind the tokens in use."""
         B, H, S, D = keys.shape
@@ -72,16 +70,10 @@ class CompressedKVCache:
         kc, vc = self.key_compressor, self.val_compressor
         kc._check_device(keys)
         vc._check_device(keys)
-        k, v = _rows_view(keys), _rows_view(values)
-        if v.dtype != k.dtype:
-            v = v.to(k.dtype)
         # one launch compresses both sides straight behind the tokens in use: no scratch, no copies
-        _lib.check(_lib.lib.tq_compress_kv(
-            k.data_ptr(), v.data_ptr(), _DTYPES[k.dtype], B, H, S, D, k.stride(0), k.stride(1), k.stride(2),
-            v.stride(0), v.stride(1), v.stride(2), prepared_constants(kc, vc).data_ptr(), kc.bits,
-            self.key_indices.data_ptr(), self.key_signs.data_ptr(), self.key_norms.data_ptr(),
-            self.key_residual_norms.data_ptr(), self.value_indices.data_ptr(), self.value_norms.data_ptr(),
-            self.capacity, self.length, resolve_mode(k.dtype, kc.mode), _stream_ptr(k.device)))
+        _lib.host.append(keys, values, prepared_constants(kc, vc), kc.bits, resolve_mode(keys.dtype, kc.mode), self.key_indices,
+                         self.key_signs, self.key_norms, self.key_residual_norms, self.value_indices, self.value_norms,
+                         self.capacity, self.length)
         self.length += S
 
     def _contiguous_prefix(self) -> tuple[dict, dict]:
@@ -99,7 +91,6 @@ class CompressedKVCache:
               "vec_norms": self.value_norms[:, :, :n].reshape(-1).contiguous(), "shape": shape}
         return ck, cv
 
-    @torch.no_grad()
     def attend(self, q: torch.Tensor, causal: bool = True, sm_scale: float | None = None,
                attention_mask: torch.Tensor | None = None) -> torch.Tensor:
         """softmax(scores * sm_scale) @ V_hat of q [B, Hq, Sq, D] over the tokens in use; with `causal` the
@@ -114,8 +105,7 @@ class CompressedKVCache:
             raise ValueError(f"queries {tuple(q.shape)} do not match the cache")
         if self.length == 0:
             raise ValueError("attention over an empty cache is undefined")
-        qv = _rows_view(q)
-        if resolve_mode(qv.dtype, self.key_compressor.mode) != _lib.TQ_MODE_BF16:
+        if resolve_mode(q.dtype, self.key_compressor.mode) != _lib.TQ_MODE_BF16:
             ck, cv = self._contiguous_prefix()
             return fused_attention(q, ck, cv, self.key_compressor, self.val_compressor, causal=causal,
                                    attention_mask=attention_mask, sm_scale=sm_scale)
@@ -127,5 +117,5 @@ class CompressedKVCache:
         # a step of a GPT-2-shaped layer over 700 tokens: 140 us with, 55 us without).
         packed = (self.key_indices, self.key_signs, self.key_norms, self.key_residual_norms, self.value_indices,
                   self.value_norms)
-        return _attend(qv, self.kv_heads, self.length, self.capacity, packed, kc, vc, sm_scale, causal, attention_mask,
+        return _attend(q, self.kv_heads, self.length, self.capacity, packed, kc, vc, sm_scale, causal, attention_mask,
                        _lib.TQ_MODE_BF16)
