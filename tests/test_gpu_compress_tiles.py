@@ -30,13 +30,17 @@ def test_short_sequences_share_tiles(B, H, S, d, bits, dtype):
     ck, cv = compress_kv(k, v, kc, vc)
     kf, vf = device_compressors(d, bits, mode="fp32")
     fk, fv = kf.compress(k), vf.compress(v)
-    # operands of 22 (fp16) and 16 (bf16) mantissa bits: coordinates within rounding of a boundary may move; an index
+    # bf16: operands of 16 mantissa bits, coordinates within rounding of a boundary may move; an index
     # that moved moves its residual, and with it a few signs of that row
     n = k.numel()
     tight = dtype == torch.float16
-    assert _bits_differ(ck["packed_key_indices"], fk["packed_key_indices"]) <= (1e-6 if tight else 3e-5) + 4 / n
-    assert _bits_differ(cv["packed_indices"], fv["packed_indices"]) <= (1e-6 if tight else 3e-5) + 4 / n
-    assert _bits_differ(ck["packed_qjl_signs"], fk["packed_qjl_signs"]) <= (2e-5 if tight else 2e-4) + 40 / n
+    # (fp16 coordinates too close to call are decided by the fp32 arithmetic: the same bytes)
+    if tight:
+        for a, b in ((ck["packed_key_indices"], fk["packed_key_indices"]), (cv["packed_indices"], fv["packed_indices"]), (ck["packed_qjl_signs"], fk["packed_qjl_signs"])):
+            assert torch.equal(a, b)
+    assert _bits_differ(ck["packed_key_indices"], fk["packed_key_indices"]) <= 3e-5 + 4 / n
+    assert _bits_differ(cv["packed_indices"], fv["packed_indices"]) <= 3e-5 + 4 / n
+    assert _bits_differ(ck["packed_qjl_signs"], fk["packed_qjl_signs"]) <= 2e-4 + 40 / n
     for a, b in ((ck["vec_norms"], fk["vec_norms"]), (ck["residual_norm"], fk["residual_norm"]), (cv["vec_norms"], fv["vec_norms"])):
         assert int((a.view(torch.int16).int() - b.view(torch.int16).int()).abs().max()) <= 1
     # the same rows behind others in a cache, one token short of its end

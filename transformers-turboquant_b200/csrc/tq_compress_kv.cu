@@ -19,8 +19,9 @@
 //     sketch MMA of tile i has finished;
 //   * fp16 inputs are exact operands of fp16 MMAs against fp16 hi + lo images of the rotations (x 128, to keep the low
 //     parts out of the subnormals) and of the sketch: 22 mantissa bits, small products first.  Against fp64 as many
-//     indices and signs differ as with the fp32 CUDA-core kernel (53 / 113 / 132 of 3.8e8 key indices, signs and value
-//     indices; fp32: 53 / 110 / 131), in 25 us instead of 171 us for the 6 x 8 x 777 keys and values of a padded prompt;
+//     indices and signs differ as with the fp32 CUDA-core kernel (53 / 113 / 132 of 4e8 key indices, signs and value
+//     indices; fp32: 53 / 110 / 131), and with the repair below the same ones: 48 us instead of 171 us for the 6 x 8 x 777
+//     keys and values of a padded prompt;
 //   * head_dim 64 takes half of tensor and shared memory, so two CTAs share an SM (8 x 12 x 1024 keys and values: 15 us
 //     instead of 38 us for a launch per side of the kernel in tq_compress_tc.cu);
 //   * the constant operands (Pi hi/lo, S_eff hi/lo for keys; Pi_v hi/lo for values) are bulk-copied from images
@@ -85,6 +86,8 @@ struct KvArgs {
   uint16_t* key_rn;
   uint8_t* val_idx;
   uint16_t* val_vn;
+  const void *k, *v;             // the inputs and their element strides (batch, head, position): fp16 repair only
+  int64_t k_stride[3], v_stride[3];
   int64_t out_stride, out_offset;  // vector (bh, s) -> output row bh * out_stride + out_offset + s
   ConstLayout L;
 };
@@ -133,6 +136,96 @@ __device__ __forceinline__ void put_field(uint32_t (&w)[B], uint32_t idx) {
   w[k] = idx * (1u << sh) + w[k];  // the field's bits are still zero there: + is |
   if constexpr (sh + B > 32) w[k + 1] = (idx >> (32 - sh)) + w[k + 1];
 }
+// Repair of fp16 decisions that the tensor-core sums leave open.
+//
+// An index or a sign whose coordinate lies within the sums' rounding of its boundary may fall either way, and a single
+// moved index moves about seven sign bytes of its vector.  A 16-bit input type with exact operands should not differ from
+// the fp32 kernel in that way, so coordinates within kOpenIndex (in units of the norm; the sums are off by 1e-8 on
+// average) and projections within kOpenSign (in units of the residual's norm; off by 1e-6) are decided by the fp32
+// kernel's own arithmetic: the functions below, one warp per open coordinate, with its order of operations.  About one
+// vector in 700 has one; the compression of 6 x 8 x 777 keys and values takes 48 us with the
+// repair and 22 us without (171 us on the fp32 kernels).
+constexpr float kOpenIndex = 1.6e-7f, kOpenSign = 6e-6f;
+
+// The fp32 kernel's norm of an fp16 row (sums of eight, then a butterfly) and this lane's normalised coordinates.
+template <int D>
+struct ExactRow {
+  static constexpr int N = D / 32;  // coordinates per lane: N lane .. N lane + N - 1
+  float x[N], norm;
+  __device__ explicit ExactRow(const __half* row) {
+    const int lane = threadIdx.x % 32, g = lane % (D / 8);
+    float ss = 0.f;
+    for (int e = 0; e < 8; ++e) {
+      const float f = __half2float(row[8 * g + e]);
+      ss = fmaf(f, f, ss);
+    }
+    for (int off = D / 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    norm = sqrtf(ss);
+    const float den = norm + 1e-8f;
+#pragma unroll
+    for (int e = 0; e < N; ++e) x[e] = __half2float(row[N * lane + e]) / den;
+  }
+};
+// sum over i = 0 .. D - 1, in that order, of in[i] * m[i]; `in` spread over the lanes as in ExactRow
+template <int D>
+__device__ __forceinline__ float exact_dot(const float (&in)[D / 32], const float* __restrict__ m) {
+  constexpr int N = D / 32;
+  float w[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) w[e] = __ldg(m + N * (threadIdx.x % 32) + e);
+  float acc = 0.f;
+#pragma unroll 4
+  for (int l = 0; l < 32; ++l)
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      acc = fmaf(__shfl_sync(0xffffffffu, in[e], l), __shfl_sync(0xffffffffu, w[e], l), acc);
+  return acc;
+}
+// Rotated coordinate of a row, as the fp32 kernel computes it (`m` is that row of the rotation).
+template <int D>
+__device__ __noinline__ float exact_coordinate(const __half* row, const float* __restrict__ m) {
+  const ExactRow<D> r(row);
+  return exact_dot<D>(r.x, m);
+}
+// Projection j of the residual of a key row, as the fp32 kernel computes it.
+template <int D, int NB>
+__device__ __noinline__ float exact_projection(const __half* row, const float* __restrict__ Pi,
+                                               const float* __restrict__ S_eff, const float* __restrict__ bnd,
+                                               const float* __restrict__ cen, int j) {
+  constexpr int N = D / 32;
+  const ExactRow<D> r(row);
+  const float np = r.norm + 1e-8f;
+  const int lane = threadIdx.x % 32;
+  float y[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) y[e] = 0.f;
+  // this lane's N rotated coordinates, sums over i in order
+#pragma unroll 1
+  for (int l0 = 0; l0 < 32; l0 += 4) {
+    float w[N][4 * N];  // 4 N columns of this lane's N rows, all loads in flight
+#pragma unroll
+    for (int o = 0; o < N; ++o)
+#pragma unroll
+      for (int c = 0; c < 4 * N; c += 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(Pi + (N * lane + o) * D + N * l0 + c));
+        w[o][c] = v.x; w[o][c + 1] = v.y; w[o][c + 2] = v.z; w[o][c + 3] = v.w;
+      }
+#pragma unroll
+    for (int c = 0; c < 4 * N; ++c) {
+      const float xs = __shfl_sync(0xffffffffu, r.x[c % N], l0 + c / N);
+#pragma unroll
+      for (int o = 0; o < N; ++o) y[o] = fmaf(xs, w[o][c], y[o]);
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < N; ++o) {
+    int idx = 0;
+    for (int b = 0; b < NB; ++b) idx += y[o] > __ldg(bnd + b) ? 1 : 0;
+    y[o] = fmaf(np, y[o], -r.norm * __ldg(cen + idx));
+  }
+  return exact_dot<D>(y, S_eff + j * D);
+}
+
 template <int FROM, int TO, class F>
 __device__ __forceinline__ void static_for(F&& f) {
   if constexpr (FROM < TO) {
@@ -376,6 +469,57 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     auto out_row = [&](uint32_t b0, uint32_t h0, uint32_t s0) {
       return ((int64_t)(b0 + row_b) * a.H + h0 + row_hh) * a.out_stride + a.out_offset + s0 + row_s;
     };
+    // where this row is in the input (fp16 repair), as one address per lane
+    auto row_address = [&](bool key, uint32_t b0, uint32_t h0, uint32_t s0) {
+      const int64_t* st = key ? a.k_stride : a.v_stride;
+      return reinterpret_cast<unsigned long long>(static_cast<const __half*>(key ? a.k : a.v) + (int64_t)(b0 + row_b) * st[0] +
+                                                  (int64_t)(h0 + row_hh) * st[1] + (int64_t)(s0 + row_s) * st[2]);
+    };
+    // Distance of a rotated coordinate to the nearest of the scaled boundaries (codebooks of 8 and more levels by symmetry,
+    // as in index_of).
+    auto distance = [](auto nb, const float (&bden)[decltype(nb)::value], float y) {
+      constexpr int NB = decltype(nb)::value, h = (NB + 1) / 2;
+      float near = NB < 7 ? fabsf(bden[0] - y) : fabsf(y);
+      if constexpr (NB < 7) {
+#pragma unroll
+        for (int j = 1; j < NB; ++j) near = fminf(near, fabsf(bden[j] - y));
+      } else {
+#pragma unroll
+        for (int j = h; j < NB; ++j) near = fminf(near, fabsf(bden[j] - fabsf(y)));
+      }
+      return near;
+    };
+    // Rotated coordinates of this warp's 32 rows x 32 coordinates, in `raw` and in tensor memory at `col`: those within
+    // `band` of a boundary are moved (in tensor memory) to the side of it that the fp32 kernel finds them on.
+    auto settle = [&](auto nb, const float* Pi, const float (&bnd)[decltype(nb)::value], const float (&bden)[decltype(nb)::value],
+                      const uint32_t (&raw)[32], uint32_t col, float band, unsigned long long addr) {
+      constexpr int NB = decltype(nb)::value;
+      uint32_t open = 0;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) open |= distance(nb, bden, __uint_as_float(raw[e])) < band ? 1u << e : 0u;
+      uint32_t lanes;
+      while ((lanes = __ballot_sync(0xffffffffu, open != 0u)) != 0u) {
+        const int l = __ffs((int)lanes) - 1;
+        const int e = __ffs((int)__shfl_sync(0xffffffffu, open, l)) - 1;
+        const float exact = exact_coordinate<D>(reinterpret_cast<const __half*>(__shfl_sync(0xffffffffu, addr, l)),
+                                                Pi + (32 * part + e) * D);
+        float y = tc::tmem_ld1(col + e);
+        if (lane == l) {
+          open &= open - 1u;
+          float near = INFINITY, at = 0.f, b = 0.f;
+#pragma unroll
+          for (int j = 0; j < NB; ++j) {
+            const float d = fabsf(bden[j] - y);
+            if (d < near) { near = d; at = bden[j]; b = bnd[j]; }
+          }
+          // the neighbour of the scaled boundary on that side
+          const float step = fmaxf(fabsf(at) * 2.4e-7f, 1e-30f);
+          y = exact > b ? at + step : at - step;
+        }
+        tc::tmem_st1(col + e, y);
+      }
+    };
+    float band_p = 0.f;  // of the previous key tile's projections
     int n_xch = 0;    // exchanges through `exch` so far in this quarter (phase of xch / xfree)
     // sum of the four parts' values of this row, in a fixed order; every part gets the same total
     auto exchange = [&](float mine, float& total_out) -> bool {
@@ -393,6 +537,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       return true;
     };
     for (int i = 0; i <= n && ok; ++i) {
+      float band_next = 0.f;
       if (i < n) {
         const int s = i % kSlots, u = i / kSlots;
         bool is_key;
@@ -434,8 +579,29 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (!(ok = tc::mbar_wait_or_abort(y_done(s), u & 1, abort_flag))) break;
         tc::fence_after_sync();
         uint32_t raw[32];
-        tc::tmem_ld32(tmem + kColYP + s * kD + lane_base + 32 * part, raw);
+        const uint32_t col_y = tmem + kColYP + s * kD + lane_base + 32 * part;
+        tc::tmem_ld32(col_y, raw);
         tc::wait_ld();
+        if constexpr (F16) {
+          // any coordinate too close to a boundary to call?
+          const bool sure = !live || !(ss_tot > 0.f) || !(den < 1e30f);
+          const float band = sure ? 0.f : kOpenIndex * den;
+          auto settle_side = [&](auto nb, const float* Pi, const float (&bnd)[decltype(nb)::value]) {
+            float bden[decltype(nb)::value], near = INFINITY;
+#pragma unroll
+            for (int j = 0; j < decltype(nb)::value; ++j) bden[j] = bnd[j] * den;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) near = fminf(near, distance(nb, bden, __uint_as_float(raw[e])));
+            if (!__any_sync(0xffffffffu, near < band)) return;
+            settle(nb, Pi, bnd, bden, raw, col_y, band, row_address(is_key, b0, h0, s0));
+            tc::tmem_ld32(col_y, raw);
+            tc::wait_ld();
+          };
+          if (is_key)
+            settle_side(std::integral_constant<int, (1 << KB) - 1>{}, reinterpret_cast<const float*>(a.consts + a.L.pi_k), bnd_k);
+          else
+            settle_side(std::integral_constant<int, (1 << VB) - 1>{}, reinterpret_cast<const float*>(a.consts + a.L.pi_v), bnd_v);
+        }
         if (is_key) {
           // y = y_raw / den is compared with the boundaries as y_raw > b * den (den > 0)
           float bden[(1 << KB) - 1];
@@ -486,6 +652,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           float rr_tot;
           if (!(ok = exchange(rr, rr_tot))) break;
           if (live && part == 0) a.key_rn[no] = fp16_bits(sqrtf(rr_tot) * (1.f / kYScale));
+          const float next_band = F16 && live && den < 1e30f ? kOpenSign * sqrtf(rr_tot) * r_scale : 0.f;
           // the residual operand of the previous key tile must have been consumed by its sketch MMAs
           if (i >= 1 && !(ok = tc::mbar_wait_or_abort(p_done((i - 1) % kSlots), ((i - 1) / kSlots) & 1, abort_flag))) break;
           tc::tmem_st16(tmem + kColRH + lane_base + 16 * part, rh);
@@ -494,6 +661,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(r_full);
+          band_next = next_band;
         } else {
           tc::fence_before_sync();
           __syncwarp();
@@ -529,8 +697,37 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (!(ok = tc::mbar_wait_or_abort(p_done(s1), ((i - 1) / kSlots) & 1, abort_flag))) break;
         tc::fence_after_sync();
         uint32_t raw[32];
-        tc::tmem_ld32(tmem + kColYP + s1 * kD + lane_base + 32 * part, raw);
+        const uint32_t col_p = tmem + kColYP + s1 * kD + lane_base + 32 * part;
+        tc::tmem_ld32(col_p, raw);
         tc::wait_ld();
+        if constexpr (F16) {
+          float near = INFINITY;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) near = fminf(near, fabsf(__uint_as_float(raw[e])));
+          if (__any_sync(0xffffffffu, near < band_p)) {
+            const unsigned long long addr = row_address(true, b0, h0, s0);
+            uint32_t open = 0, lanes;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) open |= fabsf(__uint_as_float(raw[e])) < band_p ? 1u << e : 0u;
+            while ((lanes = __ballot_sync(0xffffffffu, open != 0u)) != 0u) {
+              const int l = __ffs((int)lanes) - 1;
+              const int e = __ffs((int)__shfl_sync(0xffffffffu, open, l)) - 1;
+              const float exact = exact_projection<D, (1 << KB) - 1>(
+                  reinterpret_cast<const __half*>(__shfl_sync(0xffffffffu, addr, l)),
+                  reinterpret_cast<const float*>(a.consts + a.L.pi_k), reinterpret_cast<const float*>(a.consts + a.L.s_eff),
+                  reinterpret_cast<const float*>(a.consts + a.L.bnd_k), reinterpret_cast<const float*>(a.consts + a.L.cen_k),
+                  32 * part + e);
+              float p = tc::tmem_ld1(col_p + e);
+              if (lane == l) {
+                open &= open - 1u;
+                p = exact >= 0.f ? 1.f : -1.f;
+              }
+              tc::tmem_st1(col_p + e, p);
+            }
+            tc::tmem_ld32(col_p, raw);
+            tc::wait_ld();
+          }
+        }
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(yp_free(s1));
@@ -545,6 +742,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (live_row(b0, h0, s0))
           *reinterpret_cast<uint32_t*>(a.key_sgn + out_row(b0, h0, s0) * (kD / 8) + 4 * part) = ~neg;
       }
+      band_p = band_next;
     }
   }
   if (!ok && atomicExch(s_abort_p, 2) != 2) {  // one fault per CTA
@@ -634,7 +832,8 @@ int compress_kv(const void* k, const void* v, int dtype, int d, int64_t B, int64
   TQ_REQUIRE(tiles_s * tiles_h < ((int64_t)1 << 31) && 2 * units < ((int64_t)1 << 31), "problem too large");
   const KvArgs a{(uint32_t)(k != nullptr ? units : 0), (uint32_t)(v != nullptr ? units : 0), (uint32_t)tiles_s,
                  (uint32_t)tiles_h, (uint32_t)bs, (uint32_t)bh, (uint32_t)bb, (uint32_t)S, (uint32_t)H, (uint32_t)B, consts,
-                 key_idx, key_sgn, key_vn, key_rn, val_idx, val_vn, out_stride, out_offset, const_layout(d)};
+                 key_idx, key_sgn, key_vn, key_rn, val_idx, val_vn, k, v, {k_strides[0], k_strides[1], k_strides[2]},
+                 {v_strides[0], v_strides[1], v_strides[2]}, out_stride, out_offset, const_layout(d)};
   CUtensorMap map_k, map_v;
   if (int st = make_map(&map_k, k != nullptr ? k : v, f16, d, a, k != nullptr ? k_strides : v_strides)) return st;
   if (int st = make_map(&map_v, v != nullptr ? v : k, f16, d, a, v != nullptr ? v_strides : k_strides)) return st;

@@ -179,6 +179,17 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// One column of 32 lanes.
+__device__ __forceinline__ float tmem_ld1(uint32_t addr) {
+  uint32_t v;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;" : "=r"(v) : "r"(addr) : "memory");
+  return __uint_as_float(v);
+}
+__device__ __forceinline__ void tmem_st1(uint32_t addr, float v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};\n\ttcgen05.wait::st.sync.aligned;" ::"r"(addr),
+               "r"(__float_as_uint(v))
+               : "memory");
+}
 // 32 lanes x 32 consecutive fp32 columns: thread t of the warp gets lane (base lane + t).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
