@@ -271,7 +271,7 @@ int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq
  * rebuilt per call, and the scratch need drops to tq_attention_prepared_workspace_bytes -- zero for prefill-sized
  * calls in TQ_MODE_BF16 (`workspace` may then be NULL).  kv_capacity = Sk is the contiguous
  * layout; a larger capacity is the persistent-cache layout of tq_attention_fwd_cached, served in place for every
- * head_dim and number of queries in TQ_MODE_BF16 (TQ_MODE_FP32 takes the contiguous layout only).
+ * head_dim, number of queries and mode.
  * Replaces the attention core of the family adapters (families/llama.py:100-114, gpt2.py:90-110). */
 size_t tq_attention_prepared_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
                                              int64_t kv_capacity, int d, int mode);

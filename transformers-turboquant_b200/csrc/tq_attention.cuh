@@ -75,7 +75,7 @@ struct AttnArgs {
   int out_dtype;
   int64_t o_stride_b, o_stride_h, o_stride_s;
   // keys between the packed rows of consecutive (batch, KV head) pairs in every packed array: Sk for the
-  // contiguous [B, Hkv, Sk] layout, the capacity of a persistent cache otherwise (tensor-core mode only)
+  // contiguous [B, Hkv, Sk] layout, the capacity of a persistent cache otherwise
   int64_t kv_stride;
   MaskBits mb;  // summary of the mask; where it exists, `mask` is read in tiles of its third class only
 };
@@ -91,7 +91,7 @@ int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, in
 // fp32 mode: query preparation + CUDA-core flash kernel.  `workspace` holds q_cat fp32.
 int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
-                       cudaStream_t stream);
+                       cudaStream_t stream, bool prepared = false);
 
 // bf16 mode: tcgen05 query preparation, tcgen05 flash kernel, tcgen05 back-rotation.
 // `prepared` (optional): a constants buffer filled by prepare_constants for the same matrices; the operand images
@@ -113,6 +113,17 @@ bool decode_applies(const AttnArgs& a, int d);  // a.kv_stride != a.Sk: any key 
 size_t decode_workspace_bytes(int64_t BHq);
 int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int q_dtype, int64_t sb, int64_t sh,
                      int64_t ss, const float* Pi_k, const float* S_eff, void* q_cat, void* part_ws, cudaStream_t stream);
+
+// Merge of partial results [B * Hkv][nsplit][rows][d] (unnormalised, rotated; maxima in log2 units) and back-rotation into
+// a.out; row r of a KV head is query head kvh * G + r / Sq, position r % Sq.
+int finish_splits(const AttnArgs& a, int64_t B, int d, int rows, int nsplit, const float* part_o, const float* part_ml,
+                  cudaStream_t stream);
+
+// fp32 mode, at most 16 query rows per KV head (tq_attention_rows.cu): a.q_cat holds the fp32 query rows, `part_ws`
+// attention_rows_workspace bytes.
+bool attention_rows_applies(int64_t Hq, int64_t Sq, int64_t Hkv);
+size_t attention_rows_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
+int attention_rows(const AttnArgs& a, int64_t B, int d, int bits, void* part_ws, cudaStream_t stream);
 
 // Raw queries and the constant bf16 operands of the SM-pair kernel, which prepares its own query tile
 // (q [Pi ; coeff S]^T) and rotates its output back (o Pi_v) on the tensor pipe.

@@ -638,13 +638,13 @@ __device__ __forceinline__ void store_elem(void* base, int dtype, int64_t off, f
 }
 
 // One query row per CTA: merge the splits (O = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m)), rotate back
-// (out = O Pi_v) and store in the caller's dtype and strides; fp32 throughout.  512 threads = 128 output
+// (out = O Pi_v) and store in the caller's dtype and strides; fp32 throughout.  4 D threads = D output
 // columns x 4 parts of each sum, so that every thread has all its loads in flight at once.
-__global__ void __launch_bounds__(512) decode_finish_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+template <int D>
+__global__ void __launch_bounds__(4 * D) decode_finish_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             int nsplit, int64_t Hq, int64_t Hkv, int64_t Sq,
                                                             const float* __restrict__ Pi_v, void* __restrict__ out,
                                                             int out_dtype, int64_t osb, int64_t osh, int64_t oss) {
-  constexpr int D = 128;
   __shared__ float f_s[kMaxExtraUnits + 1];
   __shared__ float part[4][D];
   __shared__ float o_s[D];
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(512) decode_finish_kernel(const float* __restr
   const int G = (int)(Hq / Hkv);
   float pv[D / 4];  // this thread's part of column j of Pi_v: independent of the kernel before, loaded while it ends
 #pragma unroll
-  for (int c = 0; c < D / 4; ++c) pv[c] = __ldg(Pi_v + (32 * p + c) * D + j);
+  for (int c = 0; c < D / 4; ++c) pv[c] = __ldg(Pi_v + (D / 4 * p + c) * D + j);
   grid_dependency_wait();
   const int R = G * (int)Sq;
   const float* ml = part_ml + (unit * nsplit * R + r) * 2;  // split s: ml[s * R * 2], + 1
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(512) decode_finish_kernel(const float* __restr
   __syncthreads();
   float y = 0.f;
 #pragma unroll
-  for (int c = 0; c < D / 4; ++c) y = fmaf(o_s[32 * p + c], pv[c], y);
+  for (int c = 0; c < D / 4; ++c) y = fmaf(o_s[D / 4 * p + c], pv[c], y);
   part[p][j] = y;
   __syncthreads();
   if (tid < D) {
@@ -748,6 +748,16 @@ static cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+int finish_splits(const AttnArgs& a, int64_t B, int d, int rows, int nsplit, const float* part_o, const float* part_ml,
+                  cudaStream_t stream) {
+  TQ_REQUIRE(nsplit <= kMaxExtraUnits && B * a.Hkv <= 65535, "too many splits or KV heads");
+  ProfScope prof(kProfBackRotation, stream);
+  TQ_CUDA_OK(launch_dependent(d == 128 ? decode_finish_kernel<128> : decode_finish_kernel<64>,
+                              dim3((unsigned)rows, (unsigned)(B * a.Hkv)), dim3(4 * d), stream, part_o, part_ml, nsplit, a.Hq,
+                              a.Hkv, a.Sq, a.Pi_v, a.out, a.out_dtype, a.o_stride_b, a.o_stride_h, a.o_stride_s));
+  return TQ_OK;
+}
+
 int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int q_dtype, int64_t sb, int64_t sh,
                      int64_t ss, const float* Pi_k, const float* S_eff, void* q_cat, void* part_ws, cudaStream_t stream) {
   const int64_t units = B * a.Hkv;
@@ -807,11 +817,7 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
                      : (bits == 2 ? decode_kernel<2, 2, true> : bits == 3 ? decode_kernel<3, 2, true> : decode_kernel<4, 2, true>);
     TQ_CUDA_OK(launch_dependent(kern, grid, dim3(kWarps * 32), stream, da));
   }
-  ProfScope prof(kProfBackRotation, stream);
-  TQ_CUDA_OK(launch_dependent(decode_finish_kernel, dim3((unsigned)R, (unsigned)units), dim3(512), stream, part_o,
-                              part_ml, nsplit, a.Hq, a.Hkv, a.Sq, a.Pi_v, a.out, a.out_dtype, a.o_stride_b,
-                              a.o_stride_h, a.o_stride_s));
-  return TQ_OK;
+  return finish_splits(a, B, 128, R, nsplit, part_o, part_ml, stream);
 }
 
 }  // namespace tq

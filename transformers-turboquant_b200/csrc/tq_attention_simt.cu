@@ -15,6 +15,7 @@
 namespace tq {
 
 constexpr int kRows = 64;  // query rows and keys per tile
+inline size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 constexpr int kFewRows = 16;  // query rows per CTA of the few-rows preparation
 
 __device__ __forceinline__ void store8(void* base, int dtype, int64_t off, const float (&v)[8]) {
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
   if (tid < (1 << VB)) cen_v[tid] = a.cen_v[tid];
   const int64_t b = blockIdx.z, h = blockIdx.y;
   const int64_t bh = b * a.Hq + h;
-  const int64_t kv_base = (b * a.Hkv + h / (a.Hq / a.Hkv)) * a.Sk;
+  const int64_t kv_base = (b * a.Hkv + h / (a.Hq / a.Hkv)) * a.kv_stride;
   const int q0 = blockIdx.x * kRows;
   const int shift = (int)(a.Sk - a.Sq);  // query i sees keys <= i + shift when causal
   __syncthreads();
@@ -768,10 +769,16 @@ namespace tq {
 // Entry used by tq_attention_fwd (tq_api.cu) for TQ_MODE_FP32.
 int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, bool prepared) {
   float* q_cat = static_cast<float*>(workspace);
   if (int st = qprep_fp32(q, dtype, B, Hq, Sq, d, sb, sh, ss, Pi_k, S_eff, q_cat, stream)) return st;
   a.q_cat = q_cat;
+  // few query rows: split over the keys (a prepared call's workspace has room for the partial results; the packed rows are
+  // read as words)
+  const uintptr_t words = reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) |
+                          reinterpret_cast<uintptr_t>(a.val_idx);
+  if (prepared && attention_rows_applies(Hq, Sq, a.Hkv) && (words & 3u) == 0 && B * a.Hkv <= 65535 / 4)
+    return attention_rows(a, B, d, bits, reinterpret_cast<uint8_t*>(workspace) + round256((size_t)B * Hq * Sq * 2 * d * 4), stream);
   return attention_fp32(a, B, d, bits, stream);
 }
 
@@ -870,9 +877,8 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
       return st;
   }
   if (mode == TQ_MODE_FP32) {
-    TQ_REQUIRE(kv_stride == Sk, "a cache with capacity > Sk needs TQ_MODE_BF16");
     return attention_fwd_fp32(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
-                              workspace, s);
+                              workspace, s, prepared != nullptr);
   }
   return attention_fwd_bf16(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
                             workspace, s, prepared);
@@ -904,7 +910,9 @@ extern "C" int tq_prepare_constants(const float* Pi_k, const float* S_eff, const
 extern "C" size_t tq_attention_prepared_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
                                                         int64_t kv_capacity, int d, int mode) {
   if (B <= 0 || Hq <= 0 || Sq <= 0 || d <= 0 || Hkv <= 0) return 0;
-  if (mode == TQ_MODE_FP32) return ((size_t)B * Hq * Sq * 2 * d * 4 + 255) & ~(size_t)255;
+  if (mode == TQ_MODE_FP32)
+    return round256((size_t)B * Hq * Sq * 2 * d * 4) +
+           (attention_rows_applies(Hq, Sq, Hkv) && Sk > 0 ? attention_rows_workspace(B, Hq, Sq, Hkv, Sk, d) : 0);
   return workspace_bytes_bf16_prepared(B, Hq, Sq, Hkv, Sk, kv_capacity, d);
 }
 

@@ -14,8 +14,8 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from .compressors import (_attend, _require_cuda, TurboQuantCompressorMSE, TurboQuantCompressorV2, fused_attention,
-                          prepared_constants, resolve_mode)
+from .compressors import (_attend, _require_cuda, TurboQuantCompressorMSE, TurboQuantCompressorV2, prepared_constants,
+                          resolve_mode)
 
 
 class CompressedKVCache:
@@ -97,18 +97,13 @@ class CompressedKVCache:
         queries are the last Sq positions (append their keys first).  Returns [B, Hq, Sq, D] in q.dtype.
 
         `attention_mask` is an optional additive mask broadcastable to [B, 1, Sq, tokens in use] (padding).
-        Tensor-core mode reads the cache in place, whatever the number of queries; fp32 mode gathers the prefix
-        once and takes the fp32 kernels."""
+        The cache is read in place, whatever the number of queries and the arithmetic mode."""
         _require_cuda(q, "q")
         B, Hq, Sq, D = q.shape
         if (B, D) != (self.batch, self.head_dim) or Hq % self.kv_heads != 0:
             raise ValueError(f"queries {tuple(q.shape)} do not match the cache")
         if self.length == 0:
             raise ValueError("attention over an empty cache is undefined")
-        if resolve_mode(q.dtype, self.key_compressor.mode) != _lib.TQ_MODE_BF16:
-            ck, cv = self._contiguous_prefix()
-            return fused_attention(q, ck, cv, self.key_compressor, self.val_compressor, causal=causal,
-                                   attention_mask=attention_mask, sm_scale=sm_scale)
         kc, vc = self.key_compressor, self.val_compressor
         kc._check_device(q)
         vc._check_device(q)
@@ -118,4 +113,4 @@ class CompressedKVCache:
         packed = (self.key_indices, self.key_signs, self.key_norms, self.key_residual_norms, self.value_indices,
                   self.value_norms)
         return _attend(q, self.kv_heads, self.length, self.capacity, packed, kc, vc, sm_scale, causal, attention_mask,
-                       _lib.TQ_MODE_BF16)
+                       resolve_mode(q.dtype, kc.mode))
