@@ -52,3 +52,24 @@ def test_short_sequences_share_tiles(B, H, S, d, bits, dtype):
                      (cache.value_indices, cv["packed_indices"]), (cache.value_norms, cv["vec_norms"])):
         assert torch.equal(buf[:, :, 3:3 + S].reshape(-1), ref.reshape(-1))
         assert not buf[:, :, :3].any() and not buf[:, :, 3 + S:].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d,bits", [(128, 2), (128, 3), (128, 4), (64, 2), (64, 3), (64, 4)])
+@pytest.mark.parametrize("B,H,S", [(1, 1, 1), (1, 3, 1), (4, 7, 1), (2, 3, 99), (2, 12, 28), (3, 32, 32)])
+def test_few_vectors_give_the_tile_kernels_bytes(B, H, S, d, bits, dtype):
+    """fp32 mode: up to 3072 vectors go to the few-vectors kernel, the same vectors among more of them to the tile kernel."""
+    from turboquant_b200 import compress_kv
+
+    g = torch.Generator().manual_seed(B * H + S + bits)
+    k, v = (torch.randn(B, S, H, d, generator=g).cuda().to(dtype).transpose(1, 2) for _ in range(2))
+    k[0, 0, 0] = 0.0
+    k[..., 5] *= 8
+    more = torch.randn(3073 // (H * S) + 1, H, S, d, generator=g).cuda().to(dtype)
+    kc, vc = device_compressors(d, bits, mode="fp32")
+    few, many = compress_kv(k, v, kc, vc), compress_kv(torch.cat([k, more]), torch.cat([v, more]), kc, vc)
+    n = B * H * S
+    for a, b in zip(few, many):
+        for name, t in a.items():
+            if name != "shape":
+                assert torch.equal(t.reshape(n, -1), b[name].reshape(-1, t.numel() // n)[:n]), name

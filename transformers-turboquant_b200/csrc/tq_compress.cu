@@ -132,6 +132,134 @@ __global__ void __launch_bounds__(16 * (D / 8)) compress_simt_kernel(const Compr
   }
 }
 
+// Few vectors (a generation step in fp32 mode), keys and values in one launch: the tile kernel above needs its matrices in
+// shared memory before the first product (20 + 15 us for the 8 keys and values of a step).  Here a thread owns one
+// coordinate of R vectors and reads its matrix row from L2.  Every sum is taken in the order of the tile kernel, so the
+// bytes are the same.  Bound by the trip of 64 KB per matrix and CTA through L1.
+template <int D>
+__device__ __forceinline__ float butterfly_sum(const float* p) {  // as the shuffles of the tile kernel add up D / 8 parts
+  float v[D / 8];
+#pragma unroll
+  for (int g = 0; g < D / 8; ++g) v[g] = p[g];
+#pragma unroll
+  for (int off = D / 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int g = 0; g < off; ++g) v[g] += v[g + off];
+  return v[0];
+}
+template <int D, int R>
+__device__ __forceinline__ void rows_times_matrix(const float (*x)[D], const float* __restrict__ m, float (&acc)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] = 0.f;
+#pragma unroll 4
+  for (int i = 0; i < D; i += 4) {
+    const float4 w = __ldg(reinterpret_cast<const float4*>(m + i));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 v = *reinterpret_cast<const float4*>(&x[r][i]);
+      acc[r] = fmaf(v.w, w.w, fmaf(v.z, w.z, fmaf(v.y, w.y, fmaf(v.x, w.x, acc[r]))));
+    }
+  }
+}
+template <typename T, int D, int IB, bool IS_KEY, int R>
+__device__ __forceinline__ void compress_rows(const CompressArgs& a, int64_t n0) {
+  constexpr int NB = (1 << IB) - 1;
+  __shared__ __align__(16) float x[R][D];
+  __shared__ float parts[R][D / 8];
+  const int j = threadIdx.x;
+  const int64_t HS = a.H * a.S;
+  const int rows = (int)(a.n_vec - n0 < R ? a.n_vec - n0 : R);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t n = n0 + r, b = n / HS, rem = n % HS;
+    x[r][j] = r < rows ? to_float<T>(static_cast<const T*>(a.src)[b * a.stride_b + rem / a.S * a.stride_h + rem % a.S * a.stride_s + j])
+                       : 0.f;
+  }
+  auto sum_of_squares = [&](float (&total)[R]) {
+    __syncthreads();
+    for (int e = j; e < R * (D / 8); e += D) {
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float v = x[e / (D / 8)][8 * (e % (D / 8)) + c];
+        ss = fmaf(v, v, ss);
+      }
+      parts[e / (D / 8)][e % (D / 8)] = ss;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) total[r] = butterfly_sum<D>(parts[r]);
+  };
+  float norm[R], y[R];
+  sum_of_squares(norm);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    norm[r] = sqrtf(norm[r]);
+    const float den = norm[r] + 1e-8f;
+    x[r][j] = x[r][j] / den;
+  }
+  __syncthreads();
+  rows_times_matrix<D, R>(x, a.Pi + j * D, y);
+  float bnd[NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i) bnd[i] = __ldg(a.boundaries + i);
+  if constexpr (IS_KEY) __syncthreads();  // x is about to hold the residuals
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int idx = count_below<NB>(y[r], bnd);
+    uint32_t w = (uint32_t)idx << (j % 8 * IB);  // eight coordinates are IB whole bytes
+    w |= __shfl_xor_sync(0xffffffffu, w, 1);
+    w |= __shfl_xor_sync(0xffffffffu, w, 2);
+    w |= __shfl_xor_sync(0xffffffffu, w, 4);
+    const int64_t no = compress_out_row(a, n0 + r);
+    if (r < rows && j % 8 == 0) {
+      uint8_t* dst = a.packed_idx + no * (D * IB / 8) + j / 8 * IB;
+#pragma unroll
+      for (int i = 0; i < IB; ++i) dst[i] = (uint8_t)(w >> (8 * i));
+    }
+    if (r < rows && j == 0) a.vec_norms[no] = fp16_bits(norm[r]);
+    if constexpr (IS_KEY) x[r][j] = fmaf(norm[r] + 1e-8f, y[r], -norm[r] * __ldg(a.centroids + idx));
+  }
+  if constexpr (IS_KEY) {
+    float rr[R], p[R];
+    sum_of_squares(rr);
+    rows_times_matrix<D, R>(x, a.S_eff + j * D, p);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t bits = __ballot_sync(0xffffffffu, p[r] >= 0.f);
+      const int64_t no = compress_out_row(a, n0 + r);
+      if (r < rows && j % 32 == 0) {
+        uint8_t* dst = a.packed_signs + no * (D / 8) + j / 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = (uint8_t)(bits >> (8 * i));
+      }
+      if (r < rows && j == 0) a.residual_norms[no] = fp16_bits(sqrtf(rr[r]));
+    }
+  }
+}
+template <typename T, int D, int BITS, int R>
+__global__ void __launch_bounds__(D) compress_rows_kernel(const CompressArgs k, const CompressArgs v, int key_ctas) {
+  if ((int)blockIdx.x < key_ctas) compress_rows<T, D, BITS - 1, true, R>(k, (int64_t)blockIdx.x * R);
+  else compress_rows<T, D, BITS, false, R>(v, (int64_t)(blockIdx.x - key_ctas) * R);
+}
+
+// Up to this many vectors a side: 3072 take 43 us at head_dim 128 (8: 17 us) where the two
+// launches of the tile kernel take 49 us.
+constexpr int64_t kFewVectors = 3072;
+
+template <typename T, int D>
+static int launch_compress_rows(int bits, const CompressArgs& k, const CompressArgs& v, cudaStream_t stream) {
+  const int64_t n = k.n_vec > v.n_vec ? k.n_vec : v.n_vec;
+  const int R = n > 4 * sm_count() ? 8 : 4;  // one CTA per SM and side with four vectors each, then eight
+  const int kc = (int)((k.n_vec + R - 1) / R), vc = (int)((v.n_vec + R - 1) / R);
+  auto kern = R == 4 ? (bits == 2 ? compress_rows_kernel<T, D, 2, 4> : bits == 3 ? compress_rows_kernel<T, D, 3, 4> : compress_rows_kernel<T, D, 4, 4>)
+                     : (bits == 2 ? compress_rows_kernel<T, D, 2, 8> : bits == 3 ? compress_rows_kernel<T, D, 3, 8> : compress_rows_kernel<T, D, 4, 8>);
+  ProfScope prof(k.n_vec > 0 ? kProfCompressKeys : kProfCompressValues, stream);
+  kern<<<kc + vc, D, 0, stream>>>(k, v, kc);
+  TQ_CUDA_OK(cudaGetLastError());
+  return TQ_OK;
+}
+
 template <int D, bool IS_KEY>
 constexpr size_t compress_smem_bytes() {
   return sizeof(float) * (size_t)((IS_KEY ? 2 : 1) * D * D + kTileRows * (D + 4) + kTileRows);
@@ -272,6 +400,20 @@ int tq_compress_kv(const void* keys, const void* values, int dtype, int64_t B, i
   }
   const ConstLayout L = const_layout(d);
   auto f32 = [&](size_t off) { return reinterpret_cast<const float*>(c + off); };
+  const int64_t n = B * H * S;
+  if (n <= kFewVectors && !(mode == TQ_MODE_BF16 && dtype == TQ_BF16)) {  // (that combination has a kernel of its own)
+    CallScope scope(keys != nullptr ? keys : values, "keys/values", static_cast<cudaStream_t>(stream));
+    if (scope.status()) return scope.status();
+    const CompressArgs ka{keys, keys != nullptr ? n : 0, H, S, k_stride_b, k_stride_h, k_stride_s, f32(L.pi_k), f32(L.s_eff),
+                          f32(L.cen_k), f32(L.bnd_k), key_idx, key_signs, key_vec_norms, key_residual_norms, 0, kv_capacity,
+                          kv_offset};
+    const CompressArgs va{values, values != nullptr ? n : 0, H, S, v_stride_b, v_stride_h, v_stride_s, f32(L.pi_v), nullptr,
+                          nullptr, f32(L.bnd_v), val_idx, nullptr, val_vec_norms, nullptr, 0, kv_capacity, kv_offset};
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (dtype == TQ_F32) return d == 128 ? launch_compress_rows<float, 128>(bits, ka, va, s) : launch_compress_rows<float, 64>(bits, ka, va, s);
+    if (dtype == TQ_BF16) return d == 128 ? launch_compress_rows<__nv_bfloat16, 128>(bits, ka, va, s) : launch_compress_rows<__nv_bfloat16, 64>(bits, ka, va, s);
+    return d == 128 ? launch_compress_rows<__half, 128>(bits, ka, va, s) : launch_compress_rows<__half, 64>(bits, ka, va, s);
+  }
   if (keys != nullptr)
     if (int st = compress_keys_entry(keys, dtype, B, H, S, d, k_stride_b, k_stride_h, k_stride_s, f32(L.pi_k),
                                      f32(L.s_eff), f32(L.cen_k), f32(L.bnd_k), bits, key_idx, key_signs,
