@@ -182,6 +182,11 @@ int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, in
 }
 // ---- tile decode helpers -------------------------------------------------------------
 
+__device__ __forceinline__ void put8(float* dst, const float (&v)[8]) {  // 16-byte aligned
+  reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 // Decode keys [k0, k0+64) of one head into Ks[j][0:D] = C[idx], Ks[j][D:2D] = +-1, and
 // their norms into kn[j] (vector norm) and krn[j] (residual norm).  Keys past `Sk` decode
 // to zeros.
@@ -198,14 +203,18 @@ __device__ __forceinline__ void decode_key_tile(const uint8_t* __restrict__ idx,
       const int64_t n = head_base + k0 + j;
       const uint64_t w = load_fields8<IB>(idx + n * (D * IB / 8) + g * IB);
       const unsigned sb = sgn[n * G + g];
+      float v[8], sg[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        dst[c] = cen[(w >> (c * IB)) & ((1u << IB) - 1)];
-        dst[D + c] = ((sb >> c) & 1u) ? 1.f : -1.f;
+        v[c] = cen[(w >> (c * IB)) & ((1u << IB) - 1)];
+        sg[c] = ((sb >> c) & 1u) ? 1.f : -1.f;
       }
+      put8(dst, v);
+      put8(dst + D, sg);
     } else {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) { dst[c] = 0.f; dst[D + c] = 0.f; }
+      const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      put8(dst, zero);
+      put8(dst + D, zero);
     }
   }
   for (int j = tid; j < kRows; j += nthreads) {
@@ -382,10 +391,20 @@ __global__ void __launch_bounds__(256) scores_rows_kernel(const ScoreArgs a) {
 }
 
 // ---- fused attention -----------------------------------------------------------------
+//
+// One CTA per 64 query rows of a head walks the keys; where that leaves SMs idle, or a causal launch ends with its longest
+// rows alone, the keys are cut into chunks of `chunk` tiles with a CTA each, which leave unnormalised partial outputs for
+// merge_tiles_kernel (GPT-2, 12 heads x 1024 tokens: 206 us unsplit on 192 CTAs of up to 16 tiles, 115 us as 864 CTAs of two
+// tiles and the merge).
 
+struct SplitArgs {
+  int chunk, nsplit;  // key tiles per CTA, chunks of the whole key range; nsplit = 1: no partial results
+  float* part_o;      // [B*Hq][query tiles][nsplit][64][D]
+  float* part_ml;     // [B*Hq][query tiles][nsplit][64][2]: maximum, row sum
+};
 
 template <int D, int KB, int VB, bool MASK>
-__global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a, const SplitArgs x) {
   constexpr int KS = 2 * D + 4, VS = D + 4, PS = kRows + 4, G = D / 8;
   constexpr int NC = D / 16;  // output coordinates per thread in the P V product
   extern __shared__ __align__(16) float smem[];
@@ -403,8 +422,20 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
   const int64_t b = blockIdx.z, h = blockIdx.y;
   const int64_t bh = b * a.Hq + h;
   const int64_t kv_base = (b * a.Hkv + h / (a.Hq / a.Hkv)) * a.kv_stride;
-  const int q0 = blockIdx.x * kRows;
+  // longest rows first
+  const int qtiles = gridDim.x / x.nsplit, qtile = qtiles - 1 - blockIdx.x % qtiles, split = blockIdx.x / qtiles;
+  const int q0 = qtile * kRows;
   const int shift = (int)(a.Sk - a.Sq);  // query i sees keys <= i + shift when causal
+  int k_end = (int)a.Sk;
+  if (a.causal) {
+    const int last = min(q0 + kRows - 1, (int)a.Sq - 1) + shift;
+    k_end = min(k_end, last + 1);
+  }
+  const int k_begin = split * x.chunk * kRows;
+  if (x.nsplit > 1) {
+    if (k_begin >= k_end) return;  // no row of the tile sees this chunk; the merge knows
+    k_end = min(k_end, k_begin + x.chunk * kRows);
+  }
   __syncthreads();
   load_q_tile<D>(static_cast<const float*>(a.q_cat), bh * a.Sq, q0, (int)a.Sq, Qs, tid, 256);
 
@@ -416,12 +447,7 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) o[r][c] = 0.f;
   }
-  int k_end = (int)a.Sk;
-  if (a.causal) {
-    const int last = min(q0 + kRows - 1, (int)a.Sq - 1) + shift;
-    k_end = min(k_end, last + 1);
-  }
-  for (int k0 = 0; k0 < k_end; k0 += kRows) {
+  for (int k0 = k_begin; k0 < k_end; k0 += kRows) {
     __syncthreads();  // previous tile fully consumed
     decode_key_tile<D, KB>(a.key_idx, a.key_sgn, a.key_vn, a.key_rn, kv_base, k0, (int)a.Sk, cen_k, Ks, kn,
                            krn, tid, 256);
@@ -432,11 +458,13 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
         const int64_t n = kv_base + k0 + j;
         const uint64_t w = load_fields8<VB>(a.val_idx + n * (D * VB / 8) + g * VB);
         const float nv = fp16_value(a.val_vn[n]);
+        float v[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dst[c] = nv * cen_v[(w >> (c * VB)) & ((1u << VB) - 1)];
+        for (int c = 0; c < 8; ++c) v[c] = nv * cen_v[(w >> (c * VB)) & ((1u << VB) - 1)];
+        put8(dst, v);
       } else {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) dst[c] = 0.f;
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        put8(dst, zero);
       }
     }
     __syncthreads();
@@ -510,6 +538,17 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
       }
     }
   }
+  if (x.nsplit > 1) {
+    const int64_t unit = ((int64_t)bh * qtiles + qtile) * x.nsplit + split;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float* dst = x.part_o + (unit * kRows + row0 + r) * D + tx * 4;
+      *reinterpret_cast<float4*>(dst) = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+      if constexpr (NC == 8) *reinterpret_cast<float4*>(dst + D / 2) = make_float4(o[r][4], o[r][5], o[r][6], o[r][7]);
+      if (tx == 0) *reinterpret_cast<float2*>(x.part_ml + (unit * kRows + row0 + r) * 2) = make_float2(m_run[r], l_run[r]);
+    }
+    return;
+  }
   // ---- epilogue: normalise, rotate back by Pi_v, store ----------------------------------
   __syncthreads();
   float* Os = Ks;  // [64][VS]
@@ -534,6 +573,61 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a) {
       if (i < a.Sq)
         store8(a.out, a.out_dtype, b * a.o_stride_b + h * a.o_stride_h + (int64_t)i * a.o_stride_s + tx * 8, y[r]);
     }
+  }
+}
+
+// Merge of the chunks of 64 query rows and back-rotation by Pi_v.  16 x D / 8 threads; a thread owns 4 rows x 8 columns.
+template <int D>
+__global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArgs a, const SplitArgs x) {
+  constexpr int TX = D / 8, NT = 16 * TX, XS = D + 4;
+  extern __shared__ __align__(16) float smem[];
+  float* M = smem;
+  float* X = M + D * D;
+  const int tid = threadIdx.x, tx = tid % TX, row0 = tid / TX * 4;
+  const int64_t b = blockIdx.z, h = blockIdx.y, bh = b * a.Hq + h;
+  const int q0 = blockIdx.x * kRows;
+  load_matrix<D, false>(a.Pi_v, M, tid, NT);
+  int k_end = (int)a.Sk;
+  if (a.causal) k_end = min(k_end, min(q0 + kRows - 1, (int)a.Sq - 1) + (int)(a.Sk - a.Sq) + 1);
+  const int n = (k_end + x.chunk * kRows - 1) / (x.chunk * kRows);
+  const int64_t unit = (bh * gridDim.x + blockIdx.x) * x.nsplit;
+  float m[4], l[4], acc[4][8];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+  }
+  for (int s = 0; s < n; ++s)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float2 ml = __ldg(reinterpret_cast<const float2*>(x.part_ml + ((unit + s) * kRows + row0 + r) * 2));
+      const float4* p = reinterpret_cast<const float4*>(x.part_o + ((unit + s) * kRows + row0 + r) * D + tx * 8);
+      const float4 u = __ldg(p), v = __ldg(p + 1);
+      const float m_new = fmaxf(m[r], ml.x), m_use = m_new == -INFINITY ? 0.f : m_new;
+      const float f = m[r] == -INFINITY ? 0.f : __expf(m[r] - m_use), g = ml.x == -INFINITY ? 0.f : __expf(ml.x - m_use);
+      m[r] = m_new;
+      l[r] = l[r] * f + ml.y * g;
+      const float w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(w[c], g, acc[r][c] * f);
+    }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] *= inv;
+    put8(X + (row0 + r) * XS + tx * 8, acc[r]);
+  }
+  __syncthreads();
+  float y[4][8];
+  tile_gemm<D, XS>(X, M, row0, tx, y);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = q0 + row0 + r;
+    if (i < a.Sq)
+      store8(a.out, a.out_dtype, b * a.o_stride_b + h * a.o_stride_h + (int64_t)i * a.o_stride_s + tx * 8, y[r]);
   }
 }
 
@@ -641,29 +735,68 @@ int scores_fp32(const ScoreArgs& a, int64_t B, int d, int bits, cudaStream_t str
   return launch_scores<64, 3>(a, B, stream);
 }
 
+// How the tile kernel's keys are cut (the workspace is sized for causal and full calls alike).
+static SplitArgs split_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Sk, int d) {
+  const int64_t qtiles = (Sq + kRows - 1) / kRows, ktiles = (Sk + kRows - 1) / kRows, shift = Sk > Sq ? Sk - Sq : 0;
+  int64_t work = 0;  // key tiles of all query tiles of a head, causal
+  if (qtiles > 4096) work = qtiles * (shift / kRows) + qtiles * (qtiles + 1) / 2;
+  else
+    for (int64_t i = 0; i < qtiles; ++i) {
+      const int64_t end = (i + 1) * kRows + shift;
+      work += ((end < Sk ? end : Sk) + kRows - 1) / kRows;
+    }
+  // about three waves of CTAs (two per SM at head_dim 64), of at least two tiles: a chunk loads its query tile and writes
+  // its partial results
+  const int64_t slots = (int64_t)sm_count() * (d == 64 ? 2 : 1);
+  int64_t chunk = (work * B * Hq + 3 * slots - 1) / (3 * slots);
+  if (chunk < 2) chunk = 2;
+  if (chunk > ktiles) chunk = ktiles;
+  SplitArgs x{};
+  x.chunk = (int)chunk;
+  x.nsplit = (int)((ktiles + chunk - 1) / chunk);
+  return x;
+}
+static size_t split_bytes(const SplitArgs& x, int64_t B, int64_t Hq, int64_t Sq, int d) {
+  if (x.nsplit <= 1) return 0;
+  return round256((size_t)B * Hq * ((Sq + kRows - 1) / kRows) * x.nsplit * kRows * (d + 2) * sizeof(float));
+}
+
+template <int D>
+static int launch_merge(const AttnArgs& a, const SplitArgs& x, int64_t B, cudaStream_t stream) {
+  constexpr size_t smem = sizeof(float) * (D * D + kRows * (D + 4));
+  auto kern = merge_tiles_kernel<D>;
+  TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ProfScope prof(kProfBackRotation, stream);
+  kern<<<dim3((unsigned)((a.Sq + kRows - 1) / kRows), (unsigned)a.Hq, (unsigned)B), 16 * (D / 8), smem, stream>>>(a, x);
+  TQ_CUDA_OK(cudaGetLastError());
+  return TQ_OK;
+}
+
 template <int D, int BITS>
-static int launch_attention(const AttnArgs& a, int64_t B, cudaStream_t stream) {
+static int launch_attention(const AttnArgs& a, const SplitArgs& x, int64_t B, cudaStream_t stream) {
   constexpr size_t smem =
       sizeof(float) * (2 * kRows * (2 * D + 4) + kRows * (D + 4) + kRows * (kRows + 4) + 2 * kRows);
   auto kern = a.mask != nullptr || a.mb.words != nullptr ? attention_simt_kernel<D, BITS - 1, BITS, true>
                                                          : attention_simt_kernel<D, BITS - 1, BITS, false>;
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)((a.Sq + kRows - 1) / kRows), (unsigned)a.Hq, (unsigned)B);
-  ProfScope prof(kProfAttention, stream);
-  kern<<<grid, 256, smem, stream>>>(a);
-  TQ_CUDA_OK(cudaGetLastError());
-  return TQ_OK;
+  dim3 grid((unsigned)((a.Sq + kRows - 1) / kRows * x.nsplit), (unsigned)a.Hq, (unsigned)B);
+  {
+    ProfScope prof(kProfAttention, stream);
+    kern<<<grid, 256, smem, stream>>>(a, x);
+    TQ_CUDA_OK(cudaGetLastError());
+  }
+  return x.nsplit > 1 ? launch_merge<D>(a, x, B, stream) : TQ_OK;
 }
 
-int attention_fp32(const AttnArgs& a, int64_t B, int d, int bits, cudaStream_t stream) {
+int attention_fp32(const AttnArgs& a, const SplitArgs& x, int64_t B, int d, int bits, cudaStream_t stream) {
   if (d == 128) {
-    if (bits == 2) return launch_attention<128, 2>(a, B, stream);
-    if (bits == 3) return launch_attention<128, 3>(a, B, stream);
-    return launch_attention<128, 4>(a, B, stream);
+    if (bits == 2) return launch_attention<128, 2>(a, x, B, stream);
+    if (bits == 3) return launch_attention<128, 3>(a, x, B, stream);
+    return launch_attention<128, 4>(a, x, B, stream);
   }
-  if (bits == 2) return launch_attention<64, 2>(a, B, stream);
-  if (bits == 3) return launch_attention<64, 3>(a, B, stream);
-  return launch_attention<64, 4>(a, B, stream);
+  if (bits == 2) return launch_attention<64, 2>(a, x, B, stream);
+  if (bits == 3) return launch_attention<64, 3>(a, x, B, stream);
+  return launch_attention<64, 4>(a, x, B, stream);
 }
 
 template <int D, int VB>
@@ -773,13 +906,21 @@ int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
   float* q_cat = static_cast<float*>(workspace);
   if (int st = qprep_fp32(q, dtype, B, Hq, Sq, d, sb, sh, ss, Pi_k, S_eff, q_cat, stream)) return st;
   a.q_cat = q_cat;
-  // few query rows: split over the keys (a prepared call's workspace has room for the partial results; the packed rows are
-  // read as words)
-  const uintptr_t words = reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) |
-                          reinterpret_cast<uintptr_t>(a.val_idx);
-  if (prepared && attention_rows_applies(Hq, Sq, a.Hkv) && (words & 3u) == 0 && B * a.Hkv <= 65535 / 4)
-    return attention_rows(a, B, d, bits, reinterpret_cast<uint8_t*>(workspace) + round256((size_t)B * Hq * Sq * 2 * d * 4), stream);
-  return attention_fp32(a, B, d, bits, stream);
+  SplitArgs x{};
+  x.chunk = 1;
+  x.nsplit = 1;
+  if (prepared) {  // the workspace of a prepared call has room for partial results
+    uint8_t* const part = reinterpret_cast<uint8_t*>(workspace) + round256((size_t)B * Hq * Sq * 2 * d * 4);
+    // few query rows have a kernel of their own, which reads the packed rows as words
+    const uintptr_t words = reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) |
+                            reinterpret_cast<uintptr_t>(a.val_idx);
+    if (attention_rows_applies(Hq, Sq, a.Hkv) && (words & 3u) == 0 && B <= 65535 && B * a.Hkv <= 65535 / 4)
+      return attention_rows(a, B, d, bits, part, stream);
+    x = split_plan(B, Hq, Sq, a.Sk, d);
+    x.part_o = reinterpret_cast<float*>(part);
+    x.part_ml = x.part_o + (size_t)B * Hq * ((Sq + kRows - 1) / kRows) * x.nsplit * kRows * d;
+  }
+  return attention_fp32(a, x, B, d, bits, stream);
 }
 
 int check_attention_args(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
@@ -910,9 +1051,13 @@ extern "C" int tq_prepare_constants(const float* Pi_k, const float* S_eff, const
 extern "C" size_t tq_attention_prepared_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
                                                         int64_t kv_capacity, int d, int mode) {
   if (B <= 0 || Hq <= 0 || Sq <= 0 || d <= 0 || Hkv <= 0) return 0;
-  if (mode == TQ_MODE_FP32)
-    return round256((size_t)B * Hq * Sq * 2 * d * 4) +
-           (attention_rows_applies(Hq, Sq, Hkv) && Sk > 0 ? attention_rows_workspace(B, Hq, Sq, Hkv, Sk, d) : 0);
+  if (mode == TQ_MODE_FP32) {
+    const size_t q_cat = round256((size_t)B * Hq * Sq * 2 * d * 4);
+    if (Sk <= 0) return q_cat;
+    const size_t tiles = split_bytes(split_plan(B, Hq, Sq, Sk, d), B, Hq, Sq, d);
+    const size_t rows = attention_rows_applies(Hq, Sq, Hkv) ? attention_rows_workspace(B, Hq, Sq, Hkv, Sk, d) : 0;
+    return q_cat + (rows > tiles ? rows : tiles);
+  }
   return workspace_bytes_bf16_prepared(B, Hq, Sq, Hkv, Sk, kv_capacity, d);
 }
 

@@ -18,10 +18,21 @@ __device__ __forceinline__ int perm_col(int j) {
 // tile_gemm.  TRANSPOSE: MT[i][perm(j)] = M[j][i] (for x @ M^T); else MT[i][perm(j)] = M[i][j].
 template <int D, bool TRANSPOSE>
 __device__ void load_matrix(const float* __restrict__ M, float* __restrict__ MT, int tid, int nthreads) {
-  for (int e = tid; e < D * D; e += nthreads) {
-    const int a = e / D, b = e % D;
-    if (TRANSPOSE) MT[b * D + perm_col<D>(a)] = __ldg(M + e);
-    else MT[a * D + perm_col<D>(b)] = __ldg(M + e);
+  if constexpr (TRANSPOSE) {
+    // Lanes take consecutive rows and 32 bytes of each: a whole sector read, and stores to 32 columns of one row of MT
+    // (two to a bank).  Lanes along a row instead store 32 deep into one bank: 8 us of a 24 us launch at head_dim 128.
+    for (int e = tid; e < D * (D / 8); e += nthreads) {
+      const int a = e % D, b = e / D * 8, col = perm_col<D>(a);
+      const float4 u = __ldg(reinterpret_cast<const float4*>(M + a * D + b)), v = __ldg(reinterpret_cast<const float4*>(M + a * D + b) + 1);
+      const float w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) MT[(b + i) * D + col] = w[i];
+    }
+  } else {
+    for (int e = tid; e < D * (D / 4); e += nthreads) {
+      const int a = e / (D / 4), b = e % (D / 4) * 4;  // the permutation keeps groups of four columns together
+      *reinterpret_cast<float4*>(MT + a * D + perm_col<D>(b)) = __ldg(reinterpret_cast<const float4*>(M + a * D + b));
+    }
   }
 }
 
