@@ -134,7 +134,15 @@ struct PairArgs {
   const __nv_bfloat16* w_cat;    // [2d, d] = [Pi ; coeff S]
   const __nv_bfloat16* w_unrot;  // [d, d]  = Pi_v^T
   const uint32_t* luts;          // pair tables: 4^(bits-1) key entries, then 4^bits value entries (bf16x2 words)
+  int nsplit;                    // clusters that share the keys of a pair of query tiles; 1: no partial results
+  float* part_o;                 // [B*Hq][ceil(Sq / 128)][nsplit][128][d], unnormalised, rotated
+  float* part_ml;                // [B*Hq][ceil(Sq / 128)][nsplit][128][2]: running maximum (log2 units), row sum
 };
+// Clusters per pair of query tiles that the SM-pair kernel is split over, and the partial results' bytes (0 unsplit).
+int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
+size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit);
+// Merge of tiles of 128 query rows and back-rotation by Pi_v (fp32) into a.out.
+int merge_split_tiles(const AttnArgs& a, int64_t B, int d, int nsplit, float* part_o, float* part_ml, cudaStream_t stream);
 
 // SM-pair (2-CTA cluster) tensor-core kernel, head_dim 128; needs no per-query scratch.
 int attention_c2(const AttnArgs& a, const PairArgs& x, int64_t B, int d, int bits, cudaStream_t stream);

@@ -165,8 +165,9 @@ struct C2Smem {
   static_assert(2 * D <= 2 * kBN, "the Q_cat accumulator borrows both score tiles");
 };
 
+// SPLIT: the key tiles of a pair of query tiles are shared by x.nsplit clusters, which leave partial results.
 // MASK: the call has an additive mask or a mask summary (a kernel of its own: the mask handling costs the plain one 1.5 %)
-template <int D, int BITS, bool MASK, bool TRACE>
+template <int D, int BITS, bool MASK, bool SPLIT, bool TRACE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   using L = C2Smem<D, BITS>;
@@ -196,7 +197,9 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   // P V_hat issuer warp and published with the set-up barrier below; nothing before that depends on it.
   // ---- which query tile ------------------------------------------------------------------
   const int64_t b = blockIdx.z;
-  const int xpair = (int)((gridDim.x >> 1) - 1 - (blockIdx.x >> 1));  // heaviest (latest) position blocks first
+  const int xid = SPLIT ? (int)(blockIdx.x >> 1) / x.nsplit : (int)(blockIdx.x >> 1);
+  const int split = SPLIT ? (int)(blockIdx.x >> 1) % x.nsplit : 0;
+  const int xpair = (SPLIT ? (int)(gridDim.x >> 1) / x.nsplit : (int)(gridDim.x >> 1)) - 1 - xid;  // heaviest (latest) position blocks first
   int64_t head;
   int q0, q0_last;
   if (pair_heads) {
@@ -285,8 +288,10 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       if (!poisoned) {
         tc::mbar_arrive_expect_tx(w_full, L::kWBytes);
         tc::bulk_load(tc::smem_u32(smem_raw + L::kWOff), x.w_cat + (int64_t)rank * D * D, L::kWBytes, w_full);
-        tc::mbar_arrive_expect_tx(u_full, L::kUBytes);
-        tc::bulk_load(tc::smem_u32(smem_raw + L::kUOff), x.w_unrot + (int64_t)rank * (D / 2) * D, L::kUBytes, u_full);
+        if (!SPLIT) {
+          tc::mbar_arrive_expect_tx(u_full, L::kUBytes);
+          tc::bulk_load(tc::smem_u32(smem_raw + L::kUOff), x.w_unrot + (int64_t)rank * (D / 2) * D, L::kUBytes, u_full);
+        }
         // the decode tables too: nobody waits for them here, the producers do before their first tile
         tc::mbar_arrive_expect_tx(lut_full, (uint32_t)(sizeof(lutK) + sizeof(lutV)));
         tc::bulk_load(tc::smem_u32(lutK), x.luts, (uint32_t)sizeof(lutK), lut_full);
@@ -339,7 +344,25 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     for (int w = 0; w * 32 < n_tiles_live; ++w) n_tiles += __popc(map_live[w]);
   }
   // the key tile computed after tile `t` (-1: the first one)
+  int tile_skip = 0;  // live tiles of the clusters before this one
+  if (SPLIT) {
+    const int lo = (int)((int64_t)n_tiles * split / x.nsplit), hi = (int)((int64_t)n_tiles * (split + 1) / x.nsplit);
+    tile_skip = lo;
+    n_tiles = hi - lo;  // both CTAs of the pair alike
+  }
   auto next_tile = [&](int t) -> int {
+    if (SPLIT && t < 0) {
+      if (!mapped) return tile_skip;
+      int left = tile_skip;
+      for (int w = 0; w * 32 < n_tiles_live; ++w) {
+        uint32_t bits = map_live[w];
+        const int n = __popc(bits);
+        if (left >= n) { left -= n; continue; }
+        for (; left > 0; --left) bits &= bits - 1u;
+        return w * 32 + __ffs((int)bits) - 1;
+      }
+      return n_tiles_live;
+    }
     ++t;
     if (mapped) {
       for (; t < n_tiles_live; t = (t | 31) + 1) {
@@ -556,7 +579,29 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       tc::mbar_arrive(xch(quad));
       ok = tc::mbar_wait_or_abort(xch(quad), n_tiles & 1, abort_flag);
     }
-    if (ok && n_tiles > 0) {
+    if (SPLIT && ok) {
+      // partial results: this thread's half of its output row as it is, the row's maximum and sum (none: no tiles here)
+      if (n_tiles > 0) tc::fence_after_sync();
+      const int64_t qblocks = (a.Sq + kBM - 1) / kBM;
+      const int64_t prow = (((b * a.Hq + head) * qblocks + q0 / kBM) * x.nsplit + split) * kBM + row;
+      if (qi < a.Sq && chalf == 0)
+        *reinterpret_cast<float2*>(x.part_ml + prow * 2) =
+            n_tiles > 0 ? make_float2(m_run, l_run + xmax[n_tiles & 1][1][row]) : make_float2(-INFINITY, 0.f);
+      if (n_tiles > 0) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < D / NQ; c0 += 32) {
+          uint32_t raw[32];
+          tc::tmem_ld32(tmem_o + lane_base + chalf * (D / NQ) + c0, raw);
+          tc::wait_ld();
+          if (qi < a.Sq) {
+            uint4* dst = reinterpret_cast<uint4*>(x.part_o + prow * D + chalf * (D / NQ) + c0);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dst[i] = make_uint4(raw[4 * i], raw[4 * i + 1], raw[4 * i + 2], raw[4 * i + 3]);
+          }
+        }
+      }
+    }
+    if (!SPLIT && ok && n_tiles > 0) {
       tc::fence_after_sync();
       float l_tot = l_run;
 #pragma unroll
@@ -581,7 +626,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       ok = tc::mbar_wait_or_abort(e_done, 0, abort_flag);
       tr.mark(16, 999);
     }
-    if (ok && n_tiles > 0) {
+    if (!SPLIT && ok && n_tiles > 0) {
       // accumulator row -> output dtype -> shared memory (padded rows), so that whole rows leave coalesced
       tc::fence_after_sync();
       const int esz = a.out_dtype == TQ_F32 ? 4 : 2;
@@ -599,7 +644,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       ok = tc::mbar_wait_or_abort(xch(quad), (n_tiles + 1) & 1, abort_flag);
       tr.mark(24, 999);
     }
-    if (ok && n_tiles > 0) {
+    if (!SPLIT && ok && n_tiles > 0) {
       // the two warps of the quadrant store 16 of its 32 rows each
       const int esz = a.out_dtype == TQ_F32 ? 4 : 2;
       static_assert(D == 128 || D == 64, "chunks per row are derived for head_dim 64 and 128");
@@ -875,7 +920,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     if (n_tiles > 0 && (ok = tc::mbar_wait_or_abort(w_full, 0, abort_flag))) arrive_leader(qp_full);
   } else if (warp == kPvWarp && rank != 0 && lane == 0) {
     // peer CTA: ... and this half of Pi_v^T
-    if (n_tiles > 0 && (ok = tc::mbar_wait_or_abort(u_full, 0, abort_flag))) arrive_leader(u_peer);
+    if (!SPLIT && n_tiles > 0 && (ok = tc::mbar_wait_or_abort(u_full, 0, abort_flag))) arrive_leader(u_peer);
   } else if (warp == kPvWarp && rank == 0 && lane == 0) {
     // =============================== P V_hat MMA issuer (leader CTA) ===============================
     constexpr uint32_t idesc_o = tc::idesc_f16(2 * kBM, D, false, true);
@@ -897,8 +942,9 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
       tc::mma_commit2(v_empty(st), 3);
       tr.mark(6, j);
     }
-    if (ok && n_tiles > 0) ok = tc::mbar_wait_or_abort(u_full, 0, abort_flag) && tc::mbar_wait_or_abort(u_peer, 0, abort_flag);
-    if (ok && n_tiles > 0 && (ok = tc::mbar_wait_or_abort(q_full, 1, abort_flag))) {
+    if (!SPLIT && ok && n_tiles > 0)
+      ok = tc::mbar_wait_or_abort(u_full, 0, abort_flag) && tc::mbar_wait_or_abort(u_peer, 0, abort_flag);
+    if (!SPLIT && ok && n_tiles > 0 && (ok = tc::mbar_wait_or_abort(q_full, 1, abort_flag))) {
       // out tile (fp32, second score tile) = normalised bf16 output tile x Pi_v
       tc::fence_after_sync();
       const uint64_t bdesc = tc::smem_desc(tc::smem_u32(smem_raw + L::kUOff), 128, L::kSboW);
@@ -908,6 +954,10 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
                          idesc_e, ks > 0);
       tc::mma_commit2(e_done, 3);
     }
+  }
+  if (SPLIT && !dead && n_tiles == 0 && warp == kPvWarp && lane == 0) {
+    // nothing to do here, but the copies started above must land before the CTA's shared memory goes away
+    ok = tc::mbar_wait_or_abort(w_full, 0, abort_flag) && tc::mbar_wait_or_abort(lut_full, 0, abort_flag);
   }
   if (!ok && atomicExch(&s_abort, 2) != 2) {  // one fault per CTA
     atomicAdd(&g_c2_faults, 1ull);
@@ -919,40 +969,73 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
   if (warp == kCtlWarp) tc::tmem_dealloc2(tmem_base, L::kCols);
 }
 
-template <int D, int BITS>
+template <int D, int BITS, bool MASK, bool SPLIT>
 int launch_c2(const AttnArgs& a, const PairArgs& x, int64_t B, cudaStream_t stream) {
   constexpr size_t smem = C2Smem<D, BITS>::kTotal > 120 * 1024 ? C2Smem<D, BITS>::kTotal : 120 * 1024;
-#ifdef TQ_B200_TRACE  // diagnostics build only: the product library carries one instantiation per (d, bits)
-  const bool masked = a.mask != nullptr || a.mb.words != nullptr;
-  auto kern = masked ? (g_trace2_host_on ? attention_c2_kernel<D, BITS, true, true> : attention_c2_kernel<D, BITS, true, false>)
-                     : (g_trace2_host_on ? attention_c2_kernel<D, BITS, false, true> : attention_c2_kernel<D, BITS, false, false>);
+#ifdef TQ_B200_TRACE  // diagnostics build only: the product library carries no tracing instantiations
+  auto kern = g_trace2_host_on ? attention_c2_kernel<D, BITS, MASK, SPLIT, true> : attention_c2_kernel<D, BITS, MASK, SPLIT, false>;
 #else
-  auto kern = a.mask != nullptr || a.mb.words != nullptr ? attention_c2_kernel<D, BITS, true, false>
-                                                         : attention_c2_kernel<D, BITS, false, false>;
+  auto kern = attention_c2_kernel<D, BITS, MASK, SPLIT, false>;
 #endif
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pair_heads = ((a.Hq / a.Hkv) % 2 == 0) ? 1 : 0;
   const int64_t blocks = (a.Sq + kBM - 1) / kBM;
-  // x: 2 CTAs (one cluster) per pair of query tiles
-  dim3 grid((unsigned)(2 * (pair_heads ? blocks : (blocks + 1) / 2)), (unsigned)(pair_heads ? a.Hq / 2 : a.Hq),
-            (unsigned)B);
+  // x: 2 CTAs (one cluster) per pair of query tiles and split
+  dim3 grid((unsigned)(2 * (pair_heads ? blocks : (blocks + 1) / 2) * (SPLIT ? x.nsplit : 1)),
+            (unsigned)(pair_heads ? a.Hq / 2 : a.Hq), (unsigned)B);
   {
     ProfScope prof(kProfAttention, stream);
     kern<<<grid, kThreads, smem, stream>>>(a, x, pair_heads);
   }
   TQ_CUDA_OK(cudaGetLastError());
-  return TQ_OK;
+  return SPLIT ? merge_split_tiles(a, B, D, x.nsplit, x.part_o, x.part_ml, stream) : TQ_OK;
+}
+template <int D, int BITS>
+int launch_kind(const AttnArgs& a, const PairArgs& x, int64_t B, cudaStream_t stream) {
+  const bool masked = a.mask != nullptr || a.mb.words != nullptr;
+  if (x.nsplit > 1) return masked ? launch_c2<D, BITS, true, true>(a, x, B, stream) : launch_c2<D, BITS, false, true>(a, x, B, stream);
+  return masked ? launch_c2<D, BITS, true, false>(a, x, B, stream) : launch_c2<D, BITS, false, false>(a, x, B, stream);
+}
+template <int D>
+int launch_bits(const AttnArgs& a, const PairArgs& x, int64_t B, int bits, cudaStream_t stream) {
+  return bits == 2 ? launch_kind<D, 2>(a, x, B, stream) : bits == 3 ? launch_kind<D, 3>(a, x, B, stream) : launch_kind<D, 4>(a, x, B, stream);
 }
 
 }  // namespace
 
+// A few new tokens behind a long prefix are a few clusters of many key tiles each on 74 pairs of SMs.  Costs in periods of a
+// key tile (1.46 us): the set-up and end of a cluster take kFixed of them, kFixedSplit where it leaves partial results, and
+// the merge kMerge (9600 rows: 21 us).  The number of splits is the one with the least (waves of clusters) x (tiles +
+// fixed) + merge.  Measured with append (LLaMA-8B heads): 100 tokens behind 8000 take 61 us in four splits, 112 us in one;
+// 300 tokens behind 8000, 48 clusters, take 112 us in one and 122 us in three.
+int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
+  constexpr double kFixed = 6.0, kFixedSplit = 10.0, kMerge = 15.0;
+  if (Hkv <= 0 || Sk <= 0) return 1;
+  const bool pair_heads = (Hq / Hkv) % 2 == 0;
+  const int64_t blocks = (Sq + kBM - 1) / kBM, tiles = (Sk + kBN - 1) / kBN;
+  const int64_t clusters = B * (pair_heads ? Hq / 2 * blocks : Hq * ((blocks + 1) / 2)), slots = sm_count() / 2;
+  // whole tiles in front of the first query, so that no split of a causal call is empty; at least four tiles each
+  const int64_t most = (Sk > Sq ? Sk - Sq : 0) / kBN / 4;
+  int best = 1;
+  double cost = (double)((clusters + slots - 1) / slots) * ((double)tiles + kFixed);
+  for (int64_t n = 2; n <= most && n <= 32 && clusters < slots; ++n) {
+    const int64_t waves = (clusters * n + slots - 1) / slots;
+    const double c = (double)waves * ((double)((tiles + n - 1) / n) + kFixedSplit) + kMerge;
+    if (c < cost) {
+      cost = c;
+      best = (int)n;
+    }
+  }
+  return best;
+}
+size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit) {
+  if (nsplit <= 1) return 0;
+  return ((size_t)B * Hq * ((Sq + kBM - 1) / kBM) * nsplit * kBM * (d + 2) * sizeof(float) + 255) & ~(size_t)255;
+}
+
 int attention_c2(const AttnArgs& a, const PairArgs& x, int64_t B, int d, int bits, cudaStream_t stream) {
-  if (d == 128)
-    return bits == 2 ? launch_c2<128, 2>(a, x, B, stream) : bits == 3 ? launch_c2<128, 3>(a, x, B, stream)
-                                                                      : launch_c2<128, 4>(a, x, B, stream);
-  if (d == 64)
-    return bits == 2 ? launch_c2<64, 2>(a, x, B, stream) : bits == 3 ? launch_c2<64, 3>(a, x, B, stream)
-                                                                    : launch_c2<64, 4>(a, x, B, stream);
+  if (d == 128) return launch_bits<128>(a, x, B, bits, stream);
+  if (d == 64) return launch_bits<64>(a, x, B, bits, stream);
   return fail(TQ_ERR_UNSUPPORTED, "the SM-pair attention kernel is built for head_dim 64 and 128 only");
 }
 

@@ -577,7 +577,9 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a, c
 }
 
 // Merge of the chunks of 64 query rows and back-rotation by Pi_v.  16 x D / 8 threads; a thread owns 4 rows x 8 columns.
-template <int D>
+// TILE: query rows per tile of the partial results.  64: those of attention_simt_kernel; 128: those of the SM-pair kernel,
+// with maxima in log2 units and every chunk there (a maximum of -inf marks an empty one).
+template <int D, int TILE>
 __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArgs a, const SplitArgs x) {
   constexpr int TX = D / 8, NT = 16 * TX, XS = D + 4;
   extern __shared__ __align__(16) float smem[];
@@ -589,9 +591,18 @@ __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArg
   load_matrix<D, false>(a.Pi_v, M, tid, NT);
   int k_end = (int)a.Sk;
   if (a.causal) k_end = min(k_end, min(q0 + kRows - 1, (int)a.Sq - 1) + (int)(a.Sk - a.Sq) + 1);
-  const int n = (k_end + x.chunk * kRows - 1) / (x.chunk * kRows);
-  const int64_t unit = (bh * gridDim.x + blockIdx.x) * x.nsplit;
+  const int n = TILE == kRows ? (k_end + x.chunk * kRows - 1) / (x.chunk * kRows) : x.nsplit;
+  constexpr int PER = TILE / kRows;
+  const int64_t unit = (bh * ((gridDim.x + PER - 1) / PER) + blockIdx.x / PER) * x.nsplit;
+  const int trow = blockIdx.x % PER * kRows + row0;  // first row within the tile
+  auto weight = [](float d) { return TILE == kRows ? __expf(d) : exp2f(d); };
+  // the rows' maxima over the chunks, then weights and sums: two passes over a few numbers, so that the chunks' rows are
+  // loads without a chain between them
   float m[4], l[4], acc[4][8];
+  auto stats = [&](int s, int r) {
+    if (TILE != kRows && q0 + row0 + r >= a.Sq) return make_float2(-INFINITY, 0.f);  // not written
+    return __ldg(reinterpret_cast<const float2*>(x.part_ml + ((unit + s) * TILE + trow + r) * 2));
+  };
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     m[r] = -INFINITY;
@@ -599,19 +610,27 @@ __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArg
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
   }
+#pragma unroll 4
+  for (int s = 0; s < n; ++s)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) m[r] = fmaxf(m[r], stats(s, r).x);
+#pragma unroll 2
   for (int s = 0; s < n; ++s)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const float2 ml = __ldg(reinterpret_cast<const float2*>(x.part_ml + ((unit + s) * kRows + row0 + r) * 2));
-      const float4* p = reinterpret_cast<const float4*>(x.part_o + ((unit + s) * kRows + row0 + r) * D + tx * 8);
-      const float4 u = __ldg(p), v = __ldg(p + 1);
-      const float m_new = fmaxf(m[r], ml.x), m_use = m_new == -INFINITY ? 0.f : m_new;
-      const float f = m[r] == -INFINITY ? 0.f : __expf(m[r] - m_use), g = ml.x == -INFINITY ? 0.f : __expf(ml.x - m_use);
-      m[r] = m_new;
-      l[r] = l[r] * f + ml.y * g;
+      const float2 ml = stats(s, r);
+      const bool there = ml.x != -INFINITY;
+      float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
+      if (there) {
+        const float4* p = reinterpret_cast<const float4*>(x.part_o + ((unit + s) * TILE + trow + r) * D + tx * 8);
+        u = __ldg(p);
+        v = __ldg(p + 1);
+      }
+      const float g = there ? weight(ml.x - m[r]) : 0.f;
+      l[r] = fmaf(ml.y, g, l[r]);
       const float w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(w[c], g, acc[r][c] * f);
+      for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(w[c], g, acc[r][c]);
     }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -761,15 +780,20 @@ static size_t split_bytes(const SplitArgs& x, int64_t B, int64_t Hq, int64_t Sq,
   return round256((size_t)B * Hq * ((Sq + kRows - 1) / kRows) * x.nsplit * kRows * (d + 2) * sizeof(float));
 }
 
-template <int D>
+template <int D, int TILE>
 static int launch_merge(const AttnArgs& a, const SplitArgs& x, int64_t B, cudaStream_t stream) {
   constexpr size_t smem = sizeof(float) * (D * D + kRows * (D + 4));
-  auto kern = merge_tiles_kernel<D>;
+  auto kern = merge_tiles_kernel<D, TILE>;
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ProfScope prof(kProfBackRotation, stream);
   kern<<<dim3((unsigned)((a.Sq + kRows - 1) / kRows), (unsigned)a.Hq, (unsigned)B), 16 * (D / 8), smem, stream>>>(a, x);
   TQ_CUDA_OK(cudaGetLastError());
   return TQ_OK;
+}
+
+int merge_split_tiles(const AttnArgs& a, int64_t B, int d, int nsplit, float* part_o, float* part_ml, cudaStream_t stream) {
+  const SplitArgs x{0, nsplit, part_o, part_ml};
+  return d == 128 ? launch_merge<128, 128>(a, x, B, stream) : launch_merge<64, 128>(a, x, B, stream);
 }
 
 template <int D, int BITS>
@@ -785,7 +809,7 @@ static int launch_attention(const AttnArgs& a, const SplitArgs& x, int64_t B, cu
     kern<<<grid, 256, smem, stream>>>(a, x);
     TQ_CUDA_OK(cudaGetLastError());
   }
-  return x.nsplit > 1 ? launch_merge<D>(a, x, B, stream) : TQ_OK;
+  return x.nsplit > 1 ? launch_merge<D, kRows>(a, x, B, stream) : TQ_OK;
 }
 
 int attention_fp32(const AttnArgs& a, const SplitArgs& x, int64_t B, int d, int bits, cudaStream_t stream) {

@@ -938,7 +938,8 @@ size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t 
   a.Hq = Hq; a.Sq = Sq; a.Hkv = Hkv; a.Sk = Sk; a.kv_stride = kv_stride;
   const int64_t n_q = B * Hq * Sq;
   switch (bf16_path(a, Sq, d)) {
-    case Bf16Path::kPairs: return 0;  // everything it needs is in the constants buffer and on the chip
+    // everything it needs is in the constants buffer and on the chip, but for the partial results of a split call
+    case Bf16Path::kPairs: return attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk));
     case Bf16Path::kDecode: return round256((size_t)n_q * 2 * d * 2) + decode_workspace_bytes(B * Hq);
     default: return round256((size_t)n_q * 2 * d * 2) + round256((size_t)n_q * d * 2);
   }
@@ -992,7 +993,12 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
       build_luts_kernel<<<1, 128, 0, stream>>>(a.cen_k, a.cen_v, bits - 1, bits, const_cast<uint32_t*>(luts));
       TQ_CUDA_OK(cudaGetLastError());
     }
-    const PairArgs x{q, dtype, sb, sh, ss, w_cat, w_unrot, luts};
+    PairArgs x{q, dtype, sb, sh, ss, w_cat, w_unrot, luts, 1, nullptr, nullptr};
+    if (prepared != nullptr) {  // the workspace of a prepared call has room for partial results
+      x.nsplit = attention_c2_splits(B, Hq, Sq, a.Hkv, a.Sk);
+      x.part_o = static_cast<float*>(workspace);
+      x.part_ml = x.part_o + (size_t)B * Hq * ((Sq + kBM - 1) / kBM) * x.nsplit * kBM * d;
+    }
     return attention_c2(a, x, B, d, bits, stream);
   }
   // the attention kernel's score contraction runs on fp16 operands: its prepared queries are fp16

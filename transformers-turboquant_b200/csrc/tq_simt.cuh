@@ -20,30 +20,68 @@ template <int D, bool TRANSPOSE>
 __device__ void load_matrix(const float* __restrict__ M, float* __restrict__ MT, int tid, int nthreads) {
   if constexpr (TRANSPOSE) {
     // Lanes take consecutive rows and 32 bytes of each: a whole sector read, and stores to 32 columns of one row of MT
-    // (two to a bank).  Lanes along a row instead store 32 deep into one bank: 8 us of a 24 us launch at head_dim 128.
-    for (int e = tid; e < D * (D / 8); e += nthreads) {
-      const int a = e % D, b = e / D * 8, col = perm_col<D>(a);
-      const float4 u = __ldg(reinterpret_cast<const float4*>(M + a * D + b)), v = __ldg(reinterpret_cast<const float4*>(M + a * D + b) + 1);
-      const float w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    // (two to a bank).  Lanes along a row instead store 32 deep into one bank, and one load at a time costs a trip to L2
+    // each: the two made half of a launch of one tile per CTA.
+    constexpr int N = D * (D / 8), kAhead = 4;  // pieces whose loads are in flight together
+    for (int e0 = tid; e0 < N; e0 += kAhead * nthreads) {
+      float4 u[kAhead], v[kAhead];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) MT[(b + i) * D + col] = w[i];
+      for (int x = 0; x < kAhead; ++x) {
+        const int e = e0 + x * nthreads;
+        if (e < N) {
+          const float4* src = reinterpret_cast<const float4*>(M + e % D * D + e / D * 8);
+          u[x] = __ldg(src);
+          v[x] = __ldg(src + 1);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < kAhead; ++x) {
+        const int e = e0 + x * nthreads, b = e / D * 8, col = perm_col<D>(e % D);
+        if (e < N) {
+          const float w[8] = {u[x].x, u[x].y, u[x].z, u[x].w, v[x].x, v[x].y, v[x].z, v[x].w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) MT[(b + i) * D + col] = w[i];
+        }
+      }
     }
   } else {
-    for (int e = tid; e < D * (D / 4); e += nthreads) {
-      const int a = e / (D / 4), b = e % (D / 4) * 4;  // the permutation keeps groups of four columns together
-      *reinterpret_cast<float4*>(MT + a * D + perm_col<D>(b)) = __ldg(reinterpret_cast<const float4*>(M + a * D + b));
+    constexpr int N = D * (D / 4), kAhead = 8;
+    for (int e0 = tid; e0 < N; e0 += kAhead * nthreads) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int x = 0; x < kAhead; ++x)
+        if (e0 + x * nthreads < N) v[x] = __ldg(reinterpret_cast<const float4*>(M) + e0 + x * nthreads);
+#pragma unroll
+      for (int x = 0; x < kAhead; ++x) {
+        const int e = e0 + x * nthreads;  // the permutation keeps groups of four columns together
+        if (e < N) *reinterpret_cast<float4*>(MT + e / (D / 4) * D + perm_col<D>(e % (D / 4) * 4)) = v[x];
+      }
     }
   }
+}
+
+// Two fp32 multiply-adds in one instruction (each rounded as fmaf rounds): d = a * b + d
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
 }
 
 // acc[r][c] = sum_i X[row0+r][i] * MT[i][cols of this thread]
 template <int D, int XS>
 __device__ __forceinline__ void tile_gemm(const float* __restrict__ X, const float* __restrict__ MT,
                                           int row0, int tx, float (&acc)[4][8]) {
+  unsigned long long a2[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+    for (int c = 0; c < 4; ++c) a2[r][c] = 0ull;
 #pragma unroll 2
   for (int i4 = 0; i4 < D; i4 += 4) {
     float4 xv[4];
@@ -51,17 +89,23 @@ __device__ __forceinline__ void tile_gemm(const float* __restrict__ X, const flo
     for (int r = 0; r < 4; ++r) xv[r] = *reinterpret_cast<const float4*>(X + (row0 + r) * XS + i4);
 #pragma unroll
     for (int ii = 0; ii < 4; ++ii) {
-      const float4 m0 = *reinterpret_cast<const float4*>(MT + (i4 + ii) * D + tx * 4);
-      const float4 m1 = *reinterpret_cast<const float4*>(MT + (i4 + ii) * D + D / 2 + tx * 4);
-      const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+      const ulonglong2 m0 = *reinterpret_cast<const ulonglong2*>(MT + (i4 + ii) * D + tx * 4);
+      const ulonglong2 m1 = *reinterpret_cast<const ulonglong2*>(MT + (i4 + ii) * D + D / 2 + tx * 4);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const float xs = ii == 0 ? xv[r].x : ii == 1 ? xv[r].y : ii == 2 ? xv[r].z : xv[r].w;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(xs, m[c], acc[r][c]);
+        const unsigned long long x2 = pack2(xs, xs);
+        fma2(a2[r][0], x2, m0.x);
+        fma2(a2[r][1], x2, m0.y);
+        fma2(a2[r][2], x2, m1.x);
+        fma2(a2[r][3], x2, m1.y);
       }
     }
   }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) unpack2(a2[r][c], acc[r][2 * c], acc[r][2 * c + 1]);
 }
 
 
