@@ -1006,8 +1006,8 @@ int launch_bits(const AttnArgs& a, const PairArgs& x, int64_t B, int bits, cudaS
 // A few new tokens behind a long prefix are a few clusters of many key tiles each on 74 pairs of SMs.  Costs in periods of a
 // key tile (1.46 us): the set-up and end of a cluster take kFixed of them, kFixedSplit where it leaves partial results, and
 // the merge kMerge (9600 rows: 21 us).  The number of splits is the one with the least (waves of clusters) x (tiles +
-// fixed) + merge.  Measured with append (LLaMA-8B heads): 100 tokens behind 8000 take 61 us in four splits, 112 us in one;
-// 300 tokens behind 8000, 48 clusters, take 112 us in one and 122 us in three.
+// fixed) + merge.  Measured with append (LLaMA-8B heads): 100 tokens behind 8000 take 61 us in four splits and 112 us in one,
+// 20 behind 30000 122 and 353 us; 300 behind 8000, 48 clusters, take 112 us in one and 122 us in three.
 int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
   constexpr double kFixed = 6.0, kFixedSplit = 10.0, kMerge = 15.0;
   if (Hkv <= 0 || Sk <= 0) return 1;

@@ -3,13 +3,13 @@
 //   * estimator scores from packed keys (full fp32 matrix, small shapes)
 //   * fused causal attention from packed keys and values (flash-style online softmax,
 //     P V accumulated in the values' rotated coordinates, one back-rotation per tile)
-//   * value decompression
 // Follows compressors.py:163-224, :296-317, kernels/attention.py:380-461 and the adapter
 // core families/llama.py:100-114 of the reference.
 #include <math.h>
 
 #include "tq_common.cuh"
 #include "tq_simt.cuh"
+#include "tq_compress.cuh"
 #include "tq_attention.cuh"
 
 namespace tq {
@@ -120,9 +120,9 @@ __global__ void __launch_bounds__(8 * D) qprep_rows_kernel(const void* __restric
   const int tid = threadIdx.x, j = tid / 8, part = tid % 8;
   float4 w1[NV], w2[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) w1[i] = __ldg(reinterpret_cast<const float4*>(Pi + j * D + 4 * part + 32 * i));
+  for (int i = 0; i < NV; ++i) w1[i] = ldg4(Pi + j * D + 4 * part + 32 * i);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) w2[i] = __ldg(reinterpret_cast<const float4*>(S_eff + j * D + 4 * part + 32 * i));
+  for (int i = 0; i < NV; ++i) w2[i] = ldg4(S_eff + j * D + 4 * part + 32 * i);
   const int64_t n0 = (int64_t)blockIdx.x * rows_per_cta;
   const int R = (int)(n_q - n0 < rows_per_cta ? n_q - n0 : rows_per_cta);
   for (int e = tid; e < R * D; e += 8 * D) {
@@ -650,50 +650,6 @@ __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArg
   }
 }
 
-// ---- value decompression ---------------------------------------------------------------
-
-template <int D, int VB>
-__global__ void __launch_bounds__(16 * (D / 8)) decompress_simt_kernel(const uint8_t* __restrict__ idx,
-                                                                      const uint16_t* __restrict__ vn, int64_t n_vec,
-                                                                      const float* __restrict__ Pi,
-                                                                      const float* __restrict__ cen_g,
-                                                                      float* __restrict__ out, int num_tiles) {
-  constexpr int TX = D / 8, NT = 16 * TX, XS = D + 4;
-  extern __shared__ __align__(16) float smem[];
-  float* M = smem;
-  float* X = M + D * D;
-  __shared__ float cen[1 << VB];
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX, row0 = ty * 4;
-  if (tid < (1 << VB)) cen[tid] = cen_g[tid];
-  load_matrix<D, false>(Pi, M, tid, NT);
-  for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-    const int64_t base = static_cast<int64_t>(tile) * kRows;
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t n = base + row0 + r;
-      float* xr = X + (row0 + r) * XS + tx * 8;
-      uint64_t w = 0;
-      if (n < n_vec) w = load_fields8<VB>(idx + n * (D * VB / 8) + tx * VB);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) xr[c] = (n < n_vec) ? cen[(w >> (c * VB)) & ((1u << VB) - 1)] : 0.f;
-    }
-    __syncthreads();
-    float y[4][8];
-    tile_gemm<D, XS>(X, M, row0, tx, y);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t n = base + row0 + r;
-      if (n < n_vec) {
-        const float nv = fp16_value(vn[n]);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) y[r][c] *= nv;
-        store8(out, TQ_F32, n * D + tx * 8, y[r]);
-      }
-    }
-  }
-}
-
 // ---- host side ---------------------------------------------------------------------------
 
 template <typename T, int D>
@@ -823,20 +779,6 @@ int attention_fp32(const AttnArgs& a, const SplitArgs& x, int64_t B, int d, int 
   return launch_attention<64, 4>(a, x, B, stream);
 }
 
-template <int D, int VB>
-static int launch_decompress(const uint8_t* idx, const uint16_t* vn, int64_t n, const float* Pi, const float* cen,
-                             float* out, cudaStream_t stream) {
-  constexpr size_t smem = sizeof(float) * (D * D + kRows * (D + 4));
-  auto kern = decompress_simt_kernel<D, VB>;
-  TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int tiles = (int)((n + kRows - 1) / kRows);
-  int grid = sm_count() * 2;
-  if (grid > tiles) grid = tiles;
-  kern<<<grid, 16 * (D / 8), smem, stream>>>(idx, vn, n, Pi, cen, out, tiles);
-  TQ_CUDA_OK(cudaGetLastError());
-  return TQ_OK;
-}
-
 }  // namespace tq
 
 using namespace tq;
@@ -882,15 +824,7 @@ int tq_decompress_values(const uint8_t* packed_idx, const uint16_t* vec_norms, i
   TQ_REQUIRE(aligned16(out), "out must be 16-byte aligned");
   CallScope scope(packed_idx, "packed_idx", static_cast<cudaStream_t>(stream));
   if (scope.status()) return scope.status();
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (d == 128) {
-    if (bits == 2) return launch_decompress<128, 2>(packed_idx, vec_norms, n, Pi, centroids, out, s);
-    if (bits == 3) return launch_decompress<128, 3>(packed_idx, vec_norms, n, Pi, centroids, out, s);
-    return launch_decompress<128, 4>(packed_idx, vec_norms, n, Pi, centroids, out, s);
-  }
-  if (bits == 2) return launch_decompress<64, 2>(packed_idx, vec_norms, n, Pi, centroids, out, s);
-  if (bits == 3) return launch_decompress<64, 3>(packed_idx, vec_norms, n, Pi, centroids, out, s);
-  return launch_decompress<64, 4>(packed_idx, vec_norms, n, Pi, centroids, out, s);
+  return decompress_tc(packed_idx, vec_norms, n, d, Pi, centroids, bits, out, static_cast<cudaStream_t>(stream));
 }
 
 int tq_attention_scores(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t q_stride_b,

@@ -31,6 +31,10 @@ __device__ __forceinline__ int64_t compress_out_row(const CompressArgs& a, int64
 // bf16 inputs, rotation and sketch projection on tcgen05 (tq_compress_tc.cu).
 int compress_tc(bool is_key, int d, int index_bits, const CompressArgs& a, cudaStream_t stream);
 
+// Values back to fp32 on tcgen05 (tq_compress_tc.cu): any n > 0, any alignment of the packed rows.
+int decompress_tc(const uint8_t* idx, const uint16_t* vn, int64_t n, int d, const float* Pi, const float* cen, int bits,
+                  float* out, cudaStream_t stream);
+
 // Keys and values in one launch, tiles staged by TMA, constants from a prepared buffer (tq_compress_kv.cu):
 // bf16 and fp16 inputs in TQ_MODE_BF16.  Either input may be NULL (that side is skipped).  Strides in
 // elements (batch, head, position).  TQ_ERR_UNSUPPORTED when the driver refuses a tensor map for the strides.

@@ -306,7 +306,167 @@ int launch(const CompressArgs& a, cudaStream_t stream) {
   return TQ_OK;
 }
 
+// ---- value decompression -------------------------------------------------------------------
+//
+// out = n C[idx] Pi for tiles of 128 vectors.  Centroids (x 256) are split into three fp16 parts, the rotation (x 128) into
+// hi + lo (22 mantissa bits, scaled so that the low parts are normal numbers); the four products that matter run as tcgen05
+// MMAs, small ones first (the accumulator is truncated at every step), and the norm and 2^-15 are applied in fp32.  Against
+// fp64 the result is as close as the fp32 CUDA-core product it replaces (relative
+// errors 1.2e-7 to 2.0e-7 at either head_dim, 1.5e-7 to 2.1e-7 before).
+// A CTA converts the rotation once and walks tiles; 16384 vectors at head_dim 128 took 20 us on the CUDA cores, bound by
+// the latency of shared-memory operands at 8 warps per tile; 11 us here, most of it the conversion and the launch.
+template <int D, int VB>
+__global__ void __launch_bounds__(256, 1) decompress_tc_kernel(const uint8_t* __restrict__ idx, const uint16_t* __restrict__ vn,
+                                                               int64_t n_vec, const float* __restrict__ Pi,
+                                                               const float* __restrict__ cen, float* __restrict__ out,
+                                                               int num_tiles) {
+  constexpr int G = D / 8;
+  constexpr uint32_t MAT = D * D * 2, TILE = 128 * D * 2, SBO = G * 128;  // A: K-major, 8-row groups SBO apart
+  constexpr uint32_t LBO = G * 128;                                       // B: MN-major, 8-row groups of Pi LBO apart
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *BH = smem, *BL = BH + MAT, *AH = BL + MAT, *AL = AH + TILE, *AX = AL + TILE;
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
+  __shared__ uint32_t lut[1 << VB], lut_x[1 << VB];  // low half: fp16 hi part of the centroid, high half: lo part; what is left
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  if (tid == 0) {
+    s_abort = 0;
+    tc::mbar_init(tc::smem_u32(&bar), 1);
+    tc::fence_mbar_init();
+  }
+  if (warp == 0) tc::tmem_alloc(tc::smem_u32(&tmem_slot), D);
+  auto split = [](float v, uint32_t& hi, uint32_t& lo) {
+    const __half h = __float2half_rn(v);
+    hi = __half_as_ushort(h);
+    lo = __half_as_ushort(__float2half_rn(v - __half2float(h)));
+  };
+  if (tid < (1 << VB)) {
+    uint32_t hi, lo;
+    const float v = cen[tid] * 256.f;
+    split(v, hi, lo);
+    lut[tid] = hi | (lo << 16);
+    // (an error of a centroid would be that of every coordinate at its level)
+    const float rest = (v - __half2float(__ushort_as_half((unsigned short)hi))) - __half2float(__ushort_as_half((unsigned short)lo));
+    lut_x[tid] = __half_as_ushort(__float2half_rn(rest));
+  }
+#pragma unroll 4
+  for (int e = tid; e < D * G; e += 256) {  // eight columns of a row of Pi
+    const int i = e / G, c = e % G;
+    const float4 p0 = ldg4(Pi + i * D + 8 * c), p1 = ldg4(Pi + i * D + 8 * c + 4);
+    const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+    uint32_t h[8], l[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) split(v[x] * 128.f, h[x], l[x]);
+    const uint32_t off = (i / 8) * LBO + c * 128 + (i % 8) * 16;
+    *reinterpret_cast<uint4*>(BH + off) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+    *reinterpret_cast<uint4*>(BL + off) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_slot, bar_addr = tc::smem_u32(&bar);
+  constexpr uint32_t idesc = tc::idesc_f16(128, D, false, true);
+  const uint64_t ah = tc::smem_desc(tc::smem_u32(AH), 128, SBO), al = tc::smem_desc(tc::smem_u32(AL), 128, SBO);
+  const uint64_t ax = tc::smem_desc(tc::smem_u32(AX), 128, SBO);
+  const uint64_t bh = tc::smem_desc(tc::smem_u32(BH), LBO, 128), bl = tc::smem_desc(tc::smem_u32(BL), LBO, 128);
+  volatile int* abort_flag = &s_abort;
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    const int64_t base = (int64_t)tile * 128;
+#pragma unroll 4
+    for (int e = tid; e < 128 * G; e += 256) {
+      const int r = e % 8 + 8 * (e / (8 * G)), c = (e / 8) % G;
+      const uint64_t w = base + r < n_vec ? load_fields8<VB>(idx + (base + r) * (D * VB / 8) + c * VB) : 0ull;
+      uint32_t t[8], u[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const uint32_t i = (uint32_t)(w >> (x * VB)) & ((1u << VB) - 1);
+        t[x] = lut[i];
+        u[x] = lut_x[i];
+      }
+      const uint32_t off = (r / 8) * SBO + c * 128 + (r % 8) * 16;
+      *reinterpret_cast<uint4*>(AH + off) = make_uint4(__byte_perm(t[0], t[1], 0x5410), __byte_perm(t[2], t[3], 0x5410),
+                                                       __byte_perm(t[4], t[5], 0x5410), __byte_perm(t[6], t[7], 0x5410));
+      *reinterpret_cast<uint4*>(AL + off) = make_uint4(__byte_perm(t[0], t[1], 0x7632), __byte_perm(t[2], t[3], 0x7632),
+                                                       __byte_perm(t[4], t[5], 0x7632), __byte_perm(t[6], t[7], 0x7632));
+      *reinterpret_cast<uint4*>(AX + off) = make_uint4(u[0] | (u[1] << 16), u[2] | (u[3] << 16), u[4] | (u[5] << 16), u[6] | (u[7] << 16));
+    }
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (tid == 0) {
+      tc::fence_after_sync();
+      auto product = [&](uint64_t a, uint64_t b, uint32_t accumulate) {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          tc::mma_bf16(tmem, a + (uint64_t)(ks * 256 >> 4), b + (uint64_t)(ks * 2 * LBO >> 4), idesc, ks > 0 ? 1u : accumulate);
+      };
+      product(ax, bh, 0u);
+      product(al, bh, 1u);
+      product(ah, bl, 1u);
+      product(ah, bh, 1u);
+      tc::mma_commit(bar_addr);
+    }
+    if (!(ok = tc::mbar_wait_or_abort(bar_addr, phase, abort_flag))) break;
+    phase ^= 1;
+    tc::fence_after_sync();
+    const int64_t n = base + (warp % 4) * 32 + lane;
+    const float scale = n < n_vec ? fp16_value(vn[n]) * (1.f / 32768.f) : 0.f;
+#pragma unroll
+    for (int c0 = 0; c0 < D / 2; c0 += 32) {
+      const int col = warp / 4 * (D / 2) + c0;
+      uint32_t raw[32];
+      tc::tmem_ld32(tmem + ((uint32_t)((warp % 4) * 32) << 16) + col, raw);
+      tc::wait_ld();
+      if (n < n_vec) {
+        float4* dst = reinterpret_cast<float4*>(out + n * D + col);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          dst[i] = make_float4(__uint_as_float(raw[4 * i]) * scale, __uint_as_float(raw[4 * i + 1]) * scale,
+                               __uint_as_float(raw[4 * i + 2]) * scale, __uint_as_float(raw[4 * i + 3]) * scale);
+      }
+    }
+    tc::fence_before_sync();
+    __syncthreads();  // the next tile overwrites the operand tiles and the accumulator
+    tc::fence_after_sync();
+  }
+  if (!ok && atomicExch(&s_abort, 2) != 2) {  // one fault per CTA
+    atomicAdd(&g_compress_faults, 1ull);
+    notify_host_of_fault(g_fault_mailbox_compress);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, D);
+}
+
+template <int D, int VB>
+int launch_decompress(const uint8_t* idx, const uint16_t* vn, int64_t n, const float* Pi, const float* cen, float* out,
+                      cudaStream_t stream) {
+  constexpr size_t smem = (size_t)2 * D * D * 2 + (size_t)3 * 128 * D * 2;
+  auto kern = decompress_tc_kernel<D, VB>;
+  TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t tiles = (n + 127) / 128;
+  TQ_REQUIRE(tiles < ((int64_t)1 << 31), "too many vectors");
+  const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+  kern<<<grid, 256, smem, stream>>>(idx, vn, n, Pi, cen, out, (int)tiles);
+  TQ_CUDA_OK(cudaGetLastError());
+  return TQ_OK;
+}
+
 }  // namespace
+
+int decompress_tc(const uint8_t* idx, const uint16_t* vn, int64_t n, int d, const float* Pi, const float* cen, int bits,
+                  float* out, cudaStream_t stream) {
+  if (d == 128)
+    return bits == 2 ? launch_decompress<128, 2>(idx, vn, n, Pi, cen, out, stream)
+           : bits == 3 ? launch_decompress<128, 3>(idx, vn, n, Pi, cen, out, stream)
+                       : launch_decompress<128, 4>(idx, vn, n, Pi, cen, out, stream);
+  return bits == 2 ? launch_decompress<64, 2>(idx, vn, n, Pi, cen, out, stream)
+         : bits == 3 ? launch_decompress<64, 3>(idx, vn, n, Pi, cen, out, stream)
+                     : launch_decompress<64, 4>(idx, vn, n, Pi, cen, out, stream);
+}
 
 int compress_tc(bool is_key, int d, int ib, const CompressArgs& a, cudaStream_t stream) {
   if (is_key) {

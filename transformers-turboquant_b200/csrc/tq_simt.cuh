@@ -14,6 +14,12 @@ __device__ __forceinline__ int perm_col(int j) {
   return (e >> 2) * (D / 2) + tx * 4 + (e & 3);
 }
 
+// Four floats of a matrix that may start at any 4-byte address (one load where it is 16-byte aligned, as tensors are).
+__device__ __forceinline__ float4 ldg4(const float* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
 // Copy a row-major [D, D] fp32 matrix into shared memory as the right-hand side of
 // tile_gemm.  TRANSPOSE: MT[i][perm(j)] = M[j][i] (for x @ M^T); else MT[i][perm(j)] = M[i][j].
 template <int D, bool TRANSPOSE>
@@ -29,9 +35,9 @@ __device__ void load_matrix(const float* __restrict__ M, float* __restrict__ MT,
       for (int x = 0; x < kAhead; ++x) {
         const int e = e0 + x * nthreads;
         if (e < N) {
-          const float4* src = reinterpret_cast<const float4*>(M + e % D * D + e / D * 8);
-          u[x] = __ldg(src);
-          v[x] = __ldg(src + 1);
+          const float* src = M + e % D * D + e / D * 8;
+          u[x] = ldg4(src);
+          v[x] = ldg4(src + 4);
         }
       }
 #pragma unroll
@@ -50,7 +56,7 @@ __device__ void load_matrix(const float* __restrict__ M, float* __restrict__ MT,
       float4 v[kAhead];
 #pragma unroll
       for (int x = 0; x < kAhead; ++x)
-        if (e0 + x * nthreads < N) v[x] = __ldg(reinterpret_cast<const float4*>(M) + e0 + x * nthreads);
+        if (e0 + x * nthreads < N) v[x] = ldg4(M + 4 * (e0 + x * nthreads));
 #pragma unroll
       for (int x = 0; x < kAhead; ++x) {
         const int e = e0 + x * nthreads;  // the permutation keeps groups of four columns together
