@@ -270,7 +270,7 @@ int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq
 /* tq_attention_fwd / tq_attention_fwd_cached with the constants taken from a prepared buffer: no operand is
  * rebuilt per call, and the scratch need drops to tq_attention_prepared_workspace_bytes -- zero for most
  * prefill-sized calls in TQ_MODE_BF16 (`workspace` may then be NULL); long prefixes behind few queries and
- * TQ_MODE_FP32 keep partial results there.  kv_capacity = Sk is the contiguous
+ * TQ_MODE_FP32 keep partial results there and are served unsplit, slower, without the room.  kv_capacity = Sk is the contiguous
  * layout; a larger capacity is the persistent-cache layout of tq_attention_fwd_cached, served in place for every
  * head_dim, number of queries and mode.
  * Replaces the attention core of the family adapters (families/llama.py:100-114, gpt2.py:90-110). */

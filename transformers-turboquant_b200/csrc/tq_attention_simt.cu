@@ -955,7 +955,21 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
                                : tq_attention_workspace_bytes(B, Hq, Sq, d, mode);
   size_t mask_need = 0;
   if (src != nullptr) mask_bits_layout(src->nb, Sq, Sk, nullptr, &mask_need);
-  const size_t need = call_need + mask_need;
+  size_t need = call_need + mask_need;
+  // A prepared call without room for partial results (no scratch at all for the SM-pair kernel, the query rows alone in
+  // fp32 mode) is served unsplit.
+  bool split = prepared != nullptr;
+  if (split && src == nullptr && (workspace == nullptr || workspace_bytes < need)) {
+    const bool rows16 = d == 128 && (Hq / Hkv) * Sq <= 16;
+    if (mode == TQ_MODE_FP32) {
+      need = round256((size_t)B * Hq * Sq * 2 * d * 4);
+      split = false;
+    } else if (!rows16 && need == attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk))) {
+      need = 0;
+      split = false;
+      workspace = nullptr;
+    }
+  }
   if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
     return fail(TQ_ERR_WORKSPACE, "workspace of %zu bytes needed (256-byte aligned), got %zu", need,
                 workspace_bytes);
@@ -977,7 +991,7 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   }
   if (mode == TQ_MODE_FP32) {
     return attention_fwd_fp32(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
-                              workspace, s, prepared != nullptr);
+                              workspace, s, split);
   }
   return attention_fwd_bf16(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
                             workspace, s, prepared);

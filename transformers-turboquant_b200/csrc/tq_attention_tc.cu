@@ -994,7 +994,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
       TQ_CUDA_OK(cudaGetLastError());
     }
     PairArgs x{q, dtype, sb, sh, ss, w_cat, w_unrot, luts, 1, nullptr, nullptr};
-    if (prepared != nullptr) {  // the workspace of a prepared call has room for partial results
+    if (prepared != nullptr && workspace != nullptr) {  // room for partial results (NULL: an unsplit call)
       x.nsplit = attention_c2_splits(B, Hq, Sq, a.Hkv, a.Sk);
       x.part_o = static_cast<float*>(workspace);
       x.part_ml = x.part_o + (size_t)B * Hq * ((Sq + kBM - 1) / kBM) * x.nsplit * kBM * d;
