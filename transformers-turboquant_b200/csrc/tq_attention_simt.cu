@@ -139,15 +139,19 @@ __global__ void __launch_bounds__(8 * D) qprep_rows_kernel(const void* __restric
     else static_cast<float*>(q_cat)[at] = v;
   };
   auto project = [&](const float (*in)[D], const float4 (&w)[NV], int r) {
-    float acc = 0.f;
+    // The order of a sum is fixed: groups of four columns, last column first, then halves folded onto each other (a
+    // butterfly over D / 4 lanes that hold a group each gives the same bits).  The 16-bit result rounds these sums, so
+    // another order moves the scores by a bf16 step here and there.
+    float g[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const float4 v = *reinterpret_cast<const float4*>(&in[r][4 * part + 32 * i]);
-      acc = fmaf(w[i].x, v.x, fmaf(w[i].y, v.y, fmaf(w[i].z, v.z, fmaf(w[i].w, v.w, acc))));
+      g[i] = fmaf(w[i].x, v.x, fmaf(w[i].y, v.y, fmaf(w[i].z, v.z, w[i].w * v.w)));
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    float acc = NV == 4 ? (g[0] + g[2 % NV]) + (g[1] + g[3 % NV]) : g[0] + g[1];
+    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
     acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    return acc + __shfl_xor_sync(0xffffffffu, acc, 4);
+    return acc + __shfl_xor_sync(0xffffffffu, acc, 1);
   };
   __syncthreads();
 #pragma unroll 2
