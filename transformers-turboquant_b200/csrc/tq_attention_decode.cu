@@ -678,7 +678,8 @@ __global__ void __launch_bounds__(4 * D) decode_finish_kernel(const float* __res
   for (int s = p; s < nsplit; s += 4) acc = fmaf(part_o[((unit * nsplit + s) * R + r) * D + j], f_s[s], acc);
   part[p][j] = acc;
   __syncthreads();
-  if (tid < D) o_s[tid] = l > 0.f ? (part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid]) / l : 0.f;
+  // no visible key: zeros; a sum of NaN (a query or a key that is not finite) makes the whole row NaN
+  if (tid < D) o_s[tid] = l == 0.f ? 0.f : (part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid]) / l;
   __syncthreads();
   float y = 0.f;
 #pragma unroll

@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a, c
 
 // Merge of the chunks of 64 query rows and back-rotation by Pi_v.  16 x D / 8 threads; a thread owns 4 rows x 8 columns.
 // TILE: query rows per tile of the partial results.  64: those of attention_simt_kernel; 128: those of the SM-pair kernel,
-// with maxima in log2 units and every chunk there (a maximum of -inf marks an empty one).
+// with maxima in log2 units and every chunk there (a maximum of -inf with a sum of 0 marks an empty one).
 template <int D, int TILE>
 __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArgs a, const SplitArgs x) {
   constexpr int TX = D / 8, NT = 16 * TX, XS = D + 4;
@@ -623,7 +623,8 @@ __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArg
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const float2 ml = stats(s, r);
-      const bool there = ml.x != -INFINITY;
+      // an empty chunk; one whose scores are all NaN has no maximum either (maxima ignore NaN), but a sum of NaN
+      const bool there = ml.x != -INFINITY || ml.y != 0.f;
       float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
       if (there) {
         const float4* p = reinterpret_cast<const float4*>(x.part_o + ((unit + s) * TILE + trow + r) * D + tx * 8);
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(16 * (D / 8)) merge_tiles_kernel(const AttnArg
     }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+    const float inv = l[r] == 0.f ? 0.f : 1.f / l[r];  // (NaN stays NaN)
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[r][c] *= inv;
     put8(X + (row0 + r) * XS + tx * 8, acc[r]);
