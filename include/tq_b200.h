@@ -168,8 +168,15 @@ int tq_rope(const void* q, const void* k, int dtype, int64_t B, int64_t Hq, int6
  * constants taken from a prepared buffer.  keys, values: [B, H, S, d] of `dtype` with their own element strides;
  * either may be NULL, which skips that side.  Vector (b, h, s) goes to row (b*H + h)*kv_capacity + kv_offset + s
  * of every output array (kv_capacity = S, kv_offset = 0: the contiguous layout of the separate calls).
- * bf16 inputs of head_dim 128 in TQ_MODE_BF16 take the fused kernel (TMA-staged tiles, rotation and sketch on
- * tcgen05); anything else runs the per-side kernels, same bytes.
+ * bf16 and fp16 inputs in TQ_MODE_BF16 take the fused kernel (TMA-staged tiles, rotation and sketch on tcgen05), fp32
+ * mode up to 3072 vectors a side one launch on the CUDA cores; anything else, strides that no tensor map describes and fp16
+ * outputs at odd addresses run the per-side kernels.  The fused kernel writes the bytes of tq_compress_keys /
+ * tq_compress_values but for coordinates within rounding of a boundary: bf16 at head_dim 64 is sketched from 22 mantissa
+ * bits where the per-side kernel takes 16, fp16 decides open coordinates as the fp32 kernel does, and norms are summed in
+ * another order (one fp16 step).
+ * Alignment of the outputs (also of tq_compress_keys, tq_compress_values and tq_append_*): norms 2 bytes; bf16 inputs in
+ * TQ_MODE_BF16 want packed indices of 1 or 3 bits on 4 bytes, 2 bits on 8, 4 bits on 16, and signs on 4; otherwise packed
+ * rows may start anywhere.  Anything else is refused with TQ_ERR_INVALID_ARG before a launch.
  * Replaces TurboQuantCompressorV2.compress + TurboQuantCompressorMSE.compress as the family adapters call them
  * back to back (src/transformers_turboquant/families/llama.py:103-104; compressors.py:98-161, :270-294). */
 int tq_compress_kv(const void* keys, const void* values, int dtype, int64_t B, int64_t H, int64_t S, int d,

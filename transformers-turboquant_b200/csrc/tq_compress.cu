@@ -324,6 +324,21 @@ static int check_states(const void* p, int dtype, int64_t B, int64_t H, int64_t 
   return TQ_OK;
 }
 
+// The tensor-core kernels store a thread's 32 indices as one word or vector of `index_bits` words, 32 signs as a word;
+// the CUDA-core kernels store bytes.
+static bool wide_stores_fit(const uint8_t* packed_idx, int index_bits, const uint8_t* packed_signs) {
+  const uintptr_t unit = index_bits == 4 ? 16 : index_bits == 2 ? 8 : 4;
+  return reinterpret_cast<uintptr_t>(packed_idx) % unit == 0 && reinterpret_cast<uintptr_t>(packed_signs) % 4 == 0;
+}
+static int check_outputs(const uint8_t* packed_idx, int index_bits, const uint8_t* packed_signs, const uint16_t* vec_norms,
+                         const uint16_t* residual_norms, int dtype, int mode) {
+  TQ_REQUIRE(((reinterpret_cast<uintptr_t>(vec_norms) | reinterpret_cast<uintptr_t>(residual_norms)) & 1u) == 0,
+             "norms must be 2-byte aligned");
+  TQ_REQUIRE(!(mode == TQ_MODE_BF16 && dtype == TQ_BF16) || wide_stores_fit(packed_idx, index_bits, packed_signs),
+             "packed rows of bf16 inputs must be aligned to %d bytes (signs: 4)", index_bits == 4 ? 16 : index_bits == 2 ? 8 : 4);
+  return TQ_OK;
+}
+
 }  // namespace tq
 
 using namespace tq;
@@ -341,6 +356,7 @@ static int compress_keys_entry(const void* keys, int dtype, int64_t B, int64_t H
   if (n == 0) return TQ_OK;
   TQ_REQUIRE(Pi && S_eff && centroids && boundaries, "NULL constant pointer");
   TQ_REQUIRE(packed_idx && packed_signs && vec_norms && residual_norms, "NULL output pointer");
+  if (int st = check_outputs(packed_idx, bits - 1, packed_signs, vec_norms, residual_norms, dtype, mode)) return st;
   CallScope scope(keys, "keys", static_cast<cudaStream_t>(stream));
   if (scope.status()) return scope.status();
   CompressArgs a{keys, n, H, S, stride_b, stride_h, stride_s, Pi, S_eff, centroids, boundaries,
@@ -359,6 +375,7 @@ static int compress_values_entry(const void* values, int dtype, int64_t B, int64
   if (n == 0) return TQ_OK;
   TQ_REQUIRE(Pi && boundaries, "NULL constant pointer");
   TQ_REQUIRE(packed_idx && vec_norms, "NULL output pointer");
+  if (int st = check_outputs(packed_idx, bits, nullptr, vec_norms, nullptr, dtype, mode)) return st;
   CallScope scope(values, "values", static_cast<cudaStream_t>(stream));
   if (scope.status()) return scope.status();
   CompressArgs a{values, n, H, S, stride_b, stride_h, stride_s, Pi, nullptr, nullptr, boundaries,
@@ -388,8 +405,15 @@ int tq_compress_kv(const void* keys, const void* values, int dtype, int64_t B, i
   if (B * H * S == 0) return TQ_OK;
   TQ_REQUIRE(keys == nullptr || (key_idx && key_signs && key_vec_norms && key_residual_norms), "NULL key output pointer");
   TQ_REQUIRE(values == nullptr || (val_idx && val_vec_norms), "NULL value output pointer");
+  if (keys != nullptr)
+    if (int st = check_outputs(key_idx, bits - 1, key_signs, key_vec_norms, key_residual_norms, dtype, mode)) return st;
+  if (values != nullptr)
+    if (int st = check_outputs(val_idx, bits, nullptr, val_vec_norms, nullptr, dtype, mode)) return st;
   const uint8_t* c = static_cast<const uint8_t*>(constants);
-  if (compress_kv_applies(dtype, d, mode)) {
+  // (fp16 rows at addresses that the fused kernel cannot store to go to the kernels that store bytes)
+  const bool fit = (keys == nullptr || wide_stores_fit(key_idx, bits - 1, key_signs)) &&
+                   (values == nullptr || wide_stores_fit(val_idx, bits, nullptr));
+  if (compress_kv_applies(dtype, d, mode) && fit) {
     CallScope scope(keys != nullptr ? keys : values, "keys/values", static_cast<cudaStream_t>(stream));
     if (scope.status()) return scope.status();
     const int64_t ks[3] = {k_stride_b, k_stride_h, k_stride_s}, vs[3] = {v_stride_b, v_stride_h, v_stride_s};
