@@ -104,10 +104,11 @@ __device__ __forceinline__ float bf16_value(uint32_t b) { return __uint_as_float
 // Codebooks of 8 and more levels use the symmetry of the boundaries (b[NB-1-j] = -b[j], b[(NB-1)/2] = 0): the sign
 // of y and the count m of positive boundaries below |y| give idx = h + m for y > 0 and h - 1 - m otherwise
 // (h = (NB+1)/2), with half the subtractions.  The one difference: a NEGATIVE y that equals a boundary exactly
-// lands one level higher than the strict count would put it (part of the documented tie budget).
-template <int NB>
+// lands one level higher than the strict count would put it (part of the documented tie budget).  SYM false: boundaries
+// that a caller replaced by ones without that symmetry, counted as they are.
+template <int NB, bool SYM>
 __device__ __forceinline__ uint32_t index_of(float y, const float (&bd)[NB]) {
-  if constexpr (NB < 7) {
+  if constexpr (NB < 7 || !SYM) {
     uint32_t idx = 0;
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
@@ -129,6 +130,13 @@ __device__ __forceinline__ uint32_t index_of(float y, const float (&bd)[NB]) {
     return (uint32_t)(h - 1) - m + pos * (2u * m + 1u);
   }
 }
+template <int NB>
+__device__ __forceinline__ bool symmetric(const float (&b)[NB]) {
+  bool s = NB < 7 || b[NB / 2] == 0.f;
+#pragma unroll
+  for (int j = 0; NB >= 7 && j < NB / 2; ++j) s = s && b[j] == -b[NB - 1 - j];
+  return s;
+}
 // OR the B-bit field of coordinate E (of this thread's 32) into the thread's B packed words (LSB-first bit stream)
 template <int B, int E>
 __device__ __forceinline__ void put_field(uint32_t (&w)[B], uint32_t idx) {
@@ -136,6 +144,52 @@ __device__ __forceinline__ void put_field(uint32_t (&w)[B], uint32_t idx) {
   w[k] = idx * (1u << sh) + w[k];  // the field's bits are still zero there: + is |
   if constexpr (sh + B > 32) w[k + 1] = (idx >> (32 - sh)) + w[k + 1];
 }
+template <int B, int E>
+__device__ __forceinline__ uint32_t get_field(const uint32_t (&w)[B]) {
+  constexpr int pos = E * B, k = pos / 32, sh = pos % 32;
+  uint32_t v = w[k] >> sh;
+  if constexpr (sh + B > 32) v |= w[k + 1] << (32 - sh);
+  return v & ((1u << B) - 1);
+}
+// fp16 inputs: passes over a warp's 32 rows x 32 coordinates (in tensor memory at `col`) for boundaries that are counted as
+// they are, scaled by `den`.  Not inlined: inside the kernel they would cost the passes for symmetric boundaries registers
+// (4 bits, 8 x 8 x 4096 keys and values: 227 us inlined, 185 us so).
+template <int B>
+__device__ __noinline__ void index_any(uint32_t col, const float* __restrict__ bnd, float den, uint32_t (&packed)[B]) {
+  constexpr int NB = (1 << B) - 1;
+  uint32_t raw[32];
+  tc::tmem_ld32(col, raw);
+  tc::wait_ld();
+  uint64_t word = 0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) packed[j] = 0;
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    uint32_t idx = 0;
+#pragma unroll 1
+    for (int j = 0; j < NB; ++j) idx += __uint_as_float(raw[e]) > __ldg(bnd + j) * den ? 1u : 0u;
+    const int bit = e * B, k = bit / 32, sh = bit % 32;
+    word = (uint64_t)idx << sh;
+    packed[k] |= (uint32_t)word;
+    if (sh + B > 32) packed[k + 1 < B ? k + 1 : k] |= (uint32_t)(word >> 32);
+  }
+}
+// ... bit e set where coordinate e lies within `band` of a boundary
+template <int NB>
+__device__ __noinline__ uint32_t open_any(uint32_t col, const float* __restrict__ bnd, float den, float band) {
+  uint32_t raw[32], open = 0;
+  tc::tmem_ld32(col, raw);
+  tc::wait_ld();
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    float near = INFINITY;
+#pragma unroll 1
+    for (int j = 0; j < NB; ++j) near = fminf(near, fabsf(__ldg(bnd + j) * den - __uint_as_float(raw[e])));
+    open |= near < band ? 1u << e : 0u;
+  }
+  return open;
+}
+
 // Repair of fp16 decisions that the tensor-core sums leave open.
 //
 // An index or a sign whose coordinate lies within the sums' rounding of its boundary may fall either way, and a single
@@ -460,6 +514,15 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     for (int j = 0; j < (1 << KB) - 1; ++j) bnd_k[j] = __ldg(reinterpret_cast<const float*>(a.consts + a.L.bnd_k) + j);
 #pragma unroll
     for (int j = 0; j < (1 << VB) - 1; ++j) bnd_v[j] = __ldg(reinterpret_cast<const float*>(a.consts + a.L.bnd_v) + j);
+    const bool sym_k = symmetric(bnd_k), sym_v = symmetric(bnd_v);
+    // boundaries scaled for a tile's pass: from registers where symmetry needs half of them only, else loaded again
+    auto scaled = [](auto sym, const float* src, const auto& bnd, float den, auto& bden) {
+#pragma unroll
+      for (int j = 0; j < (int)(sizeof(bden) / sizeof(float)); ++j) {
+        if constexpr (decltype(sym)::value) bden[j] = bnd[j] * den;
+        else bden[j] = *static_cast<const volatile float*>(src + j) * den;
+      }
+    };
     // this row of a tile: batch element, head and position relative to the tile's first (rows past the box hold nothing)
     const uint32_t row_h = (uint32_t)row / a.box_s, row_s = (uint32_t)row - row_h * a.box_s;
     const uint32_t row_b = row_h / a.box_h, row_hh = row_h - row_b * a.box_h;
@@ -489,14 +552,11 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       }
       return near;
     };
-    // Rotated coordinates of this warp's 32 rows x 32 coordinates, in `raw` and in tensor memory at `col`: those within
-    // `band` of a boundary are moved (in tensor memory) to the side of it that the fp32 kernel finds them on.
-    auto settle = [&](auto nb, const float* Pi, const float (&bnd)[decltype(nb)::value], const float (&bden)[decltype(nb)::value],
-                      const uint32_t (&raw)[32], uint32_t col, float band, unsigned long long addr) {
+    // Rotated coordinates of this warp's 32 rows x 32 coordinates in tensor memory at `col`: the open ones (a mask per
+    // lane) are moved to the side of their boundary that the fp32 kernel finds them on.
+    auto settle = [&](auto nb, uint32_t open, const float* Pi, const float* bnd, float den, uint32_t col, unsigned long long addr) {
       constexpr int NB = decltype(nb)::value;
-      uint32_t open = 0;
-#pragma unroll
-      for (int e = 0; e < 32; ++e) open |= distance(nb, bden, __uint_as_float(raw[e])) < band ? 1u << e : 0u;
+      const float mine = lane < NB ? __ldg(bnd + lane) : INFINITY;  // a boundary per lane
       uint32_t lanes;
       while ((lanes = __ballot_sync(0xffffffffu, open != 0u)) != 0u) {
         const int l = __ffs((int)lanes) - 1;
@@ -504,14 +564,13 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         const float exact = exact_coordinate<D>(reinterpret_cast<const __half*>(__shfl_sync(0xffffffffu, addr, l)),
                                                 Pi + (32 * part + e) * D);
         float y = tc::tmem_ld1(col + e);
+        // the boundary nearest lane l's coordinate
+        const float den_l = __shfl_sync(0xffffffffu, den, l);
+        const uint32_t d = __float_as_uint(fabsf(mine * den_l - __shfl_sync(0xffffffffu, y, l)));  // (ordered as the floats are)
+        const uint32_t nearest = __ballot_sync(0xffffffffu, d == __reduce_min_sync(0xffffffffu, d));
+        const float b = __shfl_sync(0xffffffffu, mine, __ffs((int)nearest) - 1), at = b * den_l;
         if (lane == l) {
           open &= open - 1u;
-          float near = INFINITY, at = 0.f, b = 0.f;
-#pragma unroll
-          for (int j = 0; j < NB; ++j) {
-            const float d = fabsf(bden[j] - y);
-            if (d < near) { near = d; at = bden[j]; b = bnd[j]; }
-          }
           // the neighbour of the scaled boundary on that side
           const float step = fmaxf(fabsf(at) * 2.4e-7f, 1e-30f);
           y = exact > b ? at + step : at - step;
@@ -586,27 +645,35 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           // any coordinate too close to a boundary to call?
           const bool sure = !live || !(ss_tot > 0.f) || !(den < 1e30f);
           const float band = sure ? 0.f : kOpenIndex * den;
-          auto settle_side = [&](auto nb, const float* Pi, const float (&bnd)[decltype(nb)::value]) {
-            float bden[decltype(nb)::value], near = INFINITY;
+          auto settle_side = [&](auto nb, bool sym, const float* Pi, const float* src, const float (&bnd)[decltype(nb)::value]) {
+            constexpr int NB = decltype(nb)::value;
+            uint32_t open = 0;
+            if (NB < 7 || sym) {
+              float bden[NB], near = INFINITY;
 #pragma unroll
-            for (int j = 0; j < decltype(nb)::value; ++j) bden[j] = bnd[j] * den;
+              for (int j = 0; j < NB; ++j) bden[j] = bnd[j] * den;
 #pragma unroll
-            for (int e = 0; e < 32; ++e) near = fminf(near, distance(nb, bden, __uint_as_float(raw[e])));
-            if (!__any_sync(0xffffffffu, near < band)) return;
-            settle(nb, Pi, bnd, bden, raw, col_y, band, row_address(is_key, b0, h0, s0));
+              for (int e = 0; e < 32; ++e) near = fminf(near, distance(nb, bden, __uint_as_float(raw[e])));
+              if (!__any_sync(0xffffffffu, near < band)) return;
+#pragma unroll
+              for (int e = 0; e < 32; ++e) open |= distance(nb, bden, __uint_as_float(raw[e])) < band ? 1u << e : 0u;
+            } else {
+              open = open_any<NB>(col_y, src, den, band);
+              if (!__any_sync(0xffffffffu, open != 0u)) return;
+            }
+            settle(nb, open, Pi, src, den, col_y, row_address(is_key, b0, h0, s0));
             tc::tmem_ld32(col_y, raw);
             tc::wait_ld();
           };
           if (is_key)
-            settle_side(std::integral_constant<int, (1 << KB) - 1>{}, reinterpret_cast<const float*>(a.consts + a.L.pi_k), bnd_k);
+            settle_side(std::integral_constant<int, (1 << KB) - 1>{}, sym_k, reinterpret_cast<const float*>(a.consts + a.L.pi_k),
+                        reinterpret_cast<const float*>(a.consts + a.L.bnd_k), bnd_k);
           else
-            settle_side(std::integral_constant<int, (1 << VB) - 1>{}, reinterpret_cast<const float*>(a.consts + a.L.pi_v), bnd_v);
+            settle_side(std::integral_constant<int, (1 << VB) - 1>{}, sym_v, reinterpret_cast<const float*>(a.consts + a.L.pi_v),
+                        reinterpret_cast<const float*>(a.consts + a.L.bnd_v), bnd_v);
         }
         if (is_key) {
           // y = y_raw / den is compared with the boundaries as y_raw > b * den (den > 0)
-          float bden[(1 << KB) - 1];
-#pragma unroll
-          for (int j = 0; j < (1 << KB) - 1; ++j) bden[j] = bnd_k[j] * den;
           float rr = 0.f;
           uint32_t packed[KB], rh[16], rl[16];
 #pragma unroll
@@ -615,31 +682,52 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           // brings the residual's coordinates (at most about the norm) to at most about 64: a power of two
           const float r_scale = __uint_as_float(
               (uint32_t)max(127 + 6 - (F16 ? 7 : 0) + 127 - (int)(__float_as_uint(den1) >> 23), 1) << 23);
-          static_for<0, 16>([&](auto pc) {
-            constexpr int pr = decltype(pc)::value;  // coordinates 2 pr, 2 pr + 1 of this thread's 32
-            float res[2];
+          auto index_pass = [&](auto sym, auto given) {
+            constexpr bool GIVEN = decltype(given)::value;  // the indices are in `packed` already
+            float bden[(1 << KB) - 1];
+            scaled(sym, reinterpret_cast<const float*>(a.consts + a.L.bnd_k), bnd_k, den, bden);
+            static_for<0, 16>([&](auto pc) {
+              constexpr int pr = decltype(pc)::value;  // coordinates 2 pr, 2 pr + 1 of this thread's 32
+              float res[2];
+  #pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const float yr = __uint_as_float(raw[2 * pr + h]);
+                uint32_t idx;
+                if constexpr (GIVEN) {
+                  idx = h == 0 ? get_field<KB, 2 * pr>(packed) : get_field<KB, 2 * pr + 1>(packed);
+                } else {
+                  idx = index_of<(1 << KB) - 1, decltype(sym)::value>(yr, bden);
+                  if (h == 0) put_field<KB, 2 * pr>(packed, idx);
+                  else put_field<KB, 2 * pr + 1>(packed, idx);
+                }
+                res[h] = fmaf(neg_nv, cen_s[idx], yr);   // residual in rotated coordinates
+                rr = fmaf(res[h], res[h], rr);
+              }
+              // split into bf16 hi (truncated: the upper halves of the two words, one byte permute) and lo = the
+              // exact remainder, rounded; hi + lo carries ~16 mantissa bits
+              if constexpr (SK16) {
+                const float r0 = res[0] * r_scale, r1 = res[1] * r_scale;
+                rh[pr] = tc::pack_f16x2(r0, r1);
+                const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&rh[pr]));
+                rl[pr] = tc::pack_f16x2(r0 - h.x, r1 - h.y);
+              } else {
+                const uint32_t w0 = __float_as_uint(res[0]), w1 = __float_as_uint(res[1]);
+                rh[pr] = __byte_perm(w0, w1, 0x7632);
+                rl[pr] = tc::pack_bf16x2(res[0] - __uint_as_float(w0 & 0xffff0000u), res[1] - __uint_as_float(w1 & 0xffff0000u));
+              }
+            });
+          };
+          if (KB < 3 || sym_k) {
+            index_pass(std::true_type{}, std::false_type{});
+          } else if constexpr (KB >= 3 && F16) {
+            uint32_t given[KB];
+            index_any<KB>(col_y, reinterpret_cast<const float*>(a.consts + a.L.bnd_k), den, given);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const float yr = __uint_as_float(raw[2 * pr + h]);
-              const uint32_t idx = index_of<(1 << KB) - 1>(yr, bden);
-              if (h == 0) put_field<KB, 2 * pr>(packed, idx);
-              else put_field<KB, 2 * pr + 1>(packed, idx);
-              res[h] = fmaf(neg_nv, cen_s[idx], yr);   // residual in rotated coordinates
-              rr = fmaf(res[h], res[h], rr);
-            }
-            // split into bf16 hi (truncated: the upper halves of the two words, one byte permute) and lo = the
-            // exact remainder, rounded; hi + lo carries ~16 mantissa bits
-            if constexpr (SK16) {
-              const float r0 = res[0] * r_scale, r1 = res[1] * r_scale;
-              rh[pr] = tc::pack_f16x2(r0, r1);
-              const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&rh[pr]));
-              rl[pr] = tc::pack_f16x2(r0 - h.x, r1 - h.y);
-            } else {
-              const uint32_t w0 = __float_as_uint(res[0]), w1 = __float_as_uint(res[1]);
-              rh[pr] = __byte_perm(w0, w1, 0x7632);
-              rl[pr] = tc::pack_bf16x2(res[0] - __uint_as_float(w0 & 0xffff0000u), res[1] - __uint_as_float(w1 & 0xffff0000u));
-            }
-          });
+            for (int j = 0; j < KB; ++j) packed[j] = given[j];
+            index_pass(std::true_type{}, std::true_type{});
+          } else if constexpr (KB >= 3) {
+            index_pass(std::false_type{}, std::false_type{});
+          }
           if (live) {
             uint32_t* dst = reinterpret_cast<uint32_t*>(a.key_idx + no * (kD * KB / 8) + 4 * KB * part);
             if constexpr (KB == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
@@ -663,19 +751,31 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           if (lane == 0) tc::mbar_arrive(r_full);
           band_next = next_band;
         } else {
+          uint32_t given[VB];
+          if constexpr (VB >= 3 && F16)
+            if (!sym_v) index_any<VB>(col_y, reinterpret_cast<const float*>(a.consts + a.L.bnd_v), den, given);
           tc::fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(yp_free(s));  // the accumulator slot is in registers now
-          float bden[(1 << VB) - 1];
-#pragma unroll
-          for (int j = 0; j < (1 << VB) - 1; ++j) bden[j] = bnd_v[j] * den;
           uint32_t packed[VB];
 #pragma unroll
           for (int j = 0; j < VB; ++j) packed[j] = 0;
-          static_for<0, 32>([&](auto ec) {
-            constexpr int e = decltype(ec)::value;
-            put_field<VB, e>(packed, index_of<(1 << VB) - 1>(__uint_as_float(raw[e]), bden));
-          });
+          auto index_pass = [&](auto sym) {
+            float bden[(1 << VB) - 1];
+            scaled(sym, reinterpret_cast<const float*>(a.consts + a.L.bnd_v), bnd_v, den, bden);
+            static_for<0, 32>([&](auto ec) {
+              constexpr int e = decltype(ec)::value;
+              put_field<VB, e>(packed, index_of<(1 << VB) - 1, decltype(sym)::value>(__uint_as_float(raw[e]), bden));
+            });
+          };
+          if (VB < 3 || sym_v) {
+            index_pass(std::true_type{});
+          } else if constexpr (VB >= 3 && F16) {
+#pragma unroll
+            for (int j = 0; j < VB; ++j) packed[j] = given[j];
+          } else if constexpr (VB >= 3) {
+            index_pass(std::false_type{});
+          }
           if (live) {
             uint32_t* dst = reinterpret_cast<uint32_t*>(a.val_idx + no * (kD * VB / 8) + 4 * VB * part);
             if constexpr (VB == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
