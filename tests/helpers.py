@@ -49,6 +49,44 @@ def oracle_value_dict_to_device(cv: dict) -> dict:
             "vec_norms": cv["vec_norms"].cuda().contiguous(), "shape": cv["shape"]}
 
 
+def unpack_fields(packed: torch.Tensor, bits: int, d: int) -> torch.Tensor:
+    """Packed rows [..., d * bits / 8] as whole numbers [..., d] (fields LSB first), without the package's kernels."""
+    rows = packed.reshape(-1, d * bits // 8)
+    stream = (rows[:, :, None] >> torch.arange(8, dtype=torch.uint8, device=rows.device)) & 1
+    weights = 1 << torch.arange(bits, device=rows.device)
+    return (stream.reshape(-1, d, bits).long() * weights).sum(-1).reshape(*packed.shape[:-1], d)
+
+
+def values64(packed: torch.Tensor, norms: torch.Tensor, vc) -> torch.Tensor:
+    """Decoded values [..., d] in fp64 from packed rows and their norms."""
+    dev = packed.device
+    centroids, pi = vc.centroids.double().to(dev), vc.Pi.double().to(dev)
+    return centroids[unpack_fields(packed, vc.bits, vc.head_dim)] @ pi * norms.double()[..., None]
+
+
+def scores64(q: torch.Tensor, ck: dict, kc) -> torch.Tensor:
+    """Unscaled estimator scores [B, Hq, Sq, Sk] in fp64 from packed keys."""
+    B, Hkv, Sk, d = ck["shape"]
+    rows = lambda t: t.reshape(B, Hkv, Sk, -1).repeat_interleave(q.shape[1] // Hkv, dim=1)
+    cen = kc.centroids.double()[unpack_fields(rows(ck["packed_key_indices"]), kc.bits - 1, d)]
+    sign = 2.0 * unpack_fields(rows(ck["packed_qjl_signs"]), 1, d).double() - 1.0
+    rot = q.double() @ kc.Pi.double().T
+    sketch = rot @ kc.S_eff.double().T * ((torch.pi / 2) ** 0.5 / d)
+    return (rot @ cen.transpose(2, 3)) * rows(ck["vec_norms"].double())[..., 0][:, :, None] \
+        + (sketch @ sign.transpose(2, 3)) * rows(ck["residual_norm"].double())[..., 0][:, :, None]
+
+
+def contiguous_prefix(cache) -> tuple[dict, dict]:
+    """The tokens in use of a CompressedKVCache as dense compressed dictionaries."""
+    n, shape = cache.length, (cache.batch, cache.kv_heads, cache.length, cache.head_dim)
+    packed = lambda t: t[:, :, :n].reshape(-1, t.shape[-1]).contiguous()
+    ck = {"packed_key_indices": packed(cache.key_indices), "packed_qjl_signs": packed(cache.key_signs),
+          "residual_norm": cache.key_residual_norms[:, :, :n].contiguous(), "vec_norms": cache.key_norms[:, :, :n].contiguous(),
+          "shape": shape}
+    return ck, {"packed_indices": packed(cache.value_indices), "vec_norms": cache.value_norms[:, :, :n].reshape(-1).contiguous(),
+                "shape": shape}
+
+
 def rel_err(a: torch.Tensor, b: torch.Tensor) -> float:
     """Norm-wise relative error ||a-b|| / ||b||."""
     a, b = a.double().cpu(), b.double().cpu()

@@ -312,7 +312,9 @@ int launch(const CompressArgs& a, cudaStream_t stream) {
 // hi + lo (22 mantissa bits, scaled so that the low parts are normal numbers); the four products that matter run as tcgen05
 // MMAs, small ones first (the accumulator is truncated at every step), and the norm and 2^-15 are applied in fp32.  Against
 // fp64 the result is as close as the fp32 CUDA-core product it replaces (relative
-// errors 1.2e-7 to 2.0e-7 at either head_dim, 1.5e-7 to 2.1e-7 before).
+// errors 1.2e-7 to 2.0e-7 at either head_dim, 1.5e-7 to 2.1e-7 before).  The fixed scales hold those bits for rotations whose
+// columns reach 2^-7 and stay below 2^8 and for centroids that are 0 or between 2^-9 and 2^7, as every orthonormal matrix
+// and codebook of its coordinates is; with other constants the CTA multiplies in fp32, coordinate by coordinate.
 // A CTA converts the rotation once and walks tiles; 16384 vectors at head_dim 128 took 20 us on the CUDA cores, bound by
 // the latency of shared-memory operands at 8 warps per tile; 11 us here, most of it the conversion and the launch.
 template <int D, int VB>
@@ -328,6 +330,8 @@ __global__ void __launch_bounds__(256, 1) decompress_tc_kernel(const uint8_t* __
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
+  __shared__ float cen_s[1 << VB];
+  __shared__ uint32_t s_reach[8][G];                 // per warp and eight columns: those with an entry that reaches 2^-7
   __shared__ uint32_t lut[1 << VB], lut_x[1 << VB];  // low half: fp16 hi part of the centroid, high half: lo part; what is left
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   if (tid == 0) {
@@ -341,15 +345,19 @@ __global__ void __launch_bounds__(256, 1) decompress_tc_kernel(const uint8_t* __
     hi = __half_as_ushort(h);
     lo = __half_as_ushort(__float2half_rn(v - __half2float(h)));
   };
+  bool fits = true;  // the constants suit the fixed scales (a NaN does not)
   if (tid < (1 << VB)) {
     uint32_t hi, lo;
+    cen_s[tid] = cen[tid];
     const float v = cen[tid] * 256.f;
+    fits = v == 0.f || (fabsf(v) >= 0.5f && fabsf(v) <= 32768.f);
     split(v, hi, lo);
     lut[tid] = hi | (lo << 16);
     // (an error of a centroid would be that of every coordinate at its level)
     const float rest = (v - __half2float(__ushort_as_half((unsigned short)hi))) - __half2float(__ushort_as_half((unsigned short)lo));
     lut_x[tid] = __half_as_ushort(__float2half_rn(rest));
   }
+  uint32_t reach = 0;  // (a thread's pieces are the same eight columns: 256 is a multiple of G)
 #pragma unroll 4
   for (int e = tid; e < D * G; e += 256) {  // eight columns of a row of Pi
     const int i = e / G, c = e % G;
@@ -357,14 +365,28 @@ __global__ void __launch_bounds__(256, 1) decompress_tc_kernel(const uint8_t* __
     const float v[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
     uint32_t h[8], l[8];
 #pragma unroll
-    for (int x = 0; x < 8; ++x) split(v[x] * 128.f, h[x], l[x]);
+    for (int x = 0; x < 8; ++x) {
+      split(v[x] * 128.f, h[x], l[x]);
+      fits = fits && fabsf(v[x]) <= 256.f;
+      reach |= fabsf(v[x]) >= 0.0078125f ? 1u << x : 0u;
+    }
     const uint32_t off = (i / 8) * LBO + c * 128 + (i % 8) * 16;
     *reinterpret_cast<uint4*>(BH + off) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
     *reinterpret_cast<uint4*>(BL + off) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
   }
+#pragma unroll
+  for (int off = G; off < 32; off <<= 1) reach |= __shfl_xor_sync(0xffffffffu, reach, off);
+  if (lane < G) s_reach[warp][lane] = reach;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  if (tid < G) {
+    uint32_t all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) all |= s_reach[w][tid];
+    fits = fits && all == 0xffu;
+  }
+  const bool scaled = __syncthreads_and(fits);
   const uint32_t tmem = tmem_slot, bar_addr = tc::smem_u32(&bar);
   constexpr uint32_t idesc = tc::idesc_f16(128, D, false, true);
   const uint64_t ah = tc::smem_desc(tc::smem_u32(AH), 128, SBO), al = tc::smem_desc(tc::smem_u32(AL), 128, SBO);
@@ -375,6 +397,22 @@ __global__ void __launch_bounds__(256, 1) decompress_tc_kernel(const uint8_t* __
   bool ok = true;
   for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
     const int64_t base = (int64_t)tile * 128;
+    if (!scaled) {
+#pragma unroll 1
+      for (int r = tid / D; r < 128 && base + r < n_vec; r += 256 / D) {
+        const uint8_t* row = idx + (base + r) * (D * VB / 8);
+        float acc = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < G; ++c) {
+          const uint64_t w = load_fields8<VB>(row + c * VB);
+#pragma unroll
+          for (int x = 0; x < 8; ++x)
+            acc = fmaf(cen_s[(uint32_t)(w >> (x * VB)) & ((1u << VB) - 1)], __ldg(Pi + (8 * c + x) * D + tid % D), acc);
+        }
+        out[(base + r) * D + tid % D] = acc * fp16_value(vn[base + r]);
+      }
+      continue;
+    }
 #pragma unroll 4
     for (int e = tid; e < 128 * G; e += 256) {
       const int r = e % 8 + 8 * (e / (8 * G)), c = (e / 8) % G;
