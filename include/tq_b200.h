@@ -137,6 +137,9 @@ int tq_dequantize(const uint8_t* packed, int64_t n, int d, const float* centroid
  * its own kernels only.  Arguments as for tq_compress_keys / tq_compress_values / tq_attention_fwd:
  *   Pi_k, S_eff [d, d], centroids_k [2^(bits-1)], boundaries_k [2^(bits-1) - 1]   (key side)
  *   Pi_v [d, d], centroids_v [2^bits], boundaries_v [2^bits - 1]                  (value side)
+ * Matrices and codebooks may have any size within 2^20 either way (root mean square entries against those of a rotation
+ * and of a Gaussian sketch); nothing is assumed about their structure, but rotations with orthonormal rows and symmetric
+ * codebooks are what the kernels are fast for.
  * Replaces the constants the reference's compressors hold as attributes and re-read in every call
  * (compressors.py:42-70, :230-246) and the per-call table builds of kernels/attention.py:300-330. */
 size_t tq_constants_bytes(int d, int bits);

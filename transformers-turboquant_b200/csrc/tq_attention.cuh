@@ -16,11 +16,15 @@ struct ConstLayout {
   size_t pi_k, s_eff, pi_v, cen_k, bnd_k, cen_v, bnd_v;           // fp32 originals
   size_t w_cat_pair, w_unrot_pair, luts, w_cat_plain, w_unrot_plain;  // attention: bf16 operand images, fp16 pair tables
   size_t pik_hi, pik_lo, se_hi, se_lo, piv_hi, piv_lo;            // compression: split-bf16 K-major operand images
-  size_t pik16_hi, pik16_lo, se16_hi, se16_lo, piv16_hi, piv16_lo;  // ... and split-fp16 ones (Pi x kPi16Scale)
+  size_t pik16_hi, pik16_lo, se16_hi, se16_lo, piv16_hi, piv16_lo;  // ... and split-fp16 ones, scaled by powers of two
   size_t total;
 };
-// The fp16 images of the rotations hold Pi x 128: entries of about 0.1 would put the low parts into fp16's subnormals.
+// The fp16 images of a rotation hold Pi x 128 (entries of about 0.1 would put the low parts into fp16's subnormals); a matrix
+// whose rows do not have norm 1 is brought there by another power of two.  The scales of Pi_k and Pi_v and the inverse of
+// the first are floats at word kScaleWord of the header.  Rows of the sketch, of which only signs are read, are scaled
+// each to entries of about 1.
 constexpr float kPi16Scale = 128.f;
+constexpr int kScaleWord = 4;
 constexpr uint32_t kConstMagic = 0x31425154u;  // "TQB1"
 inline ConstLayout const_layout(int d) {
   ConstLayout L{};

@@ -125,17 +125,43 @@ struct ImageArgs {
   float* copy[3];
   __nv_bfloat16 *hi[3], *lo[3];
   __half *hi16[3], *lo16[3];
-  float scale16[3];
+  float* scales;  // of Pi_k and Pi_v, and the inverse of the first
 };
+// The power of two nearest the inverse of sqrt(mean square), 1 within a factor of sqrt(2); matrices beyond 2^20 either way
+// are scaled by 2^20.
+__device__ __forceinline__ int rms_exponent(double mean_square) {
+  if (!(mean_square > 0.0) || isinf(mean_square)) return 0;
+  const double e = rint(-0.5 * log2(mean_square));
+  return e < -20.0 ? -20 : e > 20.0 ? 20 : (int)e;
+}
 __global__ void build_split_images_kernel(const ImageArgs a, int d) {
+  __shared__ double s_part[4];
   const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
   const float v = a.src[m][j * d + i];
+  double ss = 0.0;  // of the whole rotation, or of this row of the sketch
+  if (m == 1) ss = (double)v * v;
+  else
+    for (int r = 0; r < d; ++r) {
+      const double w = a.src[m][r * d + i];
+      ss += w * w;
+    }
+  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  if (i % 32 == 0) s_part[i / 32] = ss;
+  __syncthreads();
+  ss = 0.0;
+  for (int w = 0; w < d / 32; ++w) ss += s_part[w];
+  const int e = rms_exponent(ss / d);  // (a rotation has d rows of norm 1, a row of the sketch d entries of size 1)
+  const float scale16 = ldexpf(m == 1 ? 1.f : kPi16Scale, e);
+  if (j == 0 && i == 0 && m != 1) {
+    a.scales[m / 2] = scale16;
+    if (m == 0) a.scales[2] = 1.f / scale16;
+  }
   const int at = operand_index(j, i, d, d);
   a.copy[m][j * d + i] = v;
   const __nv_bfloat16 h = __float2bfloat16_rn(v);
   a.hi[m][at] = h;
   a.lo[m][at] = __float2bfloat16_rn(v - __bfloat162float(h));
-  const float w = v * a.scale16[m];
+  const float w = v * scale16;
   const __half g = __float2half_rn(w);
   a.hi16[m][at] = g;
   a.lo16[m][at] = __float2half_rn(w - __half2float(g));
@@ -175,7 +201,7 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
                       {b16(L.pik_lo), b16(L.se_lo), b16(L.piv_lo)},
                       {h16(L.pik16_hi), h16(L.se16_hi), h16(L.piv16_hi)},
                       {h16(L.pik16_lo), h16(L.se16_lo), h16(L.piv16_lo)},
-                      {kPi16Scale, 1.f, kPi16Scale}};
+                      f32(L.header) + kScaleWord};
   build_split_images_kernel<<<dim3(d, 3), d, 0, stream>>>(img, d);
   const CodebookArgs cb{{cen_k, bnd_k, cen_v, bnd_v}, {f32(L.cen_k), f32(L.bnd_k), f32(L.cen_v), f32(L.bnd_v)},
                         {1 << kb, (1 << kb) - 1, 1 << vb, (1 << vb) - 1}, reinterpret_cast<uint32_t*>(c + L.header),

@@ -17,8 +17,8 @@
 //     MMA there, so it costs no shared memory and no proxy fence; its projection overwrites the rotated
 //     coordinates it came from.  The sign pass of tile i runs after the index pass of tile i+1, under which the
 //     sketch MMA of tile i has finished;
-//   * fp16 inputs are exact operands of fp16 MMAs against fp16 hi + lo images of the rotations (x 128, to keep the low
-//     parts out of the subnormals) and of the sketch: 22 mantissa bits, small products first.  Against fp64 as many
+//   * fp16 inputs are exact operands of fp16 MMAs against fp16 hi + lo images of the rotations (scaled to rows of norm
+//     128, to keep the low parts out of the subnormals) and of the sketch: 22 mantissa bits, small products first.  Against fp64 as many
 //     indices and signs differ as with the fp32 CUDA-core kernel (53 / 113 / 132 of 4e8 key indices, signs and value
 //     indices; fp32: 53 / 110 / 131), and with the repair below the same ones: 48 us instead of 171 us for the 6 x 8 x 777
 //     keys and values of a padded prompt;
@@ -317,7 +317,9 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   // Split of the residual for the sketch: fp16 hi + lo of the residual scaled by a power of two (22 mantissa bits), or
   // bf16 hi + lo (16 bits), which needs no scaling and two operations fewer per coordinate.
   constexpr bool SK16 = F16 || D == 64;
-  constexpr float kYScale = F16 ? kPi16Scale : 1.f;  // the rotated coordinates come out times this
+  // the rotated coordinates come out times these powers of two
+  const float* const scales = reinterpret_cast<const float*>(a.consts + a.L.header) + kScaleWord;
+  const float yscale_k = F16 ? __ldg(scales) : 1.f, yscale_v = F16 ? __ldg(scales + 1) : 1.f;
   constexpr int KB = BITS - 1, VB = BITS;
   constexpr uint32_t SBO = (kD / 8) * 128;  // canonical (unswizzled) K-major images of the constant operands
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -578,6 +580,12 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         tc::tmem_st1(col + e, y);
       }
     };
+    // size of a residual's coordinates, in units of the vector's norm: of a rotated coordinate or of a centroid
+    float r_size = F16 ? kPi16Scale : SK16 ? kPi16Scale * __ldg(scales + 2) : 1.f;
+    if constexpr (SK16) {
+#pragma unroll
+      for (int j = 0; j < (1 << KB); ++j) r_size = fmaxf(r_size, yscale_k * fabsf(cen_s[j]));
+    }
     float band_p = 0.f;  // of the previous key tile's projections
     int n_xch = 0;    // exchanges through `exch` so far in this quarter (phase of xch / xfree)
     // sum of the four parts' values of this row, in a fixed order; every part gets the same total
@@ -634,7 +642,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if (lane == 0) tc::mbar_arrive(x_read(s));
         float ss_tot;
         if (!(ok = exchange(ss, ss_tot))) break;
-        const float nv = sqrtf(ss_tot), den1 = nv + 1e-8f, den = kYScale * den1;
+        const float nv = sqrtf(ss_tot), den1 = nv + 1e-8f, den = (is_key ? yscale_k : yscale_v) * den1;
         if (!(ok = tc::mbar_wait_or_abort(y_done(s), u & 1, abort_flag))) break;
         tc::fence_after_sync();
         uint32_t raw[32];
@@ -644,7 +652,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         if constexpr (F16) {
           // any coordinate too close to a boundary to call?
           const bool sure = !live || !(ss_tot > 0.f) || !(den < 1e30f);
-          const float band = sure ? 0.f : kOpenIndex * den;
+          const float band = sure ? 0.f : kOpenIndex * kPi16Scale * den1;  // (the scaled rotation's rows have norm 128)
           auto settle_side = [&](auto nb, bool sym, const float* Pi, const float* src, const float (&bnd)[decltype(nb)::value]) {
             constexpr int NB = decltype(nb)::value;
             uint32_t open = 0;
@@ -678,10 +686,9 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           uint32_t packed[KB], rh[16], rl[16];
 #pragma unroll
           for (int j = 0; j < KB; ++j) packed[j] = 0;
-          const float neg_nv = -kYScale * nv;
-          // brings the residual's coordinates (at most about the norm) to at most about 64: a power of two
-          const float r_scale = __uint_as_float(
-              (uint32_t)max(127 + 6 - (F16 ? 7 : 0) + 127 - (int)(__float_as_uint(den1) >> 23), 1) << 23);
+          const float neg_nv = -yscale_k * nv;
+          // brings the residual's coordinates to at most about 64: a power of two
+          const float r_scale = __uint_as_float((uint32_t)max(127 + 6 + 127 - (int)(__float_as_uint(r_size * den1) >> 23), 1) << 23);
           auto index_pass = [&](auto sym, auto given) {
             constexpr bool GIVEN = decltype(given)::value;  // the indices are in `packed` already
             float bden[(1 << KB) - 1];
@@ -739,7 +746,7 @@ compress_kv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           }
           float rr_tot;
           if (!(ok = exchange(rr, rr_tot))) break;
-          if (live && part == 0) a.key_rn[no] = fp16_bits(sqrtf(rr_tot) * (1.f / kYScale));
+          if (live && part == 0) a.key_rn[no] = fp16_bits(sqrtf(rr_tot) * (F16 ? __ldg(scales + 2) : 1.f));
           const float next_band = F16 && live && den < 1e30f ? kOpenSign * sqrtf(rr_tot) * r_scale : 0.f;
           // the residual operand of the previous key tile must have been consumed by its sketch MMAs
           if (i >= 1 && !(ok = tc::mbar_wait_or_abort(p_done((i - 1) % kSlots), ((i - 1) / kSlots) & 1, abort_flag))) break;
