@@ -4,14 +4,9 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import device_compressors
+from helpers import device_compressors, scores64
 
 pytestmark = pytest.mark.gpu
-
-
-def _unpack(packed, b, d):
-    from turboquant_b200.kernels import unpack_bits
-    return unpack_bits(packed, b, d).long()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
@@ -24,16 +19,10 @@ def test_scores_of_few_rows(B, Hq, Hkv, Sq, Sk, d, bits, dtype):
     ck = kc.compress(torch.randn(B, Hkv, Sk, d, generator=g).cuda())
     q = torch.randn(B, Sq, Hq, d, generator=g).cuda().to(dtype).transpose(1, 2)
     got = kc.asymmetric_attention_scores(q, ck)
-    rows = lambda t: t.double().reshape(B, Hkv, Sk, -1).repeat_interleave(Hq // Hkv, dim=1)
-    cen = rows(kc.centroids[_unpack(ck["packed_key_indices"], bits - 1, d)])
-    sign = rows(2.0 * _unpack(ck["packed_qjl_signs"], 1, d) - 1.0)
-    rot = q.double() @ kc.Pi.double().T
-    sketch = rot @ kc.S_eff.double().T * ((torch.pi / 2) ** 0.5 / d)
-    want = (rot @ cen.transpose(2, 3)) * rows(ck["vec_norms"])[..., 0][:, :, None] \
-        + (sketch @ sign.transpose(2, 3)) * rows(ck["residual_norm"])[..., 0][:, :, None]
+    want = scores64(q, ck, kc)
     # A single score may cancel, so its error is held against the size of the terms it sums, |q| |k|: fp32 sums of
     # d + d + 2 d products, a few times 2^-24 sqrt(4 d).
-    size = q.double().norm(dim=-1)[..., None] * rows(ck["vec_norms"])[..., 0][:, :, None]
+    size = q.double().norm(dim=-1)[..., None] * ck["vec_norms"].double().repeat_interleave(Hq // Hkv, dim=1)[:, :, None]
     assert float(((got - want).abs() / size).max()) < 4 * 2.0 ** -24 * (4 * d) ** 0.5
 
 

@@ -3,22 +3,23 @@
 import pytest
 import torch
 
-from helpers import device_compressors, rel_err
+from helpers import device_compressors, rel_err, scores64, values64
 
 pytestmark = pytest.mark.gpu
 
 
 def _dense(q, ck, cv, kc, vc, mask, causal):
-    """softmax(scores / sqrt(d) + mask) @ decoded values in fp64; rows whose causal range is all hidden average it."""
+    """softmax(scores / sqrt(d) + mask) @ decoded values in fp64, from the packed bytes alone; rows whose causal range is all
+    hidden average it."""
     B, Hq, Sq, d = q.shape
     _, Hkv, Sk, _ = ck["shape"]
-    s = kc.asymmetric_attention_scores(q.float(), ck).double() / d ** 0.5
+    s = scores64(q, ck, kc) / d ** 0.5
     add = torch.where(mask, 0.0, -1e30).double()[:, None] if mask.dtype == torch.bool else mask.double()[:, None]
     s = torch.maximum(s + add, torch.tensor(-60000.0 * 0.6931471805599453, dtype=torch.float64, device=q.device))
     if causal:
         i = torch.arange(Sq, device=q.device)[:, None] + (Sk - Sq)
         s = s.masked_fill(torch.arange(Sk, device=q.device) > i, float("-inf"))
-    v = vc.decompress(cv).double().repeat_interleave(Hq // Hkv, dim=1)
+    v = values64(cv["packed_indices"], cv["vec_norms"].reshape(-1), vc).reshape(B, Hkv, Sk, d).repeat_interleave(Hq // Hkv, dim=1)
     return torch.softmax(s, -1) @ v
 
 
