@@ -67,3 +67,22 @@ def test_masks_against_a_dense_evaluation(d, Hq, Hkv, Sq, Sk, kind):
     # fp32 kernels read the same bits
     f32 = fused_attention(q.float(), ck, cv, kc, vc, attention_mask=mask[:, None], mode="fp32")
     assert rel_err(f32, want) < 1e-4
+
+
+@pytest.mark.parametrize("d,Sq,Sk", [(128, 3, 127), (128, 40, 128), (64, 70, 129), (128, 40, 132), (64, 300, 512), (128, 130, 515)])
+@pytest.mark.parametrize("pitch,first", [(0, 0), (4, 0), (4, 1), (3, 2)])  # elements added to a row, and before the first
+def test_additive_values_at_any_alignment(d, Sq, Sk, pitch, first):
+    """Masks of arbitrary values: with and without a summary (up to 128 keys they are read as they are), rows that can and
+    rows that cannot be loaded four columns at a time."""
+    from turboquant_b200 import compress_kv, fused_attention
+
+    g = torch.Generator().manual_seed(Sk + pitch)
+    kc, vc = device_compressors(d, 3)
+    k, v = (torch.randn(2, 2, Sk, d, generator=g).cuda().bfloat16() for _ in range(2))
+    q = torch.randn(2, 4, Sq, d, generator=g).cuda().bfloat16()
+    ck, cv = compress_kv(k, v, kc, vc)
+    row = Sk + pitch + (-Sk) % 4 * (pitch == 4)
+    mask = torch.randn(2 * Sq * row + 8, generator=g).cuda()[first:first + 2 * Sq * row].view(2, Sq, row)[:, :, :Sk]
+    want = _dense(q, ck, cv, kc, vc, mask, True)
+    assert rel_err(fused_attention(q, ck, cv, kc, vc, attention_mask=mask[:, None]), want) < 1e-2  # 16-bit operands and output
+    assert rel_err(fused_attention(q.float(), ck, cv, kc, vc, attention_mask=mask[:, None], mode="fp32"), want) < 1e-4

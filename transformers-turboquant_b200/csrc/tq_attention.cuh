@@ -88,9 +88,10 @@ int check_attention_args(const void* q, int dtype, int64_t B, int64_t Hq, int64_
                          int64_t ss, int64_t Hkv, int64_t Sk, int bits, int mode);
 
 // q_cat rows [q Pi^T | coeff (q Pi^T) S_eff^T] of few query rows (fp32 arithmetic; bf16 or fp32 result), any dtype and
-// strides of q; row n = (b * Hq + h) * Sq + s.
+// strides of q; row n = (b * Hq + h) * Sq + s.  `beside_previous`: the kernel launched last (a mask's summary) has nothing
+// that this one reads, they may run side by side; this one does not finish before that one has.
 int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh, int64_t ss,
-               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream);
+               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream, bool beside_previous = false);
 
 // fp32 mode: query preparation + CUDA-core flash kernel.  `workspace` holds q_cat fp32.
 int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,

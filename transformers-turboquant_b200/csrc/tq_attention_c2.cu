@@ -300,6 +300,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     }
   }
   if (warp == kCtlWarp) tc::tmem_alloc2(tc::smem_u32(&tmem_slot), L::kCols);
+  if (MASK) grid_dependency_wait();  // everything up to here ran under the mask's summary
   // Maps of the masked key tiles, by the producer warps (32 tiles each at a time).  Rows without a visible key
   // average all keys of their causal range: a cluster that has one computes every tile.
   const bool mapped = MASK && a.mb.words != nullptr && n_tiles_live <= 32 * kMapWords;
@@ -438,6 +439,7 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
     }
     float m_run = -INFINITY, l_run = 0.f;
     const float cexp = a.sm_scale * kLog2e, rcexp = 1.f / cexp;  // K_hat carries the key norms: S is the raw score
+    const bool mask_by_4 = MASK && ((reinterpret_cast<uintptr_t>(a.mask) | (uintptr_t)(4 * a.mask_stride_b) | (uintptr_t)(4 * a.mask_stride_q)) & 15u) == 0;
     int kt = next_tile(-1);
     for (int j = 0; j < n_tiles && ok; ++j, kt = next_tile(kt)) {
       const int bb = j & 1, u = j >> 1, k0 = kt * kBN;
@@ -484,10 +486,26 @@ attention_c2_kernel(const AttnArgs a, const PairArgs x, const int pair_heads) {
         const float floor_raw = -60000.f * rcexp;
         if (MASK && other && qi < a.Sq) {
           const float* mrow = a.mask + b * a.mask_stride_b + (int64_t)qi * a.mask_stride_q + kc0;
+          // A thread's loads lie in a row of their own, so each costs the warp 32 sectors: four columns per load where the
+          // rows allow it, sixteen columns in flight (2 x 1000 tokens of 32 heads under a mask of arbitrary values: 126 us,
+          // 157 with one load per column and no summary in front, 171 with it).
           const float m_unit = kLog2e * rcexp;
 #pragma unroll
-          for (int c = 0; c < HC; ++c)
-            if (c <= vsk) t[c] = fmaxf(fmaf(mrow[c], m_unit, t[c]), floor_raw);
+          for (int c0 = 0; c0 < HC; c0 += 16) {
+            float mv[16];
+            if (mask_by_4 && c0 + 15 <= vsk) {
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                const float4 m4 = __ldg(reinterpret_cast<const float4*>(mrow + c0 + i));
+                mv[i] = m4.x; mv[i + 1] = m4.y; mv[i + 2] = m4.z; mv[i + 3] = m4.w;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) mv[i] = c0 + i <= vsk ? __ldg(mrow + c0 + i) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) t[c0 + i] = fmaxf(fmaf(mv[i], m_unit, t[c0 + i]), floor_raw);
+          }
         } else if (MASK && hidden) {
           // a hidden key's score is the floor, as the clamp above leaves it
 #pragma unroll
@@ -985,9 +1003,13 @@ int launch_c2(const AttnArgs& a, const PairArgs& x, int64_t B, cudaStream_t stre
             (unsigned)(pair_heads ? a.Hq / 2 : a.Hq), (unsigned)B);
   {
     ProfScope prof(kProfAttention, stream);
-    kern<<<grid, kThreads, smem, stream>>>(a, x, pair_heads);
+    if (a.mb.words != nullptr) {
+      TQ_CUDA_OK(launch_dependent(kern, grid, dim3(kThreads), smem, stream, a, x, pair_heads));
+    } else {
+      kern<<<grid, kThreads, smem, stream>>>(a, x, pair_heads);
+      TQ_CUDA_OK(cudaGetLastError());
+    }
   }
-  TQ_CUDA_OK(cudaGetLastError());
   return SPLIT ? merge_split_tiles(a, B, D, x.nsplit, x.part_o, x.part_ml, stream) : TQ_OK;
 }
 template <int D, int BITS>

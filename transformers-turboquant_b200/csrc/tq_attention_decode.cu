@@ -83,11 +83,6 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// Programmatic dependent launch: `wait` returns when the grid this one depends on has completed and its writes
-// are visible (at once when the kernel was launched without the attribute); `launch_dependents` lets the next
-// kernel of the stream start early, up to its own `wait`.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // 8x8 transpose of 16-bit elements across the warp: lane (g, t) gives row g, columns 2 t, 2 t + 1 and receives
 // column g, rows 2 t, 2 t + 1
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
@@ -270,6 +265,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) decode_kernel(const DecodeArgs
     // summary's 128-key tiles, unless some row has no visible key (it then averages all its keys).  At most 16 query
     // rows: one row group.  (Decode-sized calls over left-padded batches: a quarter of the keys and more.)
     if (a.mb.words != nullptr && k_lo < k_hi) {
+      grid_dependency_wait();  // the summary may be as young as the query rows
       const int64_t mbat = a.mb.batch ? b : 0;
       uint32_t rows_seen = 0;
       for (int c = lane; c < a.mb.NC; c += 32) rows_seen |= a.mb.rows[mbat * a.mb.NC + c];
@@ -732,29 +728,12 @@ static int resident_ctas(int bits, int nt) {
   return cached[bits][nt];
 }
 
-// Launch a kernel that may start before the previous kernel of the stream has finished (programmatic dependent
-// launch); the kernel itself waits (grid_dependency_wait) before it touches that kernel's results.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
-
 int finish_splits(const AttnArgs& a, int64_t B, int d, int rows, int nsplit, const float* part_o, const float* part_ml,
                   cudaStream_t stream) {
   TQ_REQUIRE(nsplit <= kMaxExtraUnits && B * a.Hkv <= 65535, "too many splits or KV heads");
   ProfScope prof(kProfBackRotation, stream);
   TQ_CUDA_OK(launch_dependent(d == 128 ? decode_finish_kernel<128> : decode_finish_kernel<64>,
-                              dim3((unsigned)rows, (unsigned)(B * a.Hkv)), dim3(4 * d), stream, part_o, part_ml, nsplit, a.Hq,
+                              dim3((unsigned)rows, (unsigned)(B * a.Hkv)), dim3(4 * d), 0, stream, part_o, part_ml, nsplit, a.Hq,
                               a.Hkv, a.Sq, a.Pi_v, a.out, a.out_dtype, a.o_stride_b, a.o_stride_h, a.o_stride_s));
   return TQ_OK;
 }
@@ -764,7 +743,8 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
   const int64_t units = B * a.Hkv;
   const int R = (int)((a.Hq / a.Hkv) * a.Sq);
   // spread over all SMs: 8 x 32 rows take 5 us (8 us with a CTA per KV head)
-  if (int st = qprep_rows(q, q_dtype, B * a.Hq * a.Sq, a.Hq, a.Sq, 128, sb, sh, ss, Pi_k, S_eff, q_cat, true, stream)) return st;
+  if (int st = qprep_rows(q, q_dtype, B * a.Hq * a.Sq, a.Hq, a.Sq, 128, sb, sh, ss, Pi_k, S_eff, q_cat, true, stream, a.mb.words != nullptr))
+    return st;
   // One wave of CTAs, each with at least 64 keys (one 16-key block per warp).  The SMs run their resident
   // CTAs side by side and finish with the fullest one, so among the split counts that fit, take the one that
   // fills the SMs most evenly (the largest such count: more warps per SM hide more latency).
@@ -787,12 +767,14 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
   }
   if (a.mb.words != nullptr) {
     // Under a summarised mask the splits' live ranges differ (padding), so that equal shares of the keys are not equal
-    // work: up to four waves of smaller splits, which the SMs take as they become free, of at least 256 keys each.
-    // Append and attend of batch 16 x 32 KV heads x 4000 keys, half to all of them live: 253 us reading the additive
-    // mask in one wave, 201 us (159 us now) with the summary, the trimmed ranges and these splits.
+    // work: up to four waves of smaller splits, which the SMs take as they become free, of at least 256 keys each, and of
+    // 128 for every query row whose partial results a split writes (16 rows x 8 x 32 KV heads x 4000 keys that are all live:
+    // 337 us in nine splits, 269 in two).  Append and attend of batch 16 x 32 KV heads x 4000 keys, half to all of them
+    // live: 253 us reading an additive mask in one wave, 159 us with the summary, the trimmed ranges and these splits.
+    const int64_t least = 128 * R > 256 ? 128 * R : 256;
     const int64_t most = (kMaxExtraUnits + B * a.Hq) * kRows / R / units;  // what the partial-result workspace holds
     int64_t n = (4 * slots + units - 1) / units;
-    n = n < (a.Sk + 255) / 256 ? n : (a.Sk + 255) / 256;
+    n = n < (a.Sk + least - 1) / least ? n : (a.Sk + least - 1) / least;
     n = n < kMaxExtraUnits ? n : kMaxExtraUnits;
     n = n < most ? n : most;
     if (n > nsplit) nsplit = (int)n;
@@ -816,7 +798,7 @@ int attention_decode(const AttnArgs& a, int64_t B, int bits, const void* q, int 
     else
       kern = nt == 1 ? (bits == 2 ? decode_kernel<2, 1, true> : bits == 3 ? decode_kernel<3, 1, true> : decode_kernel<4, 1, true>)
                      : (bits == 2 ? decode_kernel<2, 2, true> : bits == 3 ? decode_kernel<3, 2, true> : decode_kernel<4, 2, true>);
-    TQ_CUDA_OK(launch_dependent(kern, grid, dim3(kWarps * 32), stream, da));
+    TQ_CUDA_OK(launch_dependent(kern, grid, dim3(kWarps * 32), 0, stream, da));
   }
   return finish_splits(a, B, 128, R, nsplit, part_o, part_ml, stream);
 }

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(8 * D) qprep_rows_kernel(const void* __restric
                                                            float coeff, void* __restrict__ q_cat, int rows_per_cta) {
   constexpr int NV = D / 32;  // float4s of a matrix row per thread: columns 4 part + 32 i .. + 3
   __shared__ __align__(16) float x[kFewRows][D], y[kFewRows][D];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the split-KV kernel may start its own set-up
+  grid_launch_dependents();  // the split-KV kernel may start its own set-up
   const int tid = threadIdx.x, j = tid / 8, part = tid % 8;
   float4 w1[NV], w2[NV];
 #pragma unroll
@@ -168,10 +168,11 @@ __global__ void __launch_bounds__(8 * D) qprep_rows_kernel(const void* __restric
     const float v = project(y, w2, r);
     if (part == 0) put(r, D + j, coeff * v);
   }
+  grid_dependency_wait();  // whoever waits for this kernel waits for the one beside it too
 }
 
 int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh, int64_t ss,
-               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream) {
+               const float* Pi, const float* S_eff, void* q_cat, bool bf16_out, cudaStream_t stream, bool beside_previous) {
   const int64_t sms = sm_count();
   const int64_t even = (n_q + sms - 1) / sms;  // one wave of CTAs, while they hold that many rows
   const int per = (int)(even < kFewRows ? even : kFewRows);
@@ -180,8 +181,12 @@ int qprep_rows(const void* q, int dtype, int64_t n_q, int64_t Hq, int64_t Sq, in
   auto kern = d == 128 ? (bf16_out ? qprep_rows_kernel<128, true> : qprep_rows_kernel<128, false>)
                        : (bf16_out ? qprep_rows_kernel<64, true> : qprep_rows_kernel<64, false>);
   ProfScope prof(kProfPrepareQueries, stream);
-  kern<<<grid, 8 * d, 0, stream>>>(q, dtype, n_q, Hq, Sq, sb, sh, ss, Pi, S_eff, coeff, q_cat, per);
-  TQ_CUDA_OK(cudaGetLastError());
+  if (beside_previous) {
+    TQ_CUDA_OK(launch_dependent(kern, dim3(grid), dim3(8 * d), 0, stream, q, dtype, n_q, Hq, Sq, sb, sh, ss, Pi, S_eff, coeff, q_cat, per));
+  } else {
+    kern<<<grid, 8 * d, 0, stream>>>(q, dtype, n_q, Hq, Sq, sb, sh, ss, Pi, S_eff, coeff, q_cat, per);
+    TQ_CUDA_OK(cudaGetLastError());
+  }
   return TQ_OK;
 }
 // ---- tile decode helpers -------------------------------------------------------------
@@ -1086,8 +1091,16 @@ extern "C" int tq_attention_fwd_masked(const void* q, int dtype, int64_t B, int6
              "a mask of kind %d (or NULL) is not one the library knows", mask_kind);
   TQ_REQUIRE(mask_batches == 1 || mask_batches == B, "%lld masks for a batch of %lld", (long long)mask_batches, (long long)B);
   TQ_REQUIRE(mask_kind == TQ_MASK_BOOL || (reinterpret_cast<uintptr_t>(mask) & 3u) == 0, "an additive mask must be 4-byte aligned");
-  const MaskSource src{mask, mask_kind == TQ_MASK_BOOL, mask_batches, mask_stride_b, mask_stride_q};
   const float* dummy = reinterpret_cast<const float*>(constants);  // replaced from the buffer inside
+  // An additive mask is read as it is where its summary has no reader (fp32 mode) or nothing to skip (one tile of keys:
+  // 12 x 20 x 20 tokens take 13 us that way and 19 us with the summary in front).
+  if (mask_kind == TQ_MASK_ADDITIVE && (mode == TQ_MODE_FP32 || Sk <= 128))
+    return attention_entry(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Hkv, Sk, kv_capacity, key_idx,
+                           key_signs, key_vec_norms, key_residual_norms, val_idx, val_vec_norms, dummy, dummy, dummy,
+                           dummy, dummy, bits, sm_scale, causal, static_cast<const float*>(mask),
+                           mask_batches > 1 ? mask_stride_b : 0, mask_stride_q, out, o_stride_b, o_stride_h, o_stride_s,
+                           workspace, workspace_bytes, mode, stream, static_cast<const uint8_t*>(constants));
+  const MaskSource src{mask, mask_kind == TQ_MASK_BOOL, mask_batches, mask_stride_b, mask_stride_q};
   return attention_entry(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Hkv, Sk, kv_capacity, key_idx,
                          key_signs, key_vec_norms, key_residual_norms, val_idx, val_vec_norms, dummy, dummy, dummy,
                          dummy, dummy, bits, sm_scale, causal, nullptr, 0, 0, out, o_stride_b, o_stride_h, o_stride_s,

@@ -176,4 +176,26 @@ __device__ __forceinline__ uint64_t load_fields8(const uint8_t* src) {
   return word;
 }
 
+// Programmatic dependent launch.  `wait` returns when the kernel that this one was launched behind has finished and its writes
+// are visible (at once when the kernel was launched without the attribute); `launch_dependents` lets the next
+// kernel of the stream start.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launch a kernel that may start before the previous kernel of the stream has finished; the kernel itself waits
+// (grid_dependency_wait) before it touches that kernel's results.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 }  // namespace tq

@@ -15,7 +15,9 @@
 // kernels that made the mask additive (12 us) became this one, and the attention kernel no longer waits for 64 scattered
 // loads per thread and tile.
 //
-// Bound by the mask's bytes: one warp per row, 128 keys (four per lane) per step.
+// Bound by the mask's bytes, or for the few rows of a generation step by the latency of one load: one warp per row, several
+// where a group has fewer rows than warps, 128 keys (four per lane) per step, four steps in flight.  The kernels that read
+// the summary start their own set-up under it (programmatic dependent launch).
 #include "tq_attention.cuh"
 #include "tq_common.cuh"
 
@@ -28,6 +30,7 @@ struct MaskArgs {
   const void* mask;
   int64_t stride_b, stride_q;  // elements
   int Sq, Sk, shift, causal;
+  int warps_per_row;  // a power of two
   uint32_t* words;
   uint8_t* tiles;
   uint32_t* rows;
@@ -42,17 +45,18 @@ __global__ void __launch_bounds__(kGroupRows * 32) mask_summary_kernel(const Mas
   const int64_t b = blockIdx.z;
   const int group = blockIdx.y, chunk = blockIdx.x;
   const int t0 = chunk * kChunkTiles, t1 = min(a.T, t0 + kChunkTiles);
+  grid_launch_dependents();
   if (tid < kChunkTiles) s_cls[tid] = 0;
   if (tid == 0) s_rows = 0;
   __syncthreads();
-  const int s = group * kGroupRows + warp;
+  const int row = warp / a.warps_per_row, s = group * kGroupRows + row;
   if (s < a.Sq) {
     const int last = a.causal ? min(a.Sk - 1, s + a.shift) : a.Sk - 1;  // last key of the row's causal range
     const int64_t row_off = b * a.stride_b + (int64_t)s * a.stride_q;
     bool any_row = false;
     // kAhead tiles' loads in flight: a row is a chain of latencies otherwise (4000 keys: 23 us)
     constexpr int kAhead = 4;
-    for (int ta = t0; ta < t1; ta += kAhead) {
+    for (int ta = t0 + warp % a.warps_per_row * kAhead; ta < t1; ta += a.warps_per_row * kAhead) {
     uint32_t raw[kAhead][BOOL ? 2 : 4];
 #pragma unroll
     for (int x = 0; x < kAhead; ++x) {
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(kGroupRows * 32) mask_summary_kernel(const Mas
       if (lane == 0 && all != 0u) atomicOr(&s_cls[t - t0], all);
     }
     }
-    if (__any_sync(0xffffffffu, any_row) && lane == 0) atomicOr(&s_rows, 1u << warp);
+    if (__any_sync(0xffffffffu, any_row) && lane == 0) atomicOr(&s_rows, 1u << row);
   }
   __syncthreads();
   if (t0 + tid < t1) a.tiles[(b * a.NG + group) * (int64_t)a.T + t0 + tid] = (uint8_t)s_cls[tid];
@@ -140,7 +144,9 @@ MaskBits mask_bits_layout(int64_t nb, int64_t Sq, int64_t Sk, void* base, size_t
 int summarize_mask(const void* mask, bool boolean, int64_t nb, int64_t stride_b, int64_t stride_q, int64_t Sq, int64_t Sk,
                    int causal, const MaskBits& m, cudaStream_t stream) {
   TQ_REQUIRE(nb <= 65535 && m.NG <= 65535, "mask of %lld x %lld rows is too large", (long long)nb, (long long)Sq);
-  const MaskArgs a{mask, nb > 1 ? stride_b : 0, stride_q, (int)Sq, (int)Sk, (int)(Sk - Sq), causal,
+  int per_row = 1;
+  while (2 * per_row * Sq <= kGroupRows) per_row *= 2;
+  const MaskArgs a{mask, nb > 1 ? stride_b : 0, stride_q, (int)Sq, (int)Sk, (int)(Sk - Sq), causal, per_row,
                    const_cast<uint32_t*>(m.words), const_cast<uint8_t*>(m.tiles), const_cast<uint32_t*>(m.rows),
                    m.T, m.NG, m.NC};
   const dim3 grid((unsigned)m.NC, (unsigned)m.NG, (unsigned)nb);
