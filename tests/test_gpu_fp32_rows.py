@@ -32,3 +32,18 @@ def test_few_rows_in_fp32(B, Hq, Hkv, Sq, Sk, d, bits, mask):
     if mask is not None:
         add = torch.zeros(m.shape, device="cuda").masked_fill_(~m, torch.finfo(torch.float32).min)
         assert rel_err(cache.attend(q, attention_mask=add[:, None]), want) < 2e-5
+
+
+@pytest.mark.parametrize("d,B,Hq,Hkv,Sq,Sk", [(128, 8, 32, 32, 8, 64), (128, 8, 32, 32, 12, 64), (128, 32, 32, 32, 16, 65), (64, 32, 12, 12, 16, 64),
+                                              (64, 32, 12, 12, 8, 70)])
+def test_many_rows_over_few_keys(d, B, Hq, Hkv, Sq, Sk):
+    """Both sides of the line between the few-rows and the tile kernel where the heads fill the chip."""
+    from turboquant_b200 import compress_kv, fused_attention
+
+    g = torch.Generator().manual_seed(Sq + Sk)
+    kc, vc = device_compressors(d, 3)
+    k, v = (torch.randn(B, Hkv, Sk, d, generator=g).cuda() for _ in range(2))
+    q = torch.randn(B, Hq, Sq, d, generator=g).cuda()
+    ck, cv = compress_kv(k, v, kc, vc)
+    m = torch.ones(B, Sq, Sk, dtype=torch.bool, device="cuda")
+    assert rel_err(fused_attention(q, ck, cv, kc, vc), _dense(q, ck, cv, kc, vc, m, True)) < 2e-5  # as above

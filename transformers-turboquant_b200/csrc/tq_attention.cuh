@@ -126,7 +126,7 @@ int finish_splits(const AttnArgs& a, int64_t B, int d, int rows, int nsplit, con
 
 // fp32 mode, at most 16 query rows per KV head (tq_attention_rows.cu): a.q_cat holds the fp32 query rows, `part_ws`
 // attention_rows_workspace bytes.
-bool attention_rows_applies(int64_t Hq, int64_t Sq, int64_t Hkv);
+bool attention_rows_applies(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
 size_t attention_rows_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
 int attention_rows(const AttnArgs& a, int64_t B, int d, int bits, void* part_ws, cudaStream_t stream);
 

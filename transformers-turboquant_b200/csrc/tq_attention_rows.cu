@@ -258,7 +258,21 @@ RowsPlan rows_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
 
 }  // namespace
 
-bool attention_rows_applies(int64_t Hq, int64_t Sq, int64_t Hkv) { return Hkv > 0 && Hq / Hkv * Sq <= 16; }
+// Behind many query heads that fill the chip, short key ranges are left to the tile kernel: the finishing kernel reads Pi_v
+// once for every query row, the tile kernel rotates 64 rows back at a time.  Costs in us on 148 SMs, measured at head_dim
+// 128 / 64: this path 15 + 0.0215 / 0.008 per query row + 1.75e-4 / 1.1e-4 per key and chunk of rows, the tile kernel
+// 30 / 25 + 0.1 / 0.05 per query head and for each of its tiles of 64 keys.  32 x 32 heads of 16 rows, 64 keys: 370 us here
+// and 234 there; 500 keys: 697 and 957; 8 rows, 64 keys: 198 and 234.
+bool attention_rows_applies(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
+  if (Hkv <= 0 || Hq / Hkv * Sq > 16) return false;
+  if (B * Hq < sm_count()) return true;
+  const RowsPlan p = rows_plan(B, Hq, Sq, Hkv, Sk);
+  const bool wide = d == 128;
+  const double heads = (double)(B * Hq), chunk_keys = (double)(B * Hkv * p.chunks) * (double)Sk;
+  const double here = 15.0 + heads * (double)Sq * (wide ? 0.0215 : 0.008) + chunk_keys * (wide ? 1.75e-4 : 1.1e-4);
+  const double there = (wide ? 30.0 : 25.0) + heads * (double)((Sk + 63) / 64 + 1) * (wide ? 0.1 : 0.05);
+  return here <= there;
+}
 
 size_t attention_rows_workspace(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
   const RowsPlan p = rows_plan(B, Hq, Sq, Hkv, Sk);

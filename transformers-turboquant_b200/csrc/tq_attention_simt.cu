@@ -16,6 +16,7 @@ namespace tq {
 
 constexpr int kRows = 64;  // query rows and keys per tile
 inline size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
+constexpr int kTileThreads = 256;  // of the score and attention tile kernels
 constexpr int kFewRows = 16;  // query rows per CTA of the few-rows preparation
 
 __device__ __forceinline__ void store8(void* base, int dtype, int64_t off, const float (&v)[8]) {
@@ -203,15 +204,24 @@ template <int D, int IB>
 __device__ __forceinline__ void decode_key_tile(const uint8_t* __restrict__ idx, const uint8_t* __restrict__ sgn,
                                                 const uint16_t* __restrict__ vn, const uint16_t* __restrict__ rn,
                                                 int64_t head_base, int k0, int Sk, const float* __restrict__ cen,
-                                                float* Ks, float* kn, float* krn, int tid, int nthreads) {
-  constexpr int KS = 2 * D + 4, G = D / 8;
-  for (int e = tid; e < kRows * G; e += nthreads) {
-    const int j = e / G, g = e % G;
+                                                float* Ks, float* kn, float* krn, int tid) {
+  constexpr int KS = 2 * D + 4, G = D / 8, N = kRows * G / kTileThreads;
+  uint64_t words[N];  // all packed words of this thread are in flight together
+  uint32_t signs[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int e = tid + i * kTileThreads, j = e / G, g = e % G;
+    const int64_t n = head_base + min(k0 + j, Sk - 1);
+    words[i] = load_fields8<IB>(idx + n * (D * IB / 8) + g * IB);
+    signs[i] = sgn[n * G + g];
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int e = tid + i * kTileThreads, j = e / G, g = e % G;
     float* dst = Ks + j * KS + g * 8;
     if (k0 + j < Sk) {
-      const int64_t n = head_base + k0 + j;
-      const uint64_t w = load_fields8<IB>(idx + n * (D * IB / 8) + g * IB);
-      const unsigned sb = sgn[n * G + g];
+      const uint64_t w = words[i];
+      const uint32_t sb = signs[i];
       float v[8], sg[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -226,7 +236,7 @@ __device__ __forceinline__ void decode_key_tile(const uint8_t* __restrict__ idx,
       put8(dst + D, zero);
     }
   }
-  for (int j = tid; j < kRows; j += nthreads) {
+  for (int j = tid; j < kRows; j += kTileThreads) {
     const bool ok = k0 + j < Sk;
     kn[j] = ok ? fp16_value(vn[head_base + k0 + j]) : 0.f;
     krn[j] = ok ? fp16_value(rn[head_base + k0 + j]) : 0.f;
@@ -322,7 +332,7 @@ __global__ void __launch_bounds__(256) scores_simt_kernel(const ScoreArgs a) {
   __syncthreads();
   load_q_tile<D>(a.q_cat, bh * a.Sq, q0, (int)a.Sq, Qs, tid, 256);
   decode_key_tile<D, IB>(a.key_idx, a.key_sgn, a.key_vn, a.key_rn, (b * a.Hkv + hk) * a.Sk, k0, (int)a.Sk,
-                         cen, Ks, kn, krn, tid, 256);
+                         cen, Ks, kn, krn, tid);
   __syncthreads();
   float s[4][4];
   score_tile<D>(Qs, Ks, kn, krn, row0, tx, s);
@@ -459,14 +469,24 @@ __global__ void __launch_bounds__(256) attention_simt_kernel(const AttnArgs a, c
   for (int k0 = k_begin; k0 < k_end; k0 += kRows) {
     __syncthreads();  // previous tile fully consumed
     decode_key_tile<D, KB>(a.key_idx, a.key_sgn, a.key_vn, a.key_rn, kv_base, k0, (int)a.Sk, cen_k, Ks, kn,
-                           krn, tid, 256);
-    for (int e = tid; e < kRows * G; e += 256) {
-      const int j = e / G, g = e % G;
+                           krn, tid);
+    constexpr int NI = kRows * G / kTileThreads;
+    uint64_t words[NI];
+    float norms[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int e = tid + i * kTileThreads;
+      const int64_t n = kv_base + min(k0 + e / G, (int)a.Sk - 1);
+      words[i] = load_fields8<VB>(a.val_idx + n * (D * VB / 8) + e % G * VB);
+      norms[i] = fp16_value(a.val_vn[n]);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int e = tid + i * kTileThreads, j = e / G, g = e % G;
       float* dst = Vs + j * VS + g * 8;
       if (k0 + j < a.Sk) {
-        const int64_t n = kv_base + k0 + j;
-        const uint64_t w = load_fields8<VB>(a.val_idx + n * (D * VB / 8) + g * VB);
-        const float nv = fp16_value(a.val_vn[n]);
+        const uint64_t w = words[i];
+        const float nv = norms[i];
         float v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] = nv * cen_v[(w >> (c * VB)) & ((1u << VB) - 1)];
@@ -882,7 +902,7 @@ int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
     // few query rows have a kernel of their own, which reads the packed rows as words
     const uintptr_t words = reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) |
                             reinterpret_cast<uintptr_t>(a.val_idx);
-    if (attention_rows_applies(Hq, Sq, a.Hkv) && (words & 3u) == 0 && B <= 65535 && B * a.Hkv <= 65535 / 4)
+    if (attention_rows_applies(B, Hq, Sq, a.Hkv, a.Sk, d) && (words & 3u) == 0 && B <= 65535 && B * a.Hkv <= 65535 / 4)
       return attention_rows(a, B, d, bits, part, stream);
     x = split_plan(B, Hq, Sq, a.Sk, d);
     x.part_o = reinterpret_cast<float*>(part);
@@ -1037,7 +1057,7 @@ extern "C" size_t tq_attention_prepared_workspace_bytes(int64_t B, int64_t Hq, i
     const size_t q_cat = round256((size_t)B * Hq * Sq * 2 * d * 4);
     if (Sk <= 0) return q_cat;
     const size_t tiles = split_bytes(split_plan(B, Hq, Sq, Sk, d), B, Hq, Sq, d);
-    const size_t rows = attention_rows_applies(Hq, Sq, Hkv) ? attention_rows_workspace(B, Hq, Sq, Hkv, Sk, d) : 0;
+    const size_t rows = attention_rows_applies(B, Hq, Sq, Hkv, Sk, d) ? attention_rows_workspace(B, Hq, Sq, Hkv, Sk, d) : 0;
     return q_cat + (rows > tiles ? rows : tiles);
   }
   return workspace_bytes_bf16_prepared(B, Hq, Sq, Hkv, Sk, kv_capacity, d);
