@@ -104,8 +104,9 @@ int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
 int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
                        cudaStream_t stream, const uint8_t* prepared = nullptr);
-// scratch bytes of a bf16-mode call, by the kernel that will serve it (0 when the SM-pair kernel runs from a
-// prepared constants buffer)
+// Whether the SM-pair kernel serves a bf16-mode call (its only scratch are the partial results of a split call).
+bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride, int d);
+// scratch bytes of a bf16-mode call with a prepared constants buffer, by the kernel that will serve it
 size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                      int d);
 

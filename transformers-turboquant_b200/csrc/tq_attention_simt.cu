@@ -990,13 +990,11 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   // fp32 mode) is served unsplit.
   bool split = prepared != nullptr;
   if (split && src == nullptr && (workspace == nullptr || workspace_bytes < need)) {
-    const bool rows16 = d == 128 && (Hq / Hkv) * Sq <= 16;
     if (mode == TQ_MODE_FP32) {
       need = round256((size_t)B * Hq * Sq * 2 * d * 4);
       split = false;
-    } else if (!rows16 && need == attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk))) {
+    } else if (attention_bf16_on_sm_pairs(Hq, Sq, Hkv, Sk, kv_stride, d)) {  // (partial results are all it has scratch for)
       need = 0;
-      split = false;
       workspace = nullptr;
     }
   }

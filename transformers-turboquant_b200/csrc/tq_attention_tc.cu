@@ -958,6 +958,12 @@ static Bf16Path bf16_path(const AttnArgs& a, int64_t Sq, int d) {
   return ((d == 128 || d == 64) && use_sm_pairs()) ? Bf16Path::kPairs : Bf16Path::kSingle;
 }
 
+bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride, int d) {
+  AttnArgs a{};
+  a.Hq = Hq; a.Sq = Sq; a.Hkv = Hkv; a.Sk = Sk; a.kv_stride = kv_stride;
+  return bf16_path(a, Sq, d) == Bf16Path::kPairs;
+}
+
 size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                      int d) {
   AttnArgs a{};
