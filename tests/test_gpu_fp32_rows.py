@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from helpers import device_compressors, rel_err
+from helpers import contiguous_prefix, device_compressors, rel_err
 from test_gpu_masks import _dense, _mask
 
 pytestmark = pytest.mark.gpu
@@ -23,7 +23,7 @@ def test_few_rows_in_fp32(B, Hq, Hkv, Sq, Sk, d, bits, mask):
     q = torch.randn(B, Sq, Hq, d, generator=g).cuda().transpose(1, 2)
     cache = CompressedKVCache(kc, vc, B, Hkv, Sk + 13)
     cache.append(k, v)
-    ck, cv = cache._contiguous_prefix()
+    ck, cv = contiguous_prefix(cache)
     m = torch.ones(B, Sq, Sk, dtype=torch.bool) if mask is None else _mask(mask, B, Sq, Sk, g)
     m = m.cuda()
     want = _dense(q, ck, cv, kc, vc, m, True)

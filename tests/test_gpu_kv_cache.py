@@ -5,7 +5,7 @@ src/transformers_turboquant/patch.py:80-81, families/llama.py:100-114)."""
 import pytest
 import torch
 
-from helpers import (device_compressors, oracle_attention_from_packed, oracle_key_dict_to_device, oracle_params,
+from helpers import (contiguous_prefix, device_compressors, oracle_attention_from_packed, oracle_key_dict_to_device, oracle_params,
                      oracle_value_dict_to_device, rel_err)
 from oracle import tq_oracle as orc
 
@@ -28,7 +28,7 @@ def test_generation_loop_matches_recompression(bits):
     q = _tokens(B, Hq, prefill + steps, d, 3).cuda()
     cache = CompressedKVCache(kc, vc, B, Hkv, cap)
     cache.append(k[:, :, :prefill], v[:, :, :prefill])
-    # prefill-sized queries over the cache take the gather path
+    # prefill-sized queries over the cache
     want = fused_attention(q[:, :, :prefill], kc.compress(k[:, :, :prefill]), vc.compress(v[:, :, :prefill]), kc, vc)
     assert torch.equal(cache.attend(q[:, :, :prefill]), want)
     for t in range(prefill, prefill + steps):
@@ -120,10 +120,9 @@ def test_fully_masked_row_averages_uniformly():
 
 
 @pytest.mark.parametrize("d", [64, 128])
-def test_single_token_cache_through_the_gather_path(d):
-    """One token per head in a cache with room for more: the prefix gathered for the prefill kernels must be a
-    dense copy (for a single token `reshape` alone returns a view whose rows are a whole capacity apart).  fp32
-    queries take the gather path at both head dimensions."""
+def test_single_token_cache_read_in_place(d):
+    """One token per head in a cache with room for more: rows a whole capacity apart, as the kernels of either mode read them
+    in place, against the same token in dense arrays."""
     from turboquant_b200 import CompressedKVCache, compress_kv, fused_attention
     bits, B, Hq, Hkv = 3, 3, 4, 2
     kc, vc = device_compressors(d, bits)
@@ -135,8 +134,7 @@ def test_single_token_cache_through_the_gather_path(d):
     cache.append(k, v)
     ck, cv = compress_kv(k, v, kc, vc)
     for query, tol in ((q, 1e-6), (q.to(torch.bfloat16), 1e-6 if d == 64 else 1e-2)):
-        # same kernel on both sides through the gather path; at head_dim 128 a 16-bit query reads the cache in place
-        # with the split-KV kernel instead
+        # the same kernel on both sides, but for 16-bit queries of head_dim 128: the cache is read by the split-KV kernel
         got = cache.attend(query, causal=True)
         want = fused_attention(query, ck, cv, kc, vc, causal=True)
         assert rel_err(got, want) < tol, rel_err(got, want)
@@ -149,7 +147,7 @@ def test_single_token_cache_through_the_gather_path(d):
 @pytest.mark.parametrize("cached,new", [(0, 17), (131, 1), (300, 128), (127, 130)])
 def test_chunk_attends_in_place_over_a_strided_cache(d, bits, Hq, Hkv, cached, new):
     """Chunks of a prompt behind a prefix: the kernels read the cache rows where they are (a token stride of the
-    capacity, odd here) and give bit for bit what they give on the gathered prefix."""
+    capacity, odd here) and give bit for bit what they give on dense arrays."""
     from turboquant_b200 import CompressedKVCache, fused_attention
     kc, vc = device_compressors(d, bits, mode="bf16")
     n = cached + new
@@ -158,7 +156,7 @@ def test_chunk_attends_in_place_over_a_strided_cache(d, bits, Hq, Hkv, cached, n
     cache = CompressedKVCache(kc, vc, 2, Hkv, n + 37)
     cache.append(k[:, :, :cached], v[:, :, :cached])
     cache.append(k[:, :, cached:], v[:, :, cached:])
-    ck, cv = cache._contiguous_prefix()
+    ck, cv = contiguous_prefix(cache)
     got = cache.attend(q)
     want = fused_attention(q, ck, cv, kc, vc)
     if d == 128 and (Hq // Hkv) * new <= 16 and n < 256:

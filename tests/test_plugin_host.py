@@ -121,17 +121,25 @@ def test_mask_forms_accepted_by_the_attention_wrapper():
     integer masks are refused because their meaning would be a guess."""
     import pytest
     import torch
-    from turboquant_b200.compressors import _mask_args
+    from turboquant_b200 import _lib
+    from turboquant_b200.compressors import _mask_rows
     keep = torch.ones(2, 1, 3, 5, dtype=torch.bool)
     keep[1, 0, :, :2] = False
-    mk, ptr, sb, sq = _mask_args(keep, 2, 3, 5, "cpu")
-    assert mk.dtype == torch.float32 and mk.shape == (2, 3, 5) and (sb, sq) == (15, 5) and ptr == mk.data_ptr()
-    assert torch.equal(mk == 0, keep[:, 0]) and float(mk[1, 0, 0]) == torch.finfo(torch.float32).min
+    mk, kind = _mask_rows(keep, 2, 3, 5, "cpu")
+    assert kind == _lib.TQ_MASK_BOOL and torch.equal(mk, keep[:, 0])     # bytes as they are
+    assert mk.data_ptr() == keep.data_ptr()
     add = torch.zeros(1, 1, 3, 5, dtype=torch.float16)
-    mk, _, sb, _ = _mask_args(add, 2, 3, 5, "cpu")
-    assert mk.dtype == torch.float32 and sb == 0            # broadcast over the batch
+    mk, kind = _mask_rows(add, 2, 3, 5, "cpu")
+    assert kind == _lib.TQ_MASK_ADDITIVE and mk.dtype == torch.float32 and mk.shape == (1, 3, 5)  # one for the whole batch
+    mk, _ = _mask_rows(add[0, 0], 2, 3, 5, "cpu")
+    assert mk.shape == (1, 3, 5)
+    mk, _ = _mask_rows(keep[:, :, :1].expand(2, 1, 3, 5), 2, 3, 5, "cpu")
+    assert mk.shape == (2, 3, 5) and mk.stride() == (15, 0, 1)           # expanded rows stay expanded
+    mk, _ = _mask_rows(keep[:, :, :, :1].expand(2, 1, 3, 5), 2, 3, 5, "cpu")
+    assert mk.stride(-1) == 1                                            # ... columns are copied
     with pytest.raises(TypeError):
-        _mask_args(keep.long(), 2, 3, 5, "cpu")
+        _mask_rows(keep.long(), 2, 3, 5, "cpu")
     with pytest.raises(ValueError):
-        _mask_args(torch.zeros(2, 4, 3, 5), 2, 3, 5, "cpu")  # per-head masks
-    assert _mask_args(None, 2, 3, 5, "cpu") == (None, None, 0, 0)
+        _mask_rows(torch.zeros(2, 4, 3, 5), 2, 3, 5, "cpu")  # per-head masks
+    with pytest.raises(ValueError):
+        _mask_rows(keep[:, :, :2], 2, 3, 5, "cpu")           # too few rows

@@ -95,19 +95,6 @@ PyObject* set_error_type(PyObject*, PyObject* type) {
   Py_RETURN_NONE;
 }
 
-// rows_view(t): the tensor itself where the kernels can read it in place
-PyObject* py_rows_view(PyObject*, PyObject* o) {
-  HANDLE_TH_ERRORS
-  const at::Tensor& in = tensor(o, "states");
-  at::Tensor t = rows_view(in);
-  if (t.is_same(in)) {
-    Py_INCREF(o);
-    return o;
-  }
-  return THPVariable_Wrap(std::move(t));
-  END_HANDLE_TH_ERRORS
-}
-
 // compress(keys | None, values | None, constants, bits, mode)
 //   -> (key indices, signs, residual norms, norms, value indices, norms), None for a side that is not there
 PyObject* compress(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -336,7 +323,6 @@ PyObject* rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 #define TQ_FAST(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"set_error_type", set_error_type, METH_O, nullptr},
-                         {"rows_view", py_rows_view, METH_O, nullptr},
                          TQ_FAST("compress", compress),
                          TQ_FAST("append", append),
                          TQ_FAST("attend", attend),

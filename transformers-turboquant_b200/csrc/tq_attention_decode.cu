@@ -702,8 +702,8 @@ static bool decode_enabled() {
 
 bool decode_applies(const AttnArgs& a, int d) {
   const bool shape_ok = d == 128 && a.Hkv > 0 && (a.Hq / a.Hkv) * a.Sq <= kRows;
-  if (a.kv_stride != a.Sk) return shape_ok;  // a persistent cache: the only kernel that reads strided rows
-  return decode_enabled() && shape_ok && a.Sk >= 4 * kBlockKeys * kWarps;
+  // a persistent cache takes it at any length, so that a sequence stays on one kernel while it grows
+  return decode_enabled() && shape_ok && (a.kv_stride != a.Sk || a.Sk >= 4 * kBlockKeys * kWarps);
 }
 
 

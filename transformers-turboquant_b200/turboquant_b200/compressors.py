@@ -272,17 +272,6 @@ def _mask_rows(attention_mask: torch.Tensor, B: int, Sq: int, Sk: int, dev):
     return mk, kind
 
 
-def _mask_args(attention_mask, B: int, Sq: int, Sk: int, dev):
-    """A mask as the C entry points with an additive fp32 mask take it: (tensor, pointer, batch stride, row stride),
-    boolean masks turned into the additive form; (None, None, 0, 0) for no mask."""
-    if attention_mask is None:
-        return None, None, 0, 0
-    mk, kind = _mask_rows(attention_mask, B, Sq, Sk, dev)
-    if kind == _lib.TQ_MASK_BOOL:
-        mk = torch.zeros(mk.shape, dtype=torch.float32, device=dev).masked_fill_(~mk, torch.finfo(torch.float32).min)
-    return mk, mk.data_ptr(), (mk.stride(0) if mk.shape[0] == B and B > 1 else 0), mk.stride(1)
-
-
 def _attend(q: torch.Tensor, Hkv: int, Sk: int, capacity: int, packed: tuple, kc, vc, sm_scale, causal: bool,
             attention_mask, mode: int) -> torch.Tensor:
     """One attention call over `packed` = (key indices, signs, norms, residual norms, value indices, norms)."""

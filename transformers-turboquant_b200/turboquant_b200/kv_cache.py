@@ -76,21 +76,6 @@ class CompressedKVCache:
                          self.capacity, self.length)
         self.length += S
 
-    def _contiguous_prefix(self) -> tuple[dict, dict]:
-        """The tokens in use as the contiguous dictionaries `compress()` returns (copies: the cache rows are
-        `capacity` apart).  `reshape` alone is not enough: for a single token per head it returns a strided view."""
-        n, shape = self.length, (self.batch, self.kv_heads, self.length, self.head_dim)
-
-        def rows(t):
-            return t[:, :, :n].reshape(-1, t.shape[-1]).contiguous()
-
-        ck = {"packed_key_indices": rows(self.key_indices), "packed_qjl_signs": rows(self.key_signs),
-              "vec_norms": self.key_norms[:, :, :n].contiguous(),
-              "residual_norm": self.key_residual_norms[:, :, :n].contiguous(), "shape": shape}
-        cv = {"packed_indices": rows(self.value_indices),
-              "vec_norms": self.value_norms[:, :, :n].reshape(-1).contiguous(), "shape": shape}
-        return ck, cv
-
     def attend(self, q: torch.Tensor, causal: bool = True, sm_scale: float | None = None,
                attention_mask: torch.Tensor | None = None) -> torch.Tensor:
         """softmax(scores * sm_scale) @ V_hat of q [B, Hq, Sq, D] over the tokens in use; with `causal` the
