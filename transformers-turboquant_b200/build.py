@@ -1,11 +1,12 @@
 """Build libtq_b200.so (CUDA kernels + C ABI) for sm_100a with nvcc, in-tree.
 
-    python transformers-turboquant_b200/build.py [--force] [--verbose] [--trace]
+    python transformers-turboquant_b200/build.py [--force] [--verbose] [--trace] [--no-host]
 
 Each csrc/*.cu is compiled to an object in build/ (only when its sources changed) and
 the objects are linked into turboquant_b200/libtq_b200.so; csrc/host/tq_host.cpp becomes turboquant_b200/_tq_host.so.  nvcc cross-compiles, so no
 GPU is needed.  `-Xptxas -v` output (registers, spills, shared memory per kernel) is
-kept in build/ptxas_<file>.log.  `--trace` (implies a full rebuild) adds the diagnostic
+kept in build/ptxas_<file>.log.  `--no-host` leaves _tq_host.so out: programs that use the C library alone need neither torch
+nor g++.  `--trace` (implies a full rebuild) adds the diagnostic
 instantiations of the attention kernels that tq_trace_enable / tq_trace_read need; the
 default product build leaves them out.
 """
@@ -35,28 +36,36 @@ def _newest(paths):
 
 def build_host(force: bool = False) -> str:
     """The CPython module with the native tails of the entry points (linked against libtq_b200.so beside it; torch's own
-    libraries are in the process already when it is imported)."""
-    deps = [HOST_SRC, os.path.join(INCLUDE, "tq_b200.h"), LIB, os.path.abspath(__file__)]
-    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) > _newest(deps):
-        return HOST_LIB
+    libraries are in the process already when it is imported).  Built again when this Python or this torch is another one
+    than it was built for."""
     import sysconfig
 
     import torch
 
+    abi = int(torch.compiled_with_cxx11_abi())
+    built_for = f"python {sys.version} {sys.executable} torch {torch.__version__} {os.path.dirname(torch.__file__)} abi {abi}\n"
+    stamp = os.path.join(BUILD, "tq_host.stamp")
+    deps = [HOST_SRC, os.path.join(INCLUDE, "tq_b200.h"), LIB, os.path.abspath(__file__)]
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) > _newest(deps) and os.path.exists(stamp):
+        with open(stamp) as fh:
+            if fh.read() == built_for:
+                return HOST_LIB
     root = os.path.join(os.path.dirname(torch.__file__), "include")
     includes = [INCLUDE, root, os.path.join(root, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
                 os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
-    res = subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC",
-                          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[x for i in includes for x in ("-I", i)], HOST_SRC, "-o", HOST_LIB, "-L", os.path.dirname(LIB),
+    res = subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+                          *[x for i in includes for x in ("-I", i)], HOST_SRC, "-o", HOST_LIB, "-L", os.path.dirname(LIB),
                           "-l:libtq_b200.so", "-L", os.path.join(os.path.dirname(torch.__file__), "lib"), "-lc10", "-lc10_cuda",
                           "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"],
                          capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
+    with open(stamp, "w") as fh:
+        fh.write(built_for)
     return HOST_LIB
 
 
-def build(force: bool = False, verbose: bool = False, trace: bool = False) -> str:
+def build(force: bool = False, verbose: bool = False, trace: bool = False, host: bool = True) -> str:
     os.makedirs(BUILD, exist_ok=True)
     flags = FLAGS + (["-DTQ_B200_TRACE=1"] if trace else [])
     # a library built with tracing is a different product: switching the option rebuilds everything
@@ -95,9 +104,11 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> st
                               "-lcudart"], capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
-    build_host(force)
+    if host:
+        build_host(force)
     return LIB
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, trace="--trace" in sys.argv))
+    print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, trace="--trace" in sys.argv,
+                host="--no-host" not in sys.argv))
