@@ -300,7 +300,8 @@ int tq_attention_fwd_prepared(const void* q, int dtype, int64_t B, int64_t Hq, i
 /* tq_attention_fwd_prepared under a mask the library first summarises into visibility bits (one small launch): additive
  * fp32 (TQ_MASK_ADDITIVE) or bytes of which 0 hides a key (TQ_MASK_BOOL, what HF's sdpa path hands over for padded
  * batches).  `mask_batches` is 1 (one mask for every batch element) or B; strides in elements, rows contiguous.
- * Tiles of keys that no row of a tile of queries sees are not computed. */
+ * Tiles of keys that no row of a tile of queries sees are not computed.  (Additive masks in TQ_MODE_FP32 and over at most
+ * 128 keys are read as they are.)  A mask that hides every key of a row makes it the average over its causal range. */
 #define TQ_MASK_ADDITIVE 0
 #define TQ_MASK_BOOL 1
 size_t tq_attention_masked_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,

@@ -150,7 +150,7 @@ size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsp
 // Merge of tiles of 128 query rows and back-rotation by Pi_v (fp32) into a.out.
 int merge_split_tiles(const AttnArgs& a, int64_t B, int d, int nsplit, float* part_o, float* part_ml, cudaStream_t stream);
 
-// SM-pair (2-CTA cluster) tensor-core kernel, head_dim 128; needs no per-query scratch.
+// SM-pair (2-CTA cluster) tensor-core kernel, head_dim 64 and 128; scratch only for the partial results of a split call.
 int attention_c2(const AttnArgs& a, const PairArgs& x, int64_t B, int d, int bits, cudaStream_t stream);
 int read_c2_faults(unsigned long long* out);
 int trace_enable_c2(int on);

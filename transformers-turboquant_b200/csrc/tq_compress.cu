@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(D) compress_rows_kernel(const CompressArgs k, 
   else compress_rows<T, D, BITS, false, R>(v, (int64_t)(blockIdx.x - key_ctas) * R);
 }
 
-// Up to this many vectors a side: 3072 take 43 us at head_dim 128 (8: 17 us) where the two
-// launches of the tile kernel take 49 us.
+// Up to this many vectors a side: from a cold L2, 3072 take 48 us at head_dim 128 and 23 us at 64 (8: 22 and 16 us) where the
+// two launches of the tile kernel take 52 and 32 us.
 constexpr int64_t kFewVectors = 3072;
 
 template <typename T, int D>

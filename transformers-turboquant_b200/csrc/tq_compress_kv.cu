@@ -194,9 +194,13 @@ __device__ __noinline__ uint32_t open_any(uint32_t col, const float* __restrict_
 //
 // An index or a sign whose coordinate lies within the sums' rounding of its boundary may fall either way, and a single
 // moved index moves about seven sign bytes of its vector.  A 16-bit input type with exact operands should not differ from
-// the fp32 kernel in that way, so coordinates within kOpenIndex (in units of the norm; the sums are off by 1e-8 on
-// average) and projections within kOpenSign (in units of the residual's norm; off by 1e-6) are decided by the fp32
-// kernel's own arithmetic: the functions below, one warp per open coordinate, with its order of operations.  About one
+// the fp32 kernel in that way, so coordinates within kOpenIndex (in units of the norm) and projections within kOpenSign (in
+// units of the residual's norm) are decided by the fp32 kernel's own arithmetic: the functions below, one warp per open
+// coordinate, with its order of operations.  The bands follow from that kernel's rounding, the larger of the two: a sum of d
+// multiply-adds whose partial sums are about as large as the boundary is off by 2^-25 of it sqrt(d) / 2 times or so, 1.8e-8 rms
+// near a boundary (measured against fp64: 1.6e-8 to 1.8e-8 at 3 and 4 bits, either head_dim), and passes that error on to a
+// projection sqrt(d) fold against a residual of 0.1 to 0.4 of the norm (0.5e-6 to 1.3e-6 rms measured; the tensor-core
+// sums: 1e-8).  Nine and five times that leave less than one decision in 1e10 to chance.  About one
 // vector in 700 has one; the compression of 6 x 8 x 777 keys and values takes 48 us with the
 // repair and 22 us without (171 us on the fp32 kernels).
 constexpr float kOpenIndex = 1.6e-7f, kOpenSign = 6e-6f;

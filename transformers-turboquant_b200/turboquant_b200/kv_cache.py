@@ -92,9 +92,9 @@ class CompressedKVCache:
         kc, vc = self.key_compressor, self.val_compressor
         kc._check_device(q)
         vc._check_device(q)
-        # The prefill kernels follow the token stride of the cache as the split-KV kernel does: gathering the prefix
-        # first took six strided copies per call (a 300-token chunk behind 8 000 tokens: 149 us with, 115 us without;
-        # a step of a GPT-2-shaped layer over 700 tokens: 140 us with, 55 us without).
+        # The prefill kernels follow the token stride of the cache as the split-KV kernel does: dense copies of the
+        # prefix are six strided copies per call (a 300-token chunk behind 8 000 tokens: 149 us with them, 115 us
+        # without; a step of a GPT-2-shaped layer over 700 tokens: 140 and 55 us).
         packed = (self.key_indices, self.key_signs, self.key_norms, self.key_residual_norms, self.value_indices,
                   self.value_norms)
         return _attend(q, self.kv_heads, self.length, self.capacity, packed, kc, vc, sm_scale, causal, attention_mask,
