@@ -278,8 +278,10 @@ int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq
                      void* workspace, size_t workspace_bytes, int mode, void* stream);
 
 /* tq_attention_fwd / tq_attention_fwd_cached with the constants taken from a prepared buffer: no operand is
- * rebuilt per call, and the scratch need drops to tq_attention_prepared_workspace_bytes -- zero for most
- * prefill-sized calls in TQ_MODE_BF16 (`workspace` may then be NULL); long prefixes behind few queries and
+ * rebuilt per call, and the scratch need is tq_attention_prepared_workspace_bytes.  In TQ_MODE_BF16, calls in which many
+ * queries meet each key expand keys and values once per call to fp16 rows there (4 d bytes a token and KV head, 128 MiB at a
+ * time and no more) and attend over those; without the room (`workspace` may be NULL) they are served from the packed bytes,
+ * slower.  Other prefill-sized calls need none, but for long prefixes behind few queries, which with
  * TQ_MODE_FP32 keep partial results there and are served unsplit, slower, without the room.  kv_capacity = Sk is the contiguous
  * layout; a larger capacity is the persistent-cache layout of tq_attention_fwd_cached, served in place for every
  * head_dim, number of queries and mode.

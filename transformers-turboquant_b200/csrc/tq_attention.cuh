@@ -17,6 +17,7 @@ struct ConstLayout {
   size_t w_cat_pair, w_unrot_pair, luts, w_cat_plain, w_unrot_plain;  // attention: bf16 operand images, fp16 pair tables
   size_t pik_hi, pik_lo, se_hi, se_lo, piv_hi, piv_lo;            // compression: split-bf16 K-major operand images
   size_t pik16_hi, pik16_lo, se16_hi, se16_lo, piv16_hi, piv16_lo;  // ... and split-fp16 ones, scaled by powers of two
+  size_t x_key, x_val;  // expansion: fp16 images of Pi_k^T and (S_eff Pi_k)^T, of Pi_v^T, scaled by powers of two
   size_t total;
 };
 // The fp16 images of a rotation hold Pi x 128 (entries of about 0.1 would put the low parts into fp16's subnormals); a matrix
@@ -25,6 +26,9 @@ struct ConstLayout {
 // each to entries of about 1.
 constexpr float kPi16Scale = 128.f;
 constexpr int kScaleWord = 4;
+// ... and, at this word, what the accumulators of the expansion are multiplied by: of indices, of signs (sqrt(pi/2)/d
+// included), of values.
+constexpr int kExpandScaleWord = 8;
 constexpr uint32_t kConstMagic = 0x31425154u;  // "TQB1"
 inline ConstLayout const_layout(int d) {
   ConstLayout L{};
@@ -40,6 +44,7 @@ inline ConstLayout const_layout(int d) {
   L.piv_hi = take(m16); L.piv_lo = take(m16);
   L.pik16_hi = take(m16); L.pik16_lo = take(m16); L.se16_hi = take(m16); L.se16_lo = take(m16);
   L.piv16_hi = take(m16); L.piv16_lo = take(m16);
+  L.x_key = take(2 * m16); L.x_val = take(m16);
   L.total = off;
   return L;
 }
@@ -146,6 +151,8 @@ struct PairArgs {
 };
 // Clusters per pair of query tiles that the SM-pair kernel is split over, and the partial results' bytes (0 unsplit).
 int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
+// What that kernel is expected to take, in microseconds (the estimate behind the splits).
+double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
 size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit);
 // Merge of tiles of 128 query rows and back-rotation by Pi_v (fp32) into a.out.
 int merge_split_tiles(const AttnArgs& a, int64_t B, int d, int nsplit, float* part_o, float* part_ml, cudaStream_t stream);

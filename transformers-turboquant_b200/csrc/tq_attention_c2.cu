@@ -1030,25 +1030,37 @@ int launch_bits(const AttnArgs& a, const PairArgs& x, int64_t B, int bits, cudaS
 // the merge kMerge (9600 rows: 21 us).  The number of splits is the one with the least (waves of clusters) x (tiles +
 // fixed) + merge.  Measured with append (LLaMA-8B heads): 100 tokens behind 8000 take 61 us in four splits and 112 us in one,
 // 20 behind 30000 122 and 353 us; 300 behind 8000, 48 clusters, take 112 us in one and 122 us in three.
-int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
+static double c2_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int* splits) {
   constexpr double kFixed = 6.0, kFixedSplit = 10.0, kMerge = 15.0;
-  if (Hkv <= 0 || Sk <= 0) return 1;
+  *splits = 1;
+  if (Hkv <= 0 || Sk <= 0) return 0.0;
   const bool pair_heads = (Hq / Hkv) % 2 == 0;
   const int64_t blocks = (Sq + kBM - 1) / kBM, tiles = (Sk + kBN - 1) / kBN;
   const int64_t clusters = B * (pair_heads ? Hq / 2 * blocks : Hq * ((blocks + 1) / 2)), slots = sm_count() / 2;
   // whole tiles in front of the first query, so that no split of a causal call is empty; at least four tiles each
   const int64_t most = (Sk > Sq ? Sk - Sq : 0) / kBN / 4;
-  int best = 1;
   double cost = (double)((clusters + slots - 1) / slots) * ((double)tiles + kFixed);
   for (int64_t n = 2; n <= most && n <= 32 && clusters < slots; ++n) {
     const int64_t waves = (clusters * n + slots - 1) / slots;
     const double c = (double)waves * ((double)((tiles + n - 1) / n) + kFixedSplit) + kMerge;
     if (c < cost) {
       cost = c;
-      best = (int)n;
+      *splits = (int)n;
     }
   }
-  return best;
+  // (causal prompts: the average cluster walks fewer tiles than the first ones)
+  if (4 * Sq >= Sk && clusters > slots)
+    cost = (double)tiles + kFixed + ((double)clusters / (double)slots - 1.0) * (((double)Sk - 0.5 * (double)Sq) / kBN + kFixed);
+  return cost;
+}
+int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
+  int splits;
+  c2_plan(B, Hq, Sq, Hkv, Sk, &splits);
+  return splits;
+}
+double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
+  int splits;
+  return 4.0 + 1.46 * c2_plan(B, Hq, Sq, Hkv, Sk, &splits);
 }
 size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit) {
   if (nsplit <= 1) return 0;

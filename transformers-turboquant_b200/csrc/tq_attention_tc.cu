@@ -20,6 +20,7 @@
 
 #include "tq_attention.cuh"
 #include "tq_common.cuh"
+#include "tq_dense.cuh"
 #include "tq_rows.cuh"
 #include "tq_simt.cuh"
 #include "tq_tcgen05.cuh"
@@ -166,6 +167,45 @@ __global__ void build_split_images_kernel(const ImageArgs a, int d) {
   a.hi16[m][at] = g;
   a.lo16[m][at] = __float2half_rn(w - __half2float(g));
 }
+// Operand images of the expansion (blockIdx.y: Pi_k^T, (S_eff Pi_k)^T, Pi_v^T), K-major fp16, scaled to entries of about 1.
+__global__ void build_expand_images_kernel(const float* __restrict__ Pi_k, const float* __restrict__ S_eff,
+                                           const float* __restrict__ Pi_v, int d, float coeff, __half* __restrict__ x_key,
+                                           __half* __restrict__ x_val, float* __restrict__ scales) {
+  __shared__ float s_part[2][4];
+  const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
+  const float* Pi = m == 2 ? Pi_v : Pi_k;
+  float pp = 0.f, ss = 0.f, acc = 0.f;
+#pragma unroll 8
+  for (int r = 0; r < d; ++r) {
+    const float p = Pi[r * d + i];
+    pp = fmaf(p, p, pp);
+    if (m == 1) {
+      const float s = S_eff[r * d + i];
+      ss = fmaf(s, s, ss);
+      acc = fmaf(S_eff[j * d + r], p, acc);
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    pp += __shfl_xor_sync(0xffffffffu, pp, off);
+    ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  }
+  if (i % 32 == 0) {
+    s_part[0][i / 32] = pp;
+    s_part[1][i / 32] = ss;
+  }
+  __syncthreads();
+  pp = ss = 0.f;
+  for (int w = 0; w < d / 32; ++w) {
+    pp += s_part[0][w];
+    ss += s_part[1][w];
+  }
+  // rows of a rotation have norm 1, entries 1/sqrt(d); entries of a sketch are of size 1, rotated or not
+  const int e = rms_exponent(pp / (float)d) + (m == 1 ? rms_exponent(ss / ((float)d * d)) : 3);
+  const float scale = ldexpf(1.f, e);
+  if (j == 0 && i == 0) scales[m] = ldexpf(m == 1 ? coeff : 1.f, -e);
+  const float v = (m == 1 ? acc : Pi[j * d + i]) * scale;
+  (m == 2 ? x_val : x_key + (m == 1 ? d * d : 0))[operand_index(i, j, d, d)] = __float2half_rn(v);
+}
 // The header, the codebooks and the pair tables (one block).
 struct CodebookArgs {
   const float* src[4];
@@ -210,6 +250,8 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
   const float coeff = sqrtf(1.5707963267948966f) / (float)d;
   build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, coeff, b16(L.w_cat_pair), d, b16(L.w_cat_plain), 0);
   build_wunrot_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.w_unrot_pair), d / 2, b16(L.w_unrot_plain), 0);
+  build_expand_images_kernel<<<dim3(d, 3), d, 0, stream>>>(Pi_k, S_eff, Pi_v, d, coeff, h16(L.x_key), h16(L.x_val),
+                                                           f32(L.header) + kExpandScaleWord);
   TQ_CUDA_OK(cudaGetLastError());
   return TQ_OK;
 }
@@ -971,7 +1013,9 @@ size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t 
   const int64_t n_q = B * Hq * Sq;
   switch (bf16_path(a, Sq, d)) {
     // everything it needs is in the constants buffer and on the chip, but for the partial results of a split call
-    case Bf16Path::kPairs: return attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk));
+    case Bf16Path::kPairs:
+      if (attention_dense_applies(B, Hq, Sq, Hkv, Sk, d)) return attention_dense_bytes(B, Hq, Sq, Hkv, Sk, d);
+      return attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk));
     case Bf16Path::kDecode: return round256((size_t)n_q * 2 * d * 2) + decode_workspace_bytes(B * Hq);
     default: return round256((size_t)n_q * 2 * d * 2) + round256((size_t)n_q * d * 2);
   }
@@ -1006,6 +1050,10 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
   ws += round256((size_t)n_q * 2 * d * 2);
   __nv_bfloat16* o_rot = reinterpret_cast<__nv_bfloat16*>(ws);
 
+  // (packed rows are read in words there)
+  if (pairs && prepared != nullptr && workspace != nullptr && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d) &&
+      ((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) | reinterpret_cast<uintptr_t>(a.val_idx)) & 3u) == 0)
+    return attention_dense(a, B, d, bits, q, dtype, sb, sh, ss, prepared, workspace, stream);
   if (path == Bf16Path::kDecode)  // its own small kernels on both sides of the split-KV kernel; none of the operand images
     return attention_decode(a, B, bits, q, dtype, sb, sh, ss, Pi_k, S_eff, q_cat,
                             prepared != nullptr ? reinterpret_cast<uint8_t*>(o_rot)
@@ -1026,7 +1074,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
       TQ_CUDA_OK(cudaGetLastError());
     }
     PairArgs x{q, dtype, sb, sh, ss, w_cat, w_unrot, luts, 1, nullptr, nullptr};
-    if (prepared != nullptr && workspace != nullptr) {  // room for partial results (NULL: an unsplit call)
+    if (prepared != nullptr && workspace != nullptr && !attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d)) {  // room for partial results (NULL: an unsplit call)
       x.nsplit = attention_c2_splits(B, Hq, Sq, a.Hkv, a.Sk);
       x.part_o = static_cast<float*>(workspace);
       x.part_ml = x.part_o + (size_t)B * Hq * ((Sq + kBM - 1) / kBM) * x.nsplit * kBM * d;

@@ -119,6 +119,13 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t bar, uint32_t parity
     }
   }
 }
+// As mbar_wait_or_abort for a phase that is about to complete: a suspended wait wakes up some hundred cycles late.
+__device__ __forceinline__ bool mbar_spin_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (int i = 0; i < 128; ++i)
+    if (mbar_test(bar, parity)) return true;
+  return mbar_wait_or_abort(bar, parity, abort_flag);
+}
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -177,6 +184,17 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 // Arrive on `bar` once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// One lane of a converged warp (the same one each time).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(is));
+  return is != 0;
 }
 
 // One column of 32 lanes.
