@@ -159,10 +159,9 @@ def measured_peaks():
 
 
 def attention_flops(batch, seq, heads=HQ):
-    """Algorithmic flops of one launch of the fused attention kernel: 2d (q.K_hat) + 2d (q_s.sign) + 2d (P.V_hat)
-    per causal pair, plus per query row the preparation q [Pi ; coeff S]^T (2 * 2d * d) and the output
-    back-rotation (2 d^2)."""
-    return 6.0 * D * causal_pairs(batch, seq, heads) + 6.0 * D * D * batch * heads * seq
+    """Flops of one launch of the attention kernel over expanded keys and values: 2d (q.K') + 2d (P.V') per causal pair
+    (the expansion is a launch of its own)."""
+    return 4.0 * D * causal_pairs(batch, seq, heads)
 
 
 # ---------------------------------------------------------------------------------------------------------
@@ -451,13 +450,13 @@ def head_dim64_section(ctx: Ctx, bits: int, batch: int = B, steps: int = 10, war
             return tq.fused_attention(q, ck, cv, kc, vc, causal=True, mode="bf16")
 
         ms, _ = timed_steps(ctx, step, steps, warm)
-        flops = batch * hq * (seq * (seq + 1) / 2) * 6 * d
+        flops = batch * hq * (seq * (seq + 1) / 2) * 4 * d
         out[name] = {"ms_per_step": ms, "keys_per_s": batch * hkv * seq * ctx.world / (ms * 1e-3),
                      "tflops": flops / (ms * 1e-3) / 1e12, "frac_of_burst_bf16": flops / (ms * 1e-3) / 1e12 / peaks["tflops_burst"],
                      "shape": {"batch_per_gpu": batch, "q_heads": hq, "kv_heads": hkv, "seq": seq, "head_dim": d}}
         del q, k, v
-    return {"dtype": "bf16", "bits": bits, "steps": steps, "warmup": warm, "kernel": "attention_c2_kernel<64, bits>",
-            "flops": "6 d per visible (query, key) pair", **out}
+    return {"dtype": "bf16", "bits": bits, "steps": steps, "warmup": warm, "kernel": "attention_dense_kernel<64>",
+            "flops": "4 d per visible (query, key) pair", **out}
 
 
 def rope_section(ctx: Ctx, steps: int = 20, warm: int = 3):
@@ -553,7 +552,7 @@ def decode_section(ctx: Ctx, bits: int, steps: int = 50, warm: int = 3):
                          "frac": achieved / peaks["hbm_gbs"], "traffic": None, "kernel": "decode_kernel",
                          "ms_per_launch": kern_ms, "algorithmic_bytes_per_launch": keys * bytes_per_key,
                          "peak_source": peaks["source"] + ", copy bandwidth"},
-            "kernel_ms": {"prepare_queries": ms_sum[2] / max(launches[2], 1), "decode": kern_ms,
+            "kernel_ms": {"expand_keys_and_values": ms_sum[2] / max(launches[2], 1), "decode": kern_ms,
                           "merge_and_back_rotation": ms_sum[4] / max(launches[4], 1)},
             "generation_step_ms": gen_ms,  # append one token per sequence to the cache, then attend
             "uncompressed_bf16_cache_sdpa_ms_per_call": sdpa_ms,
@@ -646,11 +645,9 @@ def run_headline(args):
     attn_ms = ms_sum[3] / max(launches[3], 1)
     flops = attention_flops(batch, seq)
     achieved = flops / (attn_ms * 1e-3) / 1e12
-    # DRAM bytes per launch: one ncu capture of this kernel at batch 1 (profiles/attention_c2_kernel_b1_s8192.md:
-    # dram__bytes_read.sum + dram__bytes_write.sum = 103.3 MB; raw queries in, outputs out, packed keys and
-    # values), scaled by the batch, which it is proportional to; the algorithmic bytes beside it
+    # (what the call cannot do without; the expanded rows between its two kernels fit the L2 but for a part)
     algorithmic_bytes = batch * (2 * HQ * seq * D * 2 + HKV * seq * ((16 * (bits - 1) + 16 + 4) + (16 * bits + 2)))
-    traffic = 103.3e6 * batch if (seq == S and D == 128 and bits == 3) else None
+    traffic = None
     roofline = {"bound": "tensor", "achieved": achieved, "unit": "TFLOP/s",
                 "peak": peaks["tflops_burst"], "frac": achieved / peaks["tflops_burst"],
                 "frac_burst": achieved / peaks["tflops_burst"], "frac_sustained": None,
@@ -659,12 +656,12 @@ def run_headline(args):
                              "against the sustained peak",
                 "peak_burst": peaks["tflops_burst"], "peak_sustained": peaks["tflops_sustained"],
                 "traffic": traffic, "algorithmic_bytes_per_launch": algorithmic_bytes,
-                "flops_per_launch": flops, "kernel": "attention_c2_kernel", "ms_per_launch": attn_ms,
+                "flops_per_launch": flops, "kernel": "attention_dense_kernel", "ms_per_launch": attn_ms,
                 "peak_source": peaks["source"],
                 "kernel_ms": {"compress": (ms_sum[0] + ms_sum[1]) / max(args.steps, 1),
                               "compress_keys": ms_sum[0] / max(launches[0], 1),
                               "compress_values": ms_sum[1] / max(launches[1], 1),
-                              "prepare_queries": ms_sum[2] / max(launches[2], 1),
+                              "expand_keys_and_values": ms_sum[2] / max(launches[2], 1),
                               "attention": attn_ms, "back_rotation": ms_sum[4] / max(launches[4], 1)}}
     comp_ms = (ms_sum[0] + ms_sum[1]) / max(args.steps, 1)
     comp_bytes = batch * HKV * seq * (2 * D * 2 + (16 * (bits - 1) + 16 + 4) + (16 * bits + 2))

@@ -87,7 +87,7 @@ int tq_selftest_wait_expiry(void* stream, int64_t limit_cycles, int64_t* waited_
 enum {
   TQ_PROF_COMPRESS_KEYS = 0,
   TQ_PROF_COMPRESS_VALUES = 1,
-  TQ_PROF_PREPARE_QUERIES = 2,
+  TQ_PROF_PREPARE_QUERIES = 2,  /* query preparation, or the expansion of keys and values */
   TQ_PROF_ATTENTION = 3,
   TQ_PROF_BACK_ROTATION = 4,
   TQ_PROF_KINDS = 5

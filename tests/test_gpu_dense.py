@@ -42,7 +42,7 @@ def _check(q, ck, cv, kc, vc, **kw):
 
 # rows of a group around one tile (128), two (a CTA) and three; groups of 1, 3 and 7 heads; ragged ends of the keys
 @pytest.mark.parametrize("d", [64, 128])
-@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk", [(32, 12, 12, 127, 127), (32, 12, 12, 128, 129), (16, 16, 16, 257, 257),
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk", [(32, 12, 12, 127, 127), (32, 16, 4, 32, 129), (16, 16, 16, 257, 257),
                                             (16, 12, 4, 85, 130), (16, 14, 2, 55, 1000), (8, 16, 4, 700, 900)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_edges_of_tiles(B, Hq, Hkv, Sq, Sk, d, causal):

@@ -152,7 +152,7 @@ struct PairArgs {
 // Clusters per pair of query tiles that the SM-pair kernel is split over, and the partial results' bytes (0 unsplit).
 int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
 // What that kernel is expected to take, in microseconds (the estimate behind the splits).
-double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
+double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
 size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit);
 // Merge of tiles of 128 query rows and back-rotation by Pi_v (fp32) into a.out.
 int merge_split_tiles(const AttnArgs& a, int64_t B, int d, int nsplit, float* part_o, float* part_ml, cudaStream_t stream);

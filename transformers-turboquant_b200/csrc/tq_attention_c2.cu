@@ -1058,9 +1058,9 @@ int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t 
   c2_plan(B, Hq, Sq, Hkv, Sk, &splits);
   return splits;
 }
-double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {
+double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
   int splits;
-  return 4.0 + 1.46 * c2_plan(B, Hq, Sq, Hkv, Sk, &splits);
+  return 4.0 + (d == 64 ? 1.25 : 1.46) * c2_plan(B, Hq, Sq, Hkv, Sk, &splits);
 }
 size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit) {
   if (nsplit <= 1) return 0;

@@ -707,9 +707,9 @@ DensePlan dense_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
       p.nsplit = (int)s;
     }
   }
-  // (causal prompts: the average block walks fewer tiles than the longest)
+  // (causal prompts: the average block walks fewer tiles than the first ones)
   if (4 * Sq >= Sk && units > slots)
-    cost = std::max((double)p.T + kFixed, (double)units / (double)slots * (((double)Sk - 0.5 * (double)Sq) / kBN + kFixed));
+    cost = (double)p.T + kFixed + ((double)units / (double)slots - 1.0) * (((double)Sk - 0.5 * (double)Sq) / kBN + kFixed);
   p.us = kLaunchUs + (double)groups * cost * kPeriodUs + (double)(all * p.T * d) * kExpandUs;
   if (p.nsplit > 1) p.part_bytes = round256((size_t)units * 2 * p.nsplit * kBM * (d + 2) * sizeof(float));
   return p;
@@ -722,10 +722,10 @@ bool attention_dense_applies(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int
   const DensePlan p = dense_plan(B, Hq, Sq, Hkv, Sk, d);
   // Expansion pays where a key is met by many tiles of queries.  Few queries behind a prefix, and calls of one or two key tiles,
   // are the SM-pair kernel's: either one's time is estimated (over 533 calls of 1 to 512 tokens behind 0 to 30000, 2 to 32 KV
-  // heads and 1 to 16 sequences both estimates are right within 5 % in the mean, and two calls go to the slower kernel by more
-  // than 2 %).  64 tokens behind 2000 (1 sequence, 32 / 8 heads): 37 and 38 us; 128 behind 8000 (4 sequences): 113 and 148;
+  // heads and 1 to 16 sequences both estimates are right within 10 % (rms), no call goes to the slower kernel by more than 3 %
+  // here, and what the rule leaves to the SM-pair kernel would gain 0.7 % in the mean).  64 tokens behind 2000 (1 sequence, 32 / 8 heads): 37 and 38 us; 128 behind 8000 (4 sequences): 113 and 148;
   // 512 behind 8000 (4 sequences, 16 / 2 heads): 217 and 161; 16 x 64 tokens: 41 and 24.
-  return p.kv_bytes > 0 && p.us < 0.98 * attention_c2_us(B, Hq, Sq, Hkv, Sk) && B * Hkv < ((int64_t)1 << 31) && p.rows < ((int64_t)1 << 31) - kRows &&
+  return p.kv_bytes > 0 && p.us < 0.98 * attention_c2_us(B, Hq, Sq, Hkv, Sk, d) && B * Hkv < ((int64_t)1 << 31) && p.rows < ((int64_t)1 << 31) - kRows &&
          p.pairs * p.blocks * 32 < ((int64_t)1 << 31) && p.pairs <= 65535;
 }
 size_t attention_dense_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
@@ -738,13 +738,15 @@ int attention_dense(const AttnArgs& a, int64_t B, int d, int bits, const void* q
   const DensePlan p = dense_plan(B, a.Hq, a.Sq, a.Hkv, a.Sk, d);
   const ConstLayout L = const_layout(d);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  ProfScope prof(kProfAttention, stream);
   for (int64_t p0 = 0; p0 < B * a.Hkv; p0 += p.pairs) {
     const int pairs = (int)std::min<int64_t>(B * a.Hkv - p0, p.pairs);
     const ExpandArgs e{a.key_idx, a.key_sgn, a.key_vn, a.key_rn, a.val_idx, a.val_vn, a.kv_stride, a.Sk, constants + L.x_key,
                        constants + L.x_val, reinterpret_cast<const uint32_t*>(constants + L.luts),
                        reinterpret_cast<const float*>(constants + L.header) + kExpandScaleWord, p0, pairs, (int)p.T, 0, ws};
-    if (int st = expand_kv(e, d, bits, stream)) return st;
+    {
+      ProfScope prof(kProfPrepareQueries, stream);
+      if (int st = expand_kv(e, d, bits, stream)) return st;
+    }
     const int group = (int)std::min<int64_t>(pairs, std::max<int64_t>(1, kGroupBytes / (p.T * 2 * kBN * d * 2)));
     DenseArgs x{q, q_dtype, sb, sh, ss, ws, (int)p.T, (int)p.rows, FastDiv((uint32_t)(a.Hq / a.Hkv)), FastDiv((uint32_t)a.Hkv), p0,
                 (int)p.blocks, pairs, p.nsplit, FastDiv((uint32_t)(group * p.blocks)),
@@ -754,6 +756,7 @@ int attention_dense(const AttnArgs& a, int64_t B, int d, int bits, const void* q
       x.part_o = reinterpret_cast<float*>(ws + p.kv_bytes);
       x.part_ml = x.part_o + (size_t)p.pairs * p.blocks * 2 * p.nsplit * kBM * d;
     }
+    ProfScope prof(kProfAttention, stream);
     if (int st = d == 128 ? launch_kind<128>(a, x, stream) : launch_kind<64>(a, x, stream)) return st;
   }
   return TQ_OK;

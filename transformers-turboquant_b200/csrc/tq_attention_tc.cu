@@ -4,7 +4,8 @@
 //                    decoded to bf16 operand tiles in shared memory, S = [q_rot | q_s] * K_hat^T and
 //                    O += P * V_hat run as tcgen05 MMAs with fp32 accumulators in tensor memory,
 //                    causal online softmax on the CUDA cores in between.
-// Nothing of size Sq x Sk and no decompressed K/V ever reaches HBM.
+// Nothing of size Sq x Sk reaches HBM, and no decompressed K/V from these kernels (tq_expand.cu expands them where queries
+// meet them often enough).
 //
 // Estimator algebra (reference compressors.py:201-224, kernels/attention.py:380-461):
 //   score(q,k) = n_k <q_rot, C[idx_k]> + coeff rn_k <q_s, sgn_k>
