@@ -32,6 +32,20 @@ def test_rope_equals_hf_bit_for_bit(dtype, B, Hq, Hkv, S, d, broadcast):
     assert torch.equal(got_q, want_q) and torch.equal(got_k, want_k)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_any_bit_pattern_rounds_as_separate_kernels_round(dtype):
+    """Subnormals, values near overflow, zeros of either sign and infinities: the same bits; NaN where HF has NaN."""
+    from transformers.models.llama.modeling_llama import apply_rotary_pos_emb
+    from turboquant_b200 import rope
+    g = torch.Generator(device="cuda").manual_seed(3)
+    bits = lambda *shape: torch.randint(-32768, 32768, shape, generator=g, device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    q, k, cos, sin = bits(2, 700, 8, 128).transpose(1, 2), bits(2, 700, 2, 128).transpose(1, 2), bits(1, 700, 128), bits(1, 700, 128)
+    for got, want in zip(rope(q, k, cos, sin), apply_rotary_pos_emb(q, k, cos, sin)):
+        nan = want.isnan()
+        assert torch.equal(got.isnan(), nan)
+        assert torch.equal(got.view(torch.int16)[~nan], want.view(torch.int16)[~nan])
+
+
 def test_rope_rejects_what_it_does_not_cover():
     from turboquant_b200 import rope
     from turboquant_b200.rotary import rope_applies

@@ -54,23 +54,6 @@ constexpr int kLoadWarp = 8, kMmaWarp = 9;
 constexpr int kMapWords = 64;         // tiles of the mask maps / 32: masks of more keys are read without skipping
 constexpr int kBars = 2 * kSlots + 21;
 
-// Division of any 32-bit n by a launch constant (Granlund and Montgomery, 1994).
-struct FastDiv {
-  uint32_t d, m, s1, s2;
-  FastDiv() = default;
-  explicit FastDiv(uint32_t v) : d(v) {
-    int l = 0;
-    while (l < 32 && (1ull << l) < v) ++l;
-    m = (uint32_t)(((1ull << 32) * ((1ull << l) - v)) / v + 1);
-    s1 = l < 1 ? l : 1;
-    s2 = l > 1 ? l - 1 : 0;
-  }
-  __device__ __forceinline__ uint32_t div(uint32_t n) const {
-    const uint32_t t = __umulhi(m, n);
-    return (t + ((n - t) >> s1)) >> s2;
-  }
-};
-
 struct DenseArgs {
   const void* q;
   int q_dtype;

@@ -180,6 +180,23 @@ __device__ __forceinline__ uint64_t load_fields8(const uint8_t* src) {
   return word;
 }
 
+// Division of any 32-bit n by a launch constant (Granlund and Montgomery, 1994).
+struct FastDiv {
+  uint32_t d, m, s1, s2;
+  FastDiv() = default;
+  explicit FastDiv(uint32_t v) : d(v) {
+    int l = 0;
+    while (l < 32 && (1ull << l) < v) ++l;
+    m = (uint32_t)(((1ull << 32) * ((1ull << l) - v)) / v + 1);
+    s1 = l < 1 ? l : 1;
+    s2 = l > 1 ? l - 1 : 0;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const {
+    const uint32_t t = __umulhi(m, n);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
+
 // Programmatic dependent launch.  `wait` returns when the kernel that this one was launched behind has finished and its writes
 // are visible (at once when the kernel was launched without the attribute); `launch_dependents` lets the next
 // kernel of the stream start.

@@ -22,82 +22,88 @@ struct RopeArgs {
   int64_t B, Hq, Hkv, S;
   int64_t qsb, qsh, qss, ksb, ksh, kss, csb, css;  // element strides
   int d;
+  FastDiv div_c, div_h, div_s;  // chunks of half a row, heads, positions
 };
 
+// Two elements (fp32: one) as a unit of arithmetic.  The packed 16-bit instructions round each product and sum once, which is
+// what rounding the fp32 result does: a product of 16-bit numbers is exact in fp32, and 24 bits are enough (2 p + 2) for the
+// second rounding of a sum to change nothing.  `_rn` forms: never contracted to a fused multiply-add.
 template <int DTYPE>
-struct Elem;
+struct Pair;
 template <>
-struct Elem<TQ_BF16> {
-  using T = __nv_bfloat16;
-  static __device__ __forceinline__ float up(T v) { return __bfloat162float(v); }
-  static __device__ __forceinline__ float rn(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-  static __device__ __forceinline__ T down(float v) { return __float2bfloat16_rn(v); }
+struct Pair<TQ_BF16> {
+  using T = __nv_bfloat162;
+  static __device__ __forceinline__ T mul(T a, T b) { return __hmul2_rn(a, b); }
+  static __device__ __forceinline__ T add(T a, T b) { return __hadd2_rn(a, b); }
+  static __device__ __forceinline__ T sub(T a, T b) { return __hsub2_rn(a, b); }
 };
 template <>
-struct Elem<TQ_F16> {
-  using T = __half;
-  static __device__ __forceinline__ float up(T v) { return __half2float(v); }
-  static __device__ __forceinline__ float rn(float v) { return __half2float(__float2half_rn(v)); }
-  static __device__ __forceinline__ T down(float v) { return __float2half_rn(v); }
+struct Pair<TQ_F16> {
+  using T = __half2;
+  static __device__ __forceinline__ T mul(T a, T b) { return __hmul2_rn(a, b); }
+  static __device__ __forceinline__ T add(T a, T b) { return __hadd2_rn(a, b); }
+  static __device__ __forceinline__ T sub(T a, T b) { return __hsub2_rn(a, b); }
 };
 template <>
-struct Elem<TQ_F32> {
+struct Pair<TQ_F32> {
   using T = float;
-  static __device__ __forceinline__ float up(T v) { return v; }
-  static __device__ __forceinline__ float rn(float v) { return v; }
-  static __device__ __forceinline__ T down(float v) { return v; }
+  static __device__ __forceinline__ T mul(T a, T b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ T add(T a, T b) { return __fadd_rn(a, b); }
+  static __device__ __forceinline__ T sub(T a, T b) { return __fsub_rn(a, b); }
 };
 
 // 16 bytes of a row
-template <typename T>
+template <int DTYPE>
 struct alignas(16) Chunk {
-  T v[16 / sizeof(T)];
+  typename Pair<DTYPE>::T v[4];
 };
 
 // One work item = one 16-byte chunk of the first half of a row and its partner in the second half.
 // Items are numbered in the memory order of the projection output ([B, S, H, D]: consecutive threads read
 // consecutive bytes); each output row is written in two 16-byte-per-thread runs.
 // IDX: uint32_t when the item count fits (64-bit divisions would otherwise dominate the instruction stream).
+// Eight CTAs per SM at 32 registers (8 x 4096 tokens of 32 + 8 heads: 129 us; six at 40: 137; two items per thread at 56: 150,
+// at 48: 192; one item per thread without the loop: 139).
 template <int DTYPE, typename IDX>
-__global__ void __launch_bounds__(256) rope_kernel(const RopeArgs a) {
-  using E = Elem<DTYPE>;
-  using T = typename E::T;
-  constexpr int N = 16 / (int)sizeof(T);  // elements per chunk
-  const int half = a.d / 2;
-  const IDX cpr = (IDX)(half / N);  // chunks per half row
-  const IDX H = (IDX)(a.Hq + a.Hkv), S = (IDX)a.S;
+__global__ void __launch_bounds__(256, 8) rope_kernel(const RopeArgs a) {
+  using P = Pair<DTYPE>;
+  using C = Chunk<DTYPE>;
+  constexpr int64_t E = DTYPE == TQ_F32 ? 4 : 2;  // bytes of an element
+  const int half = a.d / 2 * (int)E;  // bytes of half a row
+  const IDX cpr = (IDX)a.div_c.d, H = (IDX)(a.Hq + a.Hkv), S = (IDX)a.S;
   const IDX items = (IDX)a.B * S * H * cpr;
   for (IDX it = (IDX)blockIdx.x * blockDim.x + threadIdx.x; it < items; it += (IDX)gridDim.x * blockDim.x) {
-    const int c = (int)(it % cpr);
-    IDX r = it / cpr;
-    const int64_t h = (int64_t)(r % H);
-    r /= H;
-    const int64_t s = (int64_t)(r % S), b = (int64_t)(r / S);
+    IDX row, pos, b;
+    if constexpr (sizeof(IDX) == 4) {
+      row = a.div_c.div(it);
+      pos = a.div_h.div(row);
+      b = a.div_s.div(pos);
+    } else {
+      row = it / cpr;
+      pos = row / H;
+      b = pos / S;
+    }
+    const int c = (int)(it - row * cpr) * 16;
+    const int64_t h = (int64_t)(row - pos * H), s = (int64_t)(pos - b * S), bb = (int64_t)b;
     const bool is_q = h < a.Hq;
     const int64_t hh = is_q ? h : h - a.Hq;
-    const T* src = is_q ? static_cast<const T*>(a.q) + b * a.qsb + hh * a.qsh + s * a.qss
-                        : static_cast<const T*>(a.k) + b * a.ksb + hh * a.ksh + s * a.kss;
-    T* dst = is_q ? static_cast<T*>(a.q_out) + ((b * a.Hq + hh) * a.S + s) * a.d
-                  : static_cast<T*>(a.k_out) + ((b * a.Hkv + hh) * a.S + s) * a.d;
-    const T* cs = static_cast<const T*>(a.cos) + b * a.csb + s * a.css;
-    const T* sn = static_cast<const T*>(a.sin) + b * a.csb + s * a.css;
-    const Chunk<T> xlo = *reinterpret_cast<const Chunk<T>*>(src + c * N);
-    const Chunk<T> xhi = *reinterpret_cast<const Chunk<T>*>(src + half + c * N);
-    const Chunk<T> clo = *reinterpret_cast<const Chunk<T>*>(cs + c * N);
-    const Chunk<T> chi = *reinterpret_cast<const Chunk<T>*>(cs + half + c * N);
-    const Chunk<T> slo = *reinterpret_cast<const Chunk<T>*>(sn + c * N);
-    const Chunk<T> shi = *reinterpret_cast<const Chunk<T>*>(sn + half + c * N);
-    Chunk<T> olo, ohi;
+    const uint8_t* src = static_cast<const uint8_t*>(is_q ? a.q : a.k) +
+                         (is_q ? bb * a.qsb + hh * a.qsh + s * a.qss : bb * a.ksb + hh * a.ksh + s * a.kss) * E + c;
+    uint8_t* dst = static_cast<uint8_t*>(is_q ? a.q_out : a.k_out) + ((bb * (is_q ? a.Hq : a.Hkv) + hh) * a.S + s) * a.d * E + c;
+    const int64_t at = (bb * a.csb + s * a.css) * E + c;
+    const uint8_t *cs = static_cast<const uint8_t*>(a.cos) + at, *sn = static_cast<const uint8_t*>(a.sin) + at;
+    const C xlo = *reinterpret_cast<const C*>(src), xhi = *reinterpret_cast<const C*>(src + half);
+    const C clo = *reinterpret_cast<const C*>(cs), chi = *reinterpret_cast<const C*>(cs + half);
+    const C slo = *reinterpret_cast<const C*>(sn), shi = *reinterpret_cast<const C*>(sn + half);
+    C olo, ohi;
 #pragma unroll
-    for (int e = 0; e < N; ++e) {
-      const float lo = E::up(xlo.v[e]), hi = E::up(xhi.v[e]);
-      // out[i] = x[i] cos[i] - x[i + d/2] sin[i];  out[i + d/2] = x[i + d/2] cos[i + d/2] + x[i] sin[i + d/2];
-      // each product and the sum rounded to the tensor dtype (no fused multiply-add)
-      olo.v[e] = E::down(__fadd_rn(E::rn(__fmul_rn(lo, E::up(clo.v[e]))), E::rn(__fmul_rn(-hi, E::up(slo.v[e])))));
-      ohi.v[e] = E::down(__fadd_rn(E::rn(__fmul_rn(hi, E::up(chi.v[e]))), E::rn(__fmul_rn(lo, E::up(shi.v[e])))));
+    for (int e = 0; e < 4; ++e) {
+      // out[i] = x[i] cos[i] - x[i + d/2] sin[i];  out[i + d/2] = x[i + d/2] cos[i + d/2] + x[i] sin[i + d/2]
+      olo.v[e] = P::sub(P::mul(xlo.v[e], clo.v[e]), P::mul(xhi.v[e], slo.v[e]));
+      ohi.v[e] = P::add(P::mul(xhi.v[e], chi.v[e]), P::mul(xlo.v[e], shi.v[e]));
     }
-    *reinterpret_cast<Chunk<T>*>(dst + c * N) = olo;
-    *reinterpret_cast<Chunk<T>*>(dst + half + c * N) = ohi;
+    *reinterpret_cast<C*>(dst) = olo;
+    *reinterpret_cast<C*>(dst + half) = ohi;
   }
 }
 
@@ -129,7 +135,8 @@ extern "C" int tq_rope(const void* q, const void* k, int dtype, int64_t B, int64
   CallScope scope(Hq > 0 ? q : k, "q", s);
   if (scope.status()) return scope.status();
   const RopeArgs a{q, k, cos, sin, q_out, k_out, B, Hq, Hkv, S, q_stride_b, q_stride_h, q_stride_s,
-                   k_stride_b, k_stride_h, k_stride_s, cs_stride_b, cs_stride_s, d};
+                   k_stride_b, k_stride_h, k_stride_s, cs_stride_b, cs_stride_s, d,
+                   FastDiv((uint32_t)(d / 2 / n)), FastDiv((uint32_t)(Hq + Hkv)), FastDiv((uint32_t)S)};
   const int64_t items = B * S * (Hq + Hkv) * (d / 2 / n);
   int dev = 0, sms = 148;
   TQ_CUDA_OK(cudaGetDevice(&dev));
