@@ -128,6 +128,9 @@ struct ImageArgs {
   __nv_bfloat16 *hi[3], *lo[3];
   __half *hi16[3], *lo16[3];
   float* scales;  // of Pi_k and Pi_v, and the inverse of the first
+  __half *x_key, *x_val;  // (blockIdx.y from 3 on) images of the expansion, sqrt(pi/2)/d, scales
+  float coeff;
+  float* x_scales;
 };
 // The power of two nearest the inverse of sqrt(mean square), 1 within a factor of sqrt(2); matrices beyond 2^20 either way
 // are scaled by 2^20.
@@ -136,44 +139,12 @@ __device__ __forceinline__ int rms_exponent(double mean_square) {
   const double e = rint(-0.5 * log2(mean_square));
   return e < -20.0 ? -20 : e > 20.0 ? 20 : (int)e;
 }
-__global__ void build_split_images_kernel(const ImageArgs a, int d) {
-  __shared__ double s_part[4];
-  const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
-  const float v = a.src[m][j * d + i];
-  double ss = 0.0;  // of the whole rotation, or of this row of the sketch
-  if (m == 1) ss = (double)v * v;
-  else
-    for (int r = 0; r < d; ++r) {
-      const double w = a.src[m][r * d + i];
-      ss += w * w;
-    }
-  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-  if (i % 32 == 0) s_part[i / 32] = ss;
-  __syncthreads();
-  ss = 0.0;
-  for (int w = 0; w < d / 32; ++w) ss += s_part[w];
-  const int e = rms_exponent(ss / d);  // (a rotation has d rows of norm 1, a row of the sketch d entries of size 1)
-  const float scale16 = ldexpf(m == 1 ? 1.f : kPi16Scale, e);
-  if (j == 0 && i == 0 && m != 1) {
-    a.scales[m / 2] = scale16;
-    if (m == 0) a.scales[2] = 1.f / scale16;
-  }
-  const int at = operand_index(j, i, d, d);
-  a.copy[m][j * d + i] = v;
-  const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  a.hi[m][at] = h;
-  a.lo[m][at] = __float2bfloat16_rn(v - __bfloat162float(h));
-  const float w = v * scale16;
-  const __half g = __float2half_rn(w);
-  a.hi16[m][at] = g;
-  a.lo16[m][at] = __float2half_rn(w - __half2float(g));
-}
-// Operand images of the expansion (blockIdx.y: Pi_k^T, (S_eff Pi_k)^T, Pi_v^T), K-major fp16, scaled to entries of about 1.
-__global__ void build_expand_images_kernel(const float* __restrict__ Pi_k, const float* __restrict__ S_eff,
-                                           const float* __restrict__ Pi_v, int d, float coeff, __half* __restrict__ x_key,
-                                           __half* __restrict__ x_val, float* __restrict__ scales) {
+// Operand images of the expansion (m: Pi_k^T, (S_eff Pi_k)^T, Pi_v^T), K-major fp16, scaled to entries of about 1.
+__device__ __forceinline__ void build_expand_images(const float* __restrict__ Pi_k, const float* __restrict__ S_eff,
+                                                    const float* __restrict__ Pi_v, int d, float coeff, __half* __restrict__ x_key,
+                                                    __half* __restrict__ x_val, float* __restrict__ scales, int m) {
   __shared__ float s_part[2][4];
-  const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
+  const int j = blockIdx.x, i = threadIdx.x;
   const float* Pi = m == 2 ? Pi_v : Pi_k;
   float pp = 0.f, ss = 0.f, acc = 0.f;
 #pragma unroll 8
@@ -207,6 +178,42 @@ __global__ void build_expand_images_kernel(const float* __restrict__ Pi_k, const
   const float v = (m == 1 ? acc : Pi[j * d + i]) * scale;
   (m == 2 ? x_val : x_key + (m == 1 ? d * d : 0))[operand_index(i, j, d, d)] = __float2half_rn(v);
 }
+__global__ void build_split_images_kernel(const ImageArgs a, int d) {
+  __shared__ double s_part[4];
+  const int j = blockIdx.x, i = threadIdx.x, m = blockIdx.y;
+  if (m >= 3) {
+    build_expand_images(a.src[0], a.src[1], a.src[2], d, a.coeff, a.x_key, a.x_val, a.x_scales, m - 3);
+    return;
+  }
+  const float v = a.src[m][j * d + i];
+  double ss = 0.0;  // of the whole rotation, or of this row of the sketch
+  if (m == 1) ss = (double)v * v;
+  else
+    for (int r = 0; r < d; ++r) {
+      const double w = a.src[m][r * d + i];
+      ss += w * w;
+    }
+  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  if (i % 32 == 0) s_part[i / 32] = ss;
+  __syncthreads();
+  ss = 0.0;
+  for (int w = 0; w < d / 32; ++w) ss += s_part[w];
+  const int e = rms_exponent(ss / d);  // (a rotation has d rows of norm 1, a row of the sketch d entries of size 1)
+  const float scale16 = ldexpf(m == 1 ? 1.f : kPi16Scale, e);
+  if (j == 0 && i == 0 && m != 1) {
+    a.scales[m / 2] = scale16;
+    if (m == 0) a.scales[2] = 1.f / scale16;
+  }
+  const int at = operand_index(j, i, d, d);
+  a.copy[m][j * d + i] = v;
+  const __nv_bfloat16 h = __float2bfloat16_rn(v);
+  a.hi[m][at] = h;
+  a.lo[m][at] = __float2bfloat16_rn(v - __bfloat162float(h));
+  const float w = v * scale16;
+  const __half g = __float2half_rn(w);
+  a.hi16[m][at] = g;
+  a.lo16[m][at] = __float2half_rn(w - __half2float(g));
+}
 // The header, the codebooks and the pair tables (one block).
 struct CodebookArgs {
   const float* src[4];
@@ -236,23 +243,22 @@ int prepare_constants(const float* Pi_k, const float* S_eff, const float* cen_k,
   auto b16 = [&](size_t off) { return reinterpret_cast<__nv_bfloat16*>(c + off); };
   auto h16 = [&](size_t off) { return reinterpret_cast<__half*>(c + off); };
   const int kb = bits - 1, vb = bits;
+  const float coeff = sqrtf(1.5707963267948966f) / (float)d;
   const ImageArgs img{{Pi_k, S_eff, Pi_v},
                       {f32(L.pi_k), f32(L.s_eff), f32(L.pi_v)},
                       {b16(L.pik_hi), b16(L.se_hi), b16(L.piv_hi)},
                       {b16(L.pik_lo), b16(L.se_lo), b16(L.piv_lo)},
                       {h16(L.pik16_hi), h16(L.se16_hi), h16(L.piv16_hi)},
                       {h16(L.pik16_lo), h16(L.se16_lo), h16(L.piv16_lo)},
-                      f32(L.header) + kScaleWord};
-  build_split_images_kernel<<<dim3(d, 3), d, 0, stream>>>(img, d);
+                      f32(L.header) + kScaleWord,
+                      h16(L.x_key), h16(L.x_val), coeff, f32(L.header) + kExpandScaleWord};
+  build_split_images_kernel<<<dim3(d, 6), d, 0, stream>>>(img, d);
   const CodebookArgs cb{{cen_k, bnd_k, cen_v, bnd_v}, {f32(L.cen_k), f32(L.bnd_k), f32(L.cen_v), f32(L.bnd_v)},
                         {1 << kb, (1 << kb) - 1, 1 << vb, (1 << vb) - 1}, reinterpret_cast<uint32_t*>(c + L.header),
                         reinterpret_cast<uint32_t*>(c + L.luts), d, bits};
   copy_codebooks_kernel<<<1, 128, 0, stream>>>(cb);
-  const float coeff = sqrtf(1.5707963267948966f) / (float)d;
   build_wcat_kernel<<<d, d, 0, stream>>>(Pi_k, S_eff, d, coeff, b16(L.w_cat_pair), d, b16(L.w_cat_plain), 0);
   build_wunrot_kernel<<<d, d, 0, stream>>>(Pi_v, d, b16(L.w_unrot_pair), d / 2, b16(L.w_unrot_plain), 0);
-  build_expand_images_kernel<<<dim3(d, 3), d, 0, stream>>>(Pi_k, S_eff, Pi_v, d, coeff, h16(L.x_key), h16(L.x_val),
-                                                           f32(L.header) + kExpandScaleWord);
   TQ_CUDA_OK(cudaGetLastError());
   return TQ_OK;
 }
