@@ -217,8 +217,6 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
   }
   if (warp == kMmaWarp) tc::tmem_alloc(tc::smem_u32(&tmem_slot), 4 * D);
   grid_dependency_wait();
-  // The attention kernel may start: what it reads before it waits for this one (the queries) was there before this line.
-  grid_launch_dependents();
   if (tid == 0) {
     s_dead = *reinterpret_cast<volatile unsigned long long*>(&g_expand_faults) != 0ull ? 1 : 0;  // an earlier launch gave up
     s_abort = 0;
@@ -230,6 +228,10 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  // The attention kernel may start: what it reads before it waits for this one (the queries) was there before this line.  It
+  // takes all tensor memory of its SM at once and keeps it until it ends, so the barrier between the allocation above and this
+  // line has to stay: a CTA of this kernel that found none left would wait for a kernel that waits for it.
+  grid_launch_dependents();
   const uint32_t tmem = tmem_slot;
   bool ok = true;
   if (!s_dead) {
