@@ -257,9 +257,12 @@ __global__ void __launch_bounds__(kThreads, 1) attention_dense_kernel(const Attn
     float cexp = a.sm_scale * kLog2e;
     {
       // rows scaled by a power of two to fp16, into the operand tile
-      auto scale_of = [&](float m) {  // 2^(13 - exponent of m); a row of zeros or with an infinity stays as it is
+      // 2^(13 - exponent of m), 1 for a row of zeros or with an infinity; at most 2^64 cexp, so that 1 / cexp and with it the
+      // hidden keys' floor and the mask's unit stay finite.  A smaller row has scores below 2^-64: fp16 may flush it.
+      const uint32_t most = (__float_as_uint(cexp) >> 23) + 64u;
+      auto scale_of = [&](float m) {
         const uint32_t e = __float_as_uint(m) >> 23;
-        return e == 0u || e >= 255u ? 1.f : __uint_as_float((267u - max(e, 14u)) << 23);
+        return __uint_as_float(min(e == 0u || e >= 255u ? 127u : 267u - max(e, 14u), most) << 23);
       };
       float scale = 1.f;
       uint8_t* q_rows = smem + L::kQOff + w * L::kTile + warp % 4 * 4 * L::kSbo;  // this warp's 32 rows
