@@ -51,7 +51,7 @@ constexpr int kRows = 2 * kBM;        // rows of a CTA
 constexpr int kSlots = 5;             // ring of K' and V' tiles
 constexpr int kThreads = 384;
 constexpr int kLoadWarp = 8, kMmaWarp = 9;
-constexpr int kMapWords = 64;         // tiles of the mask maps / 32: masks of more keys are read without skipping
+constexpr int kMapWords = kMapTiles / 32;  // masks of more keys are read without skipping
 constexpr int kBars = 2 * kSlots + 21;
 
 struct DenseArgs {
@@ -724,11 +724,15 @@ int attention_dense(const AttnArgs& a, int64_t B, int d, int bits, const void* q
   const DensePlan p = dense_plan(B, a.Hq, a.Sq, a.Hkv, a.Sk, d);
   const ConstLayout L = const_layout(d);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
+  // Key tiles that a mask hides from every query are not expanded, where there are any to speak of: in front of a chunk.  (Prompts
+  // have those of their padding, whose rows average all keys of their causal range.)
+  const bool skip = a.mb.words != nullptr && p.T <= kMapTiles && a.Sk >= 2 * a.Sq;
   for (int64_t p0 = 0; p0 < B * a.Hkv; p0 += p.pairs) {
     const int pairs = (int)std::min<int64_t>(B * a.Hkv - p0, p.pairs);
     const ExpandArgs e{a.key_idx, a.key_sgn, a.key_vn, a.key_rn, a.val_idx, a.val_vn, a.kv_stride, a.Sk, constants + L.x_key,
                        constants + L.x_val, reinterpret_cast<const uint32_t*>(constants + L.luts),
-                       reinterpret_cast<const float*>(constants + L.header) + kExpandScaleWord, p0, pairs, (int)p.T, 0, ws};
+                       reinterpret_cast<const float*>(constants + L.header) + kExpandScaleWord, p0, pairs, (int)p.T, 0,
+                       skip ? a.mb : MaskBits{}, (int)a.Sq, 0, a.Hkv, ws};
     {
       ProfScope prof(kProfPrepareQueries, stream);
       if (int st = expand_kv(e, d, bits, stream)) return st;

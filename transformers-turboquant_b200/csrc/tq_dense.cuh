@@ -16,9 +16,15 @@ struct ExpandArgs {
   const float* scales;           // of index, sign and value accumulators
   int64_t pair0;                 // first pair
   int pairs, T, key_ctas;        // pairs, tiles of a pair; CTAs of the key side (set by the launcher)
+  MaskBits mb;                   // words != NULL: tiles that it hides from every query are left out
+  int Sq, parts;                 // queries; threads that share a tile's classes (set by the launcher)
+  int64_t Hkv;
   uint8_t* dst;
 };
 int expand_kv(const ExpandArgs& a, int d, int bits, cudaStream_t stream);
+
+// Tiles of the maps that the dense kernel skips masked key tiles by; where there are more, it reads every tile.
+constexpr int kMapTiles = 2048;
 
 // Whether a bf16-mode call of the SM-pair kernel's is served by expansion and the dense kernel when it has the scratch for it,
 // and that scratch.

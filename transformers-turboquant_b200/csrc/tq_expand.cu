@@ -13,6 +13,11 @@
 // A CTA does key tiles or value tiles: eight warps decode, one issues the MMAs, eight store, with two operand and two
 // accumulator slots between them.  Output tiles have the canonical core-matrix layout (16 bytes of eight consecutive rows
 // adjacent), which is the K-major operand of q K'^T and the MN-major operand of P V' at once: one contiguous copy each.
+#include <limits.h>
+
+#include <algorithm>
+#include <type_traits>
+
 #include "tq_attention.cuh"
 #include "tq_common.cuh"
 #include "tq_dense.cuh"
@@ -53,6 +58,74 @@ __device__ __forceinline__ uint4 signs8(uint32_t bits) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// Limits of a call whose hidden tiles are left out: tiles of a CTA, words of the map of tiles that are computed, and what a CTA
+// reads of the mask's summary to draw it.
+constexpr int kOwnTiles = 256, kLiveWords = 256, kListMapThreads = 384, kSummaryReads = 30 * kThreads;
+
+struct LiveMap {
+  uint32_t words[kLiveWords];  // [batch elements][(T + 31) / 32]: some query sees a key of the tile
+  uint8_t all[kLiveWords];     // [batch elements]: a row sees nothing and averages all keys of its causal range
+  int count[kLiveWords];       // [batch elements]: tiles that are computed
+  int tile[kOwnTiles + 1];     // this CTA's tiles, then one past the last of all
+};
+// This CTA's share of the tiles that some query computes, spread evenly over the CTAs.  `m.words` and `m.all` are zeros.  The
+// expansion waits for it, so the two halves of the summary are read side by side, and threads find their tiles without diverging.
+__device__ __forceinline__ void list_tiles(const ExpandArgs& a, int cta, int ctas, LiveMap& m) {
+  const int tid = threadIdx.x, W = (a.T + 31) / 32, b0 = a.mb.batch ? (int)(a.pair0 / a.Hkv) : 0;
+  const int nb = a.mb.batch ? (int)((a.pair0 + a.pairs - 1) / a.Hkv) - b0 + 1 : 1;
+  if (tid < kListMapThreads) {
+    for (int e = tid; e < nb * a.T * a.parts; e += kListMapThreads) {
+      const int bt = e / a.parts, bi = bt / a.T, t = bt - bi * a.T;
+      const uint8_t* cls = a.mb.tiles + (int64_t)(b0 + bi) * a.mb.NG * a.T + t;
+      uint32_t seen = 0;
+#pragma unroll 8
+      for (int g = e - bt * a.parts; g < a.mb.NG; g += a.parts) seen |= cls[(int64_t)g * a.T];
+      if ((seen & 1u) != 0u) atomicOr(&m.words[bi * W + t / 32], 1u << (t % 32));
+    }
+  } else {
+    for (int e = tid - kListMapThreads; e < nb * a.mb.NG; e += kThreads - kListMapThreads) {
+      const int bi = e / a.mb.NG, g = e - bi * a.mb.NG;
+      const uint32_t* rows = a.mb.rows + ((int64_t)b0 * a.mb.NG + e) * a.mb.NC;
+      uint32_t seen = 0;
+#pragma unroll 8
+      for (int c = 0; c < a.mb.NC; ++c) seen |= rows[c];
+      if ((~seen & ((1u << min(16, a.Sq - 16 * g)) - 1u)) != 0u) m.all[bi] = 1;
+    }
+  }
+  __syncthreads();
+  if (tid < nb) {
+    int n = 0;
+    for (int w = 0; w < W; ++w) n += __popc(m.words[tid * W + w]);
+    m.count[tid] = m.all[tid] ? a.T : n;
+  }
+  __syncthreads();
+  if (tid <= kOwnTiles) {
+    const int Hkv = (int)a.Hkv, head0 = a.mb.batch ? (int)(a.pair0 - (int64_t)b0 * Hkv) : 0;  // (of the first pair)
+    int at = tid < kOwnTiles ? cta + tid * ctas : INT_MAX, pair = 0, bi = 0, n = 1;
+    for (; bi < nb; ++bi) {
+      const int next = a.mb.batch ? min(a.pairs, (bi + 1) * Hkv - head0) : a.pairs;
+      n = m.count[bi];
+      if (at < n * (next - pair)) break;
+      at -= n * (next - pair);
+      pair = next;
+    }
+    int tile = a.pairs * a.T;
+    if (bi < nb) {
+      int t = at % n;
+      tile = (pair + at / n) * a.T;
+      if (!m.all[bi]) {  // the t-th bit of the map
+        int w = bi * W;
+        for (int c; (c = __popc(m.words[w])) <= t; ++w) t -= c;
+        uint32_t bits = m.words[w];
+        for (; t > 0; --t) bits &= bits - 1u;
+        t = (w - bi * W) * 32 + __ffs((int)bits) - 1;
+      }
+      tile += t;
+    }
+    m.tile[tid] = tile;
+  }
+}
+
 struct ExpandBars {
   uint32_t base;
   __device__ uint32_t a_full(int s) const { return base + 8u * s; }         // operand decoded: a decoding warp's arrival each
@@ -62,16 +135,24 @@ struct ExpandBars {
   __device__ uint32_t constants() const { return base + 8u * 8; }
 };
 
-template <int D, int BITS, bool KEY>
+// The tiles of a CTA: cta, cta + ctas, ..., or those of a list; `tiles` or more behind the last.
+template <bool LIST>
+struct OwnTiles {
+  int cta, ctas, tiles;
+  const int* list;
+  __device__ __forceinline__ int at(int i) const { return LIST ? list[i] : cta + i * ctas; }
+};
+
+template <int D, int BITS, bool KEY, bool LIST>
 __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem, const uint32_t* lut, const ExpandBars bar, uint32_t tmem,
-                                             volatile int* abort_flag, int cta, int ctas) {
+                                             volatile int* abort_flag, const OwnTiles<LIST> own) {
   constexpr int G = D / 8, NB = D / 32, B = KEY ? BITS - 1 : BITS;  // chunks and 32-coordinate blocks of a row, bits of an index
   constexpr int W = B + (KEY ? 1 : 0), NI = 128 * NB / (32 * kDecodeWarps);  // words of a block, blocks per decoding thread
   constexpr uint32_t MAT = D * D * 2, TILE = 128 * D * 2, SBO = G * 128;
   constexpr uint32_t kA = (KEY ? 2 : 1) * MAT, kASlot = (KEY ? 2 : 1) * TILE;  // operand slots behind the matrices
   const int tid = threadIdx.x, lane = tid % 32;
   const int warp = __shfl_sync(0xffffffffu, tid / 32, 0);
-  const int tiles = a.pairs * a.T;
+  const int tiles = own.tiles;
   bool ok = true;
   if (warp < kDecodeWarps) {
     uint32_t w[NI][W];
@@ -89,9 +170,9 @@ __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem,
         if (KEY) w[i][B] = live ? reinterpret_cast<const uint32_t*>(a.key_sgn + row * G)[c] : 0u;
       }
     };
-    int tile = cta;
+    int tile = own.at(0);
     if (tile < tiles) load(tile);
-    for (int i = 0; tile < tiles && ok; ++i, tile += ctas) {
+    for (int i = 0; tile < tiles && ok; ++i) {
       const int s = i & 1;
       if (i >= 2 && !(ok = tc::mbar_spin_or_abort(bar.a_empty(s), ((i >> 1) - 1) & 1, abort_flag))) break;
 #pragma unroll
@@ -106,7 +187,8 @@ __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem,
           if (KEY) *reinterpret_cast<uint4*>(dst + TILE + x * 128) = signs8(w[n][B] >> (8 * x));
         }
       }
-      if (tile + ctas < tiles) load(tile + ctas);
+      tile = own.at(i + 1);
+      if (tile < tiles) load(tile);
       tc::fence_async_smem();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(bar.a_full(s));
@@ -121,14 +203,16 @@ __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem,
       n0 = key < a.Sk ? (KEY ? a.key_vn : a.val_vn)[at] : (uint16_t)0;
       if (KEY) n1 = key < a.Sk ? a.key_rn[at] : (uint16_t)0;
     };
-    if (cta < tiles) load(cta);
-    for (int i = 0, tile = cta; tile < tiles && ok; ++i, tile += ctas) {
+    int tile = own.at(0);
+    if (tile < tiles) load(tile);
+    for (int i = 0, ahead; tile < tiles && ok; ++i, tile = ahead) {
       const int s = i & 1;
       const float f0 = fp16_value(n0) * scale0, f1 = fp16_value(n1) * scale1;
       // results stay finite where the norms are (a key of length 6e4 may come out a little longer than fp16 reaches)
       const bool finite = (n0 & 0x7c00u) != 0x7c00u && (n1 & 0x7c00u) != 0x7c00u;
       const bool live = tile % a.T * 128 + row < a.Sk;
-      if (tile + ctas < tiles) load(tile + ctas);
+      ahead = own.at(i + 1);
+      if (ahead < tiles) load(ahead);
       if (!(ok = tc::mbar_spin_or_abort(bar.d_full(s), (i >> 1) & 1, abort_flag))) break;
       tc::fence_after_sync();
       uint8_t* out = a.dst + ((int64_t)tile * 2 + (KEY ? 0 : 1)) * TILE + (row / 8) * SBO + (row % 8) * 16;
@@ -172,7 +256,7 @@ __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem,
     const bool leader = tc::elect_one();
     ok = tc::mbar_wait_or_abort(bar.constants(), 0, abort_flag);
     int i = 0;
-    for (int tile = cta; tile < tiles && ok; ++i, tile += ctas) {
+    for (int tile = own.at(0); tile < tiles && ok; tile = own.at(++i)) {
       const int s = i & 1;
       if (!(ok = tc::mbar_spin_or_abort(bar.a_full(s), (i >> 1) & 1, abort_flag))) break;
       if (i >= 2 && !(ok = tc::mbar_spin_or_abort(bar.d_empty(s), ((i >> 1) - 1) & 1, abort_flag))) break;
@@ -198,7 +282,7 @@ __device__ __forceinline__ bool expand_tiles(const ExpandArgs& a, uint8_t* smem,
   return ok;
 }
 
-template <int D, int BITS>
+template <int D, int BITS, bool LIST>
 __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs a) {
   constexpr uint32_t MAT = D * D * 2;
   constexpr int NK = 1 << (2 * (BITS - 1)), NV = 1 << (2 * BITS);
@@ -207,8 +291,10 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
   __shared__ __align__(8) uint64_t bars[9];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort, s_dead;
+  __shared__ std::conditional_t<LIST, LiveMap, int> live;
   const int tid = threadIdx.x, warp = tid / 32;
   const bool key = (int)blockIdx.x < a.key_ctas;
+  const int cta = key ? blockIdx.x : blockIdx.x - a.key_ctas, ctas = key ? a.key_ctas : gridDim.x - a.key_ctas;
   const ExpandBars bar{tc::smem_u32(&bars[0])};
   if (tid == 0) {
     for (int i = 0; i < 9; ++i) tc::mbar_init(bar.base + 8 * i, i < 2 ? kDecodeWarps : i == 6 || i == 7 ? kStoreWarps : 1);
@@ -216,6 +302,10 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
     tc::fence_async_smem();
   }
   if (warp == kMmaWarp) tc::tmem_alloc(tc::smem_u32(&tmem_slot), 4 * D);
+  if constexpr (LIST) {
+    if (tid < kLiveWords) live.words[tid] = live.all[tid] = 0;
+    __syncthreads();
+  }
   grid_dependency_wait();
   if (tid == 0) {
     s_dead = *reinterpret_cast<volatile unsigned long long*>(&g_expand_faults) != 0ull ? 1 : 0;  // an earlier launch gave up
@@ -225,6 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
     tc::bulk_load(tc::smem_u32(smem), key ? a.w_key : a.w_val, bytes, bar.constants());
   }
   for (int e = tid; e < (key ? NK : NV); e += kThreads) lut[e] = a.luts[(key ? 0 : NK) + e];
+  if constexpr (LIST) list_tiles(a, cta, ctas, live);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -235,8 +326,10 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
   const uint32_t tmem = tmem_slot;
   bool ok = true;
   if (!s_dead) {
-    if (key) ok = expand_tiles<D, BITS, true>(a, smem, lut, bar, tmem, &s_abort, blockIdx.x, a.key_ctas);
-    else ok = expand_tiles<D, BITS, false>(a, smem, lut, bar, tmem, &s_abort, blockIdx.x - a.key_ctas, gridDim.x - a.key_ctas);
+    OwnTiles<LIST> own{cta, ctas, a.pairs * a.T, nullptr};
+    if constexpr (LIST) own.list = live.tile;
+    if (key) ok = expand_tiles<D, BITS, true>(a, smem, lut, bar, tmem, &s_abort, own);
+    else ok = expand_tiles<D, BITS, false>(a, smem, lut, bar, tmem, &s_abort, own);
   }
   if (warp == kMmaWarp) tc::mbar_wait_bounded(bar.constants(), 0, 400000000ll);  // (landed long ago but for a CTA that gave up)
   if (!ok && atomicExch(&s_abort, 2) != 2) {  // one fault per CTA
@@ -248,12 +341,11 @@ __global__ void __launch_bounds__(kThreads, 1) expand_kv_kernel(const ExpandArgs
   if (warp == kMmaWarp) tc::tmem_dealloc(tmem, 4 * D);
 }
 
-template <int D, int BITS>
-int launch(const ExpandArgs& args, cudaStream_t stream) {
+template <int D, int BITS, bool LIST>
+int launch(ExpandArgs a, cudaStream_t stream) {
   constexpr size_t smem = (size_t)2 * D * D * 2 + (size_t)2 * 2 * 128 * D * 2;
-  auto kern = expand_kv_kernel<D, BITS>;
+  auto kern = expand_kv_kernel<D, BITS, LIST>;
   TQ_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  ExpandArgs a = args;
   const int64_t tiles = (int64_t)a.pairs * a.T;
   // A CTA per tile where that many fit the chip; otherwise three fifths of the CTAs take the keys, which cost twice the
   // MMAs and half as much again of everything else.
@@ -270,11 +362,29 @@ int launch(const ExpandArgs& args, cudaStream_t stream) {
   return TQ_OK;
 }
 
+// Tiles that a mask hides from every query are left out where the map of them is drawn in a few rounds of loads, about 2 us.
+// 32 / 8 heads of 128 under a window of 64 keys, us with all tiles expanded and so: 256 tokens behind 7936, 4 sequences, 93 and
+// 38; 64 behind 29936 91 and 38; 300 behind 8000 50 and 40 (the SM-pair kernel: 23).  A mask that hides a tenth: 64 behind 4032,
+// 8 sequences, 16 / 2 heads, 60.6 and 62.3; 64 behind 29936 123 and 122.  The summary of more queries takes longer to look
+// through than its tiles are worth beside the attention over them.
+bool lists_tiles(ExpandArgs& a) {
+  if (a.mb.words == nullptr) return false;
+  const int64_t tiles = (int64_t)a.pairs * a.T, sms = sm_count();
+  const int64_t nb = a.mb.batch ? (a.pair0 + a.pairs - 1) / a.Hkv - a.pair0 / a.Hkv + 1 : 1;
+  a.parts = (int)std::max<int64_t>(1, std::min<int64_t>(a.mb.NG, kListMapThreads / (nb * a.T)));
+  return (2 * tiles <= sms || tiles <= kOwnTiles * (sms - sms * 3 / 5)) && nb * ((a.T + 31) / 32) <= kLiveWords &&
+         nb * a.mb.NG * ((int64_t)a.T + a.mb.NC) <= kSummaryReads;
+}
+template <int D>
+int launch_bits(ExpandArgs a, int bits, cudaStream_t stream) {
+  if (lists_tiles(a)) return bits == 2 ? launch<D, 2, true>(a, stream) : bits == 3 ? launch<D, 3, true>(a, stream) : launch<D, 4, true>(a, stream);
+  return bits == 2 ? launch<D, 2, false>(a, stream) : bits == 3 ? launch<D, 3, false>(a, stream) : launch<D, 4, false>(a, stream);
+}
+
 }  // namespace
 
 int expand_kv(const ExpandArgs& a, int d, int bits, cudaStream_t stream) {
-  if (d == 128) return bits == 2 ? launch<128, 2>(a, stream) : bits == 3 ? launch<128, 3>(a, stream) : launch<128, 4>(a, stream);
-  return bits == 2 ? launch<64, 2>(a, stream) : bits == 3 ? launch<64, 3>(a, stream) : launch<64, 4>(a, stream);
+  return d == 128 ? launch_bits<128>(a, bits, stream) : launch_bits<64>(a, bits, stream);
 }
 
 }  // namespace tq
