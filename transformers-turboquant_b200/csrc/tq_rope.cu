@@ -10,6 +10,7 @@
 // HBM-bound: 2 x (B (Hq + Hkv) S D) elements in + out, plus the cos/sin rows (shared by all heads: L2).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <string.h>
 
 #include "tq_common.cuh"
 
@@ -52,18 +53,31 @@ struct Pair<TQ_F32> {
   static __device__ __forceinline__ T sub(T a, T b) { return __fsub_rn(a, b); }
 };
 
-// 16 bytes of a row
+// 16 bytes of a row.  They move as one vector: a copy of the struct is four copies of its elements, whose stores leave half-filled
+// lines behind where half a row is less than a line (8 x 1024 tokens, 12 + 12 heads of 64, bf16: 18.2 us so, 8.7 as vectors;
+// 4 x 4096, 32 + 8 heads of 64: 52 and 32).
 template <int DTYPE>
-struct alignas(16) Chunk {
+struct Chunk {
   typename Pair<DTYPE>::T v[4];
+  static __device__ __forceinline__ Chunk load(const uint8_t* p) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    Chunk c;
+    memcpy(&c, &u, 16);
+    return c;
+  }
+  __device__ __forceinline__ void store(uint8_t* p) const {
+    uint4 u;
+    memcpy(&u, this, 16);
+    *reinterpret_cast<uint4*>(p) = u;
+  }
 };
 
 // One work item = one 16-byte chunk of the first half of a row and its partner in the second half.
 // Items are numbered in the memory order of the projection output ([B, S, H, D]: consecutive threads read
 // consecutive bytes); each output row is written in two 16-byte-per-thread runs.
 // IDX: uint32_t when the item count fits (64-bit divisions would otherwise dominate the instruction stream).
-// Eight CTAs per SM at 32 registers (8 x 4096 tokens of 32 + 8 heads: 129 us; six at 40: 137; two items per thread at 56: 150,
-// at 48: 192; one item per thread without the loop: 139).
+// Eight CTAs per SM at 32 registers (8 x 4096 tokens of 32 + 8 heads of 128: 119 us, as six at 40 or four at 44; 1000 tokens: 4.1
+// us, and 4.3 or 4.4).
 template <int DTYPE, typename IDX>
 __global__ void __launch_bounds__(256, 8) rope_kernel(const RopeArgs a) {
   using P = Pair<DTYPE>;
@@ -92,9 +106,8 @@ __global__ void __launch_bounds__(256, 8) rope_kernel(const RopeArgs a) {
     uint8_t* dst = static_cast<uint8_t*>(is_q ? a.q_out : a.k_out) + ((bb * (is_q ? a.Hq : a.Hkv) + hh) * a.S + s) * a.d * E + c;
     const int64_t at = (bb * a.csb + s * a.css) * E + c;
     const uint8_t *cs = static_cast<const uint8_t*>(a.cos) + at, *sn = static_cast<const uint8_t*>(a.sin) + at;
-    const C xlo = *reinterpret_cast<const C*>(src), xhi = *reinterpret_cast<const C*>(src + half);
-    const C clo = *reinterpret_cast<const C*>(cs), chi = *reinterpret_cast<const C*>(cs + half);
-    const C slo = *reinterpret_cast<const C*>(sn), shi = *reinterpret_cast<const C*>(sn + half);
+    const C xlo = C::load(src), xhi = C::load(src + half);
+    const C clo = C::load(cs), chi = C::load(cs + half), slo = C::load(sn), shi = C::load(sn + half);
     C olo, ohi;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -102,8 +115,8 @@ __global__ void __launch_bounds__(256, 8) rope_kernel(const RopeArgs a) {
       olo.v[e] = P::sub(P::mul(xlo.v[e], clo.v[e]), P::mul(xhi.v[e], slo.v[e]));
       ohi.v[e] = P::add(P::mul(xhi.v[e], chi.v[e]), P::mul(xlo.v[e], shi.v[e]));
     }
-    *reinterpret_cast<C*>(dst) = olo;
-    *reinterpret_cast<C*>(dst + half) = ohi;
+    olo.store(dst);
+    ohi.store(dst + half);
   }
 }
 
