@@ -262,6 +262,9 @@ size_t tq_attention_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, in
  *   mask        : optional additive fp32 mask, element (b, i, k) at
  *                 mask[b*mask_stride_b + i*mask_stride_q + k]; NULL for none.
  *   out         : [B, Hq, Sq, d] of `dtype` with the given element strides.
+ *   Packed rows: norms 2 bytes aligned; in TQ_MODE_BF16 packed rows of head_dim 128 start on 16-byte boundaries and those of
+ *   head_dim 64 on 8-byte boundaries, as rows of an aligned array do.  Kernels that read them in smaller units take less; what
+ *   the kernel of a call cannot read is refused with TQ_ERR_INVALID_ARG before a launch.  In TQ_MODE_FP32 rows start anywhere.
  * Replaces the attention core of the family adapters
  * (src/transformers_turboquant/families/llama.py:100-114, gpt2.py:90-110). */
 int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d,

@@ -111,6 +111,9 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
                        cudaStream_t stream, const uint8_t* prepared = nullptr);
 // Whether the SM-pair kernel serves a bf16-mode call (its only scratch are the partial results of a split call).
 bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride, int d);
+// TQ_OK where the kernel that serves a bf16-mode call can read packed rows and norms at their addresses (`prepared`: with a
+// constants buffer; `scratch`: with any scratch).
+int check_packed_rows_bf16(const AttnArgs& a, int64_t B, int64_t Sq, int d, int bits, bool prepared, bool scratch);
 // scratch bytes of a bf16-mode call with a prepared constants buffer, by the kernel that will serve it
 size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                      int d);

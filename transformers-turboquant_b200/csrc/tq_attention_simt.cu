@@ -1001,11 +1001,13 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
     return fail(TQ_ERR_WORKSPACE, "workspace of %zu bytes needed (256-byte aligned), got %zu", need,
                 workspace_bytes);
-  CallScope scope(q, "q", static_cast<cudaStream_t>(stream));
-  if (scope.status()) return scope.status();
   AttnArgs a{nullptr, Hq, Sq, Hkv, Sk, key_idx, key_signs, key_vec_norms, key_residual_norms, val_idx,
              val_vec_norms, centroids_k, centroids_v, Pi_v, sm_scale, causal, mask, mask_stride_b, mask_stride_q,
              out, dtype, o_stride_b, o_stride_h, o_stride_s, kv_stride, MaskBits{}};
+  if (mode == TQ_MODE_BF16)
+    if (int st = check_packed_rows_bf16(a, B, Sq, d, bits, prepared != nullptr, workspace != nullptr)) return st;
+  CallScope scope(q, "q", static_cast<cudaStream_t>(stream));
+  if (scope.status()) return scope.status();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (src != nullptr) {
     a.mb = mask_bits_layout(src->nb, Sq, Sk, static_cast<uint8_t*>(workspace) + call_need, nullptr);

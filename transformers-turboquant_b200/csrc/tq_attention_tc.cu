@@ -1013,6 +1013,24 @@ bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
   return bf16_path(a, Sq, d) == Bf16Path::kPairs;
 }
 
+static bool on_words(const AttnArgs& a) {
+  return ((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) | reinterpret_cast<uintptr_t>(a.val_idx)) & 3u) == 0;
+}
+
+int check_packed_rows_bf16(const AttnArgs& a, int64_t B, int64_t Sq, int d, int bits, bool prepared, bool scratch) {
+  const Bf16Path path = bf16_path(a, Sq, d);
+  const bool expand = path == Bf16Path::kPairs && prepared && scratch && on_words(a) && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d);
+  // (the SM-pair kernel loads half a value row per CTA, in words where that is 12 bytes)
+  const unsigned keys = expand ? 4 : path == Bf16Path::kDecode ? 16 : 8;
+  const unsigned values = path == Bf16Path::kPairs && d == 64 && bits == 3 ? 4 : keys;
+  TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn)) & (keys - 1)) == 0 &&
+                 (reinterpret_cast<uintptr_t>(a.val_idx) & (values - 1)) == 0,
+             "packed rows must start on boundaries of %u bytes (keys) and %u (values) for this call in bf16 mode", keys, values);
+  TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_vn) | reinterpret_cast<uintptr_t>(a.key_rn) | reinterpret_cast<uintptr_t>(a.val_vn)) & 1u) == 0,
+             "norms must be 2-byte aligned");
+  return TQ_OK;
+}
+
 size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                      int d) {
   AttnArgs a{};
@@ -1058,8 +1076,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
   __nv_bfloat16* o_rot = reinterpret_cast<__nv_bfloat16*>(ws);
 
   // (packed rows are read in words there)
-  if (pairs && prepared != nullptr && workspace != nullptr && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d) &&
-      ((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) | reinterpret_cast<uintptr_t>(a.val_idx)) & 3u) == 0)
+  if (pairs && prepared != nullptr && workspace != nullptr && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d) && on_words(a))
     return attention_dense(a, B, d, bits, q, dtype, sb, sh, ss, prepared, workspace, stream);
   if (path == Bf16Path::kDecode)  // its own small kernels on both sides of the split-KV kernel; none of the operand images
     return attention_decode(a, B, bits, q, dtype, sb, sh, ss, Pi_k, S_eff, q_cat,
