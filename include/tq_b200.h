@@ -282,10 +282,11 @@ int tq_attention_fwd(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq
 
 /* tq_attention_fwd / tq_attention_fwd_cached with the constants taken from a prepared buffer: no operand is
  * rebuilt per call, and the scratch need is tq_attention_prepared_workspace_bytes.  In TQ_MODE_BF16, calls in which many
- * queries meet each key expand keys and values once per call to fp16 rows there (4 d bytes a token and KV head, 128 MiB at a
- * time and no more) and attend over those; without the room (`workspace` may be NULL) they are served from the packed bytes,
- * slower.  Other prefill-sized calls need none, but for long prefixes behind few queries, which with
- * TQ_MODE_FP32 keep partial results there and are served unsplit, slower, without the room.  kv_capacity = Sk is the contiguous
+ * queries meet each key expand keys and values once per call to fp16 rows there (4 d bytes a token and KV head, at most 128 MiB
+ * at a time; behind long prefixes partial results come on top, 170 MB where 300 queries of 64 heads meet 250 000 keys) and
+ * attend over those.  Other prefill-sized calls need none, but for long prefixes behind few queries, which keep partial results
+ * there, as they do with TQ_MODE_FP32.  With less than that, or with NULL, prefill-sized calls are served from the packed bytes,
+ * whole and slower; TQ_MODE_FP32 needs the query rows' part in any case.  kv_capacity = Sk is the contiguous
  * layout; a larger capacity is the persistent-cache layout of tq_attention_fwd_cached, served in place for every
  * head_dim, number of queries and mode.
  * Replaces the attention core of the family adapters (families/llama.py:100-114, gpt2.py:90-110). */
@@ -306,7 +307,10 @@ int tq_attention_fwd_prepared(const void* q, int dtype, int64_t B, int64_t Hq, i
  * fp32 (TQ_MASK_ADDITIVE) or bytes of which 0 hides a key (TQ_MASK_BOOL, what HF's sdpa path hands over for padded
  * batches).  `mask_batches` is 1 (one mask for every batch element) or B; strides in elements, rows contiguous.
  * Tiles of keys that no row of a tile of queries sees are not computed.  (Additive masks in TQ_MODE_FP32 and over at most
- * 128 keys are read as they are.)  A mask that hides every key of a row makes it the average over its causal range. */
+ * 128 keys are read as they are.)  A mask that hides every key of a row makes it the average over its causal range.
+ * The summary's scratch (tq_attention_masked_workspace_bytes less tq_attention_prepared_workspace_bytes) is always needed.  With
+ * it alone, prefill-sized TQ_MODE_BF16 calls are served as the unmasked ones are without scratch, but behind long prefixes, where
+ * that takes all of it. */
 #define TQ_MASK_ADDITIVE 0
 #define TQ_MASK_BOOL 1
 size_t tq_attention_masked_workspace_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,

@@ -103,17 +103,21 @@ int attention_fwd_fp32(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
                        cudaStream_t stream, bool prepared = false);
 
+// How a bf16-mode call of the SM-pair kernel's is served: keys and values expanded first, that kernel split over the keys, or
+// that kernel unsplit.  The first two take scratch; this is the choice for prepared calls that have it.
+enum class PairRoute { kExpand, kSplit, kWhole };
+PairRoute attention_pair_route(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
+
 // bf16 mode: tcgen05 query preparation, tcgen05 flash kernel, tcgen05 back-rotation.
 // `prepared` (optional): a constants buffer filled by prepare_constants for the same matrices; the operand images
 // are then taken from it and nothing is rebuilt.
 int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
-                       cudaStream_t stream, const uint8_t* prepared = nullptr);
-// Whether the SM-pair kernel serves a bf16-mode call (its only scratch are the partial results of a split call).
+                       cudaStream_t stream, const uint8_t* prepared, PairRoute route);
+// Whether a bf16-mode call is the SM-pair kernel's, on one of the routes above.
 bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride, int d);
-// TQ_OK where the kernel that serves a bf16-mode call can read packed rows and norms at their addresses (`prepared`: with a
-// constants buffer; `scratch`: with any scratch).
-int check_packed_rows_bf16(const AttnArgs& a, int64_t B, int64_t Sq, int d, int bits, bool prepared, bool scratch);
+// TQ_OK where the kernel that serves a bf16-mode call can read packed rows and norms at their addresses.
+int check_packed_rows_bf16(const AttnArgs& a, int64_t Sq, int d, int bits, PairRoute route);
 // scratch bytes of a bf16-mode call with a prepared constants buffer, by the kernel that will serve it
 size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int64_t kv_stride,
                                      int d);

@@ -980,32 +980,38 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
   TQ_REQUIRE(o_stride_b % al == 0 && o_stride_h % al == 0 && o_stride_s % al == 0,
              "out strides must keep every row 16-byte aligned");
   TQ_REQUIRE(sm_scale == sm_scale, "sm_scale is NaN");
-  const size_t call_need = prepared != nullptr
-                               ? tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, kv_stride, d, mode)
-                               : tq_attention_workspace_bytes(B, Hq, Sq, d, mode);
-  size_t mask_need = 0;
-  if (src != nullptr) mask_bits_layout(src->nb, Sq, Sk, nullptr, &mask_need);
-  size_t need = call_need + mask_need;
-  // A prepared call without room for partial results (no scratch at all for the SM-pair kernel, the query rows alone in
-  // fp32 mode) is served unsplit.
-  bool split = prepared != nullptr;
-  if (split && src == nullptr && (workspace == nullptr || workspace_bytes < need)) {
-    if (mode == TQ_MODE_FP32) {
-      need = round256((size_t)B * Hq * Sq * 2 * d * 4);
-      split = false;
-    } else if (attention_bf16_on_sm_pairs(Hq, Sq, Hkv, Sk, kv_stride, d)) {  // (partial results are all it has scratch for)
-      need = 0;
-      workspace = nullptr;
-    }
-  }
-  if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
-    return fail(TQ_ERR_WORKSPACE, "workspace of %zu bytes needed (256-byte aligned), got %zu", need,
-                workspace_bytes);
   AttnArgs a{nullptr, Hq, Sq, Hkv, Sk, key_idx, key_signs, key_vec_norms, key_residual_norms, val_idx,
              val_vec_norms, centroids_k, centroids_v, Pi_v, sm_scale, causal, mask, mask_stride_b, mask_stride_q,
              out, dtype, o_stride_b, o_stride_h, o_stride_s, kv_stride, MaskBits{}};
+  size_t call_need = prepared != nullptr ? tq_attention_prepared_workspace_bytes(B, Hq, Sq, Hkv, Sk, kv_stride, d, mode)
+                                         : tq_attention_workspace_bytes(B, Hq, Sq, d, mode);
+  size_t mask_need = 0;
+  if (src != nullptr) mask_bits_layout(src->nb, Sq, Sk, nullptr, &mask_need);
+  // Prepared calls without room for what only makes them faster are served without it: expanded rows and partial results in bf16
+  // mode, partial results in fp32 mode.  A masked call has scratch in any case, the summary's; where the SM-pair kernel would be
+  // split it is held to all of it, elsewhere the summary is enough.
+  const bool enough = workspace != nullptr && workspace_bytes >= call_need + mask_need;
+  bool split = prepared != nullptr;
+  PairRoute route = PairRoute::kWhole;
+  if (mode == TQ_MODE_FP32) {
+    if (split && src == nullptr && !enough) {
+      call_need = round256((size_t)B * Hq * Sq * 2 * d * 4);
+      split = false;
+    }
+  } else if (prepared != nullptr && attention_bf16_on_sm_pairs(Hq, Sq, Hkv, Sk, kv_stride, d)) {
+    const bool splits = attention_c2_splits(B, Hq, Sq, Hkv, Sk) > 1;
+    if (enough ? splits || (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 : splits && src != nullptr)
+      route = attention_pair_route(B, Hq, Sq, Hkv, Sk, d);
+    else
+      call_need = 0;
+  }
+  const size_t need = call_need + mask_need;
+  if (need == 0) workspace = nullptr;
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
+    return fail(TQ_ERR_WORKSPACE, "workspace of %zu bytes needed (256-byte aligned), got %zu", need,
+                workspace_bytes);
   if (mode == TQ_MODE_BF16)
-    if (int st = check_packed_rows_bf16(a, B, Sq, d, bits, prepared != nullptr, workspace != nullptr)) return st;
+    if (int st = check_packed_rows_bf16(a, Sq, d, bits, route)) return st;
   CallScope scope(q, "q", static_cast<cudaStream_t>(stream));
   if (scope.status()) return scope.status();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1024,7 +1030,7 @@ static int attention_entry(const void* q, int dtype, int64_t B, int64_t Hq, int6
                               workspace, s, split);
   }
   return attention_fwd_bf16(q, dtype, B, Hq, Sq, d, q_stride_b, q_stride_h, q_stride_s, Pi_k, S_eff, a, bits,
-                            workspace, s, prepared);
+                            workspace, s, prepared, route);
 }
 
 extern "C" size_t tq_constants_bytes(int d, int bits) {

@@ -1013,15 +1013,15 @@ bool attention_bf16_on_sm_pairs(int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
   return bf16_path(a, Sq, d) == Bf16Path::kPairs;
 }
 
-static bool on_words(const AttnArgs& a) {
-  return ((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn) | reinterpret_cast<uintptr_t>(a.val_idx)) & 3u) == 0;
+PairRoute attention_pair_route(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
+  if (attention_dense_applies(B, Hq, Sq, Hkv, Sk, d)) return PairRoute::kExpand;
+  return attention_c2_splits(B, Hq, Sq, Hkv, Sk) > 1 ? PairRoute::kSplit : PairRoute::kWhole;
 }
 
-int check_packed_rows_bf16(const AttnArgs& a, int64_t B, int64_t Sq, int d, int bits, bool prepared, bool scratch) {
+int check_packed_rows_bf16(const AttnArgs& a, int64_t Sq, int d, int bits, PairRoute route) {
   const Bf16Path path = bf16_path(a, Sq, d);
-  const bool expand = path == Bf16Path::kPairs && prepared && scratch && on_words(a) && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d);
   // (the SM-pair kernel loads half a value row per CTA, in words where that is 12 bytes)
-  const unsigned keys = expand ? 4 : path == Bf16Path::kDecode ? 16 : 8;
+  const unsigned keys = path == Bf16Path::kDecode ? 16 : path == Bf16Path::kPairs && route == PairRoute::kExpand ? 4 : 8;
   const unsigned values = path == Bf16Path::kPairs && d == 64 && bits == 3 ? 4 : keys;
   TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn)) & (keys - 1)) == 0 &&
                  (reinterpret_cast<uintptr_t>(a.val_idx) & (values - 1)) == 0,
@@ -1039,7 +1039,7 @@ size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t 
   switch (bf16_path(a, Sq, d)) {
     // everything it needs is in the constants buffer and on the chip, but for the partial results of a split call
     case Bf16Path::kPairs:
-      if (attention_dense_applies(B, Hq, Sq, Hkv, Sk, d)) return attention_dense_bytes(B, Hq, Sq, Hkv, Sk, d);
+      if (attention_pair_route(B, Hq, Sq, Hkv, Sk, d) == PairRoute::kExpand) return attention_dense_bytes(B, Hq, Sq, Hkv, Sk, d);
       return attention_c2_part_bytes(B, Hq, Sq, d, attention_c2_splits(B, Hq, Sq, Hkv, Sk));
     case Bf16Path::kDecode: return round256((size_t)n_q * 2 * d * 2) + decode_workspace_bytes(B * Hq);
     default: return round256((size_t)n_q * 2 * d * 2) + round256((size_t)n_q * d * 2);
@@ -1048,7 +1048,7 @@ size_t workspace_bytes_bf16_prepared(int64_t B, int64_t Hq, int64_t Sq, int64_t 
 
 int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t Sq, int d, int64_t sb, int64_t sh,
                        int64_t ss, const float* Pi_k, const float* S_eff, AttnArgs a, int bits, void* workspace,
-                       cudaStream_t stream, const uint8_t* prepared) {
+                       cudaStream_t stream, const uint8_t* prepared, PairRoute route) {
   const int64_t n_q = B * Hq * Sq;
   TQ_REQUIRE(B <= 65535 && Hq <= 65535, "batch and head counts are limited to 65535 in bf16 mode");
   TQ_REQUIRE(a.sm_scale > 0.f && a.sm_scale < 1e30f, "sm_scale must be positive and finite in bf16 mode");
@@ -1075,8 +1075,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
   ws += round256((size_t)n_q * 2 * d * 2);
   __nv_bfloat16* o_rot = reinterpret_cast<__nv_bfloat16*>(ws);
 
-  // (packed rows are read in words there)
-  if (pairs && prepared != nullptr && workspace != nullptr && attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d) && on_words(a))
+  if (pairs && route == PairRoute::kExpand)
     return attention_dense(a, B, d, bits, q, dtype, sb, sh, ss, prepared, workspace, stream);
   if (path == Bf16Path::kDecode)  // its own small kernels on both sides of the split-KV kernel; none of the operand images
     return attention_decode(a, B, bits, q, dtype, sb, sh, ss, Pi_k, S_eff, q_cat,
@@ -1098,7 +1097,7 @@ int attention_fwd_bf16(const void* q, int dtype, int64_t B, int64_t Hq, int64_t 
       TQ_CUDA_OK(cudaGetLastError());
     }
     PairArgs x{q, dtype, sb, sh, ss, w_cat, w_unrot, luts, 1, nullptr, nullptr};
-    if (prepared != nullptr && workspace != nullptr && !attention_dense_applies(B, a.Hq, Sq, a.Hkv, a.Sk, d)) {  // room for partial results (NULL: an unsplit call)
+    if (route == PairRoute::kSplit) {
       x.nsplit = attention_c2_splits(B, Hq, Sq, a.Hkv, a.Sk);
       x.part_o = static_cast<float*>(workspace);
       x.part_ml = x.part_o + (size_t)B * Hq * ((Sq + kBM - 1) / kBM) * x.nsplit * kBM * d;
