@@ -158,6 +158,9 @@ struct PairArgs {
 };
 // Clusters per pair of query tiles that the SM-pair kernel is split over, and the partial results' bytes (0 unsplit).
 int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk);
+// Keys that the average query walks, for the estimates of either prefill kernel: calls are taken for causal, but those of more
+// queries than keys cannot be.
+inline double attention_walked_keys(int64_t Sq, int64_t Sk) { return Sq > Sk ? (double)Sk : (double)Sk - 0.5 * (double)Sq; }
 // What that kernel is expected to take, in microseconds (the estimate behind the splits).
 double attention_c2_us(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d);
 size_t attention_c2_part_bytes(int64_t B, int64_t Hq, int64_t Sq, int d, int nsplit);

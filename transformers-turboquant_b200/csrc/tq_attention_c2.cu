@@ -1050,7 +1050,7 @@ static double c2_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk
   }
   // (causal prompts: the average cluster walks fewer tiles than the first ones)
   if (4 * Sq >= Sk && clusters > slots)
-    cost = (double)tiles + kFixed + ((double)clusters / (double)slots - 1.0) * (((double)Sk - 0.5 * (double)Sq) / kBN + kFixed);
+    cost = (double)tiles + kFixed + ((double)clusters / (double)slots - 1.0) * (attention_walked_keys(Sq, Sk) / kBN + kFixed);
   return cost;
 }
 int attention_c2_splits(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk) {

@@ -695,7 +695,7 @@ DensePlan dense_plan(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk,
   }
   // (causal prompts: the average block walks fewer tiles than the first ones)
   if (4 * Sq >= Sk && units > slots)
-    cost = (double)p.T + kFixed + ((double)units / (double)slots - 1.0) * (((double)Sk - 0.5 * (double)Sq) / kBN + kFixed);
+    cost = (double)p.T + kFixed + ((double)units / (double)slots - 1.0) * (attention_walked_keys(Sq, Sk) / kBN + kFixed);
   p.us = kLaunchUs + (double)groups * cost * kPeriodUs + (double)(all * p.T * d) * kExpandUs;
   if (p.nsplit > 1) p.part_bytes = round256((size_t)units * 2 * p.nsplit * kBM * (d + 2) * sizeof(float));
   return p;
