@@ -158,8 +158,24 @@ def measured_peaks():
     return {"tflops_burst": 1590.0, "tflops_sustained": 1400.0, "hbm_gbs": 6650.0, "source": "fallback"}
 
 
+def kernel_launches(step):
+    """Launches of each kernel kind in one call of `step`: a call whose expanded rows exceed 128 MiB expands and attends in
+    several rounds."""
+    from turboquant_b200 import _lib
+    _lib.check(_lib.lib.tq_profile_begin(1024))
+    step()
+    ms_sum, launches = (ctypes.c_float * 5)(), (ctypes.c_int * 5)()
+    _lib.check(_lib.lib.tq_profile_end(ms_sum, launches))
+    return list(launches)
+
+
+def kernel_ms_per_step(ms_sum, launches, per_step):
+    """Milliseconds of each kernel kind in one step, from sums over `launches` recorded launches of which a step has `per_step`."""
+    return [m / max(n, 1) * k for m, n, k in zip(ms_sum, launches, per_step)]
+
+
 def attention_flops(batch, seq, heads=HQ):
-    """Flops of one launch of the attention kernel over expanded keys and values: 2d (q.K') + 2d (P.V') per causal pair
+    """Flops of one call of the attention kernel over expanded keys and values: 2d (q.K') + 2d (P.V') per causal pair
     (the expansion is a launch of its own)."""
     return 4.0 * D * causal_pairs(batch, seq, heads)
 
@@ -432,7 +448,7 @@ def config5_section(ctx: Ctx, bits: int, steps: int = 2, warm: int = 1, seq: int
 def head_dim64_section(ctx: Ctx, bits: int, batch: int = B, steps: int = 10, warm: int = 3):
     """The op-level step (compress K and V, fused causal attention) on the headline shape with head_dim 64, the
     head dimension of every GPT-2 size, plus a GPT-2-small-shaped call (12 heads, no grouping, 1024 positions):
-    the SM-pair kernel serves both head dimensions."""
+    expansion and attention over the expanded rows serve both head dimensions."""
     import turboquant_b200 as tq
     dev, d = ctx.dev, 64
     peaks = measured_peaks()
@@ -552,7 +568,7 @@ def decode_section(ctx: Ctx, bits: int, steps: int = 50, warm: int = 3):
                          "frac": achieved / peaks["hbm_gbs"], "traffic": None, "kernel": "decode_kernel",
                          "ms_per_launch": kern_ms, "algorithmic_bytes_per_launch": keys * bytes_per_key,
                          "peak_source": peaks["source"] + ", copy bandwidth"},
-            "kernel_ms": {"expand_keys_and_values": ms_sum[2] / max(launches[2], 1), "decode": kern_ms,
+            "kernel_ms": {"prepare_queries": ms_sum[2] / max(launches[2], 1), "decode": kern_ms,
                           "merge_and_back_rotation": ms_sum[4] / max(launches[4], 1)},
             "generation_step_ms": gen_ms,  # append one token per sequence to the cache, then attend
             "uncompressed_bf16_cache_sdpa_ms_per_call": sdpa_ms,
@@ -621,11 +637,12 @@ def run_headline(args):
     warm = max(args.warmup, 3)
     for _ in range(warm):
         out = step()
+    per_step = kernel_launches(step)
     ctx.barrier()
 
     sampler = ClockSampler(ctx.local)
     sampler.start()
-    _lib.check(_lib.lib.tq_profile_begin(max(args.steps, 1)))
+    _lib.check(_lib.lib.tq_profile_begin(min(max(args.steps, 1) * max(per_step), 4096)))
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     ev0.record()
     for _ in range(args.steps):
@@ -638,11 +655,12 @@ def run_headline(args):
     ms_per_step = ctx.max_over_ranks(ev0.elapsed_time(ev1)) / args.steps
     keys_per_rank = batch * HKV * seq
     value = keys_per_rank * world / (ms_per_step * 1e-3)
-    launches_per_step = int(sum(launches)) // max(args.steps, 1)
+    launches_per_step = sum(per_step)
 
     # ---- roofline of the dominant kernel (fused attention: tensor-core bound) ---------------------------
     peaks = measured_peaks()
-    attn_ms = ms_sum[3] / max(launches[3], 1)
+    step_ms = kernel_ms_per_step(ms_sum, launches, per_step)
+    attn_ms, attn_launches = step_ms[3], max(per_step[3], 1)
     flops = attention_flops(batch, seq)
     achieved = flops / (attn_ms * 1e-3) / 1e12
     # (what the call cannot do without; the expanded rows between its two kernels fit the L2 but for a part)
@@ -655,15 +673,13 @@ def run_headline(args):
                              "conditions of the burst peak; `frac_sustained` comes from the seconds-long pass below, "
                              "against the sustained peak",
                 "peak_burst": peaks["tflops_burst"], "peak_sustained": peaks["tflops_sustained"],
-                "traffic": traffic, "algorithmic_bytes_per_launch": algorithmic_bytes,
-                "flops_per_launch": flops, "kernel": "attention_dense_kernel", "ms_per_launch": attn_ms,
+                "traffic": traffic, "algorithmic_bytes_per_launch": algorithmic_bytes / attn_launches,
+                "flops_per_launch": flops / attn_launches, "kernel": "attention_dense_kernel", "ms_per_launch": attn_ms / attn_launches,
+                "launches_per_step": attn_launches,
                 "peak_source": peaks["source"],
-                "kernel_ms": {"compress": (ms_sum[0] + ms_sum[1]) / max(args.steps, 1),
-                              "compress_keys": ms_sum[0] / max(launches[0], 1),
-                              "compress_values": ms_sum[1] / max(launches[1], 1),
-                              "expand_keys_and_values": ms_sum[2] / max(launches[2], 1),
-                              "attention": attn_ms, "back_rotation": ms_sum[4] / max(launches[4], 1)}}
-    comp_ms = (ms_sum[0] + ms_sum[1]) / max(args.steps, 1)
+                "kernel_ms": {"compress": step_ms[0] + step_ms[1], "compress_keys": step_ms[0], "compress_values": step_ms[1],
+                              "expand_keys_and_values": step_ms[2], "attention": attn_ms, "back_rotation": step_ms[4]}}
+    comp_ms = step_ms[0] + step_ms[1]
     comp_bytes = batch * HKV * seq * (2 * D * 2 + (16 * (bits - 1) + 16 + 4) + (16 * bits + 2))
     roofline["compress"] = {"bound": "hbm", "achieved": comp_bytes / (comp_ms * 1e-3) / 1e9 if comp_ms > 0 else None,
                             "peak": peaks["hbm_gbs"], "unit": "GB/s",
@@ -675,7 +691,7 @@ def run_headline(args):
         n_sus = max(50, int(3200.0 / ms_per_step))
         sampler = ClockSampler(ctx.local)
         sampler.start()
-        _lib.check(_lib.lib.tq_profile_begin(min(n_sus, 4096)))
+        _lib.check(_lib.lib.tq_profile_begin(min(n_sus * max(per_step), 4096)))
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         for _ in range(n_sus):
@@ -685,10 +701,10 @@ def run_headline(args):
         s_sum, s_launch = (ctypes.c_float * 5)(), (ctypes.c_int * 5)()
         _lib.check(_lib.lib.tq_profile_end(s_sum, s_launch))
         sus_clocks = sampler.finish()
-        sus_ms = s_sum[3] / max(s_launch[3], 1)
+        sus_ms = kernel_ms_per_step(s_sum, s_launch, per_step)[3]
         sus_ach = flops / (sus_ms * 1e-3) / 1e12
         roofline["frac_sustained"] = sus_ach / peaks["tflops_sustained"]
-        roofline["sustained_pass"] = {"steps": n_sus, "seconds": e0.elapsed_time(e1) * 1e-3, "ms_per_launch": sus_ms,
+        roofline["sustained_pass"] = {"steps": n_sus, "seconds": e0.elapsed_time(e1) * 1e-3, "ms_per_launch": sus_ms / attn_launches,
                                       "achieved": sus_ach, "peak": peaks["tflops_sustained"], "clocks": sus_clocks}
 
     # ---- end to end through the public API with pinned host buffers ----------------------------------------
