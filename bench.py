@@ -111,8 +111,13 @@ class ClockSampler(threading.Thread):
     def __init__(self, index: int):
         super().__init__(daemon=True)
         self.index, self.samples, self.reasons, self.max_mhz = index, [], set(), None
-        self._stop_evt = threading.Event()
+        self._stop_evt, self._ready = threading.Event(), threading.Event()
         self.ok = True
+
+    def start(self):
+        """Returns when sampling begins: opening NVML can take longer than the timed region (20 steps of 2 ms)."""
+        super().start()
+        self._ready.wait(timeout=10)
 
     def run(self):
         try:
@@ -125,6 +130,7 @@ class ClockSampler(threading.Thread):
                      nv.nvmlClocksThrottleReasonSwThermalSlowdown: "sw_thermal_slowdown",
                      nv.nvmlClocksThrottleReasonSwPowerCap: "sw_power_cap",
                      nv.nvmlClocksThrottleReasonHwPowerBrakeSlowdown: "hw_power_brake"}
+            self._ready.set()
             while not self._stop_evt.is_set():
                 self.samples.append(nv.nvmlDeviceGetClockInfo(h, nv.NVML_CLOCK_SM))
                 mask = nv.nvmlDeviceGetCurrentClocksThrottleReasons(h)
@@ -133,6 +139,8 @@ class ClockSampler(threading.Thread):
         except Exception as exc:  # NVML missing: report, never fail the run
             self.ok = False
             self.error = repr(exc)
+        finally:
+            self._ready.set()
 
     def finish(self):
         self._stop_evt.set()

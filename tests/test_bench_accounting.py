@@ -1,6 +1,9 @@
 """The benchmark's arithmetic on kernel times: no GPU needed."""
 
 import inspect
+import sys
+import time
+import types
 
 import bench
 
@@ -14,3 +17,20 @@ def test_rounds_of_a_call_add_up():
 def test_decode_section_names_its_kernels():
     source = inspect.getsource(bench.decode_section)
     assert '"prepare_queries"' in source and "expand" not in source
+
+
+def test_clocks_are_sampled_in_short_regions(monkeypatch):
+    # a stand-in for NVML that takes longer to open than the region lasts
+    nvml = types.ModuleType("pynvml")
+    nvml.nvmlInit = lambda: time.sleep(0.3)
+    nvml.nvmlDeviceGetHandleByIndex = lambda i: i
+    nvml.NVML_CLOCK_SM = 1
+    nvml.nvmlDeviceGetMaxClockInfo = nvml.nvmlDeviceGetClockInfo = lambda h, kind: 1965
+    nvml.nvmlDeviceGetCurrentClocksThrottleReasons = lambda h: 0
+    for i, name in enumerate(("HwSlowdown", "HwThermalSlowdown", "SwThermalSlowdown", "SwPowerCap", "HwPowerBrakeSlowdown")):
+        setattr(nvml, "nvmlClocksThrottleReason" + name, 1 << i)
+    monkeypatch.setitem(sys.modules, "pynvml", nvml)
+    sampler = bench.ClockSampler(0)
+    sampler.start()
+    time.sleep(0.05)
+    assert sampler.finish()["sm_mhz"] == 1965
