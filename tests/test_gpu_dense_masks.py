@@ -37,9 +37,9 @@ def _call(q, ck, cv, kc, vc, mask):
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("kind", ["window", "left", "shared", "blind", "all"])
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Sk", [(1, 32, 8, 300, 8300),    # split over the keys
-                                            (8, 32, 16, 400, 900),    # more tiles than CTAs
+                                            (4, 64, 16, 350, 2100),   # more tiles than CTAs
                                             (2, 32, 8, 40, 6001),     # three groups of rows, ragged
-                                            (48, 16, 16, 257, 600),   # two rounds of expansion at head_dim 128
+                                            (12, 64, 16, 257, 2050),  # two rounds of expansion at head_dim 128
                                             (32, 16, 16, 513, 513)])  # a prompt: all tiles are expanded
 def test_hidden_tiles_are_not_touched(B, Hq, Hkv, Sq, Sk, d, kind):
     from turboquant_b200 import fused_attention
@@ -70,7 +70,7 @@ def test_hidden_tiles_are_not_touched(B, Hq, Hkv, Sq, Sk, d, kind):
         return  # (several rounds share the scratch)
     tiles = torch.nn.functional.pad(mask.any(1), (0, 128 * T - Sk)).reshape(-1, T, 128).any(-1)  # some query sees a key
     tiles = tiles | ~(mask & (at <= row)).any(-1).all(-1)[:, None]                              # ... or averages all of them
-    tiles = tiles | (Sk < 2 * Sq or B * Hkv * T * d < 300 * 128)  # (all are expanded)
+    tiles = tiles | (Sk < 6 * Sq or B * Hkv * T * d < 300 * 128 or T < 16)  # (all are expanded)
     tiles = tiles.expand(B, T)[:, None].expand(B, Hkv, T).reshape(-1)
     written = (ws[:B * Hkv * T * 256 * d].reshape(B * Hkv * T, -1) != -1).all(-1)
     assert torch.equal(written, tiles)

@@ -724,9 +724,9 @@ int attention_dense(const AttnArgs& a, int64_t B, int d, int bits, const void* q
   const DensePlan p = dense_plan(B, a.Hq, a.Sq, a.Hkv, a.Sk, d);
   const ConstLayout L = const_layout(d);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  // Key tiles that a mask hides from every query are not expanded, where there are any to speak of: in front of a chunk.  (Prompts
-  // have those of their padding, whose rows average all keys of their causal range.)
-  const bool skip = a.mb.words != nullptr && p.T <= kMapTiles && a.Sk >= 2 * a.Sq;
+  // Key tiles that a mask hides from every query are not expanded, where there are any to speak of and the expansion is: in front of
+  // a chunk of few queries.  (Prompts have those of their padding, whose rows average all keys of their causal range.)
+  const bool skip = a.mb.words != nullptr && p.T <= kMapTiles && a.Sk >= 6 * a.Sq;
   for (int64_t p0 = 0; p0 < B * a.Hkv; p0 += p.pairs) {
     const int pairs = (int)std::min<int64_t>(B * a.Hkv - p0, p.pairs);
     const ExpandArgs e{a.key_idx, a.key_sgn, a.key_vn, a.key_rn, a.val_idx, a.val_vn, a.kv_stride, a.Sk, constants + L.x_key,

@@ -362,19 +362,19 @@ int launch(ExpandArgs a, cudaStream_t stream) {
   return TQ_OK;
 }
 
-// Tiles that a mask hides from every query are left out where expanding all of them takes 10 us and more, 300 tiles at head_dim
-// 128, and the map of them is drawn in a few rounds of loads: about 2 us, most of it the latency of the first.  Us with all tiles
-// expanded and so, 32 / 8 heads of 128 (nothing hidden / half of the prefix / all but a window of 64): 300 tokens behind 2700, 2
-// sequences, 78 and 81 / 60 and 60 / 37 and 31; 256 behind 7936, 4 sequences, 212 and 218 / 152 and 129 / 93 and 37; 64 behind 29936
-// 124 and 128 / 109 and 85 / 89 and 36; 164 behind 582, 3 sequences, 144 tiles, 35 and 37 / 33 and 33 / 27 and 27.  Listing them
-// under a CTA's first tile took 3 to 7 us longer.  The summary of more queries takes longer to look through than its tiles are worth
-// beside the attention over them.
+// Tiles that a mask hides from every query are left out where a KV head has 16 tiles and more, expanding all of them takes 10 us
+// (300 tiles at head_dim 128), and the map of them is drawn in a few rounds of loads: about 2 us, most of it the latency of the
+// first.  Us with all tiles expanded and so, 32 / 8 heads of 128 (nothing hidden / half of the prefix / all but a window of 64): 300
+// tokens behind 2700, 2 sequences, 78 and 81 / 60 and 60 / 37 and 31; 256 behind 7936, 4 sequences, 212 and 218 / 152 and 129 / 93
+// and 37; 64 behind 29936 124 and 128 / 109 and 85 / 89 and 36; 164 behind 582, 3 sequences, 144 tiles, 35 and 37 / 33 and 33 / 27
+// and 27; 12 behind 15, 25 sequences, 12 / 12 heads, a tile each, 39 and 43 under any.  Listing them under a CTA's first tile took 3
+// to 7 us longer.  The summary of more queries takes longer to look through than its tiles are worth beside the attention over them.
 bool lists_tiles(ExpandArgs& a, int d) {
   if (a.mb.words == nullptr) return false;
   const int64_t tiles = (int64_t)a.pairs * a.T, sms = sm_count();
   const int64_t nb = a.mb.batch ? (a.pair0 + a.pairs - 1) / a.Hkv - a.pair0 / a.Hkv + 1 : 1;
   a.parts = (int)std::max<int64_t>(1, std::min<int64_t>(a.mb.NG, kListMapThreads / (nb * a.T)));
-  return tiles * d >= 300 * 128 && tiles <= kOwnTiles * (sms - sms * 3 / 5) && nb * ((a.T + 31) / 32) <= kLiveWords &&
+  return a.T >= 16 && tiles * d >= 300 * 128 && tiles <= kOwnTiles * (sms - sms * 3 / 5) && nb * ((a.T + 31) / 32) <= kLiveWords &&
          nb * a.mb.NG * ((int64_t)a.T + a.mb.NC) <= kSummaryReads;
 }
 template <int D>
