@@ -709,10 +709,12 @@ bool attention_dense_applies(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int
   // Expansion pays where a key is met by many tiles of queries.  Few queries behind a prefix, and calls of one or two key tiles,
   // are the SM-pair kernel's: either one's time is estimated (over 533 calls of 1 to 512 tokens behind 0 to 30000, 2 to 32 KV
   // heads and 1 to 16 sequences both estimates are right within 10 % (rms), no call goes to the slower kernel by more than 3 %
-  // here, and what the rule leaves to the SM-pair kernel would gain 0.7 % in the mean).  64 tokens behind 2000 (1 sequence, 32 / 8 heads): 37 and 38 us; 128 behind 8000 (4 sequences): 113 and 148;
-  // 512 behind 8000 (4 sequences, 16 / 2 heads): 217 and 161; 16 x 64 tokens: 41 and 24.
-  return p.kv_bytes > 0 && p.us < 0.98 * attention_c2_us(B, Hq, Sq, Hkv, Sk, d) && B * Hkv < ((int64_t)1 << 31) && p.rows < ((int64_t)1 << 31) - kRows &&
-         p.pairs * p.blocks * 32 < ((int64_t)1 << 31) && p.pairs <= 65535;
+  // here, and what the rule leaves to the SM-pair kernel would gain 0.7 % in the mean).  SM-pair kernel and expansion: 64 tokens
+  // behind 2000 (1 sequence, 32 / 8 heads) 37 and 38 us; 128 behind 8000 (4 sequences) 113 and 148; 512 behind 8000 (4 sequences,
+  // 16 / 2 heads) 217 and 161; 16 x 64 tokens 41 and 24; 8192 over 512 keys (8 sequences, not causal) 1455 and 826.
+  const int64_t most = (int64_t)1 << 31;
+  return p.kv_bytes > 0 && p.us < 0.98 * attention_c2_us(B, Hq, Sq, Hkv, Sk, d) && B * Hkv < most && p.rows < most - kRows &&
+         p.pairs * p.blocks * 32 < most && p.pairs <= 65535;
 }
 size_t attention_dense_bytes(int64_t B, int64_t Hq, int64_t Sq, int64_t Hkv, int64_t Sk, int d) {
   const DensePlan p = dense_plan(B, Hq, Sq, Hkv, Sk, d);

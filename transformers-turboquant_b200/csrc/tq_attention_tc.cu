@@ -1026,7 +1026,8 @@ int check_packed_rows_bf16(const AttnArgs& a, int64_t Sq, int d, int bits, PairR
   TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_idx) | reinterpret_cast<uintptr_t>(a.key_sgn)) & (keys - 1)) == 0 &&
                  (reinterpret_cast<uintptr_t>(a.val_idx) & (values - 1)) == 0,
              "packed rows must start on boundaries of %u bytes (keys) and %u (values) for this call in bf16 mode", keys, values);
-  TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_vn) | reinterpret_cast<uintptr_t>(a.key_rn) | reinterpret_cast<uintptr_t>(a.val_vn)) & 1u) == 0,
+  TQ_REQUIRE(((reinterpret_cast<uintptr_t>(a.key_vn) | reinterpret_cast<uintptr_t>(a.key_rn) |
+               reinterpret_cast<uintptr_t>(a.val_vn)) & 1u) == 0,
              "norms must be 2-byte aligned");
   return TQ_OK;
 }
